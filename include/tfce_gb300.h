@@ -358,6 +358,22 @@ int perm_stream(int64_t n, int64_t seed, int64_t start, int64_t stop, int64_t* o
  *     (a perfect fit gives +-inf or NaN, as 0/0).  Tiles and ginv 16-byte
  *     aligned. */
 int glm_qf_design_block(int32_t kmax);
+/* Design operators of glm_tstat_tc_qf, formed on the device in FP64 (the host
+ * work of the permutation loop, cynumstats.pyx:28-29 on
+ * vertex_tfce_multiple_regression_randomise.py:90-107's permuted designs).
+ * Design d is [1, x_1 .. x_kmax-1] with column j from the base matrix
+ *   base [n][ld] double (device), + d * stride doubles (stride 0: shared):
+ *   cols [share][kmax] (device; entry 0 unused): for design d the entries of
+ *   row d % share: base column c < 256, c + 256 when the design's index row
+ *   permutes it (entry s is base[rows[s]][c]), -1 for a missing column;
+ *   rows [ceil(G / share)][n] int32 (device) or NULL: index row d / share.
+ * Writes x_tiles, ginv [G_pad][R][R], invdiag [G][kmax] (entry 0 is 0) and
+ * dof [G] as glm_tstat_tc_qf reads them, zero for the padding designs up to a
+ * multiple of glm_qf_design_block(kmax).  err (device) receives 1 for an index
+ * outside [0, n), 4 for a design without an inverse. */
+int glm_qf_designs(const double* base, int64_t ld, int64_t stride, const int32_t* rows, const int32_t* cols,
+                   int32_t share, int32_t n, int32_t n_pad, int32_t G, int32_t kmax, void* x_tiles, float* ginv,
+                   float* invdiag, float* dof, int32_t* err, void* stream);
 int glm_col_sumsq(const float* Y_centred, int64_t ldy, int32_t n, int64_t V, float* yy, void* stream);
 int glm_tstat_tc_qf(const void* y_tiles, const float* yy, int32_t n, int32_t n_pad, int64_t V,
                     const void* x_tiles, const float* ginv, const float* invdiag, const float* dof, int32_t G,

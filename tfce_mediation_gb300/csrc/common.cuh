@@ -23,6 +23,7 @@ enum DevErr : int32_t {
   kDevBadIndex = 1,   // adjacency entry outside its segment
   kDevLoopLimit = 2,  // union-find walk / retry limit reached
   kDevTooManySteps = 3,
+  kDevSingular = 4,  // a design whose cross products have no inverse
 };
 
 inline int map_dev_err(int32_t e) {

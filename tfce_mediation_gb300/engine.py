@@ -43,6 +43,22 @@ def permutations(n, seed, start, stop):
     return out
 
 
+def index_rows(perms, n, X):
+    """Permutation index rows (P, n) as numpy would read them in X[perms]:
+    integers, negative ones from the end; raises what numpy raises."""
+    perms = np.asarray(perms)
+    if perms.dtype.kind not in "iu" or perms.ndim != 2 or perms.shape[1] != n:
+        picked = X[perms]  # IndexError for what is no index
+        raise ValueError(f"permutation rows of {n} subjects expected, got designs of shape {picked.shape}")
+    if perms.size:
+        lo, hi = int(perms.min()), int(perms.max())
+        if lo < -n or hi >= n:
+            raise IndexError(f"index {lo if lo < -n else hi} is out of bounds for axis 0 with size {n}")
+        if lo < 0:
+            perms = np.where(perms < 0, perms + n, perms)
+    return perms
+
+
 class PermutationEngine:
     """Mass-univariate GLM + TFCE null distribution on one GPU.
 
@@ -179,6 +195,36 @@ class PermutationEngine:
     def _designs(self, perms):
         return DesignBatch(self.X[perms])
 
+    def _index_rows(self, perms, out=None):
+        """Index rows as int32 (P, n), written into `out` when given; raises
+        what indexing the design with them would."""
+        rows = index_rows(perms, self.n, self.X)
+        if out is None:
+            return np.ascontiguousarray(rows, np.int32)
+        out[...] = rows
+        return out
+
+    def _base(self):
+        """The design on the device, and its columns: every one permuted."""
+        if not hasattr(self, "_X_d"):
+            np.linalg.inv(self.X.T @ self.X)  # a design without an inverse raises here
+            self._cols_d = dev(np.arange(self.k, dtype=np.int32) + TensorCoreOperands.PERMUTED)
+            self._X_d = dev(self.X)
+        return self._X_d, self._cols_d
+
+    def _tmaps_of(self, perms):
+        """t maps [P][C][V] of the permutation index rows."""
+        P = perms.shape[0]
+        if not self._graph_qf() or len(self.contrasts) > 8:
+            return self.tmaps(self._designs(perms))
+        tc, out = self._tc, self._tbuf[:P]
+        base, cols = self._base()
+        rows = dev(self._index_rows(perms))
+        ops = tc.design_buffers(P, self.k)
+        tc.form_designs(base, cols, rows, P, self.k, ops)
+        tc.tstat_qf(*ops, P, self.k, self._coef, self.C, out, self.V)
+        return out
+
     def tmaps(self, designs: DesignBatch, out=None, precision=None):
         """t maps [G][C][V] for a DesignBatch (device tensor)."""
         G = designs.G
@@ -245,7 +291,7 @@ class PermutationEngine:
         P = perms.shape[0]
         if P > self.batch:
             raise ValueError("batch larger than the engine's buffers")
-        tm = self.tmaps(self._designs(perms))
+        tm = self._tmaps_of(perms)
         mx = self.sweep_max(tm, P * self.C)
         hm = self._host_max.view(-1)[: mx.numel()]
         hm.copy_(mx, non_blocking=True)
@@ -273,25 +319,30 @@ class PermutationEngine:
         return (tc is not None and self.outputs is None and self._centred and tc.quadratic_form
                 and tc.yy is not None and 2 <= self.k <= 8 and min(self.contrasts) >= 1)
 
+    def _graph_form(self):
+        """What a captured batch depends on: its size, the GLM's form and, with
+        the residual epilogue, the designs per tile."""
+        qf = self._graph_qf()
+        return self.batch, qf, None if qf or self._tc is None else self._tc.block(self.k)
+
     def _graph_slot(self, P):
         """One captured batch: pinned design operators -> device, glm_tstat,
         the sweep (counter reset included), maxima -> pinned host memory."""
         t = self.t
         n, kmax = self.n, self.k
         tc = self._tc
-        slot = {"P": P}
+        slot = {"P": P, "form": self._graph_form()}
         qf = self._graph_qf()
         slot["QF"] = qf
         if qf:
-            R, Gp = tc.qf_rows(kmax), tc.qf_padded(P, kmax)
-            keys = ("XR", "GI", "invd", "dof")
-            slot["h_XR"] = t.zeros((Gp * R, tc.n_pad), dtype=t.float32, pin_memory=True)
-            slot["h_GI"] = t.zeros((Gp, R, R), dtype=t.float32, pin_memory=True)
-            slot["d_xt"] = t.empty(int(self.lib.glm_tile_bytes(Gp * R, 256, tc.n_pad)), dtype=t.uint8,
-                                   device="cuda")
+            keys = ()
+            base, cols = self._base()
+            slot["h_rows"] = t.empty((P, n), dtype=t.int32, pin_memory=True)
+            slot["h_rows"].numpy()[...] = np.arange(n)
+            slot["d_rows"] = t.empty((P, n), dtype=t.int32, device="cuda")
+            slot["ops"] = tc.design_buffers(P, kmax)
         elif tc is not None:
             Gp, DB = tc.padded(P, kmax), tc.block(kmax)
-            slot["DB"] = DB
             keys = ("P8", "U", "Xt", "invd", "dof") + (("W",) if self._w_stride else ())
             if self._w_stride:
                 slot["h_W"] = t.zeros((P, self._w_stride), dtype=t.float32, pin_memory=True)
@@ -305,8 +356,9 @@ class PermutationEngine:
             slot["h_pinv"] = t.zeros((P, kmax, n), dtype=t.float32, pin_memory=True)
             slot["h_X"] = t.zeros((P, n, kmax), dtype=t.float32, pin_memory=True)
         # the capture warm-up runs on these before the first fill: a harmless design
-        slot["h_invd"] = t.ones((P, kmax), dtype=t.float32, pin_memory=True)
-        slot["h_dof"] = t.ones((P,), dtype=t.float32, pin_memory=True)
+        if not qf:
+            slot["h_invd"] = t.ones((P, kmax), dtype=t.float32, pin_memory=True)
+            slot["h_dof"] = t.ones((P,), dtype=t.float32, pin_memory=True)
         slot["h_max"] = t.empty((P, self.C, self.signs, self.n_seg), dtype=t.float32, pin_memory=True)
         for key in keys:
             slot["d_" + key] = t.empty(slot["h_" + key].shape, device="cuda", dtype=t.float32)
@@ -317,9 +369,9 @@ class PermutationEngine:
             for key in keys:
                 slot["d_" + key].copy_(slot["h_" + key], non_blocking=True)
             if qf:
-                tc.tile_designs_qf(slot["d_XR"], P, kmax, out=slot["d_xt"])
-                tc.tstat_qf(slot["d_xt"], slot["d_GI"], slot["d_invd"], slot["d_dof"], P, kmax, self._coef, self.C,
-                            slot["d_t"], self.V)
+                slot["d_rows"].copy_(slot["h_rows"], non_blocking=True)
+                tc.form_designs(base, cols, slot["d_rows"], P, kmax, slot["ops"])
+                tc.tstat_qf(*slot["ops"], P, kmax, self._coef, self.C, slot["d_t"], self.V)
             elif tc is not None:
                 tc.tile_designs(slot["d_P8"], P, kmax, out=slot["d_pt"])
                 tc.stat(3 if self.outputs is not None else 0, slot["d_pt"], slot["d_U"], slot["d_Xt"],
@@ -343,6 +395,7 @@ class PermutationEngine:
         side.wait_stream(t.cuda.current_stream())
         with t.cuda.stream(side):
             body_glm()
+            slot["d_t"].zero_()  # nothing to sweep: the workspace is what the warm-up is for
             body_sweep()
         t.cuda.current_stream().wait_stream(side)
         t.cuda.synchronize()
@@ -358,11 +411,12 @@ class PermutationEngine:
         return slot
 
     def _fill(self, slot, perms):
+        if slot["QF"]:
+            self._index_rows(perms, out=slot["h_rows"].numpy())
+            return
         db = DesignBatch(self.X[perms])
         P = perms.shape[0]
-        if slot["QF"]:
-            self._tc.host_operands_qf(db, XR=slot["h_XR"].numpy(), GI=slot["h_GI"].numpy())
-        elif self._tc is not None:
+        if self._tc is not None:
             self._tc.host_operands(db, P8=slot["h_P8"].numpy(), U=slot["h_U"].numpy(), Xt=slot["h_Xt"].numpy(),
                                    centred=self._centred)
             if self._w_stride:
@@ -403,9 +457,8 @@ class PermutationEngine:
         Returns the per-batch maxima, (rows, C, signs, n_seg) each."""
         t = self.t
         P = self.batch
-        DB = None if self._tc is None else self._tc.block(self.k)
-        if (not hasattr(self, "_slots") or self._slots[0]["P"] != P or self._slots[0].get("DB") != DB
-                or self._slots[0]["QF"] != self._graph_qf()):
+        form = self._graph_form()
+        if not hasattr(self, "_slots") or self._slots[0]["form"] != form:
             self._slots = [self._graph_slot(P), self._graph_slot(P)]
         if not hasattr(self, "_up_stream"):
             self._up_stream = t.cuda.Stream()
@@ -563,9 +616,39 @@ class MediationEngine:
             ta.append(tas)
         return A, B, ta
 
+    def _base(self):
+        """Base columns of the path designs on the device -- pred_x, depend_y,
+        covariates -- and the columns of each path ([1, x] and [1, dy, x] for
+        'M', pyfunc.py:131-145), those of permuted variables flagged."""
+        if not hasattr(self, "_Z_d"):
+            x, dy = self.pred_x.reshape(self.n, -1), self.depend_y.reshape(self.n, -1)
+            cov = np.zeros((self.n, 0)) if self.cov is None else self.cov.reshape(self.n, -1)
+            nx, ny, nc = x.shape[1], dy.shape[1], cov.shape[1]
+            cx = [j + TensorCoreOperands.PERMUTED for j in range(nx)]
+            cy = [nx + j + (TensorCoreOperands.PERMUTED if self.medtype == "Y" else 0) for j in range(ny)]
+            cc = [nx + ny + j for j in range(nc)]
+            paths = {"I": [cx + cc, cx + cy + cc], "M": [cx + cc, cy + cx + cc], "Y": [cy + cx + cc]}[self.medtype]
+            cols = np.full((len(paths), self.kmax), -1, np.int32)
+            for i, path in enumerate(paths):
+                cols[i, 1:1 + len(path)] = path
+            self._paths_d = dev(cols)
+            self._Z_d = dev(np.hstack([x, dy, cov]))
+        return self._Z_d, self._paths_d
+
+    def _on_device(self):
+        """Whether the path designs are formed on the device: the quadratic-form
+        GLM runs them."""
+        tc = self.inner._tc
+        return (tc is not None and tc.quadratic_form and tc.yy is not None and 2 <= self.kmax <= 8
+                and self.pred_x.ndim <= 2)
+
     def _designs(self, perms):
-        """Host work of a batch: the path designs (FP64 inverses) of the
-        permutation rows, as (DesignBatch, path-a t of medtype 'Y' or None)."""
+        """Host work of a batch, as (designs, path-a t of medtype 'Y' or None):
+        the index rows (int32) of designs formed on the device, or a
+        DesignBatch of the path designs (FP64 inverses)."""
+        if self._on_device():
+            rows = np.ascontiguousarray(index_rows(perms, self.n, self.pred_x), np.int32)
+            return rows, (np.asarray(self._paths(perms)[2], np.float32) if self.medtype == "Y" else None)
         A, B, ta = self._paths(perms)
         if self.medtype == "Y":
             return DesignBatch(B, kmax=self.kmax), np.asarray(ta, np.float32)
@@ -575,7 +658,17 @@ class MediationEngine:
         inner = self.inner
         z = self._z[:P] if out is None else out
         lib = inner.lib
-        tm = inner.tmaps(db)
+        if isinstance(db, np.ndarray):
+            tc = inner._tc
+            base, paths = self._base()
+            G = P * paths.shape[0]
+            ops = tc.design_buffers(G, self.kmax)
+            rows = dev(db)
+            tc.form_designs(base, paths, rows, G, self.kmax, ops, share=paths.shape[0])
+            tm = inner._tbuf[:G]
+            tc.tstat_qf(*ops, G, self.kmax, inner._coef, 1, tm, inner.V)
+        else:
+            tm = inner.tmaps(db)
         if self.medtype == "Y":  # tm (P, 1, V): path b
             tas = dev(ta)
             _lib.check(lib.sobel_combine(None, self.V, ptr(tas), ptr(tm), self.V, P, self.V, self.alg_code,

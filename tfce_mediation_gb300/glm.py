@@ -62,9 +62,11 @@ class DesignBatch:
 
     designs: array (G, n, k) or list of (n, k_g) arrays (float64).
     invXX: optional (G, k, k) matrices whose diagonal gives the SE factor (the
-    reference passes its own invXX to tval_int); default inv(X'X)."""
+    reference passes its own invXX to tval_int); default inv(X'X).
+    operators=False: only the stacked designs X64 and dof (designs whose
+    operators are formed on the device)."""
 
-    def __init__(self, designs, invXX=None, kmax=None):
+    def __init__(self, designs, invXX=None, kmax=None, operators=True):
         if isinstance(designs, np.ndarray) and designs.ndim == 3:
             Xs = np.array(designs, np.float64)
             mats = None
@@ -78,6 +80,11 @@ class DesignBatch:
         kmax = kmax or max(ks)
         if kmax > 8:
             raise ValueError("at most 8 regressors per design")
+        self.G, self.n, self.kmax, self.ks = G, n, kmax, ks
+        self.dof = np.asarray([n - k for k in ks], np.float64)
+        if not operators:
+            self.X64 = Xs
+            return
         invdiag = np.zeros((G, kmax), np.float64)
         inv_p = np.zeros((G, kmax, kmax), np.float64)  # inv(X'X), zero padded
         same_k = len(set(ks)) == 1
@@ -109,10 +116,8 @@ class DesignBatch:
                 Xp[g, :, :k] = m
                 invdiag[g, :k] = np.diag(inv if invXX is None else np.asarray(invXX[g], np.float64))
             self._pinv64 = pinv
-        self.G, self.n, self.kmax, self.ks = G, n, kmax, ks
         self.X64, self.invdiag64 = Xp, invdiag
         self._inv64 = inv_p
-        self.dof = np.asarray([n - k for k in ks], np.float64)
 
     @property
     def pinv64(self):
@@ -337,6 +342,37 @@ class TensorCoreOperands:
                                            ptr(out), None, stream_handle()))
         return out
 
+    PERMUTED = 256  # flag of a base column that a design's index row permutes
+
+    def design_buffers(self, G, kmax):
+        """Device operators of up to G designs of the quadratic form: (tiles,
+        ginv, invdiag, dof)."""
+        t = self.t
+        Gp, R = self.qf_padded(G, kmax), self.qf_rows(kmax)
+        return (t.empty(int(self.lib.glm_tile_bytes(Gp * R, 256, self.n_pad)), dtype=t.uint8, device="cuda"),
+                t.empty((Gp, R, R), dtype=t.float32, device="cuda"),
+                t.empty((G, kmax), dtype=t.float32, device="cuda"), t.empty(G, dtype=t.float32, device="cuda"))
+
+    def form_designs(self, base, cols, rows, G, kmax, out, stride=0, share=1):
+        """Form the operators of G designs on the device (glm_qf_designs).  base:
+        (n, c) float64, or one matrix per design `stride` apart; cols: (share,
+        kmax) int32 base columns (+ PERMUTED); rows: (G / share, n) int32 or
+        None; out: design_buffers."""
+        tiles, ginv, invd, dof = out
+        _lib.check(self.lib.glm_qf_designs(ptr(base), base.shape[-1], stride, ptr(rows), ptr(cols), share, self.n,
+                                           self.n_pad, G, kmax, ptr(tiles), ptr(ginv), ptr(invd), ptr(dof),
+                                           ptr(self.err), stream_handle()))
+
+    def form_stacked(self, X64, out=None):
+        """Operators of designs stacked as host float64 (G, n, k), the first
+        column all ones."""
+        G, n, k = X64.shape
+        out = self.design_buffers(G, k) if out is None else out
+        cols = dev(np.arange(k, dtype=np.int32))
+        base = dev(X64)
+        self.form_designs(base, cols, None, G, k, out, stride=n * k)
+        return out
+
     def tstat_qf(self, x_tiles, ginv, invd, dof, G, kmax, coef_d, n_coef, out, ldt):
         _lib.check(self.lib.glm_tstat_tc_qf(ptr(self.yt), ptr(self.yy), self.n, self.n_pad, self.V, ptr(x_tiles),
                                             ptr(ginv), ptr(invd), ptr(dof), G, kmax, ptr(coef_d), n_coef, ptr(out),
@@ -401,6 +437,10 @@ class TensorCoreOperands:
         e = int(self.err.item())
         if e:
             self.err.zero_()
+            if e == 4:
+                raise np.linalg.LinAlgError("Singular matrix")
+            if e == 1:
+                raise IndexError("a permutation index is out of bounds")
             raise RuntimeError("tensor-core GLM: a copy or MMA completion wait ran out (device code %d)" % e)
 
 
@@ -409,8 +449,10 @@ def glm_tstat_tc(Y, designs, coef, ops=None, centre=True, quadratic_form=None):
     form (glm_tstat_tc_qf) where it applies and quadratic_form is not False
     (None: the operands' setting), else the residual epilogue (glm_tstat_tc)."""
     t = require_cuda()
-    db = designs if isinstance(designs, DesignBatch) else DesignBatch(designs)
     ops = ops or TensorCoreOperands(dev(Y, t.float32), centre=centre)
+    stacked = (isinstance(designs, np.ndarray) and designs.ndim == 3 and designs.shape[2] <= 8
+               and designs.shape[1] == ops.n)
+    db = designs if isinstance(designs, DesignBatch) else DesignBatch(designs, operators=not stacked)
     keep = ops.quadratic_form
     if quadratic_form is not None:
         ops.quadratic_form = bool(quadratic_form)
@@ -419,14 +461,19 @@ def glm_tstat_tc(Y, designs, coef, ops=None, centre=True, quadratic_form=None):
     finally:
         ops.quadratic_form = keep
     if use_qf:
-        XR, GI = ops.host_operands_qf(db)
-        xt = ops.tile_designs_qf(dev(XR), db.G, db.kmax)
+        if stacked:
+            xt, gi, invd, dof = ops.form_stacked(db.X64)
+        else:
+            XR, GI = ops.host_operands_qf(db)
+            xt, gi = ops.tile_designs_qf(dev(XR), db.G, db.kmax), dev(GI)
+            invd, dof = dev(db.invdiag64.astype(np.float32)), dev(db.dof.astype(np.float32))
         out = t.empty((db.G, len(coef), ops.V), device="cuda", dtype=t.float32)
-        ops.tstat_qf(xt, dev(GI), dev(db.invdiag64.astype(np.float32)), dev(db.dof.astype(np.float32)), db.G,
-                     db.kmax, dev(np.asarray(coef, np.int32)), len(coef), out, ops.V)
+        ops.tstat_qf(xt, gi, invd, dof, db.G, db.kmax, dev(np.asarray(coef, np.int32)), len(coef), out, ops.V)
         t.cuda.synchronize()
         ops.status()
         return out
+    if stacked:
+        db = DesignBatch(designs)
     centred = ops.centred_ok(db, first_column_used=0 in list(coef))
     P8, U, Xt = ops.host_operands(db, centred=centred)
     pt = ops.tile_designs(dev(P8), db.G, db.kmax)
