@@ -78,10 +78,12 @@ int tfce_adjset_set_params(tfce_adjset* h, const float* H, const float* E);
 /* 1 if every entry has its reverse (the usual triangle-mesh / 26-neighbour
  * case), 0 otherwise. */
 int tfce_adjset_is_symmetric(const tfce_adjset* h);
-/* CTA shape of the per-component sweeps (tfce_sweep_batch with
- * accumulation 1 or 2): 3 resident CTAs of 512 threads per SM (40 registers,
- * the most sweeps in flight; the default) or 2 (64 registers, no spills).
- * The autotuner picks it per study together with the batch size. */
+/* Shape of the batched sweeps: 3 for CTAs of 256 threads, four per SM with
+ * room for 4,096 basins (local maxima of the map) each in shared memory (the
+ * default: smooth maps, up to 164k vertices), or 2 for CTAs of 512 threads, two
+ * per SM with room for 8,192; maps with more basins go to a second launch with
+ * one CTA per SM.  The autotuner picks it per study together with the batch
+ * size. */
 int tfce_adjset_set_sweep_shape(tfce_adjset* h, int32_t ctas_per_sm);
 /* Threshold groups of tfce_sweep_batch: group [n_seg] (host; ids in
  * [0, n_seg)), or NULL to give every segment its own table again.  Segments
@@ -95,7 +97,9 @@ int tfce_adjset_set_sweep_shape(tfce_adjset* h, int32_t ctas_per_sm);
  * over the maps. */
 int tfce_adjset_set_threshold_groups(tfce_adjset* h, const int32_t* group);
 
-/* How tfce_sweep_batch accumulates (the other entry points always use 0):
+/* How tfce_sweep_batch accumulates (the other entry points always use 0).  All
+ * three sweep the basins of the maps; they differ where vertex values are
+ * wanted (out_maps or vdensity):
  *   0  the reference's arithmetic: every active vertex adds its float
  *      increment to a float accumulator at every threshold
  *      (fast_tfce.hpp:72-84), so results are bit-identical to the reference
@@ -105,13 +109,12 @@ int tfce_adjset_set_threshold_groups(tfce_adjset* h, const int32_t* group);
  *      the chain of components it joined; the value is the float rounding of
  *      the exact sum of the same float increments, i.e. it differs from the
  *      reference by the reference's own float summation error (~1e-7 rel).
- *      Work per threshold is O(live components) instead of O(active vertices).
- *      A launch that asks only for maxima (out_maps NULL) without vertex
- *      weights (vdensity NULL) keeps, per component, the largest sum of any
- *      component merged into it instead of the potentials, and takes the
- *      map's maximum over the last live components: no per-vertex pass;
- *   2  as 1, but maxima-only launches keep the potentials and resolve every
- *      vertex as well (the same values; for comparisons). */
+ *   2  as 1, and maxima-only launches keep the potentials and resolve every
+ *      vertex as well (for comparisons).
+ * With 0 and 1 a launch that asks only for maxima (out_maps NULL) without
+ * vertex weights (vdensity NULL) keeps, per component, the largest float sum of
+ * any component merged into it, and takes the map's maximum over the last
+ * live components: bit-identical to 0's per-vertex sums, no per-vertex pass. */
 int tfce_adjset_set_accumulation(tfce_adjset* h, int32_t mode);
 
 /* CreateAdjSet.run(image, enhn) on host float32 arrays of length V (one

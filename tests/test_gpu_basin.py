@@ -1,0 +1,119 @@
+"""The basin form of the batched sweep at the sizes and graphs where it can go
+wrong: tile remainders (4,096 vertices a tile), one-way entries, hubs, isolated
+vertices, ties, more basins than one CTA's shared memory holds (a second
+launch) and more than all of an SM's (state in global memory).  Exact
+accumulation and maxima are compared with the oracle bit for bit; potentials
+(double sums) within 1e-5 of it."""
+import numpy as np
+import pytest
+
+from oracle import oracle
+from tfce_mediation_gb300 import adjacency as A
+
+pytestmark = pytest.mark.gpu
+
+
+def _csr(pairs, V):
+    pairs = np.unique(np.asarray(pairs, np.int64).reshape(-1, 2), axis=0)
+    pairs = pairs[pairs[:, 0] != pairs[:, 1]]
+    off = np.zeros(V + 1, np.int64)
+    np.add.at(off, pairs[:, 0] + 1, 1)
+    return np.cumsum(off), pairs[:, 1].astype(np.int32)
+
+
+def _graph(kind, V, rng):
+    i = np.arange(V)
+    ring = np.stack([i, (i + 1) % V], 1)
+    if kind == "isolated":
+        return _csr(np.zeros((0, 2)), V)
+    if kind == "ring":
+        return _csr(np.concatenate([ring, ring[:, ::-1]]), V)
+    far = np.stack([i, (i + 37) % V], 1)  # a band: every tile has neighbours in others
+    both = np.concatenate([ring, far])
+    both = np.concatenate([both, both[:, ::-1]])
+    if kind == "band":
+        return _csr(both, V)
+    if kind == "oneway":  # a third of the entries lose their reverse
+        return _csr(both[rng.random(len(both)) > 0.33], V)
+    hub = np.stack([np.zeros(V, np.int64), i], 1)  # one vertex beside every other
+    return _csr(np.concatenate([both, hub, hub[:, ::-1]]), V)
+
+
+def _maps(V, n, rng):
+    x = rng.standard_normal((n, V)).astype(np.float32)
+    for _ in range(3):
+        x[0] = (x[0] + np.roll(x[0], 1) + np.roll(x[0], -1)) / 3  # smooth, noise, ties
+    if n > 2:
+        x[2] = np.round(x[2] * 4) / 4
+    x[-1, V // 2:] = np.nan
+    x[-1, :1] = np.inf
+    return np.ascontiguousarray(x)
+
+
+def _sweep(adj, maps, signs, mode, vd=None, want_maps=False):
+    import torch
+    adj.set_accumulation(mode)
+    d = torch.from_numpy(maps).cuda()
+    V = maps.shape[1]
+    mx = torch.full((len(maps), signs, adj.n_seg), -1.0, device="cuda")
+    om = torch.full((len(maps), signs, V), -1.0, device="cuda") if want_maps else None
+    vdd = None if vd is None else torch.from_numpy(vd).cuda()
+    adj.sweep_batch(d.data_ptr(), V, len(maps), signs, None if vd is None else vdd.data_ptr(), 0, mx.data_ptr(),
+                    None if om is None else om.data_ptr(), 1 if want_maps else 0)
+    adj.status()
+    return mx.cpu().numpy(), None if om is None else om.cpu().numpy()
+
+
+@pytest.mark.parametrize("kind,V,E", [
+    ("band", 1, 1.0), ("ring", 2, 1.0), ("band", 31, 0.5), ("band", 33, 2.0), ("oneway", 500, 1.0),
+    ("band", 4095, 1.0), ("band", 4096, 0.5), ("band", 4097, 1.0), ("oneway", 8193, 1.0), ("hub", 6000, 1.0),
+    ("isolated", 9000, 1.0),   # ~4,500 basins a sign: the second launch
+    ("ring", 70_001, 1.0),     # ~23,000 basins a sign
+    ("isolated", 61_000, 0.5)])  # ~30,000: state in global memory
+def test_every_form_equals_the_oracle(kind, V, E):
+    rng = np.random.default_rng(V)
+    off, idx = _graph(kind, V, rng)
+    maps = _maps(V, 4, rng)
+    vd = (0.5 + rng.random(V)).astype(np.float32)
+    adj = A.AdjacencySet((off, idx), 2.0, E)
+    mx, _ = _sweep(adj, maps, 2, "component")
+    one, _ = _sweep(adj, maps, 1, "exact")
+    wmx, om = _sweep(adj, maps, 2, "exact", vd, want_maps=True)
+    cmx, cm = _sweep(adj, maps, 2, "component", vd, want_maps=True)
+    for m in range(len(maps)):
+        finite = maps[m][np.isfinite(maps[m])]
+        for s, sgn in enumerate((1.0, -1.0)):
+            # the oracle takes a map's maximum over finite values too
+            img = np.where(np.isfinite(maps[m]), sgn * maps[m], -np.inf).astype(np.float32)
+            top = np.float32(max((sgn * finite).max(), 0.0)) if finite.size else np.float32(0)
+            raw = oracle.tfce(off, idx, np.where(np.isfinite(img), img, 0.0).astype(np.float32), 2.0, E, hh_exact=True) \
+                if top > 0 else np.zeros(V, np.float32)
+            scaled = (raw * np.float32(top / np.float32(100.0))).astype(np.float32)
+            assert mx[m, s, 0] == scaled.max(), (m, s)
+            if s == 0:
+                assert one[m, 0, 0] == scaled.max(), m
+            want = (scaled * vd).astype(np.float32)
+            np.testing.assert_array_equal(om[m, s], want)
+            assert wmx[m, s, 0] == want.max()
+            np.testing.assert_allclose(cm[m, s], want, rtol=1e-5, atol=1e-12 * max(want.max(), 1e-30))
+            np.testing.assert_allclose(cmx[m, s, 0], want.max(), rtol=1e-5)
+
+
+def test_many_segments_of_uneven_sizes_and_launch_shapes():
+    """Segments from one vertex to several tiles, more items than SMs, both
+    shapes: every segment equals its own sweep."""
+    rng = np.random.default_rng(5)
+    sizes = [1, 40, 4096, 9001, 300, 4097]
+    parts = [_graph("band" if n > 2 else "isolated", n, rng) for n in sizes]
+    off, idx, seg = A.concat_csr(parts)
+    V = int(seg[-1])
+    maps = np.ascontiguousarray(rng.standard_normal((20, V)).astype(np.float32))
+    adj = A.AdjacencySet((off, idx), 2.0, 1.0, seg)
+    for shape in (3, 2):
+        adj.set_sweep_shape(shape)
+        mx, _ = _sweep(adj, maps, 2, "component")
+        for s, (o, i) in enumerate(parts):
+            part = np.ascontiguousarray(maps[:, seg[s]:seg[s + 1]])
+            for k, sgn in enumerate((1.0, -1.0)):
+                np.testing.assert_array_equal(mx[:, k, s], oracle.tfce_max_batch(o, i, part, 2.0, 1.0, sign=sgn,
+                                                                                 hh_exact=True))

@@ -348,8 +348,8 @@ class AdjacencySet:
         self.threshold_groups = g.copy()
 
     def set_sweep_shape(self, ctas_per_sm: int):
-        """Resident CTAs per SM of the per-component sweeps: 3 (40 registers,
-        most items in flight) or 2 (64 registers, no spills)."""
+        """Shape of the batched sweeps: 3 (more sweeps resident, each with room
+        for 4,096 local maxima of its map in shared memory) or 2 (fewer, 8,192)."""
         _lib.check(self._lib.tfce_adjset_set_sweep_shape(self._h, int(ctas_per_sm)))
         self.ctas_per_sm = int(ctas_per_sm)
 

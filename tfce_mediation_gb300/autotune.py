@@ -3,9 +3,10 @@ tensor-core GLM's designs per tile for a permutation engine.
 
 Each candidate (P, CTAs per SM) is timed on the device (CUDA events, after a
 warm-up launch) for the GLM + sweep of one batch; the one with the highest
-permutations per second wins.  The sweep runs 3 CTAs of 512 threads per SM
-(40 registers, the most items in flight) or 2 (64 registers, no spills);
-which is faster depends on the segments' sizes and list lengths.  The GLM
+permutations per second wins.  The sweep runs in shape 3 (four CTAs of 256
+threads per SM, room for 4,096 local maxima of a map each) or 2 (two of 512
+threads, 8,192); which is faster depends on the maps' smoothness and the
+segments' sizes.  The GLM
 runs as the quadratic form (t from the cross products of the centred
 designs with the data, where it applies) or with the residual epilogue, whose
 tile holds 32 designs (N = 256 MMA columns) or 16 (N = 128); the forms are

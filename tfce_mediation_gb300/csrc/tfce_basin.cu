@@ -1,0 +1,1922 @@
+// Basin form of the batched TFCE sweep: the GB300 replacement of
+// tfce_mediation/lib/fast_tfce.hpp:11-95 for every batched launch.
+//
+// The reference inserts the vertices by decreasing value and joins each to the
+// neighbours that were inserted before it.  Here every vertex first points to
+// its largest neighbour, inside a tile of up to 4,096 vertices kept in shared
+// memory.  Following the pointers gives the vertex's basin, a tree whose
+// members are connected from their own activation on.  So the component of a
+// vertex at any threshold is the component of its basin, and only the list
+// entries that join two different basins need a union: on a smooth map of 164k
+// vertices that leaves 2.5k basins and 15k pairs per sign, of 164k vertices
+// and 983k entries, and the union-find state of a sweep fits in shared memory.
+//
+//   basin_max_kernel    segment maxima of +x and -x
+//   basin_tile_kernel   one CTA per (map, tile), both signs at once (their
+//                       vertices are disjoint): activation steps, basins, and
+//                       the pairs of basins that neighbours join
+//   basin_cross_kernel  the pairs that cross a tile boundary
+//   basin_offset_kernel where each tile's entries go in the segment's lists
+//   basin_order_kernel  the segment's lists, ordered by (sign, step)
+//   basin_sweep_kernel  one CTA per (map, sign, segment): threshold steps over
+//                       the lists, union-find over basins
+//   basin_walk_kernel   vertex values of the reference's float accumulation
+//
+// Measured on one GB300 against the vertex-by-vertex sweep that batched
+// launches ran before (its state, 5 MB an item, was walked at random in DRAM):
+// 512 maps x 2 hemispheres x +/- of the L7 icosphere, smooth: 21.9 -> 4.7 ms
+// (tile 2.3, sweep 1.5, order 0.5, cross 0.2, max 0.1); unsmoothed noise, 128
+// maps: 10.1 -> 2.9 ms; 48 maps of 242k voxels, 26 neighbours, E = 0.5: 9.8 ->
+// 1.4 ms; one map: 4.64 -> 0.45 ms.
+#include <algorithm>
+#include <cmath>
+#include <cstdlib>
+#include <map>
+
+#include "basin.cuh"
+#include "host_parallel.h"
+#include "sweep_common.cuh"
+
+namespace tfgb {
+
+constexpr int kTile = 4096;            // vertices per tile at most (12 bits of a packed record)
+constexpr int kTileThreads = 512;
+constexpr int kPerThread = kTile / kTileThreads;
+constexpr int kBuckets = 256;          // sign * 128 + step
+constexpr int kTab = kBuckets + 2;     // bucket starts and the total
+constexpr uint32_t kRoot = 0x80000000u;
+constexpr uint32_t kExtent = 0x00ffffffu;
+constexpr int kPairTable = 2048;       // slots for the distinct pairs of basins of a tile
+constexpr int kCrossTable = 1024;      // the same for a chunk of boundary vertices
+constexpr int kProbes = 12;            // slots tried
+constexpr int kQueue = 96;              // neighbours that wait in a warp's queue: 31 and two rows' worth
+constexpr int kCrossThreads = 256;
+constexpr int kCrossPer = 4;
+constexpr int kCrossChunk = kCrossThreads * kCrossPer;
+constexpr int kMaxSweepThreads = 1024;
+constexpr int kTileEntries = 120000;   // list entries per tile: pairs are counted in 16 bits
+constexpr int kFindLimit = 1 << 26;
+constexpr int kAhead = 4;              // pairs of events that a thread of the sweep loads a step ahead
+constexpr uint32_t kNone = 0xffffffffu;
+
+struct TileInfo {
+  int32_t pos0;    // first list position (a multiple of 32)
+  int32_t nv;      // vertices
+  int32_t seg;
+  int32_t slice0;  // first slice (32 vertices each) of the neighbour and of the edge rows
+  int32_t bnd0;    // boundary vertices of the tile: [bnd0, bnd0 + nbnd)
+  int32_t nbnd;
+  int32_t pair0;   // first pair record
+  int32_t in_seg;  // index of the tile in its segment
+};
+
+struct ChunkInfo {
+  int32_t seg;
+  int32_t bnd0, nbnd;  // boundary vertices of the chunk
+  int32_t slice0;
+  int32_t pair0;       // first crossing-pair record
+  int32_t pad;
+};
+
+struct SegInfo {
+  int32_t tile0, ntiles, chunk0, nchunks;
+  int64_t pos0, pair0;  // first entries of the segment's ordered lists
+};
+
+struct Node {
+  float inc;
+  uint32_t next;
+};
+
+enum SweepMode { kMaxima = 0, kPotential = 1, kNodes = 2 };
+
+struct BasinArgs {
+  // request
+  const float* stats;
+  int64_t map_stride;
+  int32_t n_maps, signs, n_seg;
+  const float* vdensity;
+  float* out_max;
+  float* out_maps;
+  int32_t out_mode;
+  int64_t n_vertices;
+  const int32_t* thr_group;
+  const float* seg_H;
+  const int64_t* seg_off;
+  const int32_t* seg_rank;
+  int32_t* err;
+  // plan
+  const TileInfo* tiles;
+  const ChunkInfo* chunks;
+  const SegInfo* segs;
+  const int32_t* vert;        // vertex of a list position
+  const uint32_t* slice_off;  // first row entry of a slice; the next slice's ends it
+  const uint32_t* nbr;        // two neighbours each (4 * index in the tile), 32 lanes a row
+  const uint32_t* edge_off;   // the same for the rows that hold each pair of neighbours once
+  const uint32_t* edge;
+  const uint16_t* bnd_local;  // boundary vertex: its index in its tile
+  const int32_t* bnd_vert;    // its vertex
+  const uint16_t* bnd_tile;   // its tile in the segment
+  const uint32_t* cross_off;  // slices of the crossing lists
+  const uint32_t* cross;      // boundary vertices, 32 lanes a row
+  const double* const* seg_pow;  // extent^E, or NULL for E == 1
+  int32_t n_tiles, n_chunks, n_bnd;
+  // workspace
+  uint32_t* seg_max;    // [maps][2][n_seg] bits of max(0, max)
+  int32_t* counter;     // items taken by the first sweep launch, by the second, and queued for it
+  uint32_t* ev;         // by vertex of the tile: basin | bucket << 12, or kNone
+  uint32_t* pairs;      // pairs of basins of a tile: bucket << 24, 12 bits each
+  uint2* cpairs;        // crossing pairs: tile << 16 | 4 bits of the bucket << 12 | basin, twice
+  uint16_t* tab_ev;     // [map][tile][kBuckets] entries of every bucket
+  uint16_t* tab_pair;
+  uint32_t* tab_cross;  // [map][chunk][kBuckets]
+  uint32_t* n_pairs;    // [map][tile] and, after them, [map][chunk]
+  uint16_t* n_basin;    // [map][tile][2]
+  uint2* bnd;           // [map][boundary vertex] {float bits, basin | step << 16}
+  uint32_t* off_ev;     // [map][tile][kBuckets]: entries of earlier tiles in the bucket
+  uint32_t* off_pair;
+  uint32_t* off_cross;  // [map][chunk][kBuckets]
+  uint32_t* base_of;    // [map][tile][2] first basin number of the tile
+  uint32_t* start_ev;   // [map][seg][kTab] bucket starts of the ordered lists
+  uint32_t* start_pair;
+  uint32_t* n_basins;   // [map][seg][2]
+  void* ev_out;         // ordered: basin of an active vertex (16 bits, or 32 beyond the shared state)
+  void* pair_out;       // ordered: pairs of basins (2 x 16 or 2 x 32 bits)
+  int32_t* ord;         // ordered: vertex
+  double* base;         // ordered: potential of the component before the vertex joined
+  uint32_t* vnode;      // ordered: first node of the vertex
+  Node* nodes;
+  uint32_t* part_max;   // [items] encoded maximum
+  int64_t pos_per_map, pair_per_map, cpair_per_map, opair_per_map;
+  int64_t node_cap;
+  char* state;
+  int64_t state_bytes;
+  int32_t* queue;       // items that the first sweep launch leaves to the second
+  int32_t n_items;
+  int32_t most_first;   // basins of an item that the first launch takes
+  int32_t most_narrow;  // basins of an item whose state (but the lists) is in shared memory
+};
+
+// ---------------------------------------------------------------------------
+__device__ inline float seg_maximum(const BasinArgs& a, int64_t map, int sgn, int seg) {
+  return __uint_as_float(a.seg_max[(map * 2 + sgn) * a.n_seg + seg]);
+}
+
+// the maximum that the threshold table of (map, sign, segment) starts from
+__device__ inline float table_maximum(const BasinArgs& a, int64_t map, int sgn, int seg) {
+  if (!a.thr_group) return seg_maximum(a, map, sgn, seg);
+  const int32_t g = a.thr_group[seg];
+  float m = 0.0f;
+  for (int s = 0; s < a.n_seg; ++s)
+    if (a.thr_group[s] == g) m = fmaxf(m, seg_maximum(a, map, sgn, s));
+  return m;
+}
+
+// Activation step: the first i with x > T[i] (strict, fast_tfce.hpp:41), or L,
+// by comparing, from a guess on.
+__device__ __noinline__ int step_beside(float x, const float* T, int L, int i) {
+  if (L == 0 || !(x > T[L - 1])) return L;
+  i = max(0, min(i, L - 1));
+  while (i > 0 && x > T[i - 1]) --i;
+  while (!(x > T[i])) ++i;  // ends at L - 1
+  return i;
+}
+
+// The same from the place of x between the thresholds, in steps: T falls by dT
+// a step up to float rounding, which adds up to less than 4e-4 of a step over
+// the table, so away from a threshold by 1e-3 of a step the place gives the
+// step.  inv = 100 / tmx, or 0 for tables that are not the usual 100 or 101
+// steps of a normal float (every x is then compared).  place: 1 .. 4095, larger
+// the further x is above its threshold.
+__device__ inline int step_of(float x, const float* T, int L, float tmx, float inv, uint32_t* place) {
+  constexpr float kInt = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer, in the low bits
+  const float q = (tmx - x) * inv;
+  const float t = (q - 0.5f) + kInt;
+  const float f = q - (t - kInt);
+  int i = __float_as_int(t) - 0x4b400000;
+  *place = __float_as_uint(fmaf(-4094.0f, __saturatef(f), 4095.0f) + kInt) & 0xfffu;
+  if (f > 1e-3f && f < 0.999f) return min(i + 1, L);
+  return step_beside(x, T, L, i);
+}
+
+__device__ inline float step_scale(float tmx, int L) {
+  return (L >= 100 && L <= 101 && tmx > 1e-30f && tmx < 1e30f) ? __fdiv_rn(100.0f, tmx) : 0.0f;
+}
+
+// Block-wide exclusive scan of kBuckets counters by the first 256 threads:
+// start[b], start[kBuckets] = total.  Ends with a barrier.
+__device__ inline void scan_buckets(int* cnt, int* wsum) {
+  const int t = threadIdx.x, lane = t & 31;
+  int v = 0, inc = 0;
+  if (t < kBuckets) {
+    v = cnt[t];
+    inc = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    if (lane == 31) wsum[t >> 5] = inc;
+  }
+  __syncthreads();
+  if (t < kBuckets) {
+    int before = 0;
+    for (int w = 0; w < (t >> 5); ++w) before += wsum[w];
+    cnt[t] = before + inc - v;
+    if (t == kBuckets - 1) cnt[kBuckets] = before + inc;
+  }
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// Maxima of +x and -x of every (map, segment), finite values, at least 0.
+__global__ void __launch_bounds__(256) basin_max_kernel(BasinArgs a, int32_t parts) {
+  __shared__ float red[32];
+  const int64_t b = blockIdx.x;
+  const int part = static_cast<int>(b % parts);
+  const int seg = static_cast<int>((b / parts) % a.n_seg);
+  const int64_t map = b / parts / a.n_seg;
+  const int64_t v0 = a.seg_off[seg], n = a.seg_off[seg + 1] - v0;
+  const int64_t per = (n + parts - 1) / parts;
+  const int64_t lo = v0 + part * per, hi = min(v0 + n, lo + per);
+  const float* x = a.stats + map * a.map_stride;
+  float mp = 0.0f, mn = 0.0f;
+  for (int64_t v = lo + threadIdx.x; v < hi; v += 256) {
+    const float xv = x[v];
+    if (isfinite(xv)) {
+      mp = fmaxf(mp, xv);
+      mn = fmaxf(mn, -xv);
+    }
+  }
+  mp = block_max(mp, red);
+  mn = block_max(mn, red);
+  if (threadIdx.x == 0) {
+    if (mp > 0.0f) atomicMax(a.seg_max + (map * 2) * a.n_seg + seg, __float_as_uint(mp));
+    if (mn > 0.0f) atomicMax(a.seg_max + (map * 2 + 1) * a.n_seg + seg, __float_as_uint(mn));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Activation steps, basins and pairs of basins of one tile of one map.  Bound
+// by instruction issue (IPC 3.2 of 4; 425 warp instructions per 32 vertices,
+// a sixth each for steps, pointers and roots, the rest for the pairs).
+//
+// A vertex is one 32-bit word in shared memory: sign, 127 - step, place inside
+// the step (12 bits) and 4095 - index (12 bits).  Words of one sign order the
+// tile's vertices by step, then by value, then by index, without ties, so the
+// neighbour to point to is a running maximum and carries its own index; a
+// neighbour of the other sign is negative after the sign is taken out, an
+// inactive one 0.  Any order that keeps the steps gives the same components
+// (two-way entries; one-way ones are left to basin_cross_kernel).  Once a
+// vertex's root is known its word becomes sign, 128 - step, root, and every
+// pair of neighbours with different roots is a pair of basins, joined at the
+// later step of the two.
+__global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a) {
+  __shared__ uint32_t key[kTile];
+  __shared__ __align__(16) uint16_t lab[kTile];  // pointer, then root (2 * index in the tile)
+  uint32_t* const table = reinterpret_cast<uint32_t*>(lab);  // distinct pairs, once lab is done with
+  static_assert(kPairTable * sizeof(uint32_t) <= sizeof(lab), "the table takes lab's place");
+  __shared__ uint16_t rk[kTile];   // basin number of a root
+  __shared__ float sT[2][kMaxSteps];
+  __shared__ int cnt[kBuckets], pcnt[kBuckets];
+  __shared__ float4 sTab[2];  // maximum, steps per unit, step count
+  __shared__ int nroots[2], npairs;
+  __shared__ uint32_t sQueue[kTileThreads / 32 * kQueue];
+  const int tile = blockIdx.x % a.n_tiles;
+  const int64_t map = blockIdx.x / a.n_tiles;
+  const TileInfo ti = a.tiles[tile];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const float* x = a.stats + map * a.map_stride;
+  const int32_t* vert = a.vert + ti.pos0;
+
+  float xv[kPerThread];
+#pragma unroll
+  for (int k = 0; k < kPerThread; ++k) {
+    const int v = tid + k * kTileThreads;
+    xv[k] = (v < ti.nv) ? x[vert[v]] : 0.0f;
+  }
+  if (tid < 2) {
+    const int sgn = tid;
+    const float m = (sgn < a.signs) ? table_maximum(a, map, sgn, ti.seg) : 0.0f;
+    const int L = threshold_table(m, sT[sgn], a.err);
+    sTab[sgn] = make_float4(m, step_scale(m, L), __int_as_float(L), 0.0f);
+    nroots[sgn] = 0;
+    npairs = 0;
+  }
+  if (tid < kBuckets) cnt[tid] = pcnt[tid] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kPerThread; ++k) {
+    const int v = tid + k * kTileThreads;
+    const int sgn = xv[k] < 0.0f;
+    uint32_t w = 0;
+    if ((__float_as_uint(xv[k]) & 0x7fffffffu) - 1u < 0x7f7fffffu) {  // finite, and not 0
+      const float4 tab = sTab[sgn];
+      const int L = __float_as_int(tab.z);
+      uint32_t place;
+      const int st = step_of(fabsf(xv[k]), sT[sgn], L, tab.x, tab.y, &place);
+      if (st < L)
+        w = (__float_as_uint(xv[k]) & 0x80000000u) | (static_cast<uint32_t>(127 - st) << 24) | (place << 12) |
+            static_cast<uint32_t>(4095 - v);
+    }
+    if (v < ti.nv) key[v] = w;
+  }
+  __syncthreads();
+
+  auto at = [&](uint32_t offset) { return *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(key) + offset); };
+  // the largest neighbour
+#pragma unroll 4
+  for (int k = 0; k < kPerThread; ++k) {
+    const int v = tid + k * kTileThreads;
+    if (v < ti.nv) {
+      const uint32_t* so = a.slice_off + ti.slice0 + (v >> 5);
+      const uint32_t o1 = so[1];
+      const uint32_t kv = key[v], s = kv & 0x80000000u;
+      int best = static_cast<int>(kv ^ s);
+#pragma unroll 3
+      for (uint32_t o = so[0] + lane; o < o1; o += 32) {
+        const uint32_t two = a.nbr[o];
+        best = max(best, static_cast<int>(at(two & 0xffffu) ^ s));
+        best = max(best, static_cast<int>(at(two >> 16) ^ s));
+      }
+      lab[v] = static_cast<uint16_t>(8190 - 2 * (best & 0xfff));
+    }
+  }
+  __syncthreads();
+  // follow the pointers, two hops at a time (a root points to itself; a stored
+  // root shortens the walks that pass it); number the basins
+#pragma unroll 2
+  for (int k = 0; k < kPerThread; ++k) {
+    const int v = tid + k * kTileThreads;
+    const uint32_t w = (v < ti.nv) ? key[v] : 0u;
+    if (w) {
+      auto up = [&](uint32_t o) { return *reinterpret_cast<volatile uint16_t*>(reinterpret_cast<char*>(lab) + o); };
+      uint32_t r = up(2 * v);
+      for (int it = 0; it < kTile; ++it) {
+        const uint32_t n = up(r);
+        r = up(n);
+        if (r == n) break;
+      }
+      *reinterpret_cast<volatile uint16_t*>(lab + v) = static_cast<uint16_t>(r);
+      r >>= 1;
+      const int sgn = w >> 31;
+      const uint32_t code = ((w >> 24) & 127u) + 1u;  // 128 - step
+      const uint32_t b = sgn * kMaxSteps + kMaxSteps - code;
+      atomicAdd(&cnt[b], 1);
+      key[v] = (w & 0x80000000u) | (code << 12) | r;
+      if (r == static_cast<uint32_t>(v)) rk[v] = static_cast<uint16_t>(atomicAdd(&nroots[sgn], 1));
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < kPairTable; i += kTileThreads) table[i] = 0u;
+  __syncthreads();
+  // A pair of basins matters at the first step that joins it: the table keeps
+  // {pair, 128 - step} words and their maximum per pair.  A pair that finds no
+  // slot is written down as it comes (joining two basins again changes nothing).
+  uint32_t* pr = a.pairs + map * a.pair_per_map + ti.pair0;
+  auto emit = [&](uint32_t e) {
+    const uint32_t i = e >> 20, j = (e >> 8) & 0xfffu;
+    const uint32_t b = (key[i] >> 31) * kMaxSteps + kMaxSteps - (e & 0xffu);
+    atomicAdd(&pcnt[b], 1);
+    pr[atomicAdd(&npairs, 1)] = (b << 24) | (static_cast<uint32_t>(rk[i]) << 12) | rk[j];
+  };
+  // the neighbours of different roots wait in a queue of the warp until there
+  // are 32 for a full round
+  uint32_t* const queue = sQueue + (tid >> 5) * kQueue;
+  int nq = 0;
+  auto insert = [&](int q) {
+    const uint32_t w = at((queue[q] >> 12) << 2), u = at((queue[q] & 0xfffu) << 2);
+    const uint32_t i = w & 0xfffu, j = u & 0xfffu;
+    const uint32_t e = (min(i, j) << 20) | (max(i, j) << 8) | (min(u & 0xff000u, w & 0xff000u) >> 12);
+    uint32_t h = ((e >> 8) * 2654435761u) >> 21;
+    static_assert(kPairTable == 1 << 11, "the hash gives 11 bits");
+    for (int t = 0;; ++t) {
+      uint32_t cur = *reinterpret_cast<volatile uint32_t*>(table + h);
+      if (cur == 0u) cur = atomicCAS(&table[h], 0u, e);
+      if (cur == 0u || (cur ^ e) < 256u) {
+        if (cur != 0u && cur < e) atomicMax(&table[h], e);
+        break;
+      }
+      if (t == kProbes) {
+        emit(e);
+        break;
+      }
+      h = (h + 1) & (kPairTable - 1);
+    }
+  };
+  uint32_t* ev = a.ev + map * a.pos_per_map + ti.pos0;
+  const uint32_t below = (1u << lane) - 1u;
+  for (int k = 0; k < kPerThread; ++k) {
+    const int v = tid + k * kTileThreads;
+    if (v - lane >= ti.nv) break;
+    const uint32_t w = (v < ti.nv) ? key[v] : 0u;
+    const uint32_t* so = a.edge_off + ti.slice0 + (v >> 5);
+    const uint32_t o1 = so[1];
+    for (uint32_t o = so[0] + lane; o < o1; o += 32) {
+      const uint32_t two = a.edge[o];
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const uint32_t off = half ? two >> 16 : two & 0xffffu;
+        const uint32_t u = at(off), d = u ^ w;
+        const bool hit = (d & 0xfffu) && static_cast<int>(d) >= 0 && (u & 0xff000u) && w;
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (m) {
+          if (hit) queue[nq + __popc(m & below)] = (static_cast<uint32_t>(v) << 12) | (off >> 2);
+          nq += __popc(m);
+        }
+      }
+      while (nq >= 32) {
+        __syncwarp();
+        insert(nq - 32 + lane);
+        nq -= 32;
+        __syncwarp();
+      }
+    }
+    if (v < ti.nv)
+      ev[v] = w ? (rk[w & 0xfffu] | (((w >> 31) * kMaxSteps + kMaxSteps - ((w >> 12) & 0xffu)) << 12)) : kNone;
+  }
+  __syncwarp();
+  if (lane < nq) insert(lane);
+  // boundary vertices, for the pairs that cross tiles
+  for (int q = tid; q < ti.nbnd; q += kTileThreads) {
+    const int i = ti.bnd0 + q;
+    const uint32_t w = key[a.bnd_local[i]];
+    a.bnd[map * a.n_bnd + i] = make_uint2(w ? __float_as_uint(x[a.bnd_vert[i]]) : 0u,
+                                          w ? (rk[w & 0xfffu] | ((kMaxSteps - ((w >> 12) & 0xffu)) << 16)) : kNone);
+  }
+  __syncthreads();
+  for (int i = tid; i < kPairTable; i += kTileThreads)
+    if (table[i]) emit(table[i]);
+  __syncthreads();
+  const int64_t row = map * a.n_tiles + tile;
+  if (tid < kBuckets) {
+    a.tab_ev[row * kBuckets + tid] = static_cast<uint16_t>(cnt[tid]);
+    a.tab_pair[row * kBuckets + tid] = static_cast<uint16_t>(pcnt[tid]);
+  }
+  if (tid < 2) a.n_basin[row * 2 + tid] = static_cast<uint16_t>(nroots[tid]);
+  if (tid == 2) a.n_pairs[row] = npairs;
+}
+
+// Pairs that cross a tile boundary, and one-way entries: every boundary vertex
+// with the distinct basins of its listed neighbours that precede it by value
+// (ties by smaller vertex, the reference's insertion order).
+__global__ void __launch_bounds__(kCrossThreads) basin_cross_kernel(BasinArgs a) {
+  __shared__ int cnt[kBuckets], total;
+  __shared__ unsigned long long table[kCrossTable];  // {tile << 12 | basin, twice} << 8 | 128 - step
+  const int chunk = blockIdx.x % a.n_chunks;
+  const int64_t map = blockIdx.x / a.n_chunks;
+  const ChunkInfo ci = a.chunks[chunk];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint2* rec = a.bnd + map * a.n_bnd;
+  cnt[tid] = 0;
+  if (tid == 0) total = 0;
+  for (int i = tid; i < kCrossTable; i += kCrossThreads) table[i] = 0;
+  __syncthreads();
+  uint2* out = a.cpairs + map * a.cpair_per_map + ci.pair0;
+  // sign of a pair: that of its basins, in the top bit of the first
+  auto emit = [&](unsigned long long e) {
+    const uint32_t i = static_cast<uint32_t>(e >> 36), j = static_cast<uint32_t>(e >> 8) & 0xfffffffu;
+    const uint32_t b = (i >> 27) * kMaxSteps + kMaxSteps - static_cast<uint32_t>(e & 0xffu);
+    atomicAdd(&cnt[b], 1);
+    out[atomicAdd(&total, 1)] = make_uint2(((i << 4) & 0x7fff0000u) | ((b >> 4) << 12) | (i & 0xfffu),
+                                           ((j << 4) & 0x7fff0000u) | ((b & 15u) << 12) | (j & 0xfffu));
+  };
+#pragma unroll
+  for (int k = 0; k < kCrossPer; ++k) {
+    const int q = tid + k * kCrossThreads;
+    if (q >= ci.nbnd) break;
+    const uint2 me = rec[ci.bnd0 + q];
+    if (me.y == kNone) continue;
+    const int vme = a.bnd_vert[ci.bnd0 + q];
+    const uint32_t s = me.x & 0x80000000u;
+    const uint32_t mine = (static_cast<uint32_t>(a.bnd_tile[ci.bnd0 + q]) << 12) | (me.y & 0xfffu);
+    const int own = static_cast<int>(me.x ^ s);
+    const uint32_t code = kMaxSteps - (me.y >> 16);
+    const int sl = ci.slice0 + (q >> 5);
+    uint32_t last = mine;  // (a one-way entry may lead to the vertex's own basin, which is no pair)
+    const uint32_t o1 = a.cross_off[sl + 1];
+#pragma unroll 4
+    for (uint32_t o = a.cross_off[sl] + lane; o < o1; o += 32) {
+      const uint32_t ub = a.cross[o];
+      const uint2 r = rec[ub];
+      const int w = static_cast<int>(r.x ^ s);
+      if (w > own || (w == own && a.bnd_vert[ub] < vme)) {
+        const uint32_t other = (static_cast<uint32_t>(a.bnd_tile[ub]) << 12) | (r.y & 0xfffu);
+        if (other != last && other != mine) {
+          last = other;
+          const unsigned long long pair =
+              (static_cast<unsigned long long>(min(mine, other) | (s >> 4)) << 28) | max(mine, other);
+          const unsigned long long e = (pair << 8) | code;
+          uint32_t h = static_cast<uint32_t>((pair * 0x9e3779b97f4a7c15ull) >> 54);
+          static_assert(kCrossTable == 1 << 10, "the hash gives 10 bits");
+          for (int t = 0;; ++t) {
+            unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&table[h]);
+            if (cur == 0) cur = atomicCAS(&table[h], 0ull, e);
+            if (cur == 0 || (cur ^ e) < 256) {
+              if (cur != 0 && cur < e) atomicMax(&table[h], e);
+              break;
+            }
+            if (t == kProbes) {
+              emit(e);
+              break;
+            }
+            h = (h + 1) & (kCrossTable - 1);
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < kCrossTable; i += kCrossThreads)
+    if (table[i]) emit(table[i]);
+  __syncthreads();
+  a.tab_cross[(map * a.n_chunks + chunk) * kBuckets + tid] = static_cast<uint32_t>(cnt[tid]);
+  if (tid == 0) a.n_pairs[(int64_t)a.n_maps * a.n_tiles + map * a.n_chunks + chunk] = total;
+}
+
+// Where each tile's entries go: per bucket, the entries of the tiles (and
+// chunks) before it, and the bucket starts of the segment's lists; first basin
+// number of every tile.  One CTA per (map, segment), one thread per bucket.
+__global__ void __launch_bounds__(kBuckets) basin_offset_kernel(BasinArgs a) {
+  __shared__ int tot[kBuckets + 1], wsum[8];
+  const int seg = blockIdx.x % a.n_seg;
+  const int64_t map = blockIdx.x / a.n_seg;
+  const SegInfo si = a.segs[seg];
+  const int b = threadIdx.x;
+  const int64_t row0 = map * a.n_tiles + si.tile0, crow0 = map * a.n_chunks + si.chunk0;
+  const int64_t out = (map * a.n_seg + seg) * kTab;
+  uint32_t run = 0;
+#pragma unroll 8
+  for (int t = 0; t < si.ntiles; ++t) {
+    const uint32_t n = a.tab_ev[(row0 + t) * kBuckets + b];
+    a.off_ev[(row0 + t) * kBuckets + b] = run;
+    run += n;
+  }
+  tot[b] = run;
+  __syncthreads();
+  scan_buckets(tot, wsum);
+  a.start_ev[out + b] = tot[b];
+  if (b == 0) a.start_ev[out + kBuckets] = tot[kBuckets];
+  run = 0;
+#pragma unroll 8
+  for (int t = 0; t < si.ntiles; ++t) {
+    const uint32_t n = a.tab_pair[(row0 + t) * kBuckets + b];
+    a.off_pair[(row0 + t) * kBuckets + b] = run;
+    run += n;
+  }
+#pragma unroll 4
+  for (int c = 0; c < si.nchunks; ++c) {
+    const uint32_t n = a.tab_cross[(crow0 + c) * kBuckets + b];
+    a.off_cross[(crow0 + c) * kBuckets + b] = run;
+    run += n;
+  }
+  __syncthreads();
+  tot[b] = run;
+  __syncthreads();
+  scan_buckets(tot, wsum);
+  a.start_pair[out + b] = tot[b];
+  if (b == 0) a.start_pair[out + kBuckets] = tot[kBuckets];
+  if (b < 64) {  // one warp per sign
+    const int lane = b & 31, sgn = b >> 5;
+    uint32_t before = 0;
+    for (int t0 = 0; t0 < si.ntiles; t0 += 32) {
+      const uint32_t v = (t0 + lane < si.ntiles) ? a.n_basin[(row0 + t0 + lane) * 2 + sgn] : 0u;
+      uint32_t inc = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+      }
+      if (t0 + lane < si.ntiles) a.base_of[(row0 + t0 + lane) * 2 + sgn] = before + inc - v;
+      before += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) {
+      a.n_basins[(map * a.n_seg + seg) * 2 + sgn] = before;
+      if (sgn < a.signs && before > static_cast<uint32_t>(a.most_first))
+        a.queue[atomicAdd(a.counter + 2, 1)] = static_cast<int32_t>((map * a.signs + sgn) * a.n_seg + seg);
+    }
+  }
+}
+
+// The segment's ordered lists, with basin numbers of the whole segment: 16
+// bits a basin where the sweep keeps its state in shared memory, else 32.  One
+// CTA per (map, tile) and (map, chunk).  The order within a bucket is free.
+// A tile's vertices are put in order in shared memory first, so that the
+// segment's list is written in runs.
+template <bool kOrder>
+__global__ void __launch_bounds__(kTileThreads, 3) basin_order_kernel(BasinArgs a) {
+  __shared__ uint32_t sorted[kTile];                // basin | bucket << 24
+  __shared__ uint16_t index[kOrder ? kTile : 1];    // index in the tile
+  __shared__ int start[kBuckets + 1], wsum[8];
+  __shared__ uint32_t to_ev[kBuckets], to_pair[kBuckets];
+  const int units = a.n_tiles + a.n_chunks;
+  const int unit = blockIdx.x % units;
+  const int64_t map = blockIdx.x / units;
+  const int tid = threadIdx.x;
+  const bool is_tile = unit < a.n_tiles;
+  const int chunk = unit - a.n_tiles;
+  const int seg = is_tile ? a.tiles[unit].seg : a.chunks[chunk].seg;
+  const SegInfo si = a.segs[seg];
+  const int64_t srow = (map * a.n_seg + seg) * kTab;
+  const uint32_t* nbs = a.n_basins + (map * a.n_seg + seg) * 2;
+  const bool wide0 = nbs[0] > (uint32_t)a.most_narrow, wide1 = nbs[1] > (uint32_t)a.most_narrow;
+  // the second sign's 16-bit entries start where its 32-bit ones would
+  const uint32_t ev1 = a.start_ev[srow + kMaxSteps], pr1 = a.start_pair[srow + kMaxSteps];
+  const int64_t po = map * a.opair_per_map + si.pair0;
+  if (is_tile) {
+    const TileInfo ti = a.tiles[unit];
+    const int64_t row = map * a.n_tiles + unit;
+    const uint32_t* ev = a.ev + map * a.pos_per_map + ti.pos0;
+    uint32_t rec[kPerThread];
+#pragma unroll
+    for (int k = 0; k < kPerThread; ++k) {
+      const int v = tid + k * kTileThreads;
+      rec[k] = (v < ti.nv) ? ev[v] : kNone;
+    }
+    if (tid < kBuckets) {
+      start[tid] = a.tab_ev[row * kBuckets + tid];
+      to_ev[tid] = a.start_ev[srow + tid] + a.off_ev[row * kBuckets + tid];
+      to_pair[tid] = a.start_pair[srow + tid] + a.off_pair[row * kBuckets + tid];
+    }
+    const uint32_t base0 = a.base_of[row * 2], base1 = a.base_of[row * 2 + 1];
+    const int n_pr = static_cast<int>(a.n_pairs[row]);
+    __syncthreads();
+    scan_buckets(start, wsum);
+    if (tid < kBuckets) to_ev[tid] -= start[tid];
+    const int n_ev = start[kBuckets];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPerThread; ++k) {
+      if (rec[k] == kNone) continue;
+      const uint32_t bk = rec[k] >> 12;
+      const int p = atomicAdd(&start[bk], 1);
+      sorted[p] = ((bk >= kMaxSteps ? base1 : base0) + (rec[k] & 0xfffu)) | (bk << 24);
+      if (kOrder) index[p] = static_cast<uint16_t>(tid + k * kTileThreads);
+    }
+    __syncthreads();
+    const int64_t eo = map * a.n_vertices + si.pos0;
+    uint32_t* ev32 = reinterpret_cast<uint32_t*>(a.ev_out) + eo;
+    uint16_t* ev16 = reinterpret_cast<uint16_t*>(a.ev_out) + 2 * eo;
+#pragma unroll 4
+    for (int p = tid; p < n_ev; p += kTileThreads) {
+      const uint32_t r = sorted[p];
+      const uint32_t bk = r >> 24, id = r & 0xffffffu, d = to_ev[bk] + p;
+      const bool neg = bk >= kMaxSteps;
+      if (neg ? wide1 : wide0) ev32[d] = id;
+      else ev16[d + (neg ? ev1 : 0u)] = static_cast<uint16_t>(id);
+      if (kOrder) a.ord[eo + d] = a.vert[ti.pos0 + index[p]];
+    }
+    const uint32_t* pr = a.pairs + map * a.pair_per_map + ti.pair0;
+    for (int p = tid; p < n_pr; p += kTileThreads) {
+      const uint32_t r = pr[p];
+      const uint32_t bk = r >> 24;
+      const uint32_t d = atomicAdd(&to_pair[bk], 1u);
+      const bool neg = bk >= kMaxSteps;
+      const uint32_t base = neg ? base1 : base0;
+      const uint32_t i = base + ((r >> 12) & 0xfffu), j = base + (r & 0xfffu);
+      if (neg ? wide1 : wide0) reinterpret_cast<uint2*>(a.pair_out)[po + d] = make_uint2(i, j);
+      else reinterpret_cast<uint32_t*>(a.pair_out)[2 * po + (neg ? pr1 : 0u) + d] = (i << 16) | j;
+    }
+  } else {
+    const ChunkInfo ci = a.chunks[chunk];
+    const int64_t row = map * a.n_chunks + chunk;
+    if (tid < kBuckets) to_pair[tid] = a.start_pair[srow + tid] + a.off_cross[row * kBuckets + tid];
+    const uint32_t* base = a.base_of + (map * a.n_tiles + si.tile0) * 2;
+    const int n = static_cast<int>(a.n_pairs[(int64_t)a.n_maps * a.n_tiles + row]);
+    __syncthreads();
+    const uint2* pr = a.cpairs + map * a.cpair_per_map + ci.pair0;
+    for (int p = tid; p < n; p += kTileThreads) {
+      const uint2 r = pr[p];
+      const uint32_t bk = (((r.x >> 12) & 15u) << 4) | ((r.y >> 12) & 15u);
+      const uint32_t d = atomicAdd(&to_pair[bk], 1u);
+      const int sgn = bk >= kMaxSteps;
+      const uint32_t i = base[(r.x >> 16) * 2 + sgn] + (r.x & 0xfffu), j = base[(r.y >> 16) * 2 + sgn] + (r.y & 0xfffu);
+      if (sgn ? wide1 : wide0) reinterpret_cast<uint2*>(a.pair_out)[po + d] = make_uint2(i, j);
+      else reinterpret_cast<uint32_t*>(a.pair_out)[2 * po + (sgn ? pr1 : 0u) + d] = (i << 16) | j;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Threshold steps of one (map, sign, segment).  Bound by latency: a step is a
+// chain of a few hundred dependent instructions on shared memory, and 100
+// steps follow one another (about 2 us a step alone on an SM), so what counts
+// is how many sweeps an SM holds.  The union-find state of an item's basins is
+// private to the CTA: in shared memory, or (more basins than fit) in the CTA's
+// slot of global memory, read and written at CTA scope.
+//
+// Arrays of that state, addressed in the shared window (kShared) or in global
+// memory; every access is one explicit instruction on the state space, which
+// the threads of the CTA order with barriers or read through atomics.
+template <bool kShared, typename T>
+struct StateArray {
+  using Base = typename std::conditional<kShared, uint32_t, char*>::type;
+  Base base;
+  __device__ Base at(uint32_t i) const { return base + i * static_cast<uint32_t>(sizeof(T)); }
+  __device__ T ld(uint32_t i) const {
+    if constexpr (kShared) {
+      if constexpr (sizeof(T) == 2) {
+        uint16_t v;
+        asm volatile("ld.relaxed.cta.shared.u16 %0, [%1];" : "=h"(v) : "r"(at(i)) : "memory");
+        return v;
+      } else if constexpr (sizeof(T) == 4) {
+        uint32_t v;
+        asm volatile("ld.relaxed.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(at(i)) : "memory");
+        return v;
+      } else {
+        double v;
+        asm volatile("ld.relaxed.cta.shared.f64 %0, [%1];" : "=d"(v) : "r"(at(i)) : "memory");
+        return v;
+      }
+    } else if constexpr (sizeof(T) == 2) {
+      uint16_t v;
+      asm volatile("ld.relaxed.cta.global.u16 %0, [%1];" : "=h"(v) : "l"(glob(i)) : "memory");
+      return v;
+    } else if constexpr (sizeof(T) == 4) {
+      uint32_t v;
+      asm volatile("ld.relaxed.cta.global.u32 %0, [%1];" : "=r"(v) : "l"(glob(i)) : "memory");
+      return v;
+    } else {
+      double v;
+      asm volatile("ld.relaxed.cta.global.f64 %0, [%1];" : "=d"(v) : "l"(glob(i)) : "memory");
+      return v;
+    }
+  }
+  __device__ void st(uint32_t i, T v) const {
+    if constexpr (kShared) {
+      if constexpr (sizeof(T) == 2) asm volatile("st.relaxed.cta.shared.u16 [%0], %1;" ::"r"(at(i)), "h"(v) : "memory");
+      else if constexpr (sizeof(T) == 4)
+        asm volatile("st.relaxed.cta.shared.u32 [%0], %1;" ::"r"(at(i)), "r"(v) : "memory");
+      else asm volatile("st.relaxed.cta.shared.f64 [%0], %1;" ::"r"(at(i)), "d"(v) : "memory");
+    } else if constexpr (sizeof(T) == 2) {
+      asm volatile("st.relaxed.cta.global.u16 [%0], %1;" ::"l"(glob(i)), "h"(v) : "memory");
+    } else if constexpr (sizeof(T) == 4) {
+      asm volatile("st.relaxed.cta.global.u32 [%0], %1;" ::"l"(glob(i)), "r"(v) : "memory");
+    } else {
+      asm volatile("st.relaxed.cta.global.f64 [%0], %1;" ::"l"(glob(i)), "d"(v) : "memory");
+    }
+  }
+  __device__ uint32_t cas(uint32_t i, uint32_t expect, uint32_t v) const {
+    uint32_t old;
+    if constexpr (kShared)
+      asm volatile("atom.relaxed.cta.shared.cas.b32 %0, [%1], %2, %3;" : "=r"(old) : "r"(at(i)), "r"(expect), "r"(v) : "memory");
+    else
+      asm volatile("atom.relaxed.cta.global.cas.b32 %0, [%1], %2, %3;" : "=r"(old) : "l"(glob(i)), "r"(expect), "r"(v) : "memory");
+    return old;
+  }
+  __device__ uint32_t add(uint32_t i, uint32_t v) const {
+    uint32_t old;
+    if constexpr (kShared)
+      asm volatile("atom.relaxed.cta.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(at(i)), "r"(v) : "memory");
+    else
+      asm volatile("atom.relaxed.cta.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(glob(i)), "r"(v) : "memory");
+    return old;
+  }
+  __device__ void max_with(uint32_t i, uint32_t v) const {
+    if constexpr (kShared) asm volatile("red.relaxed.cta.shared.max.u32 [%0], %1;" ::"r"(at(i)), "r"(v) : "memory");
+    else asm volatile("red.relaxed.cta.global.max.u32 [%0], %1;" ::"l"(glob(i)), "r"(v) : "memory");
+  }
+
+ private:
+  __device__ char* glob(uint32_t i) const { return (char*)base + (size_t)i * sizeof(T); }
+};
+
+// Where a sweep keeps its state: all in shared memory; the lists of live basins
+// in global memory (read in order, a step's entries at a time); all global.
+enum StateKind { kAllShared = 0, kListsGlobal = 1, kAllGlobal = 2 };
+
+// A basin's word is its parent, or while it is a root kRoot, its age (127 - the
+// step it started at, 0 before; 7 bits) and its extent (24 bits).  The older
+// root takes the younger one in, ties by number, which keeps the trees flat:
+// a large component's root stays, and what it takes in points to it at once.
+// Ages only grow, and a root is linked by a CAS on the word that it was
+// compared with, so the order along parents is strict and walks end.
+template <int kMode, int kKind>
+struct BasinState {
+  static constexpr bool kShared = kKind != kAllGlobal;
+  using W = typename std::conditional<kMode == kPotential, double, uint32_t>::type;
+  using Idx = typename std::conditional<kShared, uint16_t, uint32_t>::type;
+  StateArray<kShared, W> w;  // maxima: largest float sum (bits); potentials: sum, or offset to the parent; nodes: last node
+  StateArray<kShared, uint32_t> word;
+  StateArray<kKind == kAllShared, Idx> list0;  // live basins; the other list holds the step's changes meanwhile
+  StateArray<kKind == kAllShared, Idx> list1;
+  __device__ BasinState(char* smem, char* global, uint32_t n) {
+    if constexpr (kShared) w.base = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    else w.base = global;
+    word.base = w.at(0) + n * static_cast<uint32_t>(sizeof(W));
+    if constexpr (kKind == kListsGlobal) list0.base = global;
+    else list0.base = word.base + n * 4u;
+    list1.base = list0.base + n * static_cast<uint32_t>(sizeof(Idx));
+  }
+};
+constexpr int state_bytes_per_basin(int mode, int kind) {
+  return (mode == kPotential ? 8 : 4) + 4 + (kind == kAllShared ? 4 : kind == kAllGlobal ? 8 : 0);
+}
+
+// One hop of a walk from x, whose word is w (not a root's); kHalve points x to
+// its grandparent.
+template <bool kHalve, typename Words>
+__device__ inline void hop(const Words& word, uint32_t& x, uint32_t& w) {
+  const uint32_t up = word.ld(w);
+  if (kHalve && !(up & kRoot)) word.st(x, up);
+  x = w;
+  w = up;
+}
+
+// Root of x, and its word.
+template <bool kHalve, typename Words>
+__device__ inline uint32_t find_basin(const Words& word, uint32_t x, uint32_t& w) {
+  w = word.ld(x);
+  while (!(w & kRoot)) hop<kHalve>(word, x, w);
+  return x;
+}
+template <bool kHalve, typename Words>
+__device__ inline uint32_t find_basin(const Words& word, uint32_t x) {
+  uint32_t w;
+  return find_basin<kHalve>(word, x, w);
+}
+
+struct SweepShared {
+  float T[kMaxSteps], HH[kMaxSteps];
+  int ev[kMaxSteps + 1], pair[kMaxSteps + 1];  // first entries of the steps
+  float red[32];
+  int L, item, n_basins, n_change;
+  int n_live[3];  // by packs modulo 3: the list's, the packed one's, and one being cleared
+};
+
+__device__ inline uint32_t enc_float(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ inline float dec_float(uint32_t u) {
+  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+}
+
+template <int kMode, int kKind>
+__device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, char* smem, char* global, int64_t map,
+                                           int sgn, int seg, int64_t item) {
+  constexpr bool kNarrow = kKind != kAllGlobal;
+  constexpr bool kHalve = kMode != kPotential;  // a linked root's parent is what its offset refers to
+  const SegInfo si = a.segs[seg];
+  const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, wbase = tid - lane;
+  const int nb = S.n_basins, L = S.L;
+  BasinState<kMode, kKind> st(smem, global, nb);
+  const int64_t eo = map * a.n_vertices + si.pos0, po = map * a.opair_per_map + si.pair0;
+  const int e1 = sgn ? S.ev[0] : 0, p1 = sgn ? S.pair[0] : 0;
+  // events are read two at a time, at even places: entry q of the list is at
+  // place q + e1 (16 bits) or q (32 bits)
+  const uint32_t* ev16 = reinterpret_cast<const uint32_t*>(a.ev_out) + eo;
+  const uint32_t* ev32 = reinterpret_cast<const uint32_t*>(a.ev_out) + eo;
+  const int shift = kNarrow ? e1 : 0;
+  const uint32_t* pair16 = reinterpret_cast<const uint32_t*>(a.pair_out) + 2 * po + p1;
+  const uint2* pair32 = reinterpret_cast<const uint2*>(a.pair_out) + po;
+  // the two events at the even place p, as far as they are in [lo, hi)
+  using Two = typename std::conditional<kNarrow, uint32_t, uint2>::type;
+  auto load_two = [&](int p, int lo, int hi) -> Two {
+    if constexpr (kNarrow) {
+      (void)lo;
+      return p < hi ? ev16[p >> 1] : 0u;
+    } else {
+      return make_uint2(p >= lo && p < hi ? ev32[p] : 0u, p + 1 >= lo && p + 1 < hi ? ev32[p + 1] : 0u);
+    }
+  };
+  auto split = [](const Two& t) -> uint2 {
+    if constexpr (kNarrow) return make_uint2(t & 0xffffu, t >> 16);
+    else return t;
+  };
+  auto load_pair = [&](int q) -> uint2 {
+    if constexpr (kNarrow) {
+      const uint32_t r = pair16[q];
+      return make_uint2(r >> 16, r & 0xffffu);
+    } else {
+      return pair32[q];
+    }
+  };
+  const double* pw = a.seg_pow[seg];
+  for (int i = tid; i < nb; i += nth) {
+    st.word.st(i, kRoot);
+    st.w.st(i, 0);
+  }
+  if (tid == 0) S.n_change = S.n_live[0] = S.n_live[1] = S.n_live[2] = 0;
+  __syncthreads();
+  uint32_t n_nodes = 0;  // nodes: ids handed out before this step
+  Node* nodes = (kMode == kNodes) ? a.nodes + item * a.node_cap : nullptr;
+  // the thread's first entries of a step are loaded a step ahead
+  int ev0 = S.ev[0], ev_end = S.ev[1], pr0 = S.pair[0], pr_end = S.pair[1];
+  Two next_ev[kAhead] = {};
+  uint2 next_pair = make_uint2(0, 0);
+  ev0 += shift;
+  ev_end += shift;
+  auto load_step = [&](int lo, int hi) {
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) next_ev[k] = load_two((lo & ~1) + 2 * (tid + k * nth), lo, hi);
+  };
+  if (L > 0) {
+    load_step(ev0, ev_end);
+    if (pr0 + tid < pr_end) next_pair = load_pair(pr0 + tid);
+  }
+  // the list of live basins, the other one, and their counters and a spare one
+  auto live = st.list0, other = st.list1;
+  int *n_live = &S.n_live[0], *n_next = &S.n_live[1], *n_spare = &S.n_live[2];
+
+  for (int i = 0; i < L; ++i) {
+    Two my_ev[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) my_ev[k] = next_ev[k];
+    const uint2 my_pair = next_pair;
+    const int ev2 = S.ev[min(i + 2, kMaxSteps)] + shift, pr2 = S.pair[min(i + 2, kMaxSteps)];
+    if (i + 1 < L) {
+      load_step(ev_end, ev2);
+      if (pr_end + tid < pr2) next_pair = load_pair(pr_end + tid);
+    }
+    if (ev_end > ev0) {
+      // (1) join the basins of the step's pairs.  A linked root hands its
+      // extent over, and its sum (maxima) or its place in the list of changes
+      // (potentials).  A warp's walks and links go in rounds, all lanes
+      // together.
+      if (pr_end > pr0) {
+        for (int q0 = pr0 + wbase; q0 < pr_end; q0 += nth) {
+          const int q = q0 + lane;
+          uint32_t x = 0, y = 0;
+          bool open = q < pr_end;
+          if (open) {
+            const uint2 r = (q == pr0 + tid) ? my_pair : load_pair(q);
+            x = r.x;
+            y = r.y;
+          }
+          for (int it = 0; __any_sync(0xffffffffu, open); ++it) {
+            if (it >= kFindLimit) {
+              if (open) set_err(a.err, kDevLoopLimit);
+              break;
+            }
+            uint32_t px = kRoot, py = kRoot;
+            if (open) {
+              px = st.word.ld(x);
+              py = st.word.ld(y);
+            }
+            while (__any_sync(0xffffffffu, !(px & py & kRoot))) {
+              if (!(px & kRoot)) hop<kHalve>(st.word, x, px);
+              if (!(py & kRoot)) hop<kHalve>(st.word, y, py);
+            }
+            if (open) {
+              if (x == y) {
+                open = false;
+              } else {
+                const uint32_t ax = px >> 24, ay = py >> 24;
+                const bool x_up = ax != ay ? ax > ay : x < y;
+                const uint32_t hi = x_up ? y : x, was = x_up ? py : px;
+                uint32_t t = x_up ? x : y;
+                if (st.word.cas(hi, was, t) == was) {
+                  open = false;
+                  const uint32_t ext = was & kExtent;
+                  if (kMode == kPotential) other.st(atomicAdd(&S.n_change, 1), hi);
+                  if (ext) {  // its vertices count with the root that it is under by now
+                    for (int k = 0; k < kFindLimit; ++k) {
+                      uint32_t wt;
+                      t = find_basin<kHalve>(st.word, t, wt);
+                      if (st.word.cas(t, wt, wt + ext) == wt) break;
+                    }
+                    if constexpr (kMode == kMaxima) {
+                      // handed to a root that is still one afterwards: a root
+                      // that is linked meanwhile reads its own sum after that
+                      const uint32_t sum = st.w.ld(hi);
+                      for (int k = 0; k < kFindLimit; ++k) {
+                        st.w.max_with(t, sum);
+                        __threadfence_block();
+                        if (st.word.ld(t) & kRoot) break;
+                        t = find_basin<kHalve>(st.word, t);
+                      }
+                    }
+                  }
+                }
+              }
+            }
+          }
+        }
+        __syncthreads();
+      }
+      // (2) potentials: linked roots keep their offset to their final root
+      if constexpr (kMode == kPotential) {
+        const int nc = (pr_end > pr0) ? S.n_change : 0;
+        for (int q = tid; q < nc; q += nth) {
+          const uint32_t d = other.ld(q);
+          const uint32_t r = find_basin<kHalve>(st.word, d);
+          st.w.st(d, st.w.ld(d) - st.w.ld(r));  // roots do not change in this phase
+          st.word.st(d, r);
+        }
+        if (nc) __syncthreads();
+      }
+      // the step's vertices join their component
+      auto join = [&](uint32_t r, uint32_t was) {
+        if (!(was & kExtent)) {  // the component's first vertices: it goes live, with its age
+          live.st(atomicAdd(n_live, 1), r);
+          st.word.add(r, static_cast<uint32_t>(kMaxSteps - 1 - i) << 24);
+        }
+      };
+      auto count_two = [&](int p, const Two& t) {
+        const uint2 two = split(t);
+        uint32_t x = two.x, y = two.y;
+        const bool on_x = p >= ev0 && p < ev_end, on_y = p + 1 >= ev0 && p + 1 < ev_end;
+        if constexpr (kMode == kPotential) {
+          auto climb = [&](uint32_t& r, int q) {
+            double sum = st.w.ld(r);
+            for (uint32_t up = st.word.ld(r); !(up & kRoot); up = st.word.ld(r)) {
+              r = up;
+              sum += st.w.ld(r);
+            }
+            a.base[eo + q - shift] = sum;
+          };
+          if (on_x) climb(x, p);
+          if (on_y) climb(y, p + 1);
+        } else {
+          uint32_t wx = kRoot, wy = kRoot;
+          if (on_x) wx = st.word.ld(x);
+          if (on_y) wy = st.word.ld(y);
+          while (!(wx & wy & kRoot)) {
+            if (!(wx & kRoot)) hop<kHalve>(st.word, x, wx);
+            if (!(wy & kRoot)) hop<kHalve>(st.word, y, wy);
+          }
+        }
+        __syncwarp();
+        // those that share the first lane's component are added at once
+        const uint32_t r0 = __shfl_sync(0xffffffffu, x, 0);
+        const unsigned sx = __ballot_sync(0xffffffffu, on_x && x == r0), sy = __ballot_sync(0xffffffffu, on_y && y == r0);
+        const bool leads = lane == __ffs(sx | sy) - 1;
+        uint32_t was_x = kExtent, was_y = kExtent, was_0 = kExtent;
+        if (leads) was_0 = st.word.add(r0, __popc(sx) + __popc(sy));
+        if (on_x && x != r0) was_x = st.word.add(x, 1u);
+        if (on_y && y != r0) was_y = st.word.add(y, 1u);
+        join(r0, was_0);
+        join(x, was_x);
+        join(y, was_y);
+      };
+      const int even = ev0 & ~1;
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k)
+        if (even + 2 * (wbase + k * nth) < ev_end) count_two(even + 2 * (tid + k * nth), my_ev[k]);
+      for (int p0 = even + 2 * (wbase + kAhead * nth); p0 < ev_end; p0 += 2 * nth)
+        count_two(p0 + 2 * lane, load_two(p0 + 2 * lane, ev0, ev_end));
+      __syncthreads();
+    }
+    // (3) every live component adds its increment.  Linked ones drop out of
+    // the list when it is packed: every eighth step, or every step where the
+    // position in the list numbers the nodes.
+    const float HH = S.HH[i];
+    const int n = *n_live;
+    const bool pack = kMode == kNodes || (i & 7) == 7;
+    // (float)(extent^E * HH): one double product, one rounding
+    // (fast_tfce.hpp:77); for E == 1 the double product of an integer below
+    // 2^24 and a float is exact, so a float product rounds alike
+    auto increment = [&](uint32_t word) {
+      const uint32_t ext = word & kExtent;
+      return pw ? __double2float_rn(__dmul_rn(pw[ext], static_cast<double>(HH))) : __fmul_rn(static_cast<float>(ext), HH);
+    };
+    auto grow = [&](uint32_t c, float inc) {
+      if constexpr (kMode == kMaxima) st.w.st(c, __float_as_uint(__fadd_rn(__uint_as_float(st.w.ld(c)), inc)));
+      if constexpr (kMode == kPotential) st.w.st(c, st.w.ld(c) + static_cast<double>(inc));
+    };
+    if (!pack) {
+      for (int q = tid; q < n; q += nth) {
+        const uint32_t c = live.ld(q);
+        const uint32_t word = st.word.ld(c);
+        if (word & kRoot) grow(c, increment(word));
+      }
+    } else {
+      for (int q0 = wbase; q0 < n; q0 += nth) {
+        const int q = q0 + lane;
+        bool root = false;
+        uint32_t c = 0;
+        float inc = 0.0f;
+        if (q < n) {
+          c = live.ld(q);
+          const uint32_t word = st.word.ld(c);
+          root = word & kRoot;
+          if (root) {
+            inc = increment(word);
+            grow(c, inc);
+          }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, root);
+        int at = 0;
+        if (lane == 0 && m) at = atomicAdd(n_next, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (root) {
+          other.st(at, c);
+          if constexpr (kMode == kNodes) {
+            const uint32_t id = n_nodes + at, last = st.w.ld(c);
+            nodes[id] = Node{inc, kNone};
+            if (last) nodes[last - 1].next = id;  // 0: no node yet
+            st.w.st(c, id + 1);
+          }
+        }
+      }
+    }
+    if (tid == 0) {
+      if (kMode == kPotential) S.n_change = 0;
+      if (pack) *n_spare = 0;  // the list before this one's: read before the last barrier
+    }
+    __syncthreads();
+    if constexpr (kMode == kNodes) {
+      // the last nodes of the linked components lead on to the joined one's,
+      // and the step's vertices start at their component's node
+      for (int q = tid; q < n; q += nth) {
+        const uint32_t c = live.ld(q);
+        const uint32_t last = st.w.ld(c);
+        if (!(st.word.ld(c) & kRoot) && last) nodes[last - 1].next = st.w.ld(find_basin<true>(st.word, c)) - 1;
+      }
+      for (int p = (ev0 & ~1) + 2 * tid; p < ev_end; p += 2 * nth) {
+        const uint2 two = split(load_two(p, ev0, ev_end));
+        if (p >= ev0) a.vnode[eo + p - shift] = st.w.ld(find_basin<true>(st.word, two.x)) - 1;
+        if (p + 1 < ev_end) a.vnode[eo + p + 1 - shift] = st.w.ld(find_basin<true>(st.word, two.y)) - 1;
+      }
+      n_nodes += *n_next;
+      __syncthreads();
+    }
+    if (pack) {
+      auto l = live;
+      live = other;
+      other = l;
+      int* c = n_live;
+      n_live = n_next;
+      n_next = n_spare;
+      n_spare = c;
+    }
+    ev0 = ev_end;
+    ev_end = ev2;
+    pr0 = pr_end;
+    pr_end = pr2;
+  }
+
+  // largest scaled value (pyfunc.py:116-118); vertices that never became
+  // active count as 0
+  const float scale = __fdiv_rn(seg_maximum(a, map, sgn, seg), 100.0f);
+  const int64_t Vs = a.seg_off[seg + 1] - a.seg_off[seg];
+  float best = (L == 0 || S.ev[L] - S.ev[0] < Vs) ? __fmul_rn(0.0f, scale) : -INFINITY;
+  if (Vs == 0) best = -INFINITY;
+  if constexpr (kMode == kMaxima) {
+    const int n = *n_live;
+    for (int q = tid; q < n; q += nth) best = fmaxf(best, __fmul_rn(__uint_as_float(st.w.ld(live.ld(q))), scale));
+  }
+  if constexpr (kMode == kPotential) {
+    float* omap = a.out_maps ? a.out_maps + (map * a.signs + sgn) * a.n_vertices : nullptr;
+    const int end = L ? S.ev[L] : 0;
+    for (int q = S.ev[0] + tid; q < end; q += nth) {
+      uint32_t r;
+      if constexpr (kNarrow) r = reinterpret_cast<const uint16_t*>(ev16)[q + shift];
+      else r = ev32[q];
+      double sum = st.w.ld(r);
+      for (int it = 0; it < kFindLimit; ++it) {
+        const uint32_t p = st.word.ld(r);
+        if (p & kRoot) break;
+        r = p;
+        sum += st.w.ld(r);
+      }
+      sum -= a.base[eo + q];
+      const int64_t v = a.ord[eo + q];
+      if (a.out_mode == 2 && omap) sum += static_cast<double>(omap[v]);
+      const float val0 = __double2float_rn(sum);
+      float val = __fmul_rn(val0, scale);
+      if (a.vdensity) val = __fmul_rn(val, a.vdensity[v]);
+      if (omap) omap[v] = (a.out_mode == 2) ? val0 : val;
+      best = fmaxf(best, val);
+    }
+  }
+  if constexpr (kMode != kNodes) {
+    best = block_max(best, S.red);
+    if (tid == 0 && a.out_max) a.out_max[item] = (best == -INFINITY) ? 0.0f : best;
+  } else {
+    if (tid == 0 && a.out_max) a.part_max[item] = enc_float(best);
+  }
+}
+
+// First launch (kSecond false): the items of up to most_first basins, all state
+// in shared memory.  Second: the queued ones, one CTA per SM with as much
+// shared memory as there is.
+template <int kMode, bool kSecond>
+__global__ void __launch_bounds__(kSecond ? kMaxSweepThreads : 512, kSecond ? 1 : 2) basin_sweep_kernel(BasinArgs a) {
+  __shared__ SweepShared S;
+  extern __shared__ __align__(16) char dyn[];
+  const int tid = threadIdx.x, nth = blockDim.x;
+  const int n_items = kSecond ? a.counter[2] : a.n_items;
+  for (;;) {
+    if (tid == 0) S.item = atomicAdd(a.counter + kSecond, 1);
+    __syncthreads();
+    const int qi = S.item;
+    if (qi >= n_items) return;
+    int64_t out;  // (map * signs + sign) * n_seg + segment
+    if (kSecond) {
+      out = a.queue[qi];
+    } else {
+      const int per_seg = a.n_items / a.n_seg;  // largest segments first
+      out = a.seg_rank ? (int64_t)(qi % per_seg) * a.n_seg + a.seg_rank[qi / per_seg] : qi;
+    }
+    const int seg = static_cast<int>(out % a.n_seg);
+    const int ms = static_cast<int>(out / a.n_seg);
+    const int sgn = ms % a.signs;
+    const int64_t map = ms / a.signs;
+    const int64_t ss = map * a.n_seg + seg;
+    const int nb = static_cast<int>(a.n_basins[ss * 2 + sgn]);
+    if (!kSecond && nb > a.most_first) {
+      __syncthreads();
+      continue;
+    }
+    for (int i = tid; i <= kMaxSteps; i += nth) {
+      S.ev[i] = static_cast<int>(a.start_ev[ss * kTab + sgn * kMaxSteps + i]);
+      S.pair[i] = static_cast<int>(a.start_pair[ss * kTab + sgn * kMaxSteps + i]);
+    }
+    if (tid == 0) {
+      S.n_basins = nb;
+      S.L = threshold_table(table_maximum(a, map, sgn, seg), S.T, a.err);
+    }
+    __syncthreads();
+    for (int i = tid; i < S.L; i += nth) S.HH[i] = pow_h(S.T[i], a.seg_H[seg]);
+    __syncthreads();
+    if (!kSecond) {
+      sweep_item<kMode, kAllShared>(a, S, dyn, nullptr, map, sgn, seg, out);
+    } else {
+      char* slot = a.state + blockIdx.x * a.state_bytes;
+      if (nb <= a.most_narrow) sweep_item<kMode, kListsGlobal>(a, S, dyn, slot, map, sgn, seg, out);
+      else sweep_item<kMode, kAllGlobal>(a, S, dyn, slot, map, sgn, seg, out);
+    }
+    __syncthreads();
+  }
+}
+
+// Fills out_maps for the vertices that never become active: 0 scaled and
+// weighted as the others are.
+__global__ void basin_fill_kernel(BasinArgs a) {
+  const int64_t V = a.n_vertices, n = (int64_t)a.n_maps * a.signs * V;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    float val = 0.0f;
+    if (a.vdensity) val = __fmul_rn(val, a.vdensity[i % V]);
+    a.out_maps[i] = val;
+  }
+}
+
+// Vertex values in the reference's arithmetic: the increments of the vertex's
+// component from its own step on, added in float in threshold order
+// (fast_tfce.hpp:72-84), along the chain of nodes.
+__global__ void __launch_bounds__(256) basin_walk_kernel(BasinArgs a) {
+  __shared__ float red[32];
+  const int ms = blockIdx.y / a.n_seg, seg = blockIdx.y % a.n_seg;
+  const int sgn = ms % a.signs;
+  const int64_t map = ms / a.signs;
+  const int64_t item = blockIdx.y;
+  const uint32_t* start = a.start_ev + (map * a.n_seg + seg) * kTab + sgn * kMaxSteps;
+  const int lo = static_cast<int>(start[0]), hi = static_cast<int>(start[kMaxSteps]);
+  const int64_t eo = map * a.n_vertices + a.segs[seg].pos0;
+  const Node* nodes = a.nodes + item * a.node_cap;
+  const float scale = __fdiv_rn(seg_maximum(a, map, sgn, seg), 100.0f);
+  float* omap = a.out_maps ? a.out_maps + (int64_t)ms * a.n_vertices : nullptr;
+  float best = -INFINITY;
+  for (int q = lo + blockIdx.x * 256 + threadIdx.x; q < hi; q += gridDim.x * 256) {
+    const int64_t v = a.ord[eo + q];
+    float acc = (a.out_mode == 2 && omap) ? omap[v] : 0.0f;
+    uint32_t id = a.vnode[eo + q];
+    for (int it = 0; it < kMaxSteps && id != kNone; ++it) {
+      const Node nd = nodes[id];
+      acc = __fadd_rn(acc, nd.inc);
+      id = nd.next;
+    }
+    float val = __fmul_rn(acc, scale);
+    if (a.vdensity) val = __fmul_rn(val, a.vdensity[v]);
+    if (omap) omap[v] = (a.out_mode == 2) ? acc : val;
+    best = fmaxf(best, val);
+  }
+  if (a.out_max) {
+    best = block_max(best, red);
+    if (threadIdx.x == 0 && best > -INFINITY) atomicMax(a.part_max + item, enc_float(best));
+  }
+}
+
+__global__ void basin_max_out_kernel(BasinArgs a) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < a.n_items; q += gridDim.x * blockDim.x) {
+    const float best = dec_float(a.part_max[q]);
+    a.out_max[q] = (best == -INFINITY) ? 0.0f : best;
+  }
+}
+
+__global__ void basin_power_kernel(double* out, int64_t n, float E) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = extent_power(static_cast<int32_t>(i), E);
+}
+
+// ---------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------
+struct BasinPlan {
+  int device = 0, sms = 0;
+  int32_t n_seg = 0, vmax = 0;
+  int64_t V = 0, n_pos = 0, n_pair = 0, n_cpair = 0, n_opair = 0;
+  int32_t n_tiles = 0, n_chunks = 0, n_bnd = 0;
+  std::vector<void*> owned;  // device tables
+  TileInfo* tiles = nullptr;
+  ChunkInfo* chunks = nullptr;
+  SegInfo* segs = nullptr;
+  int32_t* vert = nullptr;
+  uint32_t* slice_off = nullptr;
+  uint32_t* nbr = nullptr;
+  uint32_t* edge_off = nullptr;
+  uint32_t* edge = nullptr;
+  uint16_t* bnd_local = nullptr;
+  int32_t* bnd_vert = nullptr;
+  uint16_t* bnd_tile = nullptr;
+  uint32_t* cross_off = nullptr;
+  uint32_t* cross = nullptr;
+  const double** seg_pow = nullptr;
+  std::map<float, double*> powers;  // extent^E tables; kept: a captured launch reads them through seg_pow
+  // A buffer that is replaced by a larger one may still be used by a captured
+  // launch: it is kept until the plan goes.  Growth is geometric.
+  char* ws = nullptr;
+  int64_t ws_bytes = 0;
+  std::vector<void*> retired;
+};
+
+namespace {
+
+template <typename T>
+int upload(BasinPlan* p, const std::vector<T>& h, T** d) {
+  const size_t n = std::max<size_t>(1, h.size());
+  TFGB_CUDA(cudaMalloc(reinterpret_cast<void**>(d), n * sizeof(T)));
+  p->owned.push_back(*d);
+  if (!h.empty()) TFGB_CUDA(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+  return TFCE_OK;
+}
+
+int64_t up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
+
+// workspace of a launch of M maps
+struct Layout {
+  int64_t head, ev, pairs, cpairs, tab_ev, tab_pair, tab_cross, n_pairs, queue, n_basin, bnd, off_ev, off_pair, off_cross, base_of,
+      start_ev, start_pair, n_basins, ev_out, pair_out, ord, base, vnode, nodes, part, total;
+};
+
+Layout layout_of(const BasinPlan* p, int64_t M, int signs, int mode, int64_t node_cap) {
+  Layout l{};
+  int64_t o = 0;
+  auto take = [&](int64_t bytes) {
+    const int64_t at = o;
+    o += up(bytes, 256);
+    return at;
+  };
+  l.head = take(256 + M * 2 * p->n_seg * 4);
+  l.ev = take(M * p->n_pos * 4);
+  l.pairs = take(M * p->n_pair * 4);
+  l.cpairs = take(M * p->n_cpair * 8);
+  l.tab_ev = take(M * p->n_tiles * kBuckets * 2);
+  l.tab_pair = take(M * p->n_tiles * kBuckets * 2);
+  l.tab_cross = take(M * p->n_chunks * kBuckets * 4);
+  l.n_pairs = take(M * (p->n_tiles + p->n_chunks) * 4);
+  l.queue = take(M * signs * p->n_seg * 4);
+  l.n_basin = take(M * p->n_tiles * 2 * 2);
+  l.bnd = take(M * p->n_bnd * 8);
+  l.off_ev = take(M * p->n_tiles * kBuckets * 4);
+  l.off_pair = take(M * p->n_tiles * kBuckets * 4);
+  l.off_cross = take(M * p->n_chunks * kBuckets * 4);
+  l.base_of = take(M * p->n_tiles * 2 * 4);
+  l.start_ev = take(M * p->n_seg * kTab * 4);
+  l.start_pair = take(M * p->n_seg * kTab * 4);
+  l.n_basins = take(M * p->n_seg * 2 * 4);
+  l.ev_out = take(M * p->V * 4);
+  l.pair_out = take(M * p->n_opair * 8);
+  if (mode != kMaxima) l.ord = take(M * p->V * 4);
+  if (mode == kPotential) l.base = take(M * p->V * 8);
+  if (mode == kNodes) {
+    l.vnode = take(M * p->V * 4);
+    l.nodes = take(M * signs * p->n_seg * node_cap * 8);
+    l.part = take(M * signs * p->n_seg * 4);
+  }
+  l.total = o;
+  return l;
+}
+
+constexpr int64_t kWorkspaceBudget = 8LL << 30;  // maps are swept in as many launches as this asks for
+
+int64_t node_capacity(const BasinPlan* p) { return (int64_t)p->vmax * kMaxSteps; }
+
+int ensure_ws(BasinPlan* p, int64_t bytes) {
+  if (p->ws_bytes >= bytes) return TFCE_OK;
+  const int64_t want = std::max(bytes, std::min<int64_t>(2 * p->ws_bytes, kWorkspaceBudget));
+  char* fresh = nullptr;
+  TFGB_CUDA(cudaMalloc(&fresh, want));
+  if (p->ws) p->retired.push_back(p->ws);
+  p->ws = fresh;
+  p->ws_bytes = want;
+  return TFCE_OK;
+}
+
+int mode_of(const BasinRequest& r) {
+  const bool values = r.vdensity || r.out_maps;
+  if (!values && !r.potentials) return kMaxima;  // equal to the float sums bit for bit
+  return r.exact ? kNodes : kPotential;
+}
+
+// Threads, shared memory and grid of a sweep launch.
+struct SweepShape {
+  int threads, basins, smem, grid;
+};
+
+// tuning knob: fewer CTAs in flight
+int most_ctas() {
+  const char* env = std::getenv("TFCE_SWEEP_MAX_CTAS");
+  return env ? std::max(0, std::atoi(env)) : 0;
+}
+
+// The first launch of `items` sweeps.  A step of a sweep has about vmax / 128
+// entries.  Few items (one per SM at most): as many threads as the steps fill,
+// and all the shared memory.  Many: CTAs of 256 threads, four per SM with the
+// state of 4,096 basins each (dense; a smooth map of 164k vertices has 3k per
+// sign), or of 512 threads, two per SM with 8,192.
+SweepShape first_shape(const BasinPlan* p, int mode, int64_t items, bool dense) {
+  const bool few = items <= p->sms;
+  const int per_basin = state_bytes_per_basin(mode, kAllShared);
+  SweepShape s{};
+  const int most_threads = (few || !dense) ? 512 : 256;
+  s.threads = 128;
+  while (s.threads < most_threads && s.threads * 128 < p->vmax) s.threads *= 2;
+  s.basins = std::min(few ? 200 * 1024 / per_basin : dense ? 4096 : 8192, p->vmax);
+  s.smem = s.basins * per_basin;
+  const int per_sm = few ? 1 : std::max(1, std::min(1024 / s.threads, 227 * 1024 / (s.smem + 4 * 1024)));
+  s.grid = p->sms * per_sm;
+  if (const int cap = most_ctas()) s.grid = std::min(s.grid, cap);
+  return s;
+}
+
+template <int kMode, bool kSecond>
+int launch_sweep_kernel(BasinArgs& a, const SweepShape& s, cudaStream_t st) {
+  auto* kern = basin_sweep_kernel<kMode, kSecond>;
+  TFGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem));
+  kern<<<s.grid, s.threads, s.smem, st>>>(a);
+  TFGB_CUDA(cudaGetLastError());
+  return TFCE_OK;
+}
+
+template <int kMode>
+int launch_sweeps(BasinArgs& a, const SweepShape& first, const SweepShape& second, bool both, cudaStream_t st) {
+  int rc = launch_sweep_kernel<kMode, false>(a, first, st);
+  if (!rc && both) rc = launch_sweep_kernel<kMode, true>(a, second, st);
+  return rc;
+}
+
+}  // namespace
+
+int basin_resident_items(const BasinPlan* p, bool dense) {
+  return first_shape(p, kMaxima, int64_t{1} << 30, dense).grid;
+}
+
+int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_t>& packed,
+                      const std::vector<int64_t>& seg, BasinPlan** out) {
+  *out = nullptr;
+  const int64_t V = static_cast<int64_t>(off.size()) - 1;
+  const int n_seg = static_cast<int>(seg.size()) - 1;
+  const uint32_t kOne = 0x80000000u, kIdx = 0x7fffffffu;
+  // Tiles: patches grown breadth first from one vertex, so that few entries
+  // cross; a patch that cannot grow goes on from the next free vertex, so that
+  // all tiles of a segment but the last are full.  Inside a tile the vertices
+  // keep their order, so that the statistic is read in runs.
+  std::vector<int32_t> tile_of(V, -1), mark(V, -1);  // tile within the segment
+  std::vector<std::vector<std::vector<int32_t>>> grown(n_seg);
+  parallel_for(n_seg, V, [&](int64_t s) {
+    std::vector<int32_t> queue, rim;
+    int64_t scan = seg[s], left = seg[s + 1] - seg[s];
+    while (left > 0) {
+      const int32_t id = static_cast<int32_t>(grown[s].size());
+      std::vector<int32_t> members;
+      int64_t entries = 0;
+      bool full = false;
+      rim.swap(queue);  // free vertices beside the last tile
+      size_t rim_at = 0, head = 0;
+      while (!full && left > 0) {
+        while (rim_at < rim.size() && tile_of[rim[rim_at]] >= 0) ++rim_at;
+        int32_t start;
+        if (rim_at < rim.size()) {
+          start = rim[rim_at];
+        } else {
+          while (tile_of[scan] >= 0) ++scan;
+          start = static_cast<int32_t>(scan);
+        }
+        queue.assign(1, start);
+        mark[start] = id;
+        for (head = 0; head < queue.size(); ++head) {
+          const int32_t v = queue[head];
+          const int64_t deg = off[v + 1] - off[v];
+          if (static_cast<int>(members.size()) == kTile || (entries > 0 && entries + deg > kTileEntries)) {
+            full = true;
+            break;
+          }
+          entries += deg;
+          tile_of[v] = id;
+          members.push_back(v);
+          --left;
+          for (int64_t e = off[v]; e < off[v + 1]; ++e) {
+            const int32_t u = static_cast<int32_t>(packed[e] & kIdx);
+            if (tile_of[u] < 0 && mark[u] != id) {
+              mark[u] = id;
+              queue.push_back(u);
+            }
+          }
+        }
+      }
+      queue.erase(queue.begin(), queue.begin() + std::min(head, queue.size()));
+      grown[s].push_back(std::move(members));
+    }
+  });
+  std::vector<TileInfo> tiles;
+  std::vector<SegInfo> segs(n_seg);
+  std::vector<std::vector<int32_t>*> members;
+  int32_t vmax = 1;
+  for (int s = 0; s < n_seg; ++s) {
+    vmax = std::max<int32_t>(vmax, static_cast<int32_t>(seg[s + 1] - seg[s]));
+    segs[s].tile0 = static_cast<int32_t>(tiles.size());
+    segs[s].ntiles = static_cast<int32_t>(grown[s].size());
+    if (segs[s].ntiles > 32767) return TFCE_OK;  // tile numbers are 15-bit
+    for (int t = 0; t < segs[s].ntiles; ++t) {
+      TileInfo ti{};
+      ti.seg = s;
+      ti.nv = static_cast<int32_t>(grown[s][t].size());
+      ti.in_seg = t;
+      tiles.push_back(ti);
+      members.push_back(&grown[s][t]);
+    }
+  }
+  const int nt = static_cast<int>(tiles.size());
+  std::vector<uint16_t> local(V, 0);
+  parallel_for(nt, V, [&](int64_t t) {
+    std::vector<int32_t>& mem = *members[t];
+    std::sort(mem.begin(), mem.end());
+    for (size_t i = 0; i < mem.size(); ++i) local[mem[i]] = static_cast<uint16_t>(i);
+  });
+  // entries that basin_cross_kernel takes: to another tile, or one-way
+  auto crosses = [&](int64_t v, uint32_t entry) { return (entry & kOne) || tile_of[entry & kIdx] != tile_of[v]; };
+  // rows of neighbours and of pairs of neighbours, by tile
+  struct Rows {
+    std::vector<uint32_t> nbr, nbr_end, edge, edge_end;
+    int64_t n_edges = 0;
+  };
+  std::vector<Rows> rows(nt);
+  std::vector<uint8_t> is_bnd(V, 0);
+  parallel_for(nt, V, [&](int64_t t) {
+    const std::vector<int32_t>& mem = *members[t];
+    const int nv = tiles[t].nv;
+    Rows& r = rows[t];
+    std::vector<std::vector<uint16_t>> held(nv);
+    // rows of 32 lanes, two entries (4 * index) a lane; padding: the vertex itself
+    auto put = [&](std::vector<uint32_t>& rows_out, int i, size_t width, auto entry) {
+      for (size_t j = 0; j < width; j += 2)
+        for (int l = 0; l < 32; ++l) {
+          uint32_t two[2];
+          for (size_t k = 0; k < 2; ++k) {
+            const int u = i + l < nv ? entry(l, j + k) : -1;
+            two[k] = 4u * static_cast<uint32_t>(u >= 0 ? u : std::min(i + l, nv - 1));
+          }
+          rows_out.push_back(two[0] | (two[1] << 16));
+        }
+    };
+    std::vector<uint16_t> near[32];
+    for (int i = 0; i < nv; i += 32) {
+      size_t width = 0;
+      for (int l = 0; l < 32; ++l) {
+        near[l].clear();
+        if (i + l >= nv) continue;
+        const int32_t v = mem[i + l];
+        for (int64_t e = off[v]; e < off[v + 1]; ++e) {
+          if (crosses(v, packed[e])) {
+            __atomic_store_n(&is_bnd[packed[e] & kIdx], uint8_t{1}, __ATOMIC_RELAXED);
+            __atomic_store_n(&is_bnd[v], uint8_t{1}, __ATOMIC_RELAXED);
+            continue;
+          }
+          const uint16_t u = local[packed[e] & kIdx];
+          near[l].push_back(u);
+          if (u < i + l) continue;
+          // each pair of neighbours once, held by the one that holds fewer so far
+          if (held[u].size() < held[i + l].size()) held[u].push_back(static_cast<uint16_t>(i + l));
+          else held[i + l].push_back(u);
+          ++r.n_edges;
+        }
+        width = std::max(width, near[l].size());
+      }
+      put(r.nbr, i, width, [&](int l, size_t j) { return j < near[l].size() ? int(near[l][j]) : -1; });
+      r.nbr_end.push_back(static_cast<uint32_t>(r.nbr.size()));
+    }
+    for (int pass = 0; pass < 4; ++pass)  // even out: a vertex hands one to a neighbour that holds two fewer
+      for (int i = 0; i < nv; ++i)
+        for (size_t j = 0; j < held[i].size(); ++j) {
+          const int u = held[i][j];
+          if (held[u].size() + 1 < held[i].size()) {
+            held[i][j] = held[i].back();
+            held[i].pop_back();
+            held[u].push_back(static_cast<uint16_t>(i));
+          }
+        }
+    for (int i = 0; i < nv; i += 32) {
+      size_t width = 0;
+      for (int l = 0; l < 32 && i + l < nv; ++l) width = std::max(width, held[i + l].size());
+      put(r.edge, i, width, [&](int l, size_t j) { return j < held[i + l].size() ? int(held[i + l][j]) : -1; });
+      r.edge_end.push_back(static_cast<uint32_t>(r.edge.size()));
+    }
+  });
+  // the tiles one after the other
+  std::vector<int32_t> vert, bnd_vert, bnd_of(V, -1);
+  std::vector<uint32_t> slice_off(1, 0), nbr, edge_off(1, 0), edge;
+  std::vector<uint16_t> bnd_local, bnd_tile;
+  std::vector<int64_t> seg_pairs(n_seg, 0);
+  int64_t n_pair = 0;
+  for (int t = 0; t < nt; ++t) {
+    TileInfo& ti = tiles[t];
+    Rows& r = rows[t];
+    const std::vector<int32_t>& mem = *members[t];
+    ti.pos0 = static_cast<int32_t>(vert.size());
+    ti.slice0 = static_cast<int32_t>(slice_off.size()) - 1;
+    ti.bnd0 = static_cast<int32_t>(bnd_vert.size());
+    ti.pair0 = static_cast<int32_t>(n_pair);
+    for (size_t i = 0; i < r.nbr_end.size(); ++i) {
+      slice_off.push_back(static_cast<uint32_t>(nbr.size()) + r.nbr_end[i]);
+      edge_off.push_back(static_cast<uint32_t>(edge.size()) + r.edge_end[i]);
+    }
+    nbr.insert(nbr.end(), r.nbr.begin(), r.nbr.end());
+    edge.insert(edge.end(), r.edge.begin(), r.edge.end());
+    if (r.n_edges > 65535) return TFCE_OK;  // pairs are counted in 16 bits
+    seg_pairs[ti.seg] += up(r.n_edges, 8);  // pairs of basins: at most one per pair of neighbours
+    n_pair += up(r.n_edges, 8);
+    for (int i = 0; i < ti.nv; ++i) {
+      vert.push_back(mem[i]);
+      if (is_bnd[mem[i]]) {
+        bnd_of[mem[i]] = static_cast<int32_t>(bnd_vert.size());
+        bnd_local.push_back(static_cast<uint16_t>(i));
+        bnd_vert.push_back(mem[i]);
+        bnd_tile.push_back(static_cast<uint16_t>(ti.in_seg));
+      }
+    }
+    ti.nbnd = static_cast<int32_t>(bnd_vert.size()) - ti.bnd0;
+    while (vert.size() % 32) vert.push_back(0);
+    if (n_pair > 0x7fffffffLL || vert.size() > 0x7fffffffull || nbr.size() >= (1ull << 32)) return TFCE_OK;
+    r = Rows();
+  }
+  // crossing lists, in chunks of boundary vertices of one segment
+  std::vector<ChunkInfo> chunks;
+  for (int s = 0; s < n_seg; ++s) {
+    segs[s].chunk0 = static_cast<int32_t>(chunks.size());
+    if (segs[s].ntiles) {
+      const TileInfo& first = tiles[segs[s].tile0];
+      const TileInfo& last = tiles[segs[s].tile0 + segs[s].ntiles - 1];
+      for (int32_t b0 = first.bnd0; b0 < last.bnd0 + last.nbnd; b0 += kCrossChunk) {
+        ChunkInfo c{};
+        c.seg = s;
+        c.bnd0 = b0;
+        c.nbnd = std::min<int32_t>(kCrossChunk, last.bnd0 + last.nbnd - b0);
+        chunks.push_back(c);
+      }
+    }
+    segs[s].nchunks = static_cast<int32_t>(chunks.size()) - segs[s].chunk0;
+  }
+  const int n_chunks = static_cast<int>(chunks.size());
+  std::vector<Rows> crows(n_chunks);
+  parallel_for(n_chunks, V, [&](int64_t c) {
+    std::vector<uint32_t> list[32];
+    for (int i = 0; i < chunks[c].nbnd; i += 32) {
+      size_t width = 0;
+      for (int l = 0; l < 32; ++l) {
+        list[l].clear();
+        if (i + l >= chunks[c].nbnd) continue;
+        const int32_t v = bnd_vert[chunks[c].bnd0 + i + l];
+        for (int64_t e = off[v]; e < off[v + 1]; ++e)
+          if (crosses(v, packed[e])) list[l].push_back(static_cast<uint32_t>(bnd_of[packed[e] & kIdx]));
+        crows[c].n_edges += static_cast<int64_t>(list[l].size());
+        width = std::max(width, list[l].size());
+      }
+      for (size_t j = 0; j < width; ++j)
+        for (int l = 0; l < 32; ++l) {
+          const int self = std::min(i + l, chunks[c].nbnd - 1);  // padding: the vertex itself
+          crows[c].nbr.push_back(j < list[l].size() ? list[l][j] : static_cast<uint32_t>(chunks[c].bnd0 + self));
+        }
+      crows[c].nbr_end.push_back(static_cast<uint32_t>(crows[c].nbr.size()));
+    }
+  });
+  std::vector<uint32_t> cross_off(1, 0), cross;
+  int64_t n_cpair = 0;
+  for (int c = 0; c < n_chunks; ++c) {
+    chunks[c].slice0 = static_cast<int32_t>(cross_off.size()) - 1;
+    chunks[c].pair0 = static_cast<int32_t>(n_cpair);
+    for (uint32_t e : crows[c].nbr_end) cross_off.push_back(static_cast<uint32_t>(cross.size()) + e);
+    cross.insert(cross.end(), crows[c].nbr.begin(), crows[c].nbr.end());
+    n_cpair += up(crows[c].n_edges, 4);
+    seg_pairs[chunks[c].seg] += up(crows[c].n_edges, 4);
+    if (n_cpair > 0x7fffffffLL || cross.size() >= (1ull << 32)) return TFCE_OK;
+  }
+  int64_t n_opair = 0;
+  for (int s = 0; s < n_seg; ++s) {
+    segs[s].pos0 = seg[s];
+    segs[s].pair0 = n_opair;
+    n_opair += seg_pairs[s];
+  }
+  BasinPlan* p = new BasinPlan();
+  cudaGetDevice(&p->device);
+  cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
+  p->n_seg = n_seg;
+  p->vmax = vmax;
+  p->V = V;
+  p->n_pos = static_cast<int64_t>(vert.size());
+  p->n_pair = n_pair;
+  p->n_cpair = n_cpair;
+  p->n_opair = n_opair;
+  p->n_tiles = nt;
+  p->n_chunks = static_cast<int32_t>(chunks.size());
+  p->n_bnd = static_cast<int32_t>(bnd_vert.size());
+  int rc = upload(p, tiles, &p->tiles);
+  if (!rc) rc = upload(p, chunks, &p->chunks);
+  if (!rc) rc = upload(p, segs, &p->segs);
+  if (!rc) rc = upload(p, vert, &p->vert);
+  if (!rc) rc = upload(p, slice_off, &p->slice_off);
+  if (!rc) rc = upload(p, nbr, &p->nbr);
+  if (!rc) rc = upload(p, edge_off, &p->edge_off);
+  if (!rc) rc = upload(p, edge, &p->edge);
+  if (!rc) rc = upload(p, bnd_local, &p->bnd_local);
+  if (!rc) rc = upload(p, bnd_vert, &p->bnd_vert);
+  if (!rc) rc = upload(p, bnd_tile, &p->bnd_tile);
+  if (!rc) rc = upload(p, cross_off, &p->cross_off);
+  if (!rc) rc = upload(p, cross, &p->cross);
+  std::vector<const double*> none(n_seg, nullptr);
+  if (!rc) rc = upload(p, none, &p->seg_pow);
+  if (rc) {
+    basin_plan_destroy(p);
+    return rc;
+  }
+  *out = p;
+  return TFCE_OK;
+}
+
+void basin_plan_destroy(BasinPlan* p) {
+  if (!p) return;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  cudaSetDevice(p->device);
+  for (void* d : p->owned) cudaFree(d);
+  for (auto& kv : p->powers) cudaFree(kv.second);
+  for (void* d : p->retired) cudaFree(d);
+  cudaFree(p->ws);
+  cudaSetDevice(dev);
+  delete p;
+}
+
+int basin_plan_set_exponents(BasinPlan* p, const float* E) {
+  std::vector<const double*> rows(p->n_seg, nullptr);
+  for (int s = 0; s < p->n_seg; ++s) {
+    if (E[s] == 1.0f) continue;
+    auto it = p->powers.find(E[s]);
+    if (it == p->powers.end()) {
+      double* d = nullptr;
+      const int64_t n = (int64_t)p->vmax + 1;
+      TFGB_CUDA(cudaMalloc(&d, n * sizeof(double)));
+      it = p->powers.emplace(E[s], d).first;
+      basin_power_kernel<<<static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, 1216)), 256>>>(d, n, E[s]);
+      TFGB_CUDA(cudaGetLastError());
+      TFGB_CUDA(cudaStreamSynchronize(nullptr));
+    }
+    rows[s] = it->second;
+  }
+  TFGB_CUDA(cudaMemcpy(p->seg_pow, rows.data(), rows.size() * sizeof(double*), cudaMemcpyHostToDevice));
+  return TFCE_OK;
+}
+
+bool basin_takes(const BasinPlan* p, const BasinRequest& r) {
+  if (!p) return false;
+  const int mode = mode_of(r);
+  const int64_t cap = mode == kNodes ? node_capacity(p) : 0;
+  return layout_of(p, 1, r.signs, mode, cap).total <= kWorkspaceBudget;
+}
+
+int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st) {
+  const int mode = mode_of(r);
+  const int64_t cap = mode == kNodes ? node_capacity(p) : 0;
+  const int64_t one = layout_of(p, 1, r.signs, mode, cap).total;
+  // as many maps per launch as the budget holds, in launches of equal size
+  int64_t most = std::max<int64_t>(1, kWorkspaceBudget / one);
+  most = std::min<int64_t>(most, std::max<int64_t>(1, 0x7fffffffLL / std::max(1, p->n_tiles + p->n_chunks)));
+  if (mode == kNodes)  // one grid row of the walk per item
+    most = std::min<int64_t>(most, std::max<int64_t>(1, 65535 / ((int64_t)r.signs * p->n_seg)));
+  const int64_t launches = (r.n_maps + most - 1) / most;
+  const int64_t per = (r.n_maps + launches - 1) / launches;
+
+  const int64_t items_max = per * r.signs * p->n_seg;
+  SweepShape first = first_shape(p, mode, items_max, r.dense), second{};
+  second.threads = kMaxSweepThreads;
+  second.basins = std::min(std::min(222 * 1024 / state_bytes_per_basin(mode, kListsGlobal), 65535), p->vmax);
+  second.smem = second.basins * state_bytes_per_basin(mode, kListsGlobal);
+  int64_t slots2 = p->sms;
+  if (const int cap_ctas = most_ctas()) slots2 = std::min<int64_t>(slots2, cap_ctas);
+  slots2 = std::min(slots2, items_max);
+  const int slots = first.grid;
+  const bool both = first.basins < p->vmax;
+  const int64_t state = !both ? 0 : up((int64_t)p->vmax * state_bytes_per_basin(mode, kAllGlobal), 256);
+  const Layout lay = layout_of(p, per, r.signs, mode, cap);
+  const int rc = ensure_ws(p, lay.total + slots2 * state);
+  if (rc) return rc;
+
+  BasinArgs a{};
+  a.map_stride = r.map_stride;
+  a.signs = r.signs;
+  a.n_seg = p->n_seg;
+  a.vdensity = r.vdensity;
+  a.out_mode = r.out_mode;
+  a.n_vertices = p->V;
+  a.thr_group = r.thr_group;
+  a.seg_H = r.d_H;
+  a.seg_off = r.d_seg_off;
+  a.seg_rank = r.seg_rank;
+  a.err = r.err;
+  a.tiles = p->tiles;
+  a.chunks = p->chunks;
+  a.segs = p->segs;
+  a.vert = p->vert;
+  a.slice_off = p->slice_off;
+  a.nbr = p->nbr;
+  a.edge_off = p->edge_off;
+  a.edge = p->edge;
+  a.bnd_local = p->bnd_local;
+  a.bnd_vert = p->bnd_vert;
+  a.bnd_tile = p->bnd_tile;
+  a.cross_off = p->cross_off;
+  a.cross = p->cross;
+  a.seg_pow = p->seg_pow;
+  a.n_tiles = p->n_tiles;
+  a.n_chunks = p->n_chunks;
+  a.n_bnd = p->n_bnd;
+  a.counter = reinterpret_cast<int32_t*>(p->ws + lay.head);
+  a.seg_max = reinterpret_cast<uint32_t*>(p->ws + lay.head + 256);
+  auto at = [&](auto*& ptr, int64_t o) { ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(p->ws + o); };
+  at(a.ev, lay.ev);
+  at(a.pairs, lay.pairs);
+  at(a.cpairs, lay.cpairs);
+  at(a.tab_ev, lay.tab_ev);
+  at(a.tab_pair, lay.tab_pair);
+  at(a.tab_cross, lay.tab_cross);
+  at(a.n_pairs, lay.n_pairs);
+  at(a.queue, lay.queue);
+  at(a.n_basin, lay.n_basin);
+  at(a.bnd, lay.bnd);
+  at(a.off_ev, lay.off_ev);
+  at(a.off_pair, lay.off_pair);
+  at(a.off_cross, lay.off_cross);
+  at(a.base_of, lay.base_of);
+  at(a.start_ev, lay.start_ev);
+  at(a.start_pair, lay.start_pair);
+  at(a.n_basins, lay.n_basins);
+  a.ev_out = p->ws + lay.ev_out;
+  a.pair_out = p->ws + lay.pair_out;
+  at(a.ord, lay.ord);
+  at(a.base, lay.base);
+  at(a.vnode, lay.vnode);
+  at(a.nodes, lay.nodes);
+  at(a.part_max, lay.part);
+  a.pos_per_map = p->n_pos;
+  a.pair_per_map = p->n_pair;
+  a.cpair_per_map = p->n_cpair;
+  a.opair_per_map = p->n_opair;
+  a.node_cap = cap;
+  a.state = p->ws + lay.total;
+  a.state_bytes = state;
+  a.most_first = first.basins;
+  a.most_narrow = std::max(first.basins, second.basins);
+  for (int64_t m0 = 0; m0 < r.n_maps; m0 += per) {
+    const int64_t M = std::min(per, r.n_maps - m0);
+    a.n_maps = static_cast<int32_t>(M);
+    a.stats = r.stats + m0 * r.map_stride;
+    a.out_max = r.out_max ? r.out_max + m0 * r.signs * p->n_seg : nullptr;
+    a.out_maps = r.out_maps ? r.out_maps + m0 * r.signs * p->V : nullptr;
+    a.n_items = static_cast<int32_t>(M * r.signs * p->n_seg);
+    TFGB_CUDA(cudaMemsetAsync(p->ws + lay.head, 0, 256 + M * 2 * p->n_seg * 4, st));
+    // a block per (map, segment) reads about 8k values or, with many maps, all of a segment
+    const int64_t pairs_ms = M * p->n_seg;
+    const int64_t parts = std::max<int64_t>(
+        1, std::min<int64_t>((p->vmax + 8191) / 8192, (8 * p->sms + pairs_ms - 1) / pairs_ms));
+    basin_max_kernel<<<static_cast<unsigned>(pairs_ms * parts), 256, 0, st>>>(a, static_cast<int32_t>(parts));
+    if (a.out_maps && r.out_mode == 1) {
+      const int64_t n = M * r.signs * p->V;
+      basin_fill_kernel<<<static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, p->sms * 16)), 256, 0, st>>>(a);
+    }
+    if (p->n_tiles) basin_tile_kernel<<<static_cast<unsigned>(M * p->n_tiles), kTileThreads, 0, st>>>(a);
+    if (p->n_chunks)
+      basin_cross_kernel<<<static_cast<unsigned>(M * p->n_chunks), kCrossThreads, 0, st>>>(a);
+    basin_offset_kernel<<<static_cast<unsigned>(pairs_ms), kBuckets, 0, st>>>(a);
+    const unsigned units = static_cast<unsigned>(M * (p->n_tiles + p->n_chunks));
+    if (units && mode == kMaxima) basin_order_kernel<false><<<units, kTileThreads, 0, st>>>(a);
+    else if (units) basin_order_kernel<true><<<units, kTileThreads, 0, st>>>(a);
+    TFGB_CUDA(cudaGetLastError());
+    first.grid = std::min(slots, a.n_items);
+    second.grid = static_cast<int>(std::min<int64_t>(slots2, a.n_items));
+    int e;
+    if (mode == kMaxima) e = launch_sweeps<kMaxima>(a, first, second, both, st);
+    else if (mode == kPotential) e = launch_sweeps<kPotential>(a, first, second, both, st);
+    else e = launch_sweeps<kNodes>(a, first, second, both, st);
+    if (e) return e;
+    if (mode == kNodes) {
+      const dim3 g(static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((p->vmax + 255) / 256, 1024))),
+                   static_cast<unsigned>(a.n_items));
+      basin_walk_kernel<<<g, 256, 0, st>>>(a);
+      if (a.out_max)
+        basin_max_out_kernel<<<static_cast<unsigned>((a.n_items + 255) / 256), 256, 0, st>>>(a);
+      TFGB_CUDA(cudaGetLastError());
+    }
+  }
+  return TFCE_OK;
+}
+
+}  // namespace tfgb

@@ -1,7 +1,11 @@
-// TFCE sweep over adjacency sets, batched: the GB300 replacement of
+// TFCE sweep over adjacency sets: the GB300 replacement of
 // tfce_mediation/lib/fast_tfce.hpp:11-95 (reached through
 // tfce_mediation/tfce.pyx:44-45) and of the per-permutation scaling/max of
-// tfce_mediation/pyfunc.py:107-126.
+// tfce_mediation/pyfunc.py:107-126.  The adjacency handle and the C-ABI; the
+// batched launches run in the basin form (tfce_basin.cu).  The kernel here
+// sweeps vertex by vertex: it records labels and extents of every threshold,
+// serves callers that cannot allocate (tfce_sweep_batch_noalloc, a CSR that is
+// validated on the device), and graphs that the basin form does not take.
 //
 // One work item = (map, sign, segment).  One CTA sweeps one item at a time and
 // pulls the next from a global queue (persistent grid sized to the resident
@@ -18,82 +22,36 @@
 //      larger root under the smaller, so parent[x] < x and walks end).  A
 //      thread takes the next new vertex from a shared cursor, walks the roots
 //      of all its effective neighbours in lockstep (one round of loads per
-//      hop; path halving in the exact mode) and links every distinct root
-//      under the smallest with CASes issued together; a lost race falls back
-//      to a general unite; (S) the roots that were linked this step hand their
-//      extent to their final root and point at it; (A) every active vertex
-//      adds (float)(extent^E * HH_i) to its own
-//      accumulator, in threshold order -- the reference's per-vertex
-//      arithmetic, so results are bit-identical to it;
+//      hop, path halving) and links every distinct root under the smallest
+//      with CASes issued together; a lost race falls back to a general unite;
+//      (S) the roots that were linked this step hand their extent to their
+//      final root and point at it; (A) every active vertex adds
+//      (float)(extent^E * HH_i) to its own accumulator, in threshold order --
+//      the reference's per-vertex arithmetic, so results are bit-identical to
+//      it;
 //   4. the map is scaled by max/100 (and vdensity), reduced to its max, and
 //      optionally written out.
 // Every walk and retry loop is bounded; a bound sets an error word and the
 // kernel runs on to its exit.
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
 #include <mutex>
 #include <vector>
 
-#include "common.cuh"
+#include "basin.cuh"
+#include "host_parallel.h"
+#include "sweep_common.cuh"
 
 namespace tfgb {
 
-#ifdef TFGB_PHASE_PROFILE
-// Debug-only: clock64 cycles spent per phase, summed over items (thread 0).
-__device__ unsigned long long g_phase_cycles[8];
-#define TFGB_PHASE_MARK(k)                                              \
-  do {                                                                  \
-    if (threadIdx.x == 0) {                                             \
-      const long long _now = clock64();                                 \
-      atomicAdd(&g_phase_cycles[k], (unsigned long long)(_now - _pt));  \
-      _pt = _now;                                                       \
-    }                                                                   \
-  } while (0)
-// Debug-only event counters: [0] unite calls, [1] CAS attempts, [2] CAS
-// failures, [3] find hops, [4] halving writes, [5] list entries checked.
-__device__ unsigned long long g_dbg_counts[8];
-// Debug-only: cycles of each step's (U+S+A) by threshold index.
-__device__ unsigned long long g_step_cycles[128];
-#define TFGB_COUNT(k, n) atomicAdd(&g_dbg_counts[k], (unsigned long long)(n))
-#else
-#define TFGB_PHASE_MARK(k) do { } while (0)
-#define TFGB_COUNT(k, n) do { } while (0)
-#endif
-
-constexpr int kMaxSteps = 128;
-#ifndef TFGB_SWEEP_THREADS
-#define TFGB_SWEEP_THREADS 512
-#endif
-#ifndef TFGB_ACTIVE_BITMAP
-#define TFGB_ACTIVE_BITMAP 1
-#endif
 // largest activity bitmap kept in shared memory (segments up to 393,216 vertices)
 constexpr int kBitmapMaxBytes = 48 * 1024;
-#ifndef TFGB_SWEEP_MINBLOCKS
-#define TFGB_SWEEP_MINBLOCKS 3  // 3 x 512 threads per SM (40 registers; a few spills)
-#endif
-#ifndef TFGB_UBATCH
-#define TFGB_UBATCH 6
-#endif
-#ifndef TFGB_ALANES
-#define TFGB_ALANES 1
-#endif
-// path halving in the maxima-only form (no potential chains to preserve)
-#ifndef TFGB_MAX_HALVE
-#define TFGB_MAX_HALVE 0
-#endif
-#ifndef TFGB_MAX_REC8  // maxima-only form: 8-byte {float sum, extent} records
-#define TFGB_MAX_REC8 1
-#endif
-constexpr int kSweepThreads = TFGB_SWEEP_THREADS;
-constexpr int kUBatch = TFGB_UBATCH;   // list entries of one vertex looked up together
-constexpr int kALanes = TFGB_ALANES;   // positions per thread per accumulation round
-#ifndef TFGB_SLANES
-#define TFGB_SLANES 1
-#endif
-constexpr int kSLanes = TFGB_SLANES;   // dead roots per thread per size round
+constexpr int kSweepThreads = 512;
+constexpr int kSweepMinBlocks = 3;  // 3 x 512 threads per SM (40 registers; a few spills)
+constexpr int kUBatch = 6;          // list entries of one vertex looked up together
 constexpr uint32_t kOneWay = 0x80000000u;   // entry whose reverse entry is missing
 constexpr uint32_t kIndexMask = 0x7fffffffu;
 constexpr uint32_t kInactiveKey = 0xffffffffu;
@@ -146,25 +104,6 @@ struct SweepArgs {
   const int32_t* seg_rank;
 };
 
-// Per-component mode: the increments so far (root) or the potential to the
-// root joined (dead root) and the extent of a position, in one 16-byte record
-// so that the size and accumulation phases touch one sector per position.
-struct alignas(16) Rec {
-  double w;
-  int32_t size;
-  int32_t pad;
-};
-
-// Maxima-only form: {sum, extent} of a position in 8 bytes (in the Rec region
-// of the slot; four records per sector).  The sum is a float: rounding is
-// monotone, so fl(max(a, b) + x) = max(fl(a + x), fl(b + x)), and the largest
-// float sum kept per component equals the largest per-vertex float
-// accumulation of its members (fast_tfce.hpp:77-82) bit for bit.
-struct alignas(8) Rec8 {
-  float w;  // >= 0: ordered as its bit pattern
-  int32_t size;
-};
-
 struct Slot {
   uint32_t* key;
   int32_t* order;
@@ -172,10 +111,6 @@ struct Slot {
   int32_t* size;
   float* acc;
   int32_t* dead;
-  // per-component accumulation only
-  int32_t* roots_a;  // live roots after the previous threshold ...
-  int32_t* roots_b;  // ... and after this one (swapped every step)
-  Rec* rec;          // {W, extent} per position
 };
 
 __host__ __device__ inline int64_t align_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
@@ -184,18 +119,9 @@ __host__ __device__ inline int64_t slot_bytes(int32_t vcap) {
   return 6 * align_up((int64_t)vcap * 4, 256);
 }
 
-// Per-component accumulation adds two root lists and a 16-byte {W, extent}
-// record per vertex to the six int32/float arrays of the exact mode.
-__host__ __device__ inline int64_t slot_bytes_lazy(int32_t vcap) {
-  return 8 * align_up((int64_t)vcap * 4, 256) + align_up((int64_t)vcap * 16, 256);
-}
-
 __device__ inline Slot make_slot(char* base, int32_t vcap) {
   const int64_t s = align_up((int64_t)vcap * 4, 256);
   Slot sl;
-  sl.roots_a = reinterpret_cast<int32_t*>(base + 6 * s);
-  sl.roots_b = reinterpret_cast<int32_t*>(base + 7 * s);
-  sl.rec = reinterpret_cast<Rec*>(base + 8 * s);
   sl.key = reinterpret_cast<uint32_t*>(base);
   sl.order = reinterpret_cast<int32_t*>(base + s);
   sl.parent = reinterpret_cast<int32_t*>(base + 2 * s);
@@ -205,20 +131,17 @@ __device__ inline Slot make_slot(char* base, int32_t vcap) {
   return sl;
 }
 
-__device__ inline void set_err(int32_t* err, int32_t code) { atomicCAS(err, 0, code); }
-
 // dynamic shared memory of the activity bitmap for segments of up to vmax
 // vertices (0 when it would not fit: the union phase then loads every key)
 inline int bitmap_bytes(int64_t vmax) {
   const int64_t b = (vmax + 31) / 32 * 4;
-  return (TFGB_ACTIVE_BITMAP && b <= kBitmapMaxBytes) ? static_cast<int>(b) : 0;
+  return b <= kBitmapMaxBytes ? static_cast<int>(b) : 0;
 }
 
 // Union-find state of an item is private to the one CTA (one SM) sweeping it,
 // so loads and stores of it are relaxed at CTA scope: coherent with the
 // CTA's own CAS/atomics under the PTX memory model, and free to be served
 // from L1 (the hot roots of large components are read by every thread).
-#ifndef TFGB_STATE_GLOBAL_SCOPE
 __device__ inline int32_t ld_state(const int32_t* p) {
   int32_t v;
   asm volatile("ld.relaxed.cta.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -227,27 +150,19 @@ __device__ inline int32_t ld_state(const int32_t* p) {
 __device__ inline void st_state(int32_t* p, int32_t v) {
   asm volatile("st.relaxed.cta.global.s32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
 }
-#else
-__device__ inline int32_t ld_state(const int32_t* p) { return __ldcg(p); }
-__device__ inline void st_state(int32_t* p, int32_t v) { __stcg(p, v); }
-#endif
 
 // Root of x, halving the path on the way: every non-root visited is
 // re-pointed to its grandparent.  Only roots are ever linked (by CAS), and a
 // non-root's new parent is one of its ancestors, so concurrent walks and links
 // stay consistent.  parent[] entries only point to smaller positions, so the
 // walk ends; the limit is a second guard.
-template <bool kHalve = true>
 __device__ inline int32_t find_root(int32_t* parent, int32_t x, int32_t* err) {
   for (int it = 0; it < kWalkLimit; ++it) {
     const int32_t p = ld_state(parent + x);
-    TFGB_COUNT(3, 1);
     if (p == x) return x;
     const int32_t g = ld_state(parent + p);
-    TFGB_COUNT(3, 1);
     if (g == p) return p;
-    if (kHalve) st_state(parent + x, g);
-    TFGB_COUNT(4, 1);
+    st_state(parent + x, g);
     x = g;
   }
   set_err(err, kDevLoopLimit);
@@ -257,19 +172,14 @@ __device__ inline int32_t find_root(int32_t* parent, int32_t x, int32_t* err) {
 // Join the component of root-hint `a` with position b; returns the root of
 // the joined component (a hint: another thread may link it later).  A linked
 // root older than fresh_lo is appended to the dead list.
-template <bool kHalve = true>
 __device__ inline int32_t unite(int32_t* parent, int32_t a, int32_t b, int32_t* dead,
                                 int32_t* n_dead, int32_t fresh_lo, int32_t* err) {
-  TFGB_COUNT(0, 1);
   for (int it = 0; it < kWalkLimit; ++it) {
-    a = find_root<kHalve>(parent, a, err);
-    b = find_root<kHalve>(parent, b, err);
+    a = find_root(parent, a, err);
+    b = find_root(parent, b, err);
     if (a == b) return a;
     const int32_t hi = max(a, b), lo = min(a, b);
-    TFGB_COUNT(1, 1);
-    const int32_t old = atomicCAS(parent + hi, hi, lo);
-    if (old != hi) TFGB_COUNT(2, 1);
-    if (old == hi) {
+    if (atomicCAS(parent + hi, hi, lo) == hi) {
       // roots activated at this step (positions >= fresh_lo) are found by the
       // size phase in the step's own position range; older ones are listed
       if (hi < fresh_lo) dead[atomicAdd(n_dead, 1)] = hi;
@@ -293,94 +203,27 @@ __device__ inline float increment(int32_t extent, float E, int e_mode, float HH)
   return __double2float_rn(__dmul_rn(pe, static_cast<double>(HH)));
 }
 
-// HH = pow(T, H) as a float (fast_tfce.hpp:70), correctly rounded: T*T for
-// H == 2 (exact product, one rounding), otherwise the double-precision power
-// rounded once to float.  The reference calls the host libm's powf, which is
-// not always correctly rounded (glibc: <= 0.82 ulp), so at rare thresholds
-// its HH can sit one float ulp away from this value.
-__device__ inline float pow_h(float T, float H) {
-  if (H == 2.0f) return __fmul_rn(T, T);
-  if (H == 1.0f) return T;
-  return __double2float_rn(pow(static_cast<double>(T), static_cast<double>(H)));
-}
-
-__device__ inline float block_max(float v, float* red) {
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  if (w == 0) {
-    v = (l < (int)(blockDim.x >> 5)) ? red[l] : -INFINITY;
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (l == 0) red[0] = v;
-  }
-  __syncthreads();
-  const float r = red[0];
-  __syncthreads();
-  return r;
-}
-
 // kChecked = false: the handle's cleaned CSR (validated on the host, entries
 // whose reverse is missing flagged).  kChecked = true: a CSR the caller keeps
 // on the device, unvalidated and unflagged -- segment ranges and list extents
 // are checked here, and the insertion-order rule is applied to every
 // same-step entry (for a symmetric pair exactly one direction passes it, so
 // the partition is the same).
-//
-// kLazy = false: the reference's arithmetic -- every active vertex adds its
-// float increment to its own float accumulator at every threshold, so results
-// are bit-identical to the reference sweep.  kLazy = true: per-component
-// accumulation -- each live root adds its component's increment to a double
-// once per threshold; a root that is linked keeps its potential relative to
-// the root it joins, and a vertex's value is the sum of potentials along its
-// parent chain (no path halving in this mode, so a dead root's parent stays
-// the root it joined), rounded to float once.  Per threshold that is O(live
-// components) instead of O(active vertices); the result is the exact sum of
-// the same float increments, so it differs from the reference only by the
-// reference's own float summation error.
-//
-// kMaxOnly (with kLazy): only the scaled maxima are wanted and no vertex
-// weights apply.  Every vertex of a component gets the same increment from
-// the threshold it joins it on, so the largest TFCE in a component is the
-// largest sum accumulated by any of the components merged into it, plus the
-// merged component's own increments since: a root keeps that largest sum
-// (a linked root hands its sum to its final root by atomic max) and the
-// map's maximum is the largest sum among the last live roots.  No potentials
-// are kept, so there is no per-vertex resolve pass.
-//
-// kMinBlocks: resident CTAs per SM the register budget is cut for (3: 40
-// registers with a few spills, the most items in flight; 2: 64 registers, no
-// spills) -- the sweep's CTA shape, chosen per study by the autotuner.
-template <bool kChecked, bool kLazy, bool kMaxOnly = false, int kMinBlocks = TFGB_SWEEP_MINBLOCKS>
-__global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(SweepArgs a) {
-  static_assert(!kMaxOnly || kLazy, "the maxima-only form is a per-component form");
+template <bool kChecked>
+__global__ void __launch_bounds__(kSweepThreads, kSweepMinBlocks) tfce_sweep_kernel(SweepArgs a) {
   __shared__ float sT[kMaxSteps];
   __shared__ float sHH[kMaxSteps];
   __shared__ int32_t sCnt[kMaxSteps + 1];
   __shared__ int32_t sStart[kMaxSteps + 1];
   __shared__ float sRed[32];
-  __shared__ int32_t sItem, sL, sNDead, sNRoots, sNext, sGrab, sGrabS, sGrabA;
+  __shared__ int32_t sItem, sL, sNDead, sGrab, sGrabS;
   // bit v set once vertex v is active (its activation step <= the current
   // step): the union phase loads a neighbour's key only when it is set
   extern __shared__ uint32_t sAct[];
-  const bool use_bm = TFGB_ACTIVE_BITMAP && a.bm_words > 0;
+  const bool use_bm = a.bm_words > 0;
 
   Slot sl = make_slot(a.ws + (int64_t)blockIdx.x * a.ws_slot_bytes, a.vcap);
   const int tid = threadIdx.x, nth = blockDim.x;
-  // Per-component mode keeps every dead root's parent at the root it joined
-  // (no path halving), so parent[] is also the chain of the potentials; the
-  // exact mode halves paths.
-  constexpr bool kHalve = !kLazy || (kMaxOnly && TFGB_MAX_HALVE);
-  // Maxima-only form: float sums and extents in 8-byte records
-  constexpr bool kR8 = kMaxOnly && TFGB_MAX_REC8;
-  Rec8* const rec8 = reinterpret_cast<Rec8*>(sl.rec);
-  // and {vertex, packed list} of a position in one 8-byte record (the second
-  // half of the Rec region), so that bucketing scatters one store per vertex
-  int2* const vtx8 = reinterpret_cast<int2*>(sl.rec) + a.vcap;
-#ifdef TFGB_PHASE_PROFILE
-  long long _pt = clock64();
-#endif
 
   for (;;) {
     if (tid == 0) sItem = atomicAdd(a.counter, 1);
@@ -435,22 +278,8 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
         for (int32_t s2 = 0; s2 < a.n_seg; ++s2)
           if (a.thr_group[s2] == g) tmx = fmaxf(tmx, gm[s2]);
       }
-      int L = 0;
-      if (tmx > 0.0f && isfinite(tmx)) {
-        const float dT = __fdiv_rn(tmx, 100.0f);
-        float T = tmx;
-        while (T >= 0.0f) {
-          if (L >= kMaxSteps) {
-            set_err(a.err, kDevTooManySteps);
-            L = 0;
-            break;
-          }
-          sT[L] = T;
-          sHH[L] = pow_h(T, H);
-          ++L;
-          T = __fsub_rn(T, dT);
-        }
-      }
+      const int L = threshold_table(tmx, sT, a.err);
+      for (int i = 0; i < L; ++i) sHH[i] = pow_h(sT[i], H);
       sL = L;
       if (a.n_steps_out) *a.n_steps_out = L;
     }
@@ -458,7 +287,6 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
     if (use_bm)
       for (int32_t w = tid; w < (Vs + 31) / 32; w += nth) sAct[w] = 0u;
     __syncthreads();
-    TFGB_PHASE_MARK(0);
     const int L = sL;
     const float scale = isfinite(mx) ? __fdiv_rn(mx, 100.0f) : 0.0f;
 
@@ -493,8 +321,6 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
       }
       sStart[L] = s;
       sNDead = 0;
-      sNRoots = 0;
-      sNext = 0;
       sGrab = 0;
       sGrabS = 0;
     }
@@ -514,47 +340,17 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
         const int32_t p = sStart[lv] + base + __popc(peers & ((1u << lane) - 1u));
         key = (static_cast<uint32_t>(lv) << kPosBits) | static_cast<uint32_t>(p);
         if (use_bm && lv == 0) atomicOr(&sAct[v >> 5], 1u << (v & 31));
-        if constexpr (!kR8) sl.order[p] = v;
-        // maxima-only form: parents and records are set one step ahead, for
-        // a step's contiguous positions at once (below and in (A'))
-        if constexpr (!kR8) sl.parent[p] = p;
-        if constexpr (kLazy) {
-          if constexpr (!kR8) sl.rec[p] = Rec{0.0, 1, 0};
-          // the vertex's list (start relative to the segment's, degree) by
-          // position, so the union phase reads it without a dependent load;
-          // -1: out of the packed range, read the offsets
-          const int64_t e0 = a.offsets[v0 + v], deg = a.offsets[v0 + v + 1] - e0, rel = e0 - seg_e0;
-          const int32_t packed =
-              (deg <= 63 && rel >= 0 && rel < (int64_t(1) << 25)) ? static_cast<int32_t>((rel << 6) | deg) : -1;
-          if constexpr (kR8) vtx8[p] = make_int2(v, packed);
-          else reinterpret_cast<int32_t*>(sl.acc)[p] = packed;
-        } else {
-          sl.size[p] = 1;
-          sl.acc[p] = (a.out_mode == 2 && omap) ? omap[v] : 0.0f;
-        }
+        sl.order[p] = v;
+        sl.parent[p] = p;
+        sl.size[p] = 1;
+        sl.acc[p] = (a.out_mode == 2 && omap) ? omap[v] : 0.0f;
       }
       sl.key[v] = key;
     }
-    if constexpr (kR8) {
-      if (L > 0)  // the first step's positions (sStart was set before the last barrier)
-        for (int32_t q = sStart[0] + tid; q < sStart[1]; q += nth) {
-          sl.parent[q] = q;
-          rec8[q] = Rec8{0.0f, 1};
-        }
-    }
     __syncthreads();
-    TFGB_PHASE_MARK(1);
 
     // ---- 3. threshold steps
-    int32_t* cur_roots = sl.roots_a;
-    int32_t* nxt_roots = sl.roots_b;
     for (int i = 0; i < L; ++i) {
-#ifdef TFGB_PHASE_PROFILE
-      const long long _ps = clock64();
-#define TFGB_STEP_DONE() do { if (threadIdx.x == 0) atomicAdd(&g_step_cycles[i], (unsigned long long)(clock64() - _ps)); } while (0)
-#else
-#define TFGB_STEP_DONE() do { } while (0)
-#endif
       const int32_t s0 = sStart[i], s1 = sStart[i + 1];
       // (U) union newly active vertices with already-active neighbours.  A
       // vertex's list is read kUBatch entries at a time with all their key
@@ -588,12 +384,12 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
 #pragma unroll
           for (int k = 0; k < kUBatch; ++k) {
             if (par[k] != cur[k]) {
-              if (kHalve && gp[k] != par[k]) st_state(sl.parent + cur[k], gp[k]);  // halve the path
+              if (gp[k] != par[k]) st_state(sl.parent + cur[k], gp[k]);  // halve the path
               cur[k] = gp[k];
             }
           }
           if (pr != rr) {
-            if (kHalve && gr != pr) st_state(sl.parent + rr, gr);
+            if (gr != pr) st_state(sl.parent + rr, gr);
             rr = gr;
           }
         }
@@ -620,7 +416,7 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
           if (old[m] == lk[m]) {
             if (lk[m] < s0) sl.dead[atomicAdd(&sNDead, 1)] = lk[m];  // new roots: found by (S) in [s0, s1)
           } else {
-            tgt = unite<kHalve>(sl.parent, tgt, lk[m], sl.dead, &sNDead, s0, a.err);
+            tgt = unite(sl.parent, tgt, lk[m], sl.dead, &sNDead, s0, a.err);
           }
         }
         return tgt;
@@ -628,24 +424,8 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
       // each thread takes the next unprocessed vertex of the step from a
       // shared cursor, so threads with short walks do not wait for slow ones
       for (int32_t p = atomicAdd(&sGrab, 1); p < s1; p = atomicAdd(&sGrab, 1)) {
-        int32_t v = -1;  // the vertex: read when needed
-        int64_t e0, e1;
-        int32_t pk = -1;
-        if constexpr (kR8) {
-          const int2 r = vtx8[p];
-          v = r.x;
-          pk = r.y;
-        } else if constexpr (kLazy) {
-          pk = reinterpret_cast<const int32_t*>(sl.acc)[p];
-        }
-        if (pk >= 0) {
-          e0 = seg_e0 + (pk >> 6);
-          e1 = e0 + (pk & 63);
-        } else {
-          if (v < 0) v = sl.order[p];
-          e0 = a.offsets[v0 + v];
-          e1 = a.offsets[v0 + v + 1];
-        }
+        const int32_t v = sl.order[p];
+        int64_t e0 = a.offsets[v0 + v], e1 = a.offsets[v0 + v + 1];
         if constexpr (kChecked) {
           if (e0 < 0 || e1 > a.n_entries || e1 < e0) {
             set_err(a.err, kDevBadIndex);
@@ -658,7 +438,6 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
           int32_t an[kUBatch];
 #pragma unroll
           for (int k = 0; k < kUBatch; ++k) raw[k] = (eb + k < e1) ? a.indices[eb + k] : kIndexMask;
-          TFGB_COUNT(5, (e1 - eb < kUBatch) ? (e1 - eb) : kUBatch);
 #pragma unroll
           for (int k = 0; k < kUBatch; ++k) {
             const int64_t ag = static_cast<int64_t>(raw[k] & kIndexMask) - v0;
@@ -685,7 +464,6 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
             if (la == i && (kChecked || (raw[k] & kOneWay))) {
               // one-directional entry: effective only if the neighbour was
               // inserted first (larger value; ties by smaller index)
-              if (v < 0) v = sl.order[p];  // (set above in the maxima-only form)
               const float xa = sign * x[an[k]], xv = sign * x[v];
               if (!(xa > xv || (xa == xv && an[k] < v))) continue;
             }
@@ -704,258 +482,53 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
         // the next step's vertices become active (read after two more barriers)
         const int32_t s2 = sStart[i + 2];
         for (int32_t q = s1 + tid; q < s2; q += nth) {
-          const int32_t vq = kR8 ? vtx8[q].x : sl.order[q];
+          const int32_t vq = sl.order[q];
           atomicOr(&sAct[vq >> 5], 1u << (vq & 31));
         }
       }
-      TFGB_PHASE_MARK(2);
       // (S) linked roots hand their extent to their final root: the listed
       // older roots and the positions of this step that are no longer roots.
-      // Each thread takes kSLanes of them per round and walks them in
-      // lockstep from their parents; parent[d] is rewritten only when the
-      // final root is not already its parent.
+      // parent[d] is rewritten only when the final root is not already its
+      // parent.
       const int32_t nd = sNDead;
       const int32_t nsp = nd + (s1 - s0);
-      for (int32_t q0 = atomicAdd(&sGrabS, kSLanes); q0 < nsp; q0 = atomicAdd(&sGrabS, kSLanes)) {
-        int32_t d[kSLanes], c[kSLanes], pd[kSLanes];
-#pragma unroll
-        for (int k = 0; k < kSLanes; ++k) {
-          const int32_t q = q0 + k;
-          d[k] = (q < nd) ? sl.dead[q] : (q < nsp ? s0 + (q - nd) : -1);
-        }
-#pragma unroll
-        for (int k = 0; k < kSLanes; ++k) {
-          pd[k] = (d[k] >= 0) ? ld_state(sl.parent + d[k]) : -1;
-          if (pd[k] == d[k]) d[k] = -1;  // still a root
-          c[k] = (d[k] >= 0) ? pd[k] : -1;
-        }
-        for (int it = 0;; ++it) {
-          if (it >= kWalkLimit) {
-            set_err(a.err, kDevLoopLimit);
-            break;
-          }
-          int32_t par[kSLanes];
-#pragma unroll
-          for (int k = 0; k < kSLanes; ++k) par[k] = (c[k] >= 0) ? ld_state(sl.parent + c[k]) : c[k];
-          bool walking = false;
-#pragma unroll
-          for (int k = 0; k < kSLanes; ++k) walking |= (par[k] != c[k]);
-          if (!walking) break;
-          int32_t gp[kSLanes];
-#pragma unroll
-          for (int k = 0; k < kSLanes; ++k) gp[k] = (par[k] != c[k]) ? ld_state(sl.parent + par[k]) : par[k];
-#pragma unroll
-          for (int k = 0; k < kSLanes; ++k) {
-            if (par[k] != c[k]) {
-              if (kHalve && gp[k] != par[k]) st_state(sl.parent + c[k], gp[k]);  // halve the path
-              c[k] = gp[k];
-            }
-          }
-        }
-        if constexpr (kR8) {
-#pragma unroll
-          for (int k = 0; k < kSLanes; ++k) {
-            if (d[k] < 0) continue;
-            // d is no longer a root: no other thread writes its record in this
-            // phase.  Atomics on the final root: extent, and the largest sum
-            // (sums are >= 0, so their bit patterns order as the values do).
-            // A position of this step still holds its bucketing record {0, 1}:
-            // records change only on final roots, and sums only from (A') on.
-            const bool fresh = q0 + k >= nd;
-            const Rec8 rd = fresh ? Rec8{0.0f, 1} : rec8[d[k]];
-            atomicAdd(&rec8[c[k]].size, rd.size);
-            if (c[k] != pd[k]) st_state(sl.parent + d[k], c[k]);
-            if (rd.w > 0.0f) atomicMax(reinterpret_cast<unsigned int*>(&rec8[c[k]].w), __float_as_uint(rd.w));
-          }
-          continue;
-        }
-        int32_t sz[kSLanes];
-        double wd[kSLanes], wr[kSLanes];
-#pragma unroll
-        for (int k = 0; k < kSLanes; ++k) {
-          if (d[k] < 0) continue;
-          if constexpr (kLazy) {
-            const Rec rd = sl.rec[d[k]];
-            sz[k] = rd.size;
-            wd[k] = rd.w;
-            if constexpr (!kMaxOnly) wr[k] = sl.rec[c[k]].w;
-          } else {
-            sz[k] = ld_state(sl.size + d[k]);
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < kSLanes; ++k) {
-          if (d[k] < 0) continue;
-          if constexpr (kLazy) atomicAdd(&sl.rec[c[k]].size, sz[k]);
-          else atomicAdd(sl.size + c[k], sz[k]);
-          if (c[k] != pd[k]) st_state(sl.parent + d[k], c[k]);
-          if constexpr (kMaxOnly) {
-            // sums are >= 0, so their bit patterns order as the values do
-            atomicMax(reinterpret_cast<unsigned long long*>(&sl.rec[c[k]].w),
-                      static_cast<unsigned long long>(__double_as_longlong(wd[k])));
-          } else if constexpr (kLazy) {
-            sl.rec[d[k]].w = wd[k] - wr[k];
-          }
-        }
-      }
-      if constexpr (kLazy) {
-        if (tid == 0) {
-          sNext = 0;
-          sGrabA = 0;
-        }
+      for (int32_t q = atomicAdd(&sGrabS, 1); q < nsp; q = atomicAdd(&sGrabS, 1)) {
+        const int32_t d = (q < nd) ? sl.dead[q] : s0 + (q - nd);
+        const int32_t pd = ld_state(sl.parent + d);
+        if (pd == d) continue;  // still a root
+        const int32_t c = find_root(sl.parent, pd, a.err);
+        atomicAdd(sl.size + c, ld_state(sl.size + d));
+        if (c != pd) st_state(sl.parent + d, c);
       }
       __syncthreads();
-      TFGB_PHASE_MARK(3);
       if (tid == 0) {
         sNDead = 0;
         sGrabS = 0;  // read again only after two more barriers
       }
-      if constexpr (kLazy) {
-        // (A') every live root adds its component's increment once: the old
-        // live roots that survived this step plus the new vertices that are
-        // roots, compacted into the next list as they are visited
-        const float HHl = sHH[i];
-        const int32_t n_old = sNRoots;
-        const int32_t n_cand = n_old + (s1 - s0);
-        for (int32_t q0 = atomicAdd(&sGrabA, kALanes); q0 < n_cand; q0 = atomicAdd(&sGrabA, kALanes)) {
-          int32_t c[kALanes];
-          bool is_root[kALanes];
-#pragma unroll
-          for (int k = 0; k < kALanes; ++k) {
-            const int32_t q = q0 + k;
-            c[k] = (q >= n_cand) ? -1 : (q < n_old) ? cur_roots[q] : s0 + (q - n_old);
-          }
-          if constexpr (kR8) {
-            // no thread writes a record in this phase but its own root's sum
-#pragma unroll
-            for (int k = 0; k < kALanes; ++k) is_root[k] = (c[k] >= 0) && (ld_state(sl.parent + c[k]) == c[k]);
-#pragma unroll
-            for (int k = 0; k < kALanes; ++k) {
-              if (!is_root[k]) continue;
-              const Rec8 rc = rec8[c[k]];
-              rec8[c[k]].w = __fadd_rn(rc.w, increment(rc.size, E, e_mode, HHl));
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < kALanes; ++k) is_root[k] = (c[k] >= 0) && (ld_state(sl.parent + c[k]) == c[k]);
-            int32_t sz[kALanes];
-            double w[kALanes];
-#pragma unroll
-            for (int k = 0; k < kALanes; ++k) {
-              if (!is_root[k]) continue;
-              const Rec rc = sl.rec[c[k]];
-              sz[k] = rc.size;
-              w[k] = rc.w;
-            }
-#pragma unroll
-            for (int k = 0; k < kALanes; ++k)
-              if (is_root[k]) sl.rec[c[k]].w = w[k] + static_cast<double>(increment(sz[k], E, e_mode, HHl));
-          }
-          const unsigned mask = __activemask();
-          const int lane = tid & 31;
-#pragma unroll
-          for (int k = 0; k < kALanes; ++k) {
-            const unsigned roots = __ballot_sync(mask, is_root[k]);
-            if (roots) {
-              const int leader = __ffs(roots) - 1;
-              int base = 0;
-              if (lane == leader) base = atomicAdd(&sNext, __popc(roots));
-              base = __shfl_sync(mask, base, leader);
-              if (is_root[k]) nxt_roots[base + __popc(roots & ((1u << lane) - 1u))] = c[k];
-            }
-          }
-        }
-        if constexpr (kR8) {
-          // the next step's positions: read first by its union phase, after
-          // this phase's barrier
-          if (i + 1 < L)
-            for (int32_t q = s1 + tid; q < sStart[i + 2]; q += nth) {
-              sl.parent[q] = q;
-              rec8[q] = Rec8{0.0f, 1};
-            }
-        }
-        __syncthreads();
-        if (tid == 0) sNRoots = sNext;
-        int32_t* t_ = cur_roots;
-        cur_roots = nxt_roots;
-        nxt_roots = t_;
-        TFGB_PHASE_MARK(4);
-        TFGB_STEP_DONE();
-        continue;
-      }
-      // (A) per-vertex increment, threshold order.  Each thread takes kALanes
-      // positions per round and issues their loads together (the chain
-      // parent -> root -> extent is latency-bound otherwise).
+      // (A) per-vertex increment, threshold order
       const float HH = sHH[i];
-      for (int32_t base = tid; base < s1; base += kALanes * nth) {
-        int32_t pp[kALanes], rt[kALanes];
-        float ac[kALanes];
-#pragma unroll
-        for (int k = 0; k < kALanes; ++k) {
-          pp[k] = base + k * nth;
-          if (pp[k] < s1) {
-            rt[k] = ld_state(sl.parent + pp[k]);
-            ac[k] = sl.acc[pp[k]];
+      for (int32_t p = tid; p < s1; p += nth) {
+        int32_t r = ld_state(sl.parent + p);
+        const float acc = sl.acc[p];
+        if (r != p) {
+          const int32_t up = ld_state(sl.parent + r);
+          if (up != r) {
+            r = find_root(sl.parent, up, a.err);
+            st_state(sl.parent + p, r);
           }
         }
-        int32_t up[kALanes];
-#pragma unroll
-        for (int k = 0; k < kALanes; ++k)
-          up[k] = (pp[k] < s1 && rt[k] != pp[k]) ? ld_state(sl.parent + rt[k]) : -1;
-#pragma unroll
-        for (int k = 0; k < kALanes; ++k) {
-          if (up[k] >= 0 && up[k] != rt[k]) {
-            rt[k] = find_root(sl.parent, up[k], a.err);
-            st_state(sl.parent + pp[k], rt[k]);
-          }
-        }
-        int32_t ext[kALanes];
-#pragma unroll
-        for (int k = 0; k < kALanes; ++k)
-          if (pp[k] < s1) ext[k] = ld_state(sl.size + rt[k]);
-#pragma unroll
-        for (int k = 0; k < kALanes; ++k) {
-          if (pp[k] < s1) {
-            sl.acc[pp[k]] = __fadd_rn(ac[k], increment(ext[k], E, e_mode, HH));
-            if (a.labels && i < a.label_cap) {
-              const int32_t v = sl.order[pp[k]];
-              a.labels[(int64_t)i * Vs + v] = sl.order[rt[k]];
-              a.extents[(int64_t)i * Vs + v] = ext[k];
-            }
-          }
+        const int32_t ext = ld_state(sl.size + r);
+        sl.acc[p] = __fadd_rn(acc, increment(ext, E, e_mode, HH));
+        if (a.labels && i < a.label_cap) {
+          const int32_t v = sl.order[p];
+          a.labels[(int64_t)i * Vs + v] = sl.order[r];
+          a.extents[(int64_t)i * Vs + v] = ext;
         }
       }
       __syncthreads();
-      TFGB_PHASE_MARK(4);
     }
 
     // ---- 4. scale, reduce, write
-    if constexpr (kMaxOnly) {
-      float best = (n_act < Vs) ? __fmul_rn(0.0f, scale) : -INFINITY;
-      const int32_t nr = sNRoots;
-      for (int32_t q = tid; q < nr; q += nth)
-        best = fmaxf(best, __fmul_rn(kR8 ? rec8[cur_roots[q]].w : __double2float_rn(sl.rec[cur_roots[q]].w), scale));
-      best = block_max(best, sRed);
-      if (tid == 0 && a.out_max) a.out_max[item] = (best == -INFINITY) ? 0.0f : best;
-      __syncthreads();
-      TFGB_PHASE_MARK(5);
-      continue;
-    }
-    if constexpr (kLazy) {
-      // resolve every active vertex: sum of potentials along its parent chain
-      for (int32_t p = tid; p < n_act; p += nth) {
-        double sum = sl.rec[p].w;
-        int32_t c = p, l = sl.parent[p];
-        for (int it = 0; l != c && it < kWalkLimit; ++it) {
-          c = l;
-          sum += sl.rec[c].w;
-          l = sl.parent[c];
-        }
-        if (a.out_mode == 2 && omap) sum += static_cast<double>(omap[sl.order[p]]);
-        sl.acc[p] = __double2float_rn(sum);
-      }
-      __syncthreads();
-    }
     float best = (n_act < Vs) ? __fmul_rn(0.0f, scale) : -INFINITY;
     if (a.out_mode == 1 && omap) {
       for (int32_t v = tid; v < Vs; v += nth) {
@@ -978,7 +551,6 @@ __global__ void __launch_bounds__(kSweepThreads, kMinBlocks) tfce_sweep_kernel(S
     best = block_max(best, sRed);
     if (tid == 0 && a.out_max) a.out_max[item] = (best == -INFINITY) ? 0.0f : best;
     __syncthreads();
-    TFGB_PHASE_MARK(5);
   }
 }
 
@@ -1049,7 +621,7 @@ struct tfce_adjset {
   int32_t run_cap = 0;
   int32_t accumulation = 0;  // 0: reference arithmetic, 1: per-component
   bool no_max_only = false;  // accumulation 2: the potential form for maxima-only launches too
-  int32_t ctas_per_sm = TFGB_SWEEP_MINBLOCKS;  // sweep CTA shape of the per-component launches (3 or 2)
+  int32_t sweep_shape = 3;   // 3: more sweeps resident, 2: fewer, with more shared state each
   int32_t* d_group = nullptr;  // threshold group of every segment, or NULL
   float* d_segmax = nullptr;   // segment maxima of the last grouped launch
   int64_t segmax_cap = 0;
@@ -1064,6 +636,7 @@ struct tfce_adjset {
   // the next) and a launch does not end on a few long sweeps.  NULL when all
   // segments have the same size.
   int32_t* d_segrank = nullptr;
+  tfgb::BasinPlan* basin = nullptr;  // NULL: a graph that form does not take
   std::mutex mu;
 };
 
@@ -1086,6 +659,7 @@ int release(tfce_adjset* h) {
   cudaFree(h->d_group);
   cudaFree(h->d_segmax);
   cudaFree(h->d_segrank);
+  tfgb::basin_plan_destroy(h->basin);
   for (void* p : h->retired) cudaFree(p);
   h->retired.clear();
   cudaSetDevice(dev);
@@ -1096,12 +670,8 @@ int resident_slots(tfce_adjset* h) {
   if (h->max_slots) return TFCE_OK;
   int sms = 0, per_sm = 0;
   TFGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-  if (h->ctas_per_sm == 2)
-    TFGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tfgb::tfce_sweep_kernel<false, true, true, 2>,
-                                                            tfgb::kSweepThreads, tfgb::bitmap_bytes(h->vmax_seg)));
-  else
-    TFGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tfgb::tfce_sweep_kernel<false, false>,
-                                                            tfgb::kSweepThreads, tfgb::bitmap_bytes(h->vmax_seg)));
+  TFGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tfgb::tfce_sweep_kernel<false>, tfgb::kSweepThreads,
+                                                          tfgb::bitmap_bytes(h->vmax_seg)));
   h->max_slots = std::max(1, sms * std::max(1, per_sm));
   // tuning knob: fewer CTAs in flight (smaller L2 working set)
   if (const char* env = std::getenv("TFCE_SWEEP_MAX_CTAS")) {
@@ -1111,13 +681,11 @@ int resident_slots(tfce_adjset* h) {
   return TFCE_OK;
 }
 
-// One slot layout serves both accumulation modes (the per-component layout
-// is the larger), so switching modes never replaces the workspace; a launch
-// with more items than the workspace has slots replaces it by one at least
-// twice as large (capped at the resident-slot count), retiring the old one.
-int ensure_workspace(tfce_adjset* h, int32_t slots, bool lazy) {
-  (void)lazy;
-  const int64_t per = std::max(tfgb::slot_bytes_lazy(h->vmax_seg), tfgb::slot_bytes(h->vmax_seg));
+// A launch with more items than the workspace has slots replaces it by one at
+// least twice as large (capped at the resident-slot count), retiring the old
+// one.
+int ensure_workspace(tfce_adjset* h, int32_t slots) {
+  const int64_t per = tfgb::slot_bytes(h->vmax_seg);
   if (h->d_ws && h->ws_slots >= slots && h->ws_slot >= per) return TFCE_OK;
   const int32_t want = std::max(slots, std::min(h->max_slots, 2 * h->ws_slots));
   char* fresh = nullptr;
@@ -1137,10 +705,32 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
   TFGB_CHECK_ARG(items64 < (1LL << 31), "too many sweep items");
   const int32_t items = static_cast<int32_t>(items64);
   if (items == 0) return TFCE_OK;
+  if (!labels) {
+    tfgb::BasinRequest r{};
+    r.stats = stats;
+    r.map_stride = map_stride;
+    r.n_maps = n_maps;
+    r.signs = signs;
+    r.vdensity = vdensity;
+    r.floor_zero = floor_zero;
+    r.out_max = out_max;
+    r.out_maps = out_maps;
+    r.out_mode = out_mode;
+    r.exact = !lazy;
+    r.potentials = lazy && h->no_max_only;
+    r.dense = h->sweep_shape == 3;
+    r.thr_group = h->d_group;
+    r.d_H = h->d_H;
+    r.d_E = h->d_E;
+    r.d_seg_off = h->d_seg_off;
+    r.seg_rank = h->d_segrank;
+    r.err = h->d_ctrl + 1;
+    if (tfgb::basin_takes(h->basin, r)) return tfgb::basin_sweep(h->basin, r, st);
+  }
   int rs = resident_slots(h);
   if (rs) return rs;
   const int32_t slots = std::min<int32_t>(items, h->max_slots);
-  int rc = ensure_workspace(h, slots, lazy);
+  int rc = ensure_workspace(h, slots);
   if (rc) return rc;
   TFGB_CUDA(cudaMemsetAsync(h->d_ctrl, 0, sizeof(int32_t), st));  // queue counter only
   tfgb::SweepArgs a{};
@@ -1191,14 +781,7 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
     a.thr_group = h->d_group;
     a.seg_max = h->d_segmax;
   }
-  // maxima only, no vertex weights: the per-component form without potentials
-  const bool max_only = lazy && !vdensity && !out_maps && !labels && out_max && !h->no_max_only;
-  const bool two = (h->ctas_per_sm == 2);
-  if (max_only && two) tfgb::tfce_sweep_kernel<false, true, true, 2><<<slots, tfgb::kSweepThreads, bm, st>>>(a);
-  else if (max_only) tfgb::tfce_sweep_kernel<false, true, true><<<slots, tfgb::kSweepThreads, bm, st>>>(a);
-  else if (lazy && two) tfgb::tfce_sweep_kernel<false, true, false, 2><<<slots, tfgb::kSweepThreads, bm, st>>>(a);
-  else if (lazy) tfgb::tfce_sweep_kernel<false, true><<<slots, tfgb::kSweepThreads, bm, st>>>(a);
-  else tfgb::tfce_sweep_kernel<false, false><<<slots, tfgb::kSweepThreads, bm, st>>>(a);
+  tfgb::tfce_sweep_kernel<false><<<slots, tfgb::kSweepThreads, bm, st>>>(a);
   TFGB_CUDA(cudaGetLastError());
   return TFCE_OK;
 }
@@ -1286,17 +869,24 @@ int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n
     }
     off[v + 1] = static_cast<int64_t>(idx.size());
   }
-  for (int32_t v = 0; v < V; ++v) std::sort(idx.begin() + off[v], idx.begin() + off[v + 1]);
+  const int64_t blocks = (V + 4095) / 4096;
+  tfgb::parallel_for(blocks, V, [&](int64_t k) {
+    for (int64_t v = k * 4096; v < std::min<int64_t>(V, (k + 1) * 4096); ++v)
+      if (!std::is_sorted(idx.begin() + off[v], idx.begin() + off[v + 1]))
+        std::sort(idx.begin() + off[v], idx.begin() + off[v + 1]);
+  });
   std::vector<uint32_t> packed(idx.size());
-  bool symmetric = true;
-  for (int32_t v = 0; v < V; ++v) {
-    for (int64_t e = off[v]; e < off[v + 1]; ++e) {
-      const int32_t b = idx[e];
-      const bool rev = std::binary_search(idx.begin() + off[b], idx.begin() + off[b + 1], v);
-      packed[e] = static_cast<uint32_t>(b) | (rev ? 0u : tfgb::kOneWay);
-      symmetric = symmetric && rev;
-    }
-  }
+  std::atomic<bool> two_way{true};
+  tfgb::parallel_for(blocks, V, [&](int64_t k) {
+    for (int64_t v = k * 4096; v < std::min<int64_t>(V, (k + 1) * 4096); ++v)
+      for (int64_t e = off[v]; e < off[v + 1]; ++e) {
+        const int32_t b = idx[e];
+        const bool rev = std::binary_search(idx.begin() + off[b], idx.begin() + off[b + 1], static_cast<int32_t>(v));
+        packed[e] = static_cast<uint32_t>(b) | (rev ? 0u : tfgb::kOneWay);
+        if (!rev) two_way = false;
+      }
+  });
+  const bool symmetric = two_way;
 
   tfce_adjset* h = new tfce_adjset();
   cudaGetDevice(&h->device);
@@ -1346,6 +936,9 @@ int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n
     TFGB_CUDA_H(cudaMemcpy(h->d_segrank, rank.data(), sizeof(int32_t) * n_seg, cudaMemcpyHostToDevice));
   }
 #undef TFGB_CUDA_H
+  int rc = tfgb::basin_plan_create(off, packed, seg, &h->basin);
+  if (!rc && h->basin) rc = tfgb::basin_plan_set_exponents(h->basin, E);
+  if (rc) return fail(rc);
   *out = h;
   return TFCE_OK;
 }
@@ -1366,7 +959,7 @@ int tfce_adjset_set_params(tfce_adjset* h, const float* H, const float* E) {
   h->E.assign(E, E + h->n_seg);
   TFGB_CUDA(cudaMemcpy(h->d_H, H, sizeof(float) * h->n_seg, cudaMemcpyHostToDevice));
   TFGB_CUDA(cudaMemcpy(h->d_E, E, sizeof(float) * h->n_seg, cudaMemcpyHostToDevice));
-  return TFCE_OK;
+  return h->basin ? tfgb::basin_plan_set_exponents(h->basin, E) : TFCE_OK;
 }
 
 int tfce_adjset_is_symmetric(const tfce_adjset* h) { return (h && h->symmetric) ? 1 : 0; }
@@ -1376,10 +969,7 @@ int tfce_adjset_set_sweep_shape(tfce_adjset* h, int32_t ctas_per_sm) {
   TFGB_CHECK_ARG(h != nullptr, "handle is NULL");
   TFGB_CHECK_ARG(ctas_per_sm == 2 || ctas_per_sm == 3, "ctas_per_sm must be 2 or 3");
   std::lock_guard<std::mutex> lk(h->mu);
-  if (h->ctas_per_sm != ctas_per_sm) {
-    h->ctas_per_sm = ctas_per_sm;
-    h->max_slots = 0;  // recomputed for the new shape at the next launch
-  }
+  h->sweep_shape = ctas_per_sm;
   return TFCE_OK;
 }
 
@@ -1501,32 +1091,15 @@ int tfce_sweep_batch(tfce_adjset* h, const float* stats, int64_t map_stride, int
   return rc;
 }
 
-#ifdef TFGB_PHASE_PROFILE
-// Debug-only export: per-phase cycle sums since the last call (then cleared).
-int tfce_debug_step_cycles(unsigned long long* out128) {
-  TFGB_CUDA(cudaDeviceSynchronize());
-  TFGB_CUDA(cudaMemcpyFromSymbol(out128, tfgb::g_step_cycles, 128 * sizeof(unsigned long long)));
-  unsigned long long z[128] = {0};
-  TFGB_CUDA(cudaMemcpyToSymbol(tfgb::g_step_cycles, z, sizeof(z)));
-  return TFCE_OK;
-}
 
-int tfce_debug_phase_cycles(unsigned long long* out16) {
-  TFGB_CUDA(cudaDeviceSynchronize());
-  TFGB_CUDA(cudaMemcpyFromSymbol(out16, tfgb::g_phase_cycles, 8 * sizeof(unsigned long long)));
-  TFGB_CUDA(cudaMemcpyFromSymbol(out16 + 8, tfgb::g_dbg_counts, 8 * sizeof(unsigned long long)));
-  unsigned long long z[8] = {0};
-  TFGB_CUDA(cudaMemcpyToSymbol(tfgb::g_phase_cycles, z, sizeof(z)));
-  TFGB_CUDA(cudaMemcpyToSymbol(tfgb::g_dbg_counts, z, sizeof(z)));
-  return TFCE_OK;
-}
-#endif
-
-// Error word of the last batched sweep on this handle (synchronises `stream`).
 int tfce_sweep_resident_slots(tfce_adjset* h, int32_t* slots) {
   tfgb::clear_error();
   TFGB_CHECK_ARG(h != nullptr && slots != nullptr, "NULL pointer");
   std::lock_guard<std::mutex> lk(h->mu);
+  if (h->basin) {
+    *slots = tfgb::basin_resident_items(h->basin, h->sweep_shape == 3);
+    return TFCE_OK;
+  }
   const int rc = resident_slots(h);
   if (rc) return rc;
   *slots = h->max_slots;
@@ -1599,7 +1172,7 @@ int noalloc_setup(int dev, NoAllocDevice* out) {
   if (!g_noalloc_slots[dev]) {
     int sms = 0, per_sm = 0;
     TFGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    TFGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tfce_sweep_kernel<true, false>,
+    TFGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tfce_sweep_kernel<true>,
                                                             kSweepThreads, 0));
     g_noalloc_slots[dev] = std::max(1, sms * std::max(1, per_sm));
   }
@@ -1674,7 +1247,7 @@ extern "C" int tfce_sweep_batch_noalloc(const int64_t* offsets, const int32_t* i
   a.n_items = items;
   a.n_vertices = n_vertices;
   a.n_entries = n_entries;
-  tfgb::tfce_sweep_kernel<true, false><<<slots, tfgb::kSweepThreads, 0, st>>>(a);
+  tfgb::tfce_sweep_kernel<true><<<slots, tfgb::kSweepThreads, 0, st>>>(a);
   TFGB_CUDA(cudaGetLastError());
   int32_t hctrl[2] = {0, 0};
   TFGB_CUDA(cudaMemcpyAsync(hctrl, ctrl, sizeof(hctrl), cudaMemcpyDeviceToHost, st));
