@@ -27,7 +27,7 @@
 // 512 maps x 2 hemispheres x +/- of the L7 icosphere, smooth: 21.9 -> 4.7 ms
 // (tile 2.3, sweep 1.5, order 0.5, cross 0.2, max 0.1); unsmoothed noise, 128
 // maps: 10.1 -> 2.9 ms; 48 maps of 242k voxels, 26 neighbours, E = 0.5: 9.8 ->
-// 1.4 ms; one map: 4.64 -> 0.45 ms.
+// 1.3 ms; one map: 4.64 -> 0.40 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -145,8 +145,9 @@ struct BasinArgs {
   int32_t* ord;         // ordered: vertex
   double* base;         // ordered: potential of the component before the vertex joined
   uint32_t* vnode;      // ordered: first node of the vertex
-  Node* nodes;
+  Node* nodes;          // [items][node_cap]: step * basins + basin
   uint32_t* part_max;   // [items] encoded maximum
+  uint32_t* n_steps;    // [items]
   int64_t pos_per_map, pair_per_map, cpair_per_map, opair_per_map;
   int64_t node_cap;
   char* state;
@@ -794,9 +795,9 @@ struct BasinState {
   static constexpr bool kShared = kKind != kAllGlobal;
   using W = typename std::conditional<kMode == kPotential, double, uint32_t>::type;
   using Idx = typename std::conditional<kShared, uint16_t, uint32_t>::type;
-  StateArray<kShared, W> w;  // maxima: largest float sum (bits); potentials: sum, or offset to the parent; nodes: last node
+  StateArray<kShared, W> w;  // maxima: largest float sum (bits); potentials: sum, or offset to the parent
   StateArray<kShared, uint32_t> word;
-  StateArray<kKind == kAllShared, Idx> list0;  // live basins; the other list holds the step's changes meanwhile
+  StateArray<kKind == kAllShared, Idx> list0;  // live basins; they are packed from one list to the other
   StateArray<kKind == kAllShared, Idx> list1;
   __device__ BasinState(char* smem, char* global, uint32_t n) {
     if constexpr (kShared) w.base = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
@@ -821,6 +822,21 @@ __device__ inline void hop(const Words& word, uint32_t& x, uint32_t& w) {
   w = up;
 }
 
+// The same for two walks of which at least one goes on, their loads together.
+template <bool kHalve, typename Words>
+__device__ inline void hop_two(const Words& word, uint32_t& x, uint32_t& wx, uint32_t& y, uint32_t& wy) {
+  const bool up_x = !(wx & kRoot), up_y = !(wy & kRoot);
+  uint32_t ux = wx, uy = wy;
+  if (up_x) ux = word.ld(wx);
+  if (up_y) uy = word.ld(wy);
+  if (kHalve && up_x && !(ux & kRoot)) word.st(x, ux);
+  if (kHalve && up_y && !(uy & kRoot)) word.st(y, uy);
+  if (up_x) x = wx;
+  if (up_y) y = wy;
+  wx = ux;
+  wy = uy;
+}
+
 // Root of x, and its word.
 template <bool kHalve, typename Words>
 __device__ inline uint32_t find_basin(const Words& word, uint32_t x, uint32_t& w) {
@@ -838,7 +854,7 @@ struct SweepShared {
   float T[kMaxSteps], HH[kMaxSteps];
   int ev[kMaxSteps + 1], pair[kMaxSteps + 1];  // first entries of the steps
   float red[32];
-  int L, item, n_basins, n_change;
+  int L, item, n_basins;
   int n_live[3];  // by packs modulo 3: the list's, the packed one's, and one being cleared
 };
 
@@ -895,9 +911,8 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
     st.word.st(i, kRoot);
     st.w.st(i, 0);
   }
-  if (tid == 0) S.n_change = S.n_live[0] = S.n_live[1] = S.n_live[2] = 0;
+  if (tid == 0) S.n_live[0] = S.n_live[1] = S.n_live[2] = 0;
   __syncthreads();
-  uint32_t n_nodes = 0;  // nodes: ids handed out before this step
   Node* nodes = (kMode == kNodes) ? a.nodes + item * a.node_cap : nullptr;
   // the thread's first entries of a step are loaded a step ahead
   int ev0 = S.ev[0], ev_end = S.ev[1], pr0 = S.pair[0], pr_end = S.pair[1];
@@ -928,89 +943,89 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
       if (pr_end + tid < pr2) next_pair = load_pair(pr_end + tid);
     }
     if (ev_end > ev0) {
-      // (1) join the basins of the step's pairs.  A linked root hands its
-      // extent over, and its sum (maxima) or its place in the list of changes
-      // (potentials).  A warp's walks and links go in rounds, all lanes
-      // together.
-      if (pr_end > pr0) {
-        for (int q0 = pr0 + wbase; q0 < pr_end; q0 += nth) {
-          const int q = q0 + lane;
-          uint32_t x = 0, y = 0;
-          bool open = q < pr_end;
+      // (1) join the basins of the step's pairs, one pair per thread at a time;
+      // a warp's walks and links go in rounds, all lanes together.  A thread
+      // keeps the root that it linked until all pairs are through.  Then roots
+      // stand still, and its extent and its sum go to the one that it ended
+      // under, once per warp for those that share the first lane's (potentials:
+      // it keeps its offset to that one).  Handed over link by link, the many
+      // that a large component takes in waited for one another at its word
+      // (128 voxel items of a 91 x 109 x 91 mask: 532 -> 423 us; 256 items of
+      // L6 surfaces: 283 -> 219 us).
+      for (int q0 = pr0; q0 < pr_end; q0 += nth) {
+        const int q = q0 + tid;
+        uint32_t x = 0, y = 0;
+        bool open = q < pr_end;
+        bool linked = false;
+        uint32_t low = 0, ext = 0;
+        if (q0 + wbase < pr_end) {
+          uint32_t px = kRoot, py = kRoot;
           if (open) {
-            const uint2 r = (q == pr0 + tid) ? my_pair : load_pair(q);
+            const uint2 r = (q0 == pr0) ? my_pair : load_pair(q);
             x = r.x;
             y = r.y;
+            px = st.word.ld(x);
+            py = st.word.ld(y);
           }
-          for (int it = 0; __any_sync(0xffffffffu, open); ++it) {
-            if (it >= kFindLimit) {
-              if (open) set_err(a.err, kDevLoopLimit);
-              break;
+          for (int it = 0; it < kFindLimit; ++it) {
+            // both walks a hop at a time, their loads together
+            while (__any_sync(0xffffffffu, !(px & py & kRoot))) hop_two<kHalve>(st.word, x, px, y, py);
+            open = open && x != y;
+            if (open) {
+              const uint32_t ax = px >> 24, ay = py >> 24;
+              const bool x_up = ax != ay ? ax > ay : x < y;
+              const uint32_t was = x_up ? py : px;
+              low = x_up ? y : x;
+              if (st.word.cas(low, was, x_up ? x : y) == was) {
+                open = false;
+                linked = true;
+                ext = was & kExtent;
+              }
             }
-            uint32_t px = kRoot, py = kRoot;
+            if (!__any_sync(0xffffffffu, open)) break;
+            px = py = kRoot;
             if (open) {
               px = st.word.ld(x);
               py = st.word.ld(y);
             }
-            while (__any_sync(0xffffffffu, !(px & py & kRoot))) {
-              if (!(px & kRoot)) hop<kHalve>(st.word, x, px);
-              if (!(py & kRoot)) hop<kHalve>(st.word, y, py);
-            }
-            if (open) {
-              if (x == y) {
-                open = false;
-              } else {
-                const uint32_t ax = px >> 24, ay = py >> 24;
-                const bool x_up = ax != ay ? ax > ay : x < y;
-                const uint32_t hi = x_up ? y : x, was = x_up ? py : px;
-                uint32_t t = x_up ? x : y;
-                if (st.word.cas(hi, was, t) == was) {
-                  open = false;
-                  const uint32_t ext = was & kExtent;
-                  if (kMode == kPotential) other.st(atomicAdd(&S.n_change, 1), hi);
-                  if (ext) {  // its vertices count with the root that it is under by now
-                    for (int k = 0; k < kFindLimit; ++k) {
-                      uint32_t wt;
-                      t = find_basin<kHalve>(st.word, t, wt);
-                      if (st.word.cas(t, wt, wt + ext) == wt) break;
-                    }
-                    if constexpr (kMode == kMaxima) {
-                      // handed to a root that is still one afterwards: a root
-                      // that is linked meanwhile reads its own sum after that
-                      const uint32_t sum = st.w.ld(hi);
-                      for (int k = 0; k < kFindLimit; ++k) {
-                        st.w.max_with(t, sum);
-                        __threadfence_block();
-                        if (st.word.ld(t) & kRoot) break;
-                        t = find_basin<kHalve>(st.word, t);
-                      }
-                    }
-                  }
-                }
-              }
-            }
           }
+          if (open) set_err(a.err, kDevLoopLimit);
         }
         __syncthreads();
-      }
-      // (2) potentials: linked roots keep their offset to their final root
-      if constexpr (kMode == kPotential) {
-        const int nc = (pr_end > pr0) ? S.n_change : 0;
-        for (int q = tid; q < nc; q += nth) {
-          const uint32_t d = other.ld(q);
-          const uint32_t r = find_basin<kHalve>(st.word, d);
-          st.w.st(d, st.w.ld(d) - st.w.ld(r));  // roots do not change in this phase
-          st.word.st(d, r);
+        if constexpr (kMode == kPotential) {
+          if (linked) {
+            const uint32_t r = find_basin<kHalve>(st.word, low);
+            if (ext) st.word.add(r, ext);
+            st.w.st(low, st.w.ld(low) - st.w.ld(r));
+            st.word.st(low, r);
+          }
+          __syncthreads();  // vertices climb by these
+        } else {
+          linked = linked && ext;
+          const unsigned m = __ballot_sync(0xffffffffu, linked);
+          if (m) {
+            const uint32_t r = linked ? find_basin<kHalve>(st.word, low) : 0;
+            uint32_t sum = 0;
+            if (kMode == kMaxima && linked) sum = st.w.ld(low);
+            __syncwarp();
+            const int first = __ffs(m) - 1;
+            const uint32_t r0 = __shfl_sync(0xffffffffu, r, first);
+            const bool same = linked && r == r0;
+            const uint32_t all_ext = __reduce_add_sync(0xffffffffu, same ? ext : 0u);
+            const uint32_t all_sum = kMode == kMaxima ? __reduce_max_sync(0xffffffffu, same ? sum : 0u) : 0u;
+            if (lane == first) {
+              ext = all_ext;
+              sum = all_sum;
+            }
+            if (lane == first || (linked && !same)) {
+              st.word.add(r, ext);
+              if constexpr (kMode == kMaxima) st.w.max_with(r, sum);
+            }
+          }
+          if (q0 + nth < pr_end) __syncthreads();
         }
-        if (nc) __syncthreads();
       }
       // the step's vertices join their component
-      auto join = [&](uint32_t r, uint32_t was) {
-        if (!(was & kExtent)) {  // the component's first vertices: it goes live, with its age
-          live.st(atomicAdd(n_live, 1), r);
-          st.word.add(r, static_cast<uint32_t>(kMaxSteps - 1 - i) << 24);
-        }
-      };
       auto count_two = [&](int p, const Two& t) {
         const uint2 two = split(t);
         uint32_t x = two.x, y = two.y;
@@ -1030,10 +1045,11 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
           uint32_t wx = kRoot, wy = kRoot;
           if (on_x) wx = st.word.ld(x);
           if (on_y) wy = st.word.ld(y);
-          while (!(wx & wy & kRoot)) {
-            if (!(wx & kRoot)) hop<kHalve>(st.word, x, wx);
-            if (!(wy & kRoot)) hop<kHalve>(st.word, y, wy);
-          }
+          while (!(wx & wy & kRoot)) hop_two<kHalve>(st.word, x, wx, y, wy);
+        }
+        if constexpr (kMode == kNodes) {
+          if (on_x) a.vnode[eo + p - shift] = i * nb + x;
+          if (on_y) a.vnode[eo + p + 1 - shift] = i * nb + y;
         }
         __syncwarp();
         // those that share the first lane's component are added at once
@@ -1044,9 +1060,24 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
         if (leads) was_0 = st.word.add(r0, __popc(sx) + __popc(sy));
         if (on_x && x != r0) was_x = st.word.add(x, 1u);
         if (on_y && y != r0) was_y = st.word.add(y, 1u);
-        join(r0, was_0);
-        join(x, was_x);
-        join(y, was_y);
+        // a component's first vertices: it goes live, with its age
+        const bool new_0 = !(was_0 & kExtent), new_x = !(was_x & kExtent), new_y = !(was_y & kExtent);
+        if (new_0 || new_x || new_y) {
+          int at = atomicAdd(n_live, int(new_0) + int(new_x) + int(new_y));
+          const uint32_t age = static_cast<uint32_t>(kMaxSteps - 1 - i) << 24;
+          if (new_0) {
+            live.st(at++, r0);
+            st.word.add(r0, age);
+          }
+          if (new_x) {
+            live.st(at++, x);
+            st.word.add(x, age);
+          }
+          if (new_y) {
+            live.st(at, y);
+            st.word.add(y, age);
+          }
+        }
       };
       const int even = ev0 & ~1;
 #pragma unroll
@@ -1057,11 +1088,10 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
       __syncthreads();
     }
     // (3) every live component adds its increment.  Linked ones drop out of
-    // the list when it is packed: every eighth step, or every step where the
-    // position in the list numbers the nodes.
+    // the list when it is packed, every eighth step.
     const float HH = S.HH[i];
     const int n = *n_live;
-    const bool pack = kMode == kNodes || (i & 7) == 7;
+    const bool pack = (i & 7) == 7;
     // (float)(extent^E * HH): one double product, one rounding
     // (fast_tfce.hpp:77); for E == 1 the double product of an integer below
     // 2^24 and a float is exact, so a float product rounds alike
@@ -1072,64 +1102,45 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
     auto grow = [&](uint32_t c, float inc) {
       if constexpr (kMode == kMaxima) st.w.st(c, __float_as_uint(__fadd_rn(__uint_as_float(st.w.ld(c)), inc)));
       if constexpr (kMode == kPotential) st.w.st(c, st.w.ld(c) + static_cast<double>(inc));
+      if constexpr (kMode == kNodes) nodes[(int64_t)i * nb + c] = Node{inc, c};
+    };
+    // nodes: a component that was linked at this step leads on to the one that
+    // it is part of now (before, it led on to itself).  A node's place follows
+    // from its step and basin, so that vertices know theirs as they join (a
+    // pass of its own for them cost a quarter of the sweep: 414 -> 342 us)
+    auto lead_on = [&](uint32_t c) {
+      if constexpr (kMode == kNodes) {
+        if (i > 0) nodes[(int64_t)(i - 1) * nb + c].next = find_basin<kHalve>(st.word, c);
+      }
     };
     if (!pack) {
       for (int q = tid; q < n; q += nth) {
         const uint32_t c = live.ld(q);
         const uint32_t word = st.word.ld(c);
         if (word & kRoot) grow(c, increment(word));
+        else lead_on(c);
       }
     } else {
       for (int q0 = wbase; q0 < n; q0 += nth) {
         const int q = q0 + lane;
         bool root = false;
         uint32_t c = 0;
-        float inc = 0.0f;
         if (q < n) {
           c = live.ld(q);
           const uint32_t word = st.word.ld(c);
           root = word & kRoot;
-          if (root) {
-            inc = increment(word);
-            grow(c, inc);
-          }
+          if (root) grow(c, increment(word));
+          else lead_on(c);
         }
         const unsigned m = __ballot_sync(0xffffffffu, root);
         int at = 0;
         if (lane == 0 && m) at = atomicAdd(n_next, __popc(m));
         at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
-        if (root) {
-          other.st(at, c);
-          if constexpr (kMode == kNodes) {
-            const uint32_t id = n_nodes + at, last = st.w.ld(c);
-            nodes[id] = Node{inc, kNone};
-            if (last) nodes[last - 1].next = id;  // 0: no node yet
-            st.w.st(c, id + 1);
-          }
-        }
+        if (root) other.st(at, c);
       }
     }
-    if (tid == 0) {
-      if (kMode == kPotential) S.n_change = 0;
-      if (pack) *n_spare = 0;  // the list before this one's: read before the last barrier
-    }
+    if (tid == 0 && pack) *n_spare = 0;  // the list before this one's: read before the last barrier
     __syncthreads();
-    if constexpr (kMode == kNodes) {
-      // the last nodes of the linked components lead on to the joined one's,
-      // and the step's vertices start at their component's node
-      for (int q = tid; q < n; q += nth) {
-        const uint32_t c = live.ld(q);
-        const uint32_t last = st.w.ld(c);
-        if (!(st.word.ld(c) & kRoot) && last) nodes[last - 1].next = st.w.ld(find_basin<true>(st.word, c)) - 1;
-      }
-      for (int p = (ev0 & ~1) + 2 * tid; p < ev_end; p += 2 * nth) {
-        const uint2 two = split(load_two(p, ev0, ev_end));
-        if (p >= ev0) a.vnode[eo + p - shift] = st.w.ld(find_basin<true>(st.word, two.x)) - 1;
-        if (p + 1 < ev_end) a.vnode[eo + p + 1 - shift] = st.w.ld(find_basin<true>(st.word, two.y)) - 1;
-      }
-      n_nodes += *n_next;
-      __syncthreads();
-    }
     if (pack) {
       auto l = live;
       live = other;
@@ -1183,7 +1194,10 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
     best = block_max(best, S.red);
     if (tid == 0 && a.out_max) a.out_max[item] = (best == -INFINITY) ? 0.0f : best;
   } else {
-    if (tid == 0 && a.out_max) a.part_max[item] = enc_float(best);
+    if (tid == 0) {
+      a.n_steps[item] = L;
+      a.part_max[item] = enc_float(best);
+    }
   }
 }
 
@@ -1264,17 +1278,19 @@ __global__ void __launch_bounds__(256) basin_walk_kernel(BasinArgs a) {
   const int lo = static_cast<int>(start[0]), hi = static_cast<int>(start[kMaxSteps]);
   const int64_t eo = map * a.n_vertices + a.segs[seg].pos0;
   const Node* nodes = a.nodes + item * a.node_cap;
+  const uint32_t nb = a.n_basins[(map * a.n_seg + seg) * 2 + sgn], L = a.n_steps[item];
   const float scale = __fdiv_rn(seg_maximum(a, map, sgn, seg), 100.0f);
   float* omap = a.out_maps ? a.out_maps + (int64_t)ms * a.n_vertices : nullptr;
   float best = -INFINITY;
   for (int q = lo + blockIdx.x * 256 + threadIdx.x; q < hi; q += gridDim.x * 256) {
     const int64_t v = a.ord[eo + q];
     float acc = (a.out_mode == 2 && omap) ? omap[v] : 0.0f;
-    uint32_t id = a.vnode[eo + q];
-    for (int it = 0; it < kMaxSteps && id != kNone; ++it) {
-      const Node nd = nodes[id];
+    const uint32_t id = a.vnode[eo + q];
+    uint32_t c = id % nb;
+    for (uint32_t i = id / nb; i < L; ++i) {
+      const Node nd = nodes[(int64_t)i * nb + c];
       acc = __fadd_rn(acc, nd.inc);
-      id = nd.next;
+      c = nd.next;
     }
     float val = __fmul_rn(acc, scale);
     if (a.vdensity) val = __fmul_rn(val, a.vdensity[v]);
@@ -1382,7 +1398,7 @@ Layout layout_of(const BasinPlan* p, int64_t M, int signs, int mode, int64_t nod
   if (mode == kNodes) {
     l.vnode = take(M * p->V * 4);
     l.nodes = take(M * signs * p->n_seg * node_cap * 8);
-    l.part = take(M * signs * p->n_seg * 4);
+    l.part = take(2 * M * signs * p->n_seg * 4);
   }
   l.total = o;
   return l;
@@ -1866,6 +1882,7 @@ int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st) {
   at(a.vnode, lay.vnode);
   at(a.nodes, lay.nodes);
   at(a.part_max, lay.part);
+  a.n_steps = a.part_max + per * r.signs * p->n_seg;
   a.pos_per_map = p->n_pos;
   a.pair_per_map = p->n_pair;
   a.cpair_per_map = p->n_cpair;
