@@ -81,9 +81,10 @@ int tfce_adjset_is_symmetric(const tfce_adjset* h);
 /* Shape of the batched sweeps: 3 for CTAs of 256 threads, four per SM with
  * room for 4,096 basins (local maxima of the map) each in shared memory (the
  * default: smooth maps, up to 164k vertices), or 2 for CTAs of 512 threads, two
- * per SM with room for 8,192; maps with more basins go to a second launch with
- * one CTA per SM.  The autotuner picks it per study together with the batch
- * size. */
+ * per SM with room for 9,300; items with more basins than their shape holds go
+ * to launches with fewer, larger CTAs per SM beside it.  Batches of up to two
+ * items per SM take the second shape or a larger one by themselves.  The
+ * autotuner picks it per study together with the batch size. */
 int tfce_adjset_set_sweep_shape(tfce_adjset* h, int32_t ctas_per_sm);
 /* Threshold groups of tfce_sweep_batch: group [n_seg] (host; ids in
  * [0, n_seg)), or NULL to give every segment its own table again.  Segments

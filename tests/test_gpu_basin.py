@@ -117,3 +117,35 @@ def test_many_segments_of_uneven_sizes_and_launch_shapes():
             for k, sgn in enumerate((1.0, -1.0)):
                 np.testing.assert_array_equal(mx[:, k, s], oracle.tfce_max_batch(o, i, part, 2.0, 1.0, sign=sgn,
                                                                                  hh_exact=True))
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_launches_of_three_sizes_at_once(weighted):
+    """More than two items per SM, of ~300, ~8,000 and ~23,000 basins a sign:
+    three launches that do not wait for one another, and more maps behind them
+    on the stream."""
+    rng = np.random.default_rng(11)
+    sizes = [1000, 24_000, 70_001]
+    parts = [_graph("ring", n, rng) for n in sizes]
+    off, idx, seg = A.concat_csr(parts)
+    V = int(seg[-1])
+    few = np.ascontiguousarray(rng.standard_normal((3, V)).astype(np.float32))
+    pick = rng.integers(0, 3, 60)
+    maps = np.ascontiguousarray(few[pick])
+    vd = (0.5 + rng.random(V)).astype(np.float32) if weighted else None
+    adj = A.AdjacencySet((off, idx), 2.0, 1.0, seg)
+    runs = [_sweep(adj, maps, 2, "component", vd)[0] for _ in range(2)]
+    for s, (o, i) in enumerate(parts):
+        part = few[:, seg[s]:seg[s + 1]]
+        for k, sgn in enumerate((1.0, -1.0)):
+            want = np.empty(3, np.float32)
+            for m in range(3):
+                img = (sgn * part[m]).astype(np.float32)
+                raw = oracle.tfce(o, i, img, 2.0, 1.0, hh_exact=True)
+                val = (raw * np.float32(img.max() / np.float32(100.0))).astype(np.float32)
+                want[m] = val.max() if vd is None else (val * vd[seg[s]:seg[s + 1]]).astype(np.float32).max()
+            for mx in runs:
+                if weighted:
+                    np.testing.assert_allclose(mx[:, k, s], want[pick], rtol=1e-5)
+                else:
+                    np.testing.assert_array_equal(mx[:, k, s], want[pick])

@@ -349,7 +349,7 @@ class AdjacencySet:
 
     def set_sweep_shape(self, ctas_per_sm: int):
         """Shape of the batched sweeps: 3 (more sweeps resident, each with room
-        for 4,096 local maxima of its map in shared memory) or 2 (fewer, 8,192)."""
+        for 4,096 local maxima of its map in shared memory) or 2 (fewer, 9,300)."""
         _lib.check(self._lib.tfce_adjset_set_sweep_shape(self._h, int(ctas_per_sm)))
         self.ctas_per_sm = int(ctas_per_sm)
 

@@ -5,7 +5,7 @@ Each candidate (P, CTAs per SM) is timed on the device (CUDA events, after a
 warm-up launch) for the GLM + sweep of one batch; the one with the highest
 permutations per second wins.  The sweep runs in shape 3 (four CTAs of 256
 threads per SM, room for 4,096 local maxima of a map each) or 2 (two of 512
-threads, 8,192); which is faster depends on the maps' smoothness and the
+threads, 9,300); which is faster depends on the maps' smoothness and the
 segments' sizes.  The GLM
 runs as the quadratic form (t from the cross products of the centred
 designs with the data, where it applies) or with the residual epilogue, whose

@@ -55,6 +55,8 @@ constexpr int kCrossPer = 4;
 constexpr int kCrossChunk = kCrossThreads * kCrossPer;
 constexpr int kMaxSweepThreads = 1024;
 constexpr int kTileEntries = 120000;   // list entries per tile: pairs are counted in 16 bits
+constexpr int kSmBytes = 226 * 1024;   // shared memory of an SM's sweeps together
+constexpr int kSweepBytes = 3328;      // of a sweep besides its state
 constexpr int kFindLimit = 1 << 26;
 constexpr int kAhead = 4;              // pairs of events that a thread of the sweep loads a step ahead
 constexpr uint32_t kNone = 0xffffffffu;
@@ -123,7 +125,7 @@ struct BasinArgs {
   int32_t n_tiles, n_chunks, n_bnd;
   // workspace
   uint32_t* seg_max;    // [maps][2][n_seg] bits of max(0, max)
-  int32_t* counter;     // items taken by the first sweep launch, by the second, and queued for it
+  int32_t* counter;     // items taken and, of the queued ones, there are: by class (2 * class, 2 * class + 1)
   uint32_t* ev;         // by vertex of the tile: basin | bucket << 12, or kNone
   uint32_t* pairs;      // pairs of basins of a tile: bucket << 24, 12 bits each
   uint2* cpairs;        // crossing pairs: tile << 16 | 4 bits of the bucket << 12 | basin, twice
@@ -152,9 +154,11 @@ struct BasinArgs {
   int64_t node_cap;
   char* state;
   int64_t state_bytes;
-  int32_t* queue;       // items that the first sweep launch leaves to the second
+  int32_t* queue;       // [2][n_items] items of the middle and of the large class
   int32_t n_items;
-  int32_t most_first;   // basins of an item that the first launch takes
+  int32_t most_first;   // basins of an item of the small class
+  int32_t most_mid;     // of the middle class: all state in shared memory too
+  int32_t mid;          // the launch takes the middle class
   int32_t most_narrow;  // basins of an item whose state (but the lists) is in shared memory
 };
 
@@ -591,8 +595,11 @@ __global__ void __launch_bounds__(kBuckets) basin_offset_kernel(BasinArgs a) {
     }
     if (lane == 0) {
       a.n_basins[(map * a.n_seg + seg) * 2 + sgn] = before;
-      if (sgn < a.signs && before > static_cast<uint32_t>(a.most_first))
-        a.queue[atomicAdd(a.counter + 2, 1)] = static_cast<int32_t>((map * a.signs + sgn) * a.n_seg + seg);
+      if (sgn < a.signs && before > static_cast<uint32_t>(a.most_first)) {
+        const int large = before > static_cast<uint32_t>(a.most_mid);
+        a.queue[large * a.n_items + atomicAdd(a.counter + 2 * large + 3, 1)] =
+            static_cast<int32_t>((map * a.signs + sgn) * a.n_seg + seg);
+      }
     }
   }
 }
@@ -950,7 +957,7 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
       // under, once per warp for those that share the first lane's (potentials:
       // it keeps its offset to that one).  Handed over link by link, the many
       // that a large component takes in waited for one another at its word
-      // (128 voxel items of a 91 x 109 x 91 mask: 532 -> 423 us; 256 items of
+      // (96 voxel items of a 91 x 109 x 91 mask: 532 -> 423 us; 256 items of
       // L6 surfaces: 283 -> 219 us).
       for (int q0 = pr0; q0 < pr_end; q0 += nth) {
         const int q = q0 + tid;
@@ -1201,23 +1208,31 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
   }
 }
 
-// First launch (kSecond false): the items of up to most_first basins, all state
-// in shared memory.  Second: the queued ones, one CTA per SM with as much
-// shared memory as there is.
-template <int kMode, bool kSecond>
-__global__ void __launch_bounds__(kSecond ? kMaxSweepThreads : 512, kSecond ? 1 : 2) basin_sweep_kernel(BasinArgs a) {
+// One launch per class of items: those of up to most_first basins, those of up
+// to most_mid (a queue; all their state in shared memory too, with fewer CTAs
+// per SM), and (kLarge) the rest, one CTA per SM with as much shared memory as
+// there is.  The launches go out largest class first and do not wait for one
+// another: a class's CTAs take the room that the one before leaves.  The end of
+// each launch waits for the one before, so that what follows the last of them
+// follows all.
+template <int kMode, bool kLarge>
+__global__ void __launch_bounds__(kLarge ? kMaxSweepThreads : 512, kLarge ? 1 : 2) basin_sweep_kernel(BasinArgs a) {
   __shared__ SweepShared S;
   extern __shared__ __align__(16) char dyn[];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x, nth = blockDim.x;
-  const int n_items = kSecond ? a.counter[2] : a.n_items;
+  const int cls = kLarge ? 2 : a.mid;
+  int32_t* const counter = a.counter + 2 * cls;
+  const int32_t* const queue = a.queue + (kLarge ? a.n_items : 0);
+  const int n_items = cls ? counter[1] : a.n_items;
   for (;;) {
-    if (tid == 0) S.item = atomicAdd(a.counter + kSecond, 1);
+    if (tid == 0) S.item = atomicAdd(counter, 1);
     __syncthreads();
     const int qi = S.item;
-    if (qi >= n_items) return;
+    if (qi >= n_items) break;
     int64_t out;  // (map * signs + sign) * n_seg + segment
-    if (kSecond) {
-      out = a.queue[qi];
+    if (cls) {
+      out = queue[qi];
     } else {
       const int per_seg = a.n_items / a.n_seg;  // largest segments first
       out = a.seg_rank ? (int64_t)(qi % per_seg) * a.n_seg + a.seg_rank[qi / per_seg] : qi;
@@ -1228,7 +1243,7 @@ __global__ void __launch_bounds__(kSecond ? kMaxSweepThreads : 512, kSecond ? 1 
     const int64_t map = ms / a.signs;
     const int64_t ss = map * a.n_seg + seg;
     const int nb = static_cast<int>(a.n_basins[ss * 2 + sgn]);
-    if (!kSecond && nb > a.most_first) {
+    if (!cls && nb > a.most_first) {
       __syncthreads();
       continue;
     }
@@ -1243,7 +1258,7 @@ __global__ void __launch_bounds__(kSecond ? kMaxSweepThreads : 512, kSecond ? 1 
     __syncthreads();
     for (int i = tid; i < S.L; i += nth) S.HH[i] = pow_h(S.T[i], a.seg_H[seg]);
     __syncthreads();
-    if (!kSecond) {
+    if (!kLarge) {
       sweep_item<kMode, kAllShared>(a, S, dyn, nullptr, map, sgn, seg, out);
     } else {
       char* slot = a.state + blockIdx.x * a.state_bytes;
@@ -1252,6 +1267,7 @@ __global__ void __launch_bounds__(kSecond ? kMaxSweepThreads : 512, kSecond ? 1 
     }
     __syncthreads();
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Fills out_maps for the vertices that never become active: 0 scaled and
@@ -1381,7 +1397,7 @@ Layout layout_of(const BasinPlan* p, int64_t M, int signs, int mode, int64_t nod
   l.tab_pair = take(M * p->n_tiles * kBuckets * 2);
   l.tab_cross = take(M * p->n_chunks * kBuckets * 4);
   l.n_pairs = take(M * (p->n_tiles + p->n_chunks) * 4);
-  l.queue = take(M * signs * p->n_seg * 4);
+  l.queue = take(2 * M * signs * p->n_seg * 4);
   l.n_basin = take(M * p->n_tiles * 2 * 2);
   l.bnd = take(M * p->n_bnd * 8);
   l.off_ev = take(M * p->n_tiles * kBuckets * 4);
@@ -1436,39 +1452,61 @@ int most_ctas() {
   return env ? std::max(0, std::atoi(env)) : 0;
 }
 
-// The first launch of `items` sweeps.  A step of a sweep has about vmax / 128
-// entries.  Few items (one per SM at most): as many threads as the steps fill,
-// and all the shared memory.  Many: CTAs of 256 threads, four per SM with the
-// state of 4,096 basins each (dense; a smooth map of 164k vertices has 3k per
-// sign), or of 512 threads, two per SM with 8,192.
-SweepShape first_shape(const BasinPlan* p, int mode, int64_t items, bool dense) {
-  const bool few = items <= p->sms;
-  const int per_basin = state_bytes_per_basin(mode, kAllShared);
+// The launches of `items` sweeps.  A step of a sweep has about vmax / 128
+// entries and is bound by latency, so an SM holds as many items as there are.
+// Up to one per SM: as many threads as the steps fill, and all the shared
+// memory.  Up to two: CTAs of 512 threads with half of it.  More: CTAs of 256
+// threads, four per SM with the state of 4,096 basins each (dense; a smooth map
+// of 164k vertices has 3k per sign), and the items with more of them in two per
+// SM (256 unsmoothed items of 38k vertices, 5k basins each: one per SM with
+// 1,024 threads 894 us, two 654 us).  The classes run beside one another: 320
+// items of two surfaces and a voxel skeleton took 353 + 313 us in turn, 390 so.
+SweepShape shape_of(const BasinPlan* p, int per_basin, int per_sm, int basins, int most_threads) {
   SweepShape s{};
-  const int most_threads = (few || !dense) ? 512 : 256;
   s.threads = 128;
   while (s.threads < most_threads && s.threads * 128 < p->vmax) s.threads *= 2;
-  s.basins = std::min(few ? 200 * 1024 / per_basin : dense ? 4096 : 8192, p->vmax);
+  s.basins = std::min({basins, (kSmBytes / per_sm - kSweepBytes) / per_basin, p->vmax});
   s.smem = s.basins * per_basin;
-  const int per_sm = few ? 1 : std::max(1, std::min(1024 / s.threads, 227 * 1024 / (s.smem + 4 * 1024)));
-  s.grid = p->sms * per_sm;
+  const int fit = std::min(1024 / s.threads, kSmBytes / (s.smem + kSweepBytes));
+  s.grid = p->sms * (per_sm == 1 ? 1 : std::max(per_sm, fit));
   if (const int cap = most_ctas()) s.grid = std::min(s.grid, cap);
   return s;
 }
 
-template <int kMode, bool kSecond>
-int launch_sweep_kernel(BasinArgs& a, const SweepShape& s, cudaStream_t st) {
-  auto* kern = basin_sweep_kernel<kMode, kSecond>;
-  TFGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem));
-  kern<<<s.grid, s.threads, s.smem, st>>>(a);
-  TFGB_CUDA(cudaGetLastError());
+SweepShape first_shape(const BasinPlan* p, int mode, int64_t items, bool dense) {
+  const int per_basin = state_bytes_per_basin(mode, kAllShared);
+  const int per_sm = items <= p->sms ? 1 : (items <= 2 * p->sms || !dense) ? 2 : 4;
+  return shape_of(p, per_basin, per_sm, per_sm == 4 ? 4096 : 65535, per_sm == 4 ? 256 : 512);
+}
+
+// `after`: the launch starts as soon as all CTAs of the one before it have.
+template <int kMode, bool kLarge>
+int launch_sweep_kernel(BasinArgs& a, const SweepShape& s, bool after, cudaStream_t st) {
+  auto* kern = basin_sweep_kernel<kMode, kLarge>;
+  TFGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmBytes - kSweepBytes));
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(s.grid);
+  cfg.blockDim = dim3(s.threads);
+  cfg.dynamicSmemBytes = s.smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = after ? 1 : 0;
+  TFGB_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
   return TFCE_OK;
 }
 
 template <int kMode>
-int launch_sweeps(BasinArgs& a, const SweepShape& first, const SweepShape& second, bool both, cudaStream_t st) {
-  int rc = launch_sweep_kernel<kMode, false>(a, first, st);
-  if (!rc && both) rc = launch_sweep_kernel<kMode, true>(a, second, st);
+int launch_sweeps(BasinArgs& a, const SweepShape& first, const SweepShape& mid, const SweepShape& large,
+                  cudaStream_t st) {
+  int rc = TFCE_OK;
+  if (large.grid) rc = launch_sweep_kernel<kMode, true>(a, large, false, st);
+  a.mid = 1;
+  if (!rc && mid.grid) rc = launch_sweep_kernel<kMode, false>(a, mid, large.grid > 0, st);
+  a.mid = 0;
+  if (!rc) rc = launch_sweep_kernel<kMode, false>(a, first, large.grid || mid.grid, st);
   return rc;
 }
 
@@ -1812,18 +1850,26 @@ int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st) {
   const int64_t per = (r.n_maps + launches - 1) / launches;
 
   const int64_t items_max = per * r.signs * p->n_seg;
-  SweepShape first = first_shape(p, mode, items_max, r.dense), second{};
-  second.threads = kMaxSweepThreads;
-  second.basins = std::min(std::min(222 * 1024 / state_bytes_per_basin(mode, kListsGlobal), 65535), p->vmax);
-  second.smem = second.basins * state_bytes_per_basin(mode, kListsGlobal);
-  int64_t slots2 = p->sms;
-  if (const int cap_ctas = most_ctas()) slots2 = std::min<int64_t>(slots2, cap_ctas);
-  slots2 = std::min(slots2, items_max);
-  const int slots = first.grid;
-  const bool both = first.basins < p->vmax;
-  const int64_t state = !both ? 0 : up((int64_t)p->vmax * state_bytes_per_basin(mode, kAllGlobal), 256);
+  SweepShape first = first_shape(p, mode, items_max, r.dense), mid{}, large{};
+  const int per_basin = state_bytes_per_basin(mode, kAllShared), per_basin_large = state_bytes_per_basin(mode, kListsGlobal);
+  const int first_ctas = first.grid;
+  int mid_ctas = 0, large_ctas = 0;
+  mid.basins = first.basins;
+  if (items_max > 2 * p->sms && r.dense && first.basins < p->vmax) {
+    mid = shape_of(p, per_basin, 2, 65535, 512);
+    mid_ctas = mid.grid;
+  }
+  if (mid.basins < p->vmax) {
+    large.threads = kMaxSweepThreads;
+    large.basins = std::min({(kSmBytes - kSweepBytes) / per_basin_large, 65535, p->vmax});
+    large.smem = large.basins * per_basin_large;
+    large_ctas = p->sms;
+    if (const int cap_ctas = most_ctas()) large_ctas = std::min(large_ctas, cap_ctas);
+    large_ctas = static_cast<int>(std::min<int64_t>(large_ctas, items_max));
+  }
+  const int64_t state = !large_ctas ? 0 : up((int64_t)p->vmax * state_bytes_per_basin(mode, kAllGlobal), 256);
   const Layout lay = layout_of(p, per, r.signs, mode, cap);
-  const int rc = ensure_ws(p, lay.total + slots2 * state);
+  const int rc = ensure_ws(p, lay.total + large_ctas * state);
   if (rc) return rc;
 
   BasinArgs a{};
@@ -1891,7 +1937,8 @@ int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st) {
   a.state = p->ws + lay.total;
   a.state_bytes = state;
   a.most_first = first.basins;
-  a.most_narrow = std::max(first.basins, second.basins);
+  a.most_mid = mid.basins;
+  a.most_narrow = std::max(mid.basins, large.basins);
   for (int64_t m0 = 0; m0 < r.n_maps; m0 += per) {
     const int64_t M = std::min(per, r.n_maps - m0);
     a.n_maps = static_cast<int32_t>(M);
@@ -1917,12 +1964,13 @@ int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st) {
     if (units && mode == kMaxima) basin_order_kernel<false><<<units, kTileThreads, 0, st>>>(a);
     else if (units) basin_order_kernel<true><<<units, kTileThreads, 0, st>>>(a);
     TFGB_CUDA(cudaGetLastError());
-    first.grid = std::min(slots, a.n_items);
-    second.grid = static_cast<int>(std::min<int64_t>(slots2, a.n_items));
+    first.grid = std::min(first_ctas, a.n_items);
+    mid.grid = std::min(mid_ctas, a.n_items);
+    large.grid = std::min(large_ctas, a.n_items);
     int e;
-    if (mode == kMaxima) e = launch_sweeps<kMaxima>(a, first, second, both, st);
-    else if (mode == kPotential) e = launch_sweeps<kPotential>(a, first, second, both, st);
-    else e = launch_sweeps<kNodes>(a, first, second, both, st);
+    if (mode == kMaxima) e = launch_sweeps<kMaxima>(a, first, mid, large, st);
+    else if (mode == kPotential) e = launch_sweeps<kPotential>(a, first, mid, large, st);
+    else e = launch_sweeps<kNodes>(a, first, mid, large, st);
     if (e) return e;
     if (mode == kNodes) {
       const dim3 g(static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((p->vmax + 255) / 256, 1024))),
