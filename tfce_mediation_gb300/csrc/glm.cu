@@ -188,38 +188,117 @@ int launch_glm_k(int tv, const float* Y, int64_t ldy, int32_t n, int64_t V, cons
 // data, the SE rounded to float32 (se_of_slope stores it in a float32 array,
 // cynumstats.pyx:47-52) and t = double beta / that SE (tval_int, :59-64).
 // One thread per vertex, the design's pseudoinverse and rows in shared memory.
+//
+// Bound by the double pipe (2 FMA per SM and cycle, 64 times fewer than float):
+// with residuals in double too and the data converted by it, 200 subjects x
+// 305k vertices x 4 columns took 1,213 us.  The betas stay there.  sigma^2 only
+// has to decide a float32 rounding, so its residuals are formed in pairs of
+// floats, the rounding is taken where the pairs' error bound decides it
+// (Ziv 1991), and the vertices where it does not (one in some thousands, data
+// out of the float range, a near-perfect fit) redo theirs in double.  The data
+// are widened by integer operations.  The results are the same bit for bit, in
+// 605 us.
+
+// The double of a float, without the double pipe for normal numbers.
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t u = __float_as_uint(f), e = u & 0x7f800000u;
+  if (e == 0u || e == 0x7f800000u) return (u << 1) ? (double)f : __hiloint2double((int)u, 0);
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+
+__device__ __forceinline__ float two_sum(float x, float y, float& err) {  // Knuth
+  const float s = __fadd_rn(x, y), t = __fsub_rn(s, x);
+  err = __fadd_rn(__fsub_rn(x, __fsub_rn(s, t)), __fsub_rn(y, t));
+  return s;
+}
+
 template <int KMAX>
 __global__ void __launch_bounds__(256) glm_f64_kernel(
     const float* __restrict__ Y, int64_t ldy, int32_t n, int64_t V, const double* __restrict__ pinv,
     const double* __restrict__ X, const double* __restrict__ invdiag, const double* __restrict__ dof,
     const int32_t* __restrict__ coef, int32_t n_coef, int32_t what, double* __restrict__ out, int64_t ldo) {
   extern __shared__ double sm64[];
-  double* ps = sm64;              // [KMAX][n]
-  double* xs = sm64 + KMAX * n;   // [n][KMAX]
+  double* ps = sm64;                                        // [n][KMAX]
+  float2* xs = reinterpret_cast<float2*>(sm64 + KMAX * n);  // [n][KMAX]: X in pairs
+  __shared__ uint32_t x_max[KMAX];                          // bits of each column's largest |X|
   const int64_t g = blockIdx.y;
+  const double* Xg = X + g * n * KMAX;
+  if (threadIdx.x < KMAX) x_max[threadIdx.x] = 0;
+  __syncthreads();
   for (int i = threadIdx.x; i < KMAX * n; i += blockDim.x) {
-    ps[i] = pinv[g * KMAX * n + i];
-    xs[i] = X[g * n * KMAX + i];
+    ps[(i % n) * KMAX + i / n] = pinv[g * KMAX * n + i];
+    const double x = Xg[i];
+    const float hi = (float)x;
+    xs[i] = make_float2(hi, (float)(x - (double)hi));
+    atomicMax(&x_max[i % KMAX], __float_as_uint(fabsf(hi)));
   }
   __syncthreads();
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= V) return;
+  const float* Yv = Y + v;
   double b[KMAX];
 #pragma unroll
   for (int j = 0; j < KMAX; ++j) b[j] = 0.0;
+#pragma unroll 4
   for (int s = 0; s < n; ++s) {
-    const double y = (double)Y[(int64_t)s * ldy + v];
+    const double y = widen(Yv[(int64_t)s * ldy]);
 #pragma unroll
-    for (int j = 0; j < KMAX; ++j) b[j] = fma(ps[j * n + s], y, b[j]);
+    for (int j = 0; j < KMAX; ++j) b[j] = fma(ps[s * KMAX + j], y, b[j]);
   }
-  double rss = 0.0;
-  for (int s = 0; s < n; ++s) {
-    double r = (double)Y[(int64_t)s * ldy + v];
+  // RSS in pairs of floats, and the bound of its relative error (of its root)
+  double rss = 0.0, eps = 1.0;
+  if (what != kWhatBeta) {
+    float bh[KMAX], bl[KMAX], top = 0.0f, sum = 0.0f, low = 0.0f;
+    float reach = 0.0f;  // largest sum of the fit's terms
+    bool fits = true;
 #pragma unroll
-    for (int j = 0; j < KMAX; ++j) r = fma(-xs[s * KMAX + j], b[j], r);
-    rss = fma(r, r, rss);
+    for (int j = 0; j < KMAX; ++j) {
+      bh[j] = -(float)b[j];
+      bl[j] = -(float)(b[j] + (double)bh[j]);
+      const float xm = __uint_as_float(x_max[j]);
+      fits = fits && fabsf(bh[j]) <= 0x1p60f && xm <= 0x1p60f;
+      reach = __fmaf_rn(fabsf(bh[j]), xm, reach);
+    }
+#pragma unroll 4
+    for (int s = 0; s < n; ++s) {
+      float r = Yv[(int64_t)s * ldy], rl = 0.0f;
+      top = fmaxf(top, fabsf(r));
+#pragma unroll
+      for (int j = 0; j < KMAX; ++j) {
+        const float2 x = xs[s * KMAX + j];
+        const float p = __fmul_rn(x.x, bh[j]);
+        float e;
+        r = two_sum(r, p, e);
+        rl = __fadd_rn(rl, __fadd_rn(e, __fmaf_rn(x.x, bh[j], -p)));
+        rl = __fmaf_rn(x.x, bl[j], __fmaf_rn(x.y, bh[j], rl));
+      }
+      float e;
+      r = two_sum(r, rl, rl);  // the terms may have cancelled down to rl
+      const float q = __fmul_rn(r, r);
+      sum = two_sum(sum, q, e);
+      low = __fadd_rn(low, __fadd_rn(e, __fmaf_rn(__fadd_rn(r, r), rl, __fmaf_rn(r, r, -q))));
+      const float t = __fadd_rn(sum, low);  // |low| stays below an ulp of the sum
+      low = __fsub_rn(low, __fsub_rn(t, sum));
+      sum = t;
+    }
+    // A residual is off by at most 2^-47 of its terms' sum per term and
+    // operation (8 per column), a sum of n squares by n 2^-47.
+    if (fits && sum >= 0x1p-60f && sum <= 0x1p100f) {
+      rss = (double)sum + (double)low;
+      const float root = sqrtf(__fdiv_rn(sum, (float)n));
+      eps = 0x1p-43 + (double)(0x1p-47f * ((float)n + (8.0f * KMAX + 8.0f) * ((top + reach) / root)));
+    }
   }
-  const double sigma2 = rss / dof[g];
+  auto rss_double = [&]() {
+    double total = 0.0;
+    for (int s = 0; s < n; ++s) {
+      double r = (double)Yv[(int64_t)s * ldy];
+#pragma unroll
+      for (int j = 0; j < KMAX; ++j) r = fma(-Xg[s * KMAX + j], b[j], r);
+      total = fma(r, r, total);
+    }
+    return total;
+  };
   for (int c = 0; c < n_coef; ++c) {
     const int j = coef[c];
     double bj = 0.0;
@@ -231,8 +310,18 @@ __global__ void __launch_bounds__(256) glm_f64_kernel(
       *dst = CUDART_NAN;
       continue;
     }
-    const double se = (double)__double2float_rn(sqrt(sigma2 * invdiag[g * KMAX + j]));
-    *dst = (what == kWhatBeta) ? bj : (what == kWhatSE) ? se : bj / se;
+    if (what == kWhatBeta) {
+      *dst = bj;
+      continue;
+    }
+    double root = sqrt(rss / dof[g] * invdiag[g * KMAX + j]);
+    if (eps > 0.0 && !(eps < 0x1p-24 && __double2float_rn(root * (1.0 - eps)) == __double2float_rn(root * (1.0 + eps)))) {
+      rss = rss_double();
+      eps = 0.0;
+      root = sqrt(rss / dof[g] * invdiag[g * KMAX + j]);
+    }
+    const double se = (double)__double2float_rn(root);
+    *dst = (what == kWhatSE) ? se : bj / se;
   }
 }
 
@@ -261,11 +350,6 @@ __device__ __forceinline__ float sobel_z(float a, float b, int alg) {
   const float ah = __fmul_rn(a, a), bh = __fmul_rn(b, b);
   const float al = __fmaf_rn(a, a, -ah), bl = __fmaf_rn(b, b, -bh);
   const float one = alg == 0 ? 1.0f : alg == 1 ? 0.0f : -1.0f;
-  auto two_sum = [](float x, float y, float& err) {
-    const float s = __fadd_rn(x, y), t = __fsub_rn(s, x);
-    err = __fadd_rn(__fsub_rn(x, __fsub_rn(s, t)), __fsub_rn(y, t));
-    return s;
-  };
   float e0, e1;
   const float s0 = two_sum(ah, bh, e0);
   const float sh = two_sum(s0, one, e1);
