@@ -1337,6 +1337,7 @@ __global__ void basin_power_kernel(double* out, int64_t n, float E) {
 struct BasinPlan {
   int device = 0, sms = 0;
   int32_t n_seg = 0, vmax = 0;
+  int32_t basins = 0;  // of one sign of a segment at most
   int64_t V = 0, n_pos = 0, n_pair = 0, n_cpair = 0, n_opair = 0;
   int32_t n_tiles = 0, n_chunks = 0, n_bnd = 0;
   std::vector<void*> owned;  // device tables
@@ -1422,7 +1423,7 @@ Layout layout_of(const BasinPlan* p, int64_t M, int signs, int mode, int64_t nod
 
 constexpr int64_t kWorkspaceBudget = 8LL << 30;  // maps are swept in as many launches as this asks for
 
-int64_t node_capacity(const BasinPlan* p) { return (int64_t)p->vmax * kMaxSteps; }
+int64_t node_capacity(const BasinPlan* p) { return (int64_t)p->basins * kMaxSteps; }
 
 int ensure_ws(BasinPlan* p, int64_t bytes) {
   if (p->ws_bytes >= bytes) return TFCE_OK;
@@ -1465,7 +1466,7 @@ SweepShape shape_of(const BasinPlan* p, int per_basin, int per_sm, int basins, i
   SweepShape s{};
   s.threads = 128;
   while (s.threads < most_threads && s.threads * 128 < p->vmax) s.threads *= 2;
-  s.basins = std::min({basins, (kSmBytes / per_sm - kSweepBytes) / per_basin, p->vmax});
+  s.basins = std::min({basins, (kSmBytes / per_sm - kSweepBytes) / per_basin, p->basins});
   s.smem = s.basins * per_basin;
   const int fit = std::min(1024 / s.threads, kSmBytes / (s.smem + kSweepBytes));
   s.grid = p->sms * (per_sm == 1 ? 1 : std::max(per_sm, fit));
@@ -1526,50 +1527,50 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
   // cross; a patch that cannot grow goes on from the next free vertex, so that
   // all tiles of a segment but the last are full.  Inside a tile the vertices
   // keep their order, so that the statistic is read in runs.
-  std::vector<int32_t> tile_of(V, -1), mark(V, -1);  // tile within the segment
+  std::vector<int32_t> mark(V, -1), tile_of(V);
   std::vector<std::vector<std::vector<int32_t>>> grown(n_seg);
   parallel_for(n_seg, V, [&](int64_t s) {
-    std::vector<int32_t> queue, rim;
+    constexpr int32_t kTaken = 0x7fffffff;  // in mark: in a tile; else the last tile that queued the vertex
+    std::vector<int32_t> queue(seg[s + 1] - seg[s] + 1), rim;
     int64_t scan = seg[s], left = seg[s + 1] - seg[s];
     while (left > 0) {
       const int32_t id = static_cast<int32_t>(grown[s].size());
       std::vector<int32_t> members;
+      members.reserve(std::min<int64_t>(left, kTile));
       int64_t entries = 0;
       bool full = false;
-      rim.swap(queue);  // free vertices beside the last tile
-      size_t rim_at = 0, head = 0;
+      size_t rim_at = 0;  // of the free vertices beside the last tile
       while (!full && left > 0) {
-        while (rim_at < rim.size() && tile_of[rim[rim_at]] >= 0) ++rim_at;
-        int32_t start;
+        while (rim_at < rim.size() && mark[rim[rim_at]] == kTaken) ++rim_at;
+        size_t head = 0, tail = 1;
         if (rim_at < rim.size()) {
-          start = rim[rim_at];
+          queue[0] = rim[rim_at];
         } else {
-          while (tile_of[scan] >= 0) ++scan;
-          start = static_cast<int32_t>(scan);
+          while (mark[scan] == kTaken) ++scan;
+          queue[0] = static_cast<int32_t>(scan);
         }
-        queue.assign(1, start);
-        mark[start] = id;
-        for (head = 0; head < queue.size(); ++head) {
+        mark[queue[0]] = id;
+        for (; head < tail; ++head) {
           const int32_t v = queue[head];
-          const int64_t deg = off[v + 1] - off[v];
-          if (static_cast<int>(members.size()) == kTile || (entries > 0 && entries + deg > kTileEntries)) {
+          const int64_t e0 = off[v], e1 = off[v + 1];
+          if (static_cast<int>(members.size()) == kTile || (entries > 0 && entries + e1 - e0 > kTileEntries)) {
             full = true;
             break;
           }
-          entries += deg;
-          tile_of[v] = id;
+          entries += e1 - e0;
+          mark[v] = kTaken;
           members.push_back(v);
           --left;
-          for (int64_t e = off[v]; e < off[v + 1]; ++e) {
+          for (int64_t e = e0; e < e1; ++e) {
             const int32_t u = static_cast<int32_t>(packed[e] & kIdx);
-            if (tile_of[u] < 0 && mark[u] != id) {
+            if (mark[u] < id) {
               mark[u] = id;
-              queue.push_back(u);
+              queue[tail++] = u;
             }
           }
         }
+        if (full || left == 0) rim.assign(queue.begin() + head, queue.begin() + tail);
       }
-      queue.erase(queue.begin(), queue.begin() + std::min(head, queue.size()));
       grown[s].push_back(std::move(members));
     }
   });
@@ -1596,14 +1597,17 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
   parallel_for(nt, V, [&](int64_t t) {
     std::vector<int32_t>& mem = *members[t];
     std::sort(mem.begin(), mem.end());
-    for (size_t i = 0; i < mem.size(); ++i) local[mem[i]] = static_cast<uint16_t>(i);
+    for (size_t i = 0; i < mem.size(); ++i) {
+      local[mem[i]] = static_cast<uint16_t>(i);
+      tile_of[mem[i]] = tiles[t].in_seg;
+    }
   });
   // entries that basin_cross_kernel takes: to another tile, or one-way
   auto crosses = [&](int64_t v, uint32_t entry) { return (entry & kOne) || tile_of[entry & kIdx] != tile_of[v]; };
   // rows of neighbours and of pairs of neighbours, by tile
   struct Rows {
     std::vector<uint32_t> nbr, nbr_end, edge, edge_end;
-    int64_t n_edges = 0;
+    int64_t n_edges = 0, n_basins = 0;
   };
   std::vector<Rows> rows(nt);
   std::vector<uint8_t> is_bnd(V, 0);
@@ -1611,67 +1615,80 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
     const std::vector<int32_t>& mem = *members[t];
     const int nv = tiles[t].nv;
     Rows& r = rows[t];
-    std::vector<std::vector<uint16_t>> held(nv);
     // rows of 32 lanes, two entries (4 * index) a lane; padding: the vertex itself
-    auto put = [&](std::vector<uint32_t>& rows_out, int i, size_t width, auto entry) {
-      for (size_t j = 0; j < width; j += 2)
-        for (int l = 0; l < 32; ++l) {
-          uint32_t two[2];
-          for (size_t k = 0; k < 2; ++k) {
-            const int u = i + l < nv ? entry(l, j + k) : -1;
-            two[k] = 4u * static_cast<uint32_t>(u >= 0 ? u : std::min(i + l, nv - 1));
+    auto put = [&](std::vector<uint32_t>& out, std::vector<uint32_t>& ends, const std::vector<uint16_t>& list,
+                   const std::vector<int32_t>& at, const std::vector<int32_t>& count) {
+      for (int i = 0; i < nv; i += 32) {
+        int width = 0;
+        for (int v = i; v < std::min(nv, i + 32); ++v) width = std::max(width, count[v]);
+        size_t o = out.size();
+        out.resize(o + static_cast<size_t>((width + 1) / 2) * 32);
+        for (int j = 0; j < width; j += 2)
+          for (int v = i; v < i + 32; ++v) {
+            const uint32_t self = std::min(v, nv - 1);
+            const int c = v < nv ? count[v] : 0;
+            const uint32_t x = j < c ? list[at[v] + j] : self, y = j + 1 < c ? list[at[v] + j + 1] : self;
+            out[o++] = 4u * x | (4u * y << 16);
           }
-          rows_out.push_back(two[0] | (two[1] << 16));
-        }
-    };
-    std::vector<uint16_t> near[32];
-    for (int i = 0; i < nv; i += 32) {
-      size_t width = 0;
-      for (int l = 0; l < 32; ++l) {
-        near[l].clear();
-        if (i + l >= nv) continue;
-        const int32_t v = mem[i + l];
-        for (int64_t e = off[v]; e < off[v + 1]; ++e) {
-          if (crosses(v, packed[e])) {
-            __atomic_store_n(&is_bnd[packed[e] & kIdx], uint8_t{1}, __ATOMIC_RELAXED);
-            __atomic_store_n(&is_bnd[v], uint8_t{1}, __ATOMIC_RELAXED);
-            continue;
-          }
-          const uint16_t u = local[packed[e] & kIdx];
-          near[l].push_back(u);
-          if (u < i + l) continue;
-          // each pair of neighbours once, held by the one that holds fewer so far
-          if (held[u].size() < held[i + l].size()) held[u].push_back(static_cast<uint16_t>(i + l));
-          else held[i + l].push_back(u);
-          ++r.n_edges;
-        }
-        width = std::max(width, near[l].size());
+        ends.push_back(static_cast<uint32_t>(out.size()));
       }
-      put(r.nbr, i, width, [&](int l, size_t j) { return j < near[l].size() ? int(near[l][j]) : -1; });
-      r.nbr_end.push_back(static_cast<uint32_t>(r.nbr.size()));
+    };
+    std::vector<int32_t> at(nv + 1, 0), count(nv, 0), held_count(nv, 0);
+    for (int i = 0; i < nv; ++i) at[i + 1] = at[i] + static_cast<int32_t>(off[mem[i] + 1] - off[mem[i]]);
+    std::vector<uint16_t> near(at[nv]), held(at[nv]);
+    auto hold = [&](int v, int u) { held[at[v] + held_count[v]++] = static_cast<uint16_t>(u); };
+    for (int i = 0; i < nv; ++i) {
+      const int32_t v = mem[i];
+      for (int64_t e = off[v]; e < off[v + 1]; ++e) {
+        if (crosses(v, packed[e])) {
+          __atomic_store_n(&is_bnd[packed[e] & kIdx], uint8_t{1}, __ATOMIC_RELAXED);
+          __atomic_store_n(&is_bnd[v], uint8_t{1}, __ATOMIC_RELAXED);
+          continue;
+        }
+        const uint16_t u = local[packed[e] & kIdx];
+        near[at[i] + count[i]++] = u;
+        if (u < i) continue;
+        // each pair of neighbours once, held by the one that holds fewer so far
+        if (held_count[u] < held_count[i]) hold(u, i);
+        else hold(i, u);
+        ++r.n_edges;
+      }
     }
+    put(r.nbr, r.nbr_end, near, at, count);
     for (int pass = 0; pass < 4; ++pass)  // even out: a vertex hands one to a neighbour that holds two fewer
       for (int i = 0; i < nv; ++i)
-        for (size_t j = 0; j < held[i].size(); ++j) {
-          const int u = held[i][j];
-          if (held[u].size() + 1 < held[i].size()) {
-            held[i][j] = held[i].back();
-            held[i].pop_back();
-            held[u].push_back(static_cast<uint16_t>(i));
+        for (int j = 0; j < held_count[i]; ++j) {
+          const int u = held[at[i] + j];
+          if (held_count[u] + 1 < held_count[i]) {
+            held[at[i] + j] = held[at[i] + --held_count[i]];
+            hold(u, i);
           }
         }
-    for (int i = 0; i < nv; i += 32) {
-      size_t width = 0;
-      for (int l = 0; l < 32 && i + l < nv; ++l) width = std::max(width, held[i + l].size());
-      put(r.edge, i, width, [&](int l, size_t j) { return j < held[i + l].size() ? int(held[i + l][j]) : -1; });
-      r.edge_end.push_back(static_cast<uint32_t>(r.edge.size()));
+    put(r.edge, r.edge_end, held, at, held_count);
+    // Basins at most: of vertices that are all neighbours of one another only
+    // the highest can start one.  Covered greedily by triples and pairs.
+    std::vector<uint8_t> covered(nv, 0);
+    for (int i = 0; i < nv; ++i) {
+      if (covered[i]) continue;
+      covered[i] = 1;
+      ++r.n_basins;
+      int u = -1, w = -1;
+      for (int j = 0; j < count[i] && w < 0; ++j) {
+        const int x = near[at[i] + j];
+        if (covered[x]) continue;
+        if (u < 0) u = x;
+        else if (std::find(near.begin() + at[x], near.begin() + at[x] + count[x], u) != near.begin() + at[x] + count[x])
+          w = x;
+      }
+      if (u >= 0) covered[u] = 1;
+      if (w >= 0) covered[w] = 1;
     }
   });
   // the tiles one after the other
   std::vector<int32_t> vert, bnd_vert, bnd_of(V, -1);
   std::vector<uint32_t> slice_off(1, 0), nbr, edge_off(1, 0), edge;
   std::vector<uint16_t> bnd_local, bnd_tile;
-  std::vector<int64_t> seg_pairs(n_seg, 0);
+  std::vector<int64_t> seg_pairs(n_seg, 0), seg_basins(n_seg, 0);
   int64_t n_pair = 0;
   for (int t = 0; t < nt; ++t) {
     TileInfo& ti = tiles[t];
@@ -1688,6 +1705,7 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
     nbr.insert(nbr.end(), r.nbr.begin(), r.nbr.end());
     edge.insert(edge.end(), r.edge.begin(), r.edge.end());
     if (r.n_edges > 65535) return TFCE_OK;  // pairs are counted in 16 bits
+    seg_basins[ti.seg] += r.n_basins;
     seg_pairs[ti.seg] += up(r.n_edges, 8);  // pairs of basins: at most one per pair of neighbours
     n_pair += up(r.n_edges, 8);
     for (int i = 0; i < ti.nv; ++i) {
@@ -1766,6 +1784,7 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
   cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
   p->n_seg = n_seg;
   p->vmax = vmax;
+  p->basins = static_cast<int32_t>(std::max<int64_t>(1, *std::max_element(seg_basins.begin(), seg_basins.end())));
   p->V = V;
   p->n_pos = static_cast<int64_t>(vert.size());
   p->n_pair = n_pair;
@@ -1855,19 +1874,19 @@ int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st) {
   const int first_ctas = first.grid;
   int mid_ctas = 0, large_ctas = 0;
   mid.basins = first.basins;
-  if (items_max > 2 * p->sms && r.dense && first.basins < p->vmax) {
+  if (items_max > 2 * p->sms && r.dense && first.basins < p->basins) {
     mid = shape_of(p, per_basin, 2, 65535, 512);
     mid_ctas = mid.grid;
   }
-  if (mid.basins < p->vmax) {
+  if (mid.basins < p->basins) {
     large.threads = kMaxSweepThreads;
-    large.basins = std::min({(kSmBytes - kSweepBytes) / per_basin_large, 65535, p->vmax});
+    large.basins = std::min({(kSmBytes - kSweepBytes) / per_basin_large, 65535, p->basins});
     large.smem = large.basins * per_basin_large;
     large_ctas = p->sms;
     if (const int cap_ctas = most_ctas()) large_ctas = std::min(large_ctas, cap_ctas);
     large_ctas = static_cast<int>(std::min<int64_t>(large_ctas, items_max));
   }
-  const int64_t state = !large_ctas ? 0 : up((int64_t)p->vmax * state_bytes_per_basin(mode, kAllGlobal), 256);
+  const int64_t state = !large_ctas ? 0 : up((int64_t)p->basins * state_bytes_per_basin(mode, kAllGlobal), 256);
   const Layout lay = layout_of(p, per, r.signs, mode, cap);
   const int rc = ensure_ws(p, lay.total + large_ctas * state);
   if (rc) return rc;

@@ -837,13 +837,11 @@ int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n
     seg[0] = 0;
     seg[1] = V;
   }
-  std::vector<int32_t> seg_of(V);
   int32_t vmax = 1;
   for (int s = 0; s < n_seg; ++s) {
     const int64_t len = seg[s + 1] - seg[s];
     TFGB_CHECK_ARG(len <= tfgb::kMaxSegVertices, "segment larger than 2^24-1 vertices");
     vmax = std::max<int32_t>(vmax, static_cast<int32_t>(len));
-    for (int64_t v = seg[s]; v < seg[s + 1]; ++v) seg_of[v] = s;
   }
   for (int s = 0; s < n_seg; ++s) {
     TFGB_CHECK_ARG(std::isfinite(H[s]) && std::isfinite(E[s]), "H/E must be finite");
@@ -851,33 +849,45 @@ int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n
 
   // Clean the lists: validate, drop self entries, mark entries whose reverse
   // is missing.  Neighbour order inside a list never changes the partition.
-  std::vector<int64_t> off(V + 1, 0);
-  std::vector<int32_t> idx;
-  idx.reserve(static_cast<size_t>(D));
-  for (int32_t v = 0; v < V; ++v) {
-    for (int64_t e = offsets[v]; e < offsets[v + 1]; ++e) {
-      const int32_t b = indices[e];
-      if (b < 0 || b >= V) {
-        tfgb::set_error("adjacency entry %d of vertex %d outside [0, %d)", b, v, V);
-        return TFCE_EINVAL;
-      }
-      if (seg_of[b] != seg_of[v]) {
-        tfgb::set_error("adjacency entry %d of vertex %d crosses segments", b, v);
-        return TFCE_EINVAL;
-      }
-      if (b != v) idx.push_back(b);
-    }
-    off[v + 1] = static_cast<int64_t>(idx.size());
-  }
+  // An entry is rejected, the first of them, if it is outside the graph or its
+  // vertex's segment.
+  auto segment_of = [&](int64_t v) { return std::upper_bound(seg.begin(), seg.end(), v) - seg.begin() - 1; };
   const int64_t blocks = (V + 4095) / 4096;
-  tfgb::parallel_for(blocks, V, [&](int64_t k) {
-    for (int64_t v = k * 4096; v < std::min<int64_t>(V, (k + 1) * 4096); ++v)
-      if (!std::is_sorted(idx.begin() + off[v], idx.begin() + off[v + 1]))
-        std::sort(idx.begin() + off[v], idx.begin() + off[v + 1]);
+  std::vector<int64_t> off(V + 1, 0), kept(blocks + 1, 0), bad(blocks, -1);
+  tfgb::parallel_for(blocks, D, [&](int64_t k) {
+    int64_t v = k * 4096, s = segment_of(v);
+    for (; v < std::min<int64_t>(V, (k + 1) * 4096); ++v) {
+      while (v >= seg[s + 1]) ++s;
+      int64_t n = 0;
+      for (int64_t e = offsets[v]; e < offsets[v + 1]; ++e) {
+        if ((indices[e] < seg[s] || indices[e] >= seg[s + 1]) && bad[k] < 0) bad[k] = e;
+        n += indices[e] != v;
+      }
+      kept[k + 1] += n;
+    }
+  });
+  for (int64_t e : bad) {
+    if (e < 0) continue;
+    const int32_t v = static_cast<int32_t>(std::upper_bound(offsets, offsets + V + 1, e) - offsets - 1);
+    if (indices[e] < 0 || indices[e] >= V) tfgb::set_error("adjacency entry %d of vertex %d outside [0, %d)", indices[e], v, V);
+    else tfgb::set_error("adjacency entry %d of vertex %d crosses segments", indices[e], v);
+    return TFCE_EINVAL;
+  }
+  for (int64_t k = 0; k < blocks; ++k) kept[k + 1] += kept[k];
+  std::vector<int32_t> idx(kept[blocks]);
+  tfgb::parallel_for(blocks, D, [&](int64_t k) {
+    int64_t o = kept[k];
+    for (int64_t v = k * 4096; v < std::min<int64_t>(V, (k + 1) * 4096); ++v) {
+      const int64_t o0 = o;
+      for (int64_t e = offsets[v]; e < offsets[v + 1]; ++e)
+        if (indices[e] != v) idx[o++] = indices[e];
+      off[v + 1] = o;
+      if (!std::is_sorted(idx.begin() + o0, idx.begin() + o)) std::sort(idx.begin() + o0, idx.begin() + o);
+    }
   });
   std::vector<uint32_t> packed(idx.size());
   std::atomic<bool> two_way{true};
-  tfgb::parallel_for(blocks, V, [&](int64_t k) {
+  tfgb::parallel_for(blocks, D, [&](int64_t k) {
     for (int64_t v = k * 4096; v < std::min<int64_t>(V, (k + 1) * 4096); ++v)
       for (int64_t e = off[v]; e < off[v + 1]; ++e) {
         const int32_t b = idx[e];
