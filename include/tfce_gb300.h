@@ -483,10 +483,13 @@ int geodesic_take_lists(geodesic_mesh* m, int32_t* out_i, int32_t* out_j, double
  *           written only where x > 0 (0 elsewhere);
  *   mode 1 (tm_func.find_nearest): p_array of the nearer neighbour rank,
  *           for every value.
- * image and out are double [V] (device). */
+ * image and out are double [V] (device); fwer_lookup_f32 takes the image as
+ * float, with the same results. */
 int fwer_sort(double* values, int64_t n, void* stream);
 int fwer_lookup(const double* sorted_null, int64_t N, const double* image, int64_t V,
                 int32_t mode, double* out, void* stream);
+int fwer_lookup_f32(const double* sorted_null, int64_t N, const float* image, int64_t V,
+                    int32_t mode, double* out, void* stream);
 
 /* ---------------------------------------------------------------------------
  * Learned null-tail surrogate: kernels of a small MLP (no counterpart in the

@@ -119,6 +119,8 @@ SIGNATURES = {
     "fwer_sort": (ctypes.c_int, [c_vp, ctypes.c_int64, c_vp]),
     "fwer_lookup": (ctypes.c_int, [c_vp, ctypes.c_int64, c_vp, ctypes.c_int64, ctypes.c_int32,
                                    c_vp, c_vp]),
+    "fwer_lookup_f32": (ctypes.c_int, [c_vp, ctypes.c_int64, c_vp, ctypes.c_int64, ctypes.c_int32,
+                                   c_vp, c_vp]),
     "mlp_gemm": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                 c_vp, ctypes.c_int32, c_vp, ctypes.c_int32, c_vp, ctypes.c_int32, c_vp,
                                 ctypes.c_int32, c_vp, ctypes.c_int32, c_vp]),

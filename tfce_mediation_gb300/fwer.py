@@ -26,10 +26,16 @@ def sorted_null(null):
 
 def _lookup(srt, image, mode):
     t = require_cuda()
-    img = dev(np.asarray(image, np.float64) if not isinstance(image, t.Tensor) else image, t.float64)
-    out = t.empty_like(img)
-    _lib.check(_lib.load().fwer_lookup(ptr(srt), srt.numel(), ptr(img), img.numel(), mode, ptr(out),
-                                       stream_handle()))
+    if not isinstance(image, t.Tensor):
+        image = np.asarray(image)
+    # float32 images go up as they are and are widened by the lookup
+    f32 = image.dtype in (t.float32, np.float32)
+    if not isinstance(image, t.Tensor):
+        image = image.astype(np.float32 if f32 else np.float64, copy=not image.flags.writeable)
+    img = dev(image, t.float32 if f32 else t.float64)
+    out = t.empty_like(img, dtype=t.float64)
+    lookup = _lib.load().fwer_lookup_f32 if f32 else _lib.load().fwer_lookup
+    _lib.check(lookup(ptr(srt), srt.numel(), ptr(img), img.numel(), mode, ptr(out), stream_handle()))
     return out
 
 
