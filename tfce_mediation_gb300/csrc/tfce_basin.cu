@@ -44,6 +44,8 @@ constexpr int kTileThreads = 512;
 constexpr int kPerThread = kTile / kTileThreads;
 constexpr int kBuckets = 256;          // sign * 128 + step
 constexpr int kTab = kBuckets + 2;     // bucket starts and the total
+constexpr uint32_t kNegative = 0x80000000u, kPositive = 0x40000000u;  // sign of a vertex of a tile
+constexpr uint32_t kOddRow = 0x80000000u;  // in edge_off: the second entries of the row's last words are padding
 constexpr uint32_t kRoot = 0x80000000u;
 constexpr uint32_t kExtent = 0x00ffffffu;
 constexpr int kPairTable = 2048;       // slots for the distinct pairs of basins of a tile
@@ -126,10 +128,10 @@ struct BasinArgs {
   // workspace
   uint32_t* seg_max;    // [maps][2][n_seg] bits of max(0, max)
   int32_t* counter;     // items taken and, of the queued ones, there are: by class (2 * class, 2 * class + 1)
-  uint32_t* ev;         // by vertex of the tile: basin | bucket << 12, or kNone
+  uint32_t* ev;         // vertices of a tile by bucket: bucket << 24, index in the tile << 12, basin
   uint32_t* pairs;      // pairs of basins of a tile: bucket << 24, 12 bits each
   uint2* cpairs;        // crossing pairs: tile << 16 | 4 bits of the bucket << 12 | basin, twice
-  uint16_t* tab_ev;     // [map][tile][kBuckets] entries of every bucket
+  uint16_t* tab_ev;     // [map][tile][kTab] first entry of every bucket, and their number
   uint16_t* tab_pair;
   uint32_t* tab_cross;  // [map][chunk][kBuckets]
   uint32_t* n_pairs;    // [map][tile] and, after them, [map][chunk]
@@ -275,6 +277,11 @@ __global__ void __launch_bounds__(256) basin_max_kernel(BasinArgs a, int32_t par
 // vertex's root is known its word becomes sign, 128 - step, root, and every
 // pair of neighbours with different roots is a pair of basins, joined at the
 // later step of the two.
+//
+// Bound by instructions (3.3 a cycle, 420 per 32 vertices of a mesh: keys 71,
+// neighbours 81, pointers 71, pairs 154, sort 53): 2.25 ms for 512 maps x 2 L7.
+// The pairs' test reads the class of both words at once, and rows of an odd
+// width leave their last halves out (198 before).
 __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a) {
   __shared__ uint32_t key[kTile];
   __shared__ __align__(16) uint16_t lab[kTile];  // pointer, then root (2 * index in the tile)
@@ -282,7 +289,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a
   static_assert(kPairTable * sizeof(uint32_t) <= sizeof(lab), "the table takes lab's place");
   __shared__ uint16_t rk[kTile];   // basin number of a root
   __shared__ float sT[2][kMaxSteps];
-  __shared__ int cnt[kBuckets], pcnt[kBuckets];
+  __shared__ int cnt[kBuckets + 1], pcnt[kBuckets], wsum[8];
   __shared__ float4 sTab[2];  // maximum, steps per unit, step count
   __shared__ int nroots[2], npairs;
   __shared__ uint32_t sQueue[kTileThreads / 32 * kQueue];
@@ -319,61 +326,64 @@ __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a
       const int L = __float_as_int(tab.z);
       uint32_t place;
       const int st = step_of(fabsf(xv[k]), sT[sgn], L, tab.x, tab.y, &place);
-      if (st < L)
-        w = (__float_as_uint(xv[k]) & 0x80000000u) | (static_cast<uint32_t>(127 - st) << 24) | (place << 12) |
-            static_cast<uint32_t>(4095 - v);
+      if (st < L) w = (static_cast<uint32_t>(127 - st) << 24) | (place << 12) | static_cast<uint32_t>(4095 - v);
+      if (sgn) w = 0u - w;
     }
     if (v < ti.nv) key[v] = w;
   }
   __syncthreads();
 
   auto at = [&](uint32_t offset) { return *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(key) + offset); };
-  // the largest neighbour
+  // the largest neighbour (the smallest, for the negative sign)
 #pragma unroll 4
   for (int k = 0; k < kPerThread; ++k) {
     const int v = tid + k * kTileThreads;
     if (v < ti.nv) {
       const uint32_t* so = a.slice_off + ti.slice0 + (v >> 5);
       const uint32_t o1 = so[1];
-      const uint32_t kv = key[v], s = kv & 0x80000000u;
-      int best = static_cast<int>(kv ^ s);
+      const int kv = static_cast<int>(key[v]);
+      int hi = kv, lo = kv;
 #pragma unroll 3
       for (uint32_t o = so[0] + lane; o < o1; o += 32) {
         const uint32_t two = a.nbr[o];
-        best = max(best, static_cast<int>(at(two & 0xffffu) ^ s));
-        best = max(best, static_cast<int>(at(two >> 16) ^ s));
+        const int x0 = static_cast<int>(at(two & 0xffffu)), x1 = static_cast<int>(at(two >> 16));
+        hi = max(max(hi, x0), x1);
+        lo = min(min(lo, x0), x1);
       }
+      const int best = kv < 0 ? -lo : hi;
       lab[v] = static_cast<uint16_t>(8190 - 2 * (best & 0xfff));
     }
   }
   __syncthreads();
-  // follow the pointers, two hops at a time (a root points to itself; a stored
-  // root shortens the walks that pass it); number the basins
+  // Follow the pointers, two hops at a time (a root points to itself; a stored
+  // root shortens the walks that pass it; keys grow along them, so they end);
+  // number the basins.
 #pragma unroll 2
   for (int k = 0; k < kPerThread; ++k) {
     const int v = tid + k * kTileThreads;
-    const uint32_t w = (v < ti.nv) ? key[v] : 0u;
-    if (w) {
+    const int kv = (v < ti.nv) ? static_cast<int>(key[v]) : 0;
+    if (kv) {
       auto up = [&](uint32_t o) { return *reinterpret_cast<volatile uint16_t*>(reinterpret_cast<char*>(lab) + o); };
       uint32_t r = up(2 * v);
-      for (int it = 0; it < kTile; ++it) {
+      for (;;) {
         const uint32_t n = up(r);
         r = up(n);
         if (r == n) break;
       }
       *reinterpret_cast<volatile uint16_t*>(lab + v) = static_cast<uint16_t>(r);
       r >>= 1;
-      const int sgn = w >> 31;
-      const uint32_t code = ((w >> 24) & 127u) + 1u;  // 128 - step
-      const uint32_t b = sgn * kMaxSteps + kMaxSteps - code;
-      atomicAdd(&cnt[b], 1);
-      key[v] = (w & 0x80000000u) | (code << 12) | r;
+      const int sgn = kv < 0;
+      const uint32_t code = (static_cast<uint32_t>(abs(kv)) >> 24) + 1u;  // 128 - step
+      atomicAdd(&cnt[sgn * kMaxSteps + kMaxSteps - code], 1);
+      key[v] = (sgn ? kNegative : kPositive) | (code << 12) | r;
       if (r == static_cast<uint32_t>(v)) rk[v] = static_cast<uint16_t>(atomicAdd(&nroots[sgn], 1));
     }
   }
   __syncthreads();
   for (int i = tid; i < kPairTable; i += kTileThreads) table[i] = 0u;
-  __syncthreads();
+  scan_buckets(cnt, wsum);
+  const int64_t row = map * a.n_tiles + tile;
+  if (tid <= kBuckets) a.tab_ev[row * kTab + tid] = static_cast<uint16_t>(cnt[tid]);
   // A pair of basins matters at the first step that joins it: the table keeps
   // {pair, 128 - step} words and their maximum per pair.  A pair that finds no
   // slot is written down as it comes (joining two basins again changes nothing).
@@ -389,7 +399,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a
   uint32_t* const queue = sQueue + (tid >> 5) * kQueue;
   int nq = 0;
   auto insert = [&](int q) {
-    const uint32_t w = at((queue[q] >> 12) << 2), u = at((queue[q] & 0xfffu) << 2);
+    const uint32_t w = at(queue[q] >> 16), u = at(queue[q] & 0xffffu);
     const uint32_t i = w & 0xfffu, j = u & 0xfffu;
     const uint32_t e = (min(i, j) << 20) | (max(i, j) << 8) | (min(u & 0xff000u, w & 0xff000u) >> 12);
     uint32_t h = ((e >> 8) * 2654435761u) >> 21;
@@ -408,27 +418,25 @@ __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a
       h = (h + 1) & (kPairTable - 1);
     }
   };
-  uint32_t* ev = a.ev + map * a.pos_per_map + ti.pos0;
   const uint32_t below = (1u << lane) - 1u;
   for (int k = 0; k < kPerThread; ++k) {
     const int v = tid + k * kTileThreads;
     if (v - lane >= ti.nv) break;
-    const uint32_t w = (v < ti.nv) ? key[v] : 0u;
+    const uint32_t w = (v < ti.nv) ? key[v] : 0u, sign = w & (kPositive | kNegative);
     const uint32_t* so = a.edge_off + ti.slice0 + (v >> 5);
-    const uint32_t o1 = so[1];
-    for (uint32_t o = so[0] + lane; o < o1; o += 32) {
+    const uint32_t end = so[1], o1 = end & ~kOddRow;
+    // neighbours of the same sign with another root
+    auto check = [&](uint32_t off) {
+      const uint32_t u = at(off);
+      const bool hit = (u & sign) && ((u ^ w) & 0xfffu);
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      if (hit) queue[nq + __popc(m & below)] = (static_cast<uint32_t>(v) << 18) | off;
+      nq += __popc(m);
+    };
+    for (uint32_t o = (so[0] & ~kOddRow) + lane; o < o1; o += 32) {
       const uint32_t two = a.edge[o];
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const uint32_t off = half ? two >> 16 : two & 0xffffu;
-        const uint32_t u = at(off), d = u ^ w;
-        const bool hit = (d & 0xfffu) && static_cast<int>(d) >= 0 && (u & 0xff000u) && w;
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (m) {
-          if (hit) queue[nq + __popc(m & below)] = (static_cast<uint32_t>(v) << 12) | (off >> 2);
-          nq += __popc(m);
-        }
-      }
+      check(two & 0xffffu);
+      if (!(end & kOddRow) || o + 32 < o1) check(two >> 16);
       while (nq >= 32) {
         __syncwarp();
         insert(nq - 32 + lane);
@@ -436,8 +444,6 @@ __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a
         __syncwarp();
       }
     }
-    if (v < ti.nv)
-      ev[v] = w ? (rk[w & 0xfffu] | (((w >> 31) * kMaxSteps + kMaxSteps - ((w >> 12) & 0xffu)) << 12)) : kNone;
   }
   __syncwarp();
   if (lane < nq) insert(lane);
@@ -451,12 +457,25 @@ __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a
   __syncthreads();
   for (int i = tid; i < kPairTable; i += kTileThreads)
     if (table[i]) emit(table[i]);
-  __syncthreads();
-  const int64_t row = map * a.n_tiles + tile;
-  if (tid < kBuckets) {
-    a.tab_ev[row * kBuckets + tid] = static_cast<uint16_t>(cnt[tid]);
-    a.tab_pair[row * kBuckets + tid] = static_cast<uint16_t>(pcnt[tid]);
+  // the vertices in order of their buckets, in place of the keys
+  uint32_t rec[kPerThread];
+#pragma unroll
+  for (int k = 0; k < kPerThread; ++k) {
+    const int v = tid + k * kTileThreads;
+    rec[k] = (v < ti.nv) ? key[v] : 0u;
   }
+  const int n_ev = cnt[kBuckets];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kPerThread; ++k) {
+    if (rec[k] == 0u) continue;
+    const uint32_t b = (rec[k] >> 31) * kMaxSteps + kMaxSteps - ((rec[k] >> 12) & 0xffu);
+    key[atomicAdd(&cnt[b], 1)] = (b << 24) | (static_cast<uint32_t>(tid + k * kTileThreads) << 12) | rk[rec[k] & 0xfffu];
+  }
+  __syncthreads();
+  uint32_t* ev = a.ev + map * a.pos_per_map + ti.pos0;
+  for (int p = tid; p < n_ev; p += kTileThreads) ev[p] = key[p];
+  if (tid < kBuckets) a.tab_pair[row * kBuckets + tid] = static_cast<uint16_t>(pcnt[tid]);
   if (tid < 2) a.n_basin[row * 2 + tid] = static_cast<uint16_t>(nroots[tid]);
   if (tid == 2) a.n_pairs[row] = npairs;
 }
@@ -552,9 +571,9 @@ __global__ void __launch_bounds__(kBuckets) basin_offset_kernel(BasinArgs a) {
   uint32_t run = 0;
 #pragma unroll 8
   for (int t = 0; t < si.ntiles; ++t) {
-    const uint32_t n = a.tab_ev[(row0 + t) * kBuckets + b];
-    a.off_ev[(row0 + t) * kBuckets + b] = run;
-    run += n;
+    const uint16_t* start = a.tab_ev + (row0 + t) * kTab + b;
+    a.off_ev[(row0 + t) * kBuckets + b] = run - start[0];  // for a place in the tile's own order
+    run += static_cast<uint32_t>(start[1]) - start[0];
   }
   tot[b] = run;
   __syncthreads();
@@ -607,13 +626,11 @@ __global__ void __launch_bounds__(kBuckets) basin_offset_kernel(BasinArgs a) {
 // The segment's ordered lists, with basin numbers of the whole segment: 16
 // bits a basin where the sweep keeps its state in shared memory, else 32.  One
 // CTA per (map, tile) and (map, chunk).  The order within a bucket is free.
-// A tile's vertices are put in order in shared memory first, so that the
-// segment's list is written in runs.
+// A tile's vertices are in order already, so the segment's list is written in
+// runs.  Bound by the latency of a CTA's loads (512 maps x 2 L7: 525 us with the
+// sort in here, 387 with all loads issued before the first is used).
 template <bool kOrder>
-__global__ void __launch_bounds__(kTileThreads, 3) basin_order_kernel(BasinArgs a) {
-  __shared__ uint32_t sorted[kTile];                // basin | bucket << 24
-  __shared__ uint16_t index[kOrder ? kTile : 1];    // index in the tile
-  __shared__ int start[kBuckets + 1], wsum[8];
+__global__ void __launch_bounds__(kTileThreads, 4) basin_order_kernel(BasinArgs a) {
   __shared__ uint32_t to_ev[kBuckets], to_pair[kBuckets];
   const int units = a.n_tiles + a.n_chunks;
   const int unit = blockIdx.x % units;
@@ -633,48 +650,40 @@ __global__ void __launch_bounds__(kTileThreads, 3) basin_order_kernel(BasinArgs 
     const TileInfo ti = a.tiles[unit];
     const int64_t row = map * a.n_tiles + unit;
     const uint32_t* ev = a.ev + map * a.pos_per_map + ti.pos0;
-    uint32_t rec[kPerThread];
+    uint32_t rec[kPerThread];  // all loads at once: a CTA lives for little more than their latency
 #pragma unroll
     for (int k = 0; k < kPerThread; ++k) {
-      const int v = tid + k * kTileThreads;
-      rec[k] = (v < ti.nv) ? ev[v] : kNone;
+      const int p = tid + k * kTileThreads;
+      rec[k] = p < ti.nv ? ev[p] : 0u;
     }
     if (tid < kBuckets) {
-      start[tid] = a.tab_ev[row * kBuckets + tid];
       to_ev[tid] = a.start_ev[srow + tid] + a.off_ev[row * kBuckets + tid];
       to_pair[tid] = a.start_pair[srow + tid] + a.off_pair[row * kBuckets + tid];
     }
     const uint32_t base0 = a.base_of[row * 2], base1 = a.base_of[row * 2 + 1];
     const int n_pr = static_cast<int>(a.n_pairs[row]);
-    __syncthreads();
-    scan_buckets(start, wsum);
-    if (tid < kBuckets) to_ev[tid] -= start[tid];
-    const int n_ev = start[kBuckets];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-      if (rec[k] == kNone) continue;
-      const uint32_t bk = rec[k] >> 12;
-      const int p = atomicAdd(&start[bk], 1);
-      sorted[p] = ((bk >= kMaxSteps ? base1 : base0) + (rec[k] & 0xfffu)) | (bk << 24);
-      if (kOrder) index[p] = static_cast<uint16_t>(tid + k * kTileThreads);
-    }
+    const int n_ev = a.tab_ev[row * kTab + kBuckets];
+    const uint32_t* pr = a.pairs + map * a.pair_per_map + ti.pair0;
+    uint32_t first = 0;
+    if (tid < n_pr) first = pr[tid];
     __syncthreads();
     const int64_t eo = map * a.n_vertices + si.pos0;
     uint32_t* ev32 = reinterpret_cast<uint32_t*>(a.ev_out) + eo;
     uint16_t* ev16 = reinterpret_cast<uint16_t*>(a.ev_out) + 2 * eo;
-#pragma unroll 4
-    for (int p = tid; p < n_ev; p += kTileThreads) {
-      const uint32_t r = sorted[p];
-      const uint32_t bk = r >> 24, id = r & 0xffffffu, d = to_ev[bk] + p;
+#pragma unroll
+    for (int k = 0; k < kPerThread; ++k) {
+      const int p = tid + k * kTileThreads;
+      if (p >= n_ev) break;
+      const uint32_t r = rec[k];
+      const uint32_t bk = r >> 24, d = to_ev[bk] + p;
       const bool neg = bk >= kMaxSteps;
+      const uint32_t id = (neg ? base1 : base0) + (r & 0xfffu);
       if (neg ? wide1 : wide0) ev32[d] = id;
       else ev16[d + (neg ? ev1 : 0u)] = static_cast<uint16_t>(id);
-      if (kOrder) a.ord[eo + d] = a.vert[ti.pos0 + index[p]];
+      if (kOrder) a.ord[eo + d] = a.vert[ti.pos0 + ((r >> 12) & 0xfffu)];
     }
-    const uint32_t* pr = a.pairs + map * a.pair_per_map + ti.pair0;
     for (int p = tid; p < n_pr; p += kTileThreads) {
-      const uint32_t r = pr[p];
+      const uint32_t r = p == tid ? first : pr[p];
       const uint32_t bk = r >> 24;
       const uint32_t d = atomicAdd(&to_pair[bk], 1u);
       const bool neg = bk >= kMaxSteps;
@@ -1394,7 +1403,7 @@ Layout layout_of(const BasinPlan* p, int64_t M, int signs, int mode, int64_t nod
   l.ev = take(M * p->n_pos * 4);
   l.pairs = take(M * p->n_pair * 4);
   l.cpairs = take(M * p->n_cpair * 8);
-  l.tab_ev = take(M * p->n_tiles * kBuckets * 2);
+  l.tab_ev = take(M * p->n_tiles * kTab * 2);
   l.tab_pair = take(M * p->n_tiles * kBuckets * 2);
   l.tab_cross = take(M * p->n_chunks * kBuckets * 4);
   l.n_pairs = take(M * (p->n_tiles + p->n_chunks) * 4);
@@ -1630,7 +1639,7 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
             const uint32_t x = j < c ? list[at[v] + j] : self, y = j + 1 < c ? list[at[v] + j + 1] : self;
             out[o++] = 4u * x | (4u * y << 16);
           }
-        ends.push_back(static_cast<uint32_t>(out.size()));
+        ends.push_back(static_cast<uint32_t>(out.size()) | (width & 1 ? kOddRow : 0u));
       }
     };
     std::vector<int32_t> at(nv + 1, 0), count(nv, 0), held_count(nv, 0);
@@ -1699,7 +1708,7 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
     ti.bnd0 = static_cast<int32_t>(bnd_vert.size());
     ti.pair0 = static_cast<int32_t>(n_pair);
     for (size_t i = 0; i < r.nbr_end.size(); ++i) {
-      slice_off.push_back(static_cast<uint32_t>(nbr.size()) + r.nbr_end[i]);
+      slice_off.push_back(static_cast<uint32_t>(nbr.size()) + (r.nbr_end[i] & ~kOddRow));
       edge_off.push_back(static_cast<uint32_t>(edge.size()) + r.edge_end[i]);
     }
     nbr.insert(nbr.end(), r.nbr.begin(), r.nbr.end());
@@ -1719,7 +1728,7 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
     }
     ti.nbnd = static_cast<int32_t>(bnd_vert.size()) - ti.bnd0;
     while (vert.size() % 32) vert.push_back(0);
-    if (n_pair > 0x7fffffffLL || vert.size() > 0x7fffffffull || nbr.size() >= (1ull << 32)) return TFCE_OK;
+    if (n_pair > 0x7fffffffLL || vert.size() > 0x7fffffffull || nbr.size() >= (1ull << 32) || edge.size() >= (1ull << 31)) return TFCE_OK;
     r = Rows();
   }
   // crossing lists, in chunks of boundary vertices of one segment
