@@ -378,6 +378,18 @@ int glm_qf_design_block(int32_t kmax);
 int glm_qf_designs(const double* base, int64_t ld, int64_t stride, const int32_t* rows, const int32_t* cols,
                    int32_t share, int32_t n, int32_t n_pad, int32_t G, int32_t kmax, void* x_tiles, float* ginv,
                    float* invdiag, float* dof, int32_t* err, void* stream);
+/* Operands of glm_stat_tc_block for G permuted intercept designs, formed on the
+ * device in FP64: design d is [1, x_1 .. x_kmax-1] with x_j column j of
+ * base [n][ld] double (device; column 0 is not read) at the subjects of
+ * rows [G][n] int32 (device), or NULL for none permuted.  Writes p_tiles (row
+ * blocks of design_block * 8), u_rows [G_pad][kmax], x_rows
+ * [G_pad / design_block][n_sc][kmax][design_block] (centred: 1 for use with
+ * Y_centred), invdiag [G][kmax], dof [G], and for the n_rows rows of an output
+ * program (device, mode 3) weights [G][w_stride]; err as glm_qf_designs. */
+int glm_tc_designs(const double* base, int64_t ld, const int32_t* rows, int32_t n, int32_t n_pad, int32_t n_sc,
+                   int32_t G, int32_t kmax, int32_t design_block, int32_t centred, const int32_t* program,
+                   int32_t n_rows, int32_t w_stride, void* p_tiles, float* u_rows, float* x_rows, float* invdiag,
+                   float* dof, float* weights, int32_t* err, void* stream);
 int glm_col_sumsq(const float* Y_centred, int64_t ldy, int32_t n, int64_t V, float* yy, void* stream);
 int glm_tstat_tc_qf(const void* y_tiles, const float* yy, int32_t n, int32_t n_pad, int64_t V,
                     const void* x_tiles, const float* ginv, const float* invdiag, const float* dof, int32_t G,

@@ -26,6 +26,9 @@ enum DevErr : int32_t {
   kDevSingular = 4,  // a design whose cross products have no inverse
 };
 
+// output kinds of the programmed GLM epilogue (glm_stat_tc mode 3)
+constexpr int kTcOutT = 0, kTcOutNegT = 1, kTcOutF = 2, kTcOutAmp = 3, kTcOutAcro = 4, kTcOutEss = 5;
+
 inline int map_dev_err(int32_t e) {
   switch (e) {
     case kDevOk: return TFCE_OK;

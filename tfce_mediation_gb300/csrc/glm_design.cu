@@ -51,10 +51,64 @@ __device__ inline double block_sum(double v, double* red) {
   return v;
 }
 
+struct DesignShared {
+  double red[kDesignThreads / 32];
+  double mean[kDesignCols], gram[kDesignCols][2 * kDesignCols];
+};
+
+// Means and centred cross products of the columns entry(s, 0 .. kc).
+template <typename Entry>
+__device__ void centred_products(const Entry& entry, int kc, int n, DesignShared& S) {
+  const int tid = threadIdx.x;
+  for (int j = 0; j < kc; ++j) {
+    double s = 0.0;
+    for (int i = tid; i < n; i += kDesignThreads) s += entry(i, j);
+    s = block_sum(s, S.red);
+    if (tid == 0) S.mean[j] = s / n;
+  }
+  __syncthreads();
+  for (int j = 0; j < kc; ++j)
+    for (int l = j; l < kc; ++l) {
+      double s = 0.0;
+      for (int i = tid; i < n; i += kDesignThreads) s += (entry(i, j) - S.mean[j]) * (entry(i, l) - S.mean[l]);
+      s = block_sum(s, S.red);
+      if (tid == 0) S.gram[j][l] = S.gram[l][j] = s;
+    }
+  __syncthreads();
+}
+
+// Inverse of the w x w block at the left of g's rows of `ld` into the block
+// beside it, by Gauss-Jordan with row pivots (one thread).
+__device__ void invert(double* g, int ld, int w, int32_t* err) {
+  for (int j = 0; j < w; ++j)
+    for (int l = 0; l < w; ++l) g[j * ld + w + l] = (j == l) ? 1.0 : 0.0;
+  for (int j = 0; j < w; ++j) {
+    int p = j;
+    for (int r = j + 1; r < w; ++r)
+      if (fabs(g[r * ld + j]) > fabs(g[p * ld + j])) p = r;
+    if (p != j)
+      for (int l = 0; l < 2 * w; ++l) {
+        const double t = g[j * ld + l];
+        g[j * ld + l] = g[p * ld + l];
+        g[p * ld + l] = t;
+      }
+    const double pivot = g[j * ld + j];  // divided, so that equal columns leave an exact zero
+    if (pivot == 0.0) atomicCAS(err, 0, kDevSingular);
+    for (int l = 0; l < 2 * w; ++l) g[j * ld + l] = g[j * ld + l] / pivot;
+    for (int r = 0; r < w; ++r) {
+      if (r == j) continue;
+      const double f = g[r * ld + j];
+      if (f != 0.0)
+        for (int l = 0; l < 2 * w; ++l) g[r * ld + l] = fma(-f, g[j * ld + l], g[r * ld + l]);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kDesignThreads) design_kernel(DesignArgs a) {
-  __shared__ double red[kDesignThreads / 32];
-  __shared__ double mean[kDesignCols], gram[kDesignCols][2 * kDesignCols];
+  __shared__ DesignShared S;
   __shared__ int32_t sCol[kDesignCols];
+  auto& mean = S.mean;
+  auto& gram = S.gram;
   const int d = blockIdx.x, tid = threadIdx.x;
   const int kc = a.kmax - 1, R = a.R;
   const bool live = d < a.G;
@@ -74,56 +128,16 @@ __global__ void __launch_bounds__(kDesignThreads) design_kernel(DesignArgs a) {
     }
     return X[(int64_t)r * a.ld + (c & (kPermuted - 1))];
   };
-  if (live) {
-    for (int j = 0; j < kc; ++j) {
-      double s = 0.0;
-      for (int i = tid; i < a.n; i += kDesignThreads) s += entry(i, j);
-      s = block_sum(s, red);
-      if (tid == 0) mean[j] = s / a.n;
-    }
-    __syncthreads();
-    for (int j = 0; j < kc; ++j)
-      for (int l = j; l < kc; ++l) {
-        double s = 0.0;
-        for (int i = tid; i < a.n; i += kDesignThreads) s += (entry(i, j) - mean[j]) * (entry(i, l) - mean[l]);
-        s = block_sum(s, red);
-        if (tid == 0) gram[j][l] = gram[l][j] = s;
-      }
-    __syncthreads();
-  }
-  // inverse by Gauss-Jordan with row pivots; a missing column keeps a zero
-  // row and column
-  if (tid == 0) {
+  if (live) centred_products(entry, kc, a.n, S);
+  // a missing column keeps a zero row and column
+  if (tid == 0 && live) {
     int k = 1;
-    if (live) {
-      for (int j = 0; j < kc; ++j) {
-        const bool has = sCol[j] >= 0;
-        k += has;
-        for (int l = 0; l < kc; ++l) gram[j][kc + l] = (j == l) ? 1.0 : 0.0;
-        if (!has) gram[j][j] = 1.0;
-      }
-      for (int j = 0; j < kc; ++j) {
-        int p = j;
-        for (int r = j + 1; r < kc; ++r)
-          if (fabs(gram[r][j]) > fabs(gram[p][j])) p = r;
-        if (p != j)
-          for (int l = 0; l < 2 * kc; ++l) {
-            const double t = gram[j][l];
-            gram[j][l] = gram[p][l];
-            gram[p][l] = t;
-          }
-        if (gram[j][j] == 0.0) atomicCAS(a.err, 0, kDevSingular);
-        const double pivot = gram[j][j];  // divided, so that equal columns leave an exact zero
-        for (int l = 0; l < 2 * kc; ++l) gram[j][l] = gram[j][l] / pivot;
-        for (int r = 0; r < kc; ++r) {
-          if (r == j) continue;
-          const double f = gram[r][j];
-          if (f != 0.0)
-            for (int l = 0; l < 2 * kc; ++l) gram[r][l] = fma(-f, gram[j][l], gram[r][l]);
-        }
-      }
-      a.dof[d] = static_cast<float>(a.n - k);
+    for (int j = 0; j < kc; ++j) {
+      if (sCol[j] >= 0) ++k;
+      else gram[j][j] = 1.0;
     }
+    invert(&gram[0][0], 2 * kDesignCols, kc, a.err);
+    a.dof[d] = static_cast<float>(a.n - k);
   }
   // the split-BF16 tiles of glm_tile_split: 256-row blocks, 16-column steps of
   // [hi|lo][8-column block][row][8]
@@ -157,9 +171,173 @@ __global__ void __launch_bounds__(kDesignThreads) design_kernel(DesignArgs a) {
         (tid > 0 && sCol[tid - 1] >= 0) ? static_cast<float>(gram[tid - 1][kc + tid - 1]) : 0.0f;
 }
 
+// Operands of the residual-epilogue GLM (glm_stat_tc) for permuted intercept
+// designs [1, x_1 .. x_kmax-1], all columns permuted alike: tiles of the
+// pseudoinverse rows, their sums, the negated design rows, inv(X'X)'s diagonal
+// and the weights of an output program.  The host formed and uploaded them
+// batch by batch: 1.1 of the 1.9 ms that 32 permutations of a rhythm model
+// over 82k vertices took; this takes 51 us.
+struct ResidualDesignArgs {
+  const double* base;   // [n][ld]
+  int64_t ld;
+  const int32_t* rows;  // [G][n], or NULL
+  int32_t n, n_pad, n_sc, G, kmax, DB, centred;
+  const int32_t* program;  // [n_rows] {kind, column, width, weight offset}
+  int32_t n_rows, w_stride;
+  __nv_bfloat16* tiles;    // row blocks of DB * 8
+  float* u;                // [G_pad][kmax]
+  float* x;                // [G_pad / DB][n_sc][kmax][DB]
+  float* invdiag;          // [G][kmax]
+  float* dof;              // [G]
+  float* weights;          // [G][w_stride]
+  int32_t* err;
+};
+
+__global__ void __launch_bounds__(kDesignThreads) residual_design_kernel(ResidualDesignArgs a) {
+  constexpr int kAll = kDesignCols + 1;
+  __shared__ DesignShared S;
+  __shared__ double full[kAll][kAll];       // inv(X'X)
+  __shared__ double block[kAll][2 * kAll];  // a program row's block of it, and its inverse
+  const int d = blockIdx.x, tid = threadIdx.x;
+  const int kmax = a.kmax, kc = kmax - 1;
+  const bool live = d < a.G;
+  const int32_t* rows = (a.rows && live) ? a.rows + (int64_t)d * a.n : nullptr;
+  auto entry = [&](int s, int j) -> double {  // column j + 1
+    int r = s;
+    if (rows) {
+      const int p = rows[s];
+      if (static_cast<unsigned>(p) < static_cast<unsigned>(a.n)) r = p;
+      else atomicCAS(a.err, 0, kDevBadIndex);
+    }
+    return a.base[(int64_t)r * a.ld + j + 1];
+  };
+  if (live) {
+    centred_products(entry, kc, a.n, S);
+    if (tid == 0) {
+      invert(&S.gram[0][0], 2 * kDesignCols, kc, a.err);
+      double m0 = 1.0 / a.n;
+      for (int j = 0; j < kc; ++j) {
+        double gm = 0.0;
+        for (int l = 0; l < kc; ++l) {
+          full[j + 1][l + 1] = S.gram[j][kc + l];
+          gm = fma(S.gram[j][kc + l], S.mean[l], gm);
+        }
+        full[0][j + 1] = full[j + 1][0] = -gm;
+        m0 = fma(S.mean[j], gm, m0);
+      }
+      full[0][0] = m0;
+      a.dof[d] = static_cast<float>(a.n - kmax);
+      float* w = a.weights + (int64_t)d * a.w_stride;
+      for (int t = 0; t < a.n_rows; ++t) {
+        const int kind = a.program[4 * t], j = a.program[4 * t + 1], width = a.program[4 * t + 2], o = a.program[4 * t + 3];
+        const bool block_row = kind == kTcOutF || kind == kTcOutEss;
+        if (!block_row && kind != kTcOutAmp && kind != kTcOutAcro) continue;
+        const int size = block_row ? width * width : 3;
+        if (o < 0 || width < 1 || width > kAll || o + size > a.w_stride) continue;
+        const bool inside = j >= 0 && j + width <= kmax;  // else the GLM returns NaN for the row
+        if (inside && block_row) {
+          for (int p = 0; p < width; ++p)
+            for (int q = 0; q < width; ++q) block[p][q] = full[j + p][j + q];
+          invert(&block[0][0], 2 * kAll, width, a.err);
+          for (int p = 0; p < width; ++p)
+            for (int q = 0; q < width; ++q) w[o + p * width + q] = static_cast<float>(block[p][width + q]);
+        } else if (inside) {
+          w[o] = static_cast<float>(full[j][j]);
+          w[o + 1] = static_cast<float>(full[j][j + 1]);
+          w[o + 2] = static_cast<float>(full[j + 1][j + 1]);
+        } else {
+          for (int e = 0; e < size; ++e) w[o + e] = 0.0f;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // pseudoinverse entry (row j, subject s): inv(X'X) (1, x_s)'
+  auto pinv = [&](int j, int s) {
+    double v = full[j][0];
+    for (int l = 0; l < kc; ++l) v = fma(full[j][l + 1], entry(s, l), v);
+    return v;
+  };
+  const int rb = a.DB * 8, ks_count = a.n_pad / 16;
+  for (int t = tid; t < 8 * (a.n_pad / 8); t += kDesignThreads) {
+    const int j = t % 8, c0 = (t / 8) * 8;
+    __align__(16) __nv_bfloat16 h[8];
+    __align__(16) __nv_bfloat16 l[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int c = c0 + e;
+      const float x = (live && j < kmax && c < a.n) ? static_cast<float>(pinv(j, c)) : 0.0f;
+      h[e] = __float2bfloat16_rn(x);
+      l[e] = __float2bfloat16_rn(x - __bfloat162float(h[e]));
+    }
+    const int64_t row = (int64_t)d * 8 + j;
+    const int64_t blk = row / rb, r = row % rb;
+    const int ks = c0 / 16, kb = (c0 % 16) / 8;
+    __nv_bfloat16* at = a.tiles + ((blk * ks_count + ks) * 2 * rb * 16 + (int64_t)kb * rb * 8 + r * 8);
+    *reinterpret_cast<uint4*>(at) = *reinterpret_cast<const uint4*>(h);
+    *reinterpret_cast<uint4*>(at + (int64_t)rb * 16) = *reinterpret_cast<const uint4*>(l);
+  }
+  float* x = a.x + (int64_t)(d / a.DB) * a.n_sc * kmax * a.DB + d % a.DB;
+  for (int t = tid; t < a.n_sc * kmax; t += kDesignThreads) {
+    const int s = t / kmax, j = t % kmax;
+    double v = 0.0;
+    if (live && s < a.n) {
+      if (j == 0) v = a.centred ? 0.0 : -1.0;
+      else v = a.centred ? S.mean[j - 1] - entry(s, j - 1) : -entry(s, j - 1);
+    }
+    x[(int64_t)t * a.DB] = static_cast<float>(v);
+  }
+  // the rows sum to those of the identity's first column
+  if (tid < kmax) {
+    a.u[(int64_t)d * kmax + tid] = (live && tid == 0) ? 1.0f : 0.0f;
+    if (live) a.invdiag[(int64_t)d * kmax + tid] = static_cast<float>(full[tid][tid]);
+  }
+}
+
 }  // namespace tfgb
 
 extern "C" {
+
+int glm_tc_designs(const double* base, int64_t ld, const int32_t* rows, int32_t n, int32_t n_pad, int32_t n_sc,
+                   int32_t G, int32_t kmax, int32_t design_block, int32_t centred, const int32_t* program,
+                   int32_t n_rows, int32_t w_stride, void* p_tiles, float* u_rows, float* x_rows, float* invdiag,
+                   float* dof, float* weights, int32_t* err, void* stream) {
+  tfgb::clear_error();
+  TFGB_CHECK_ARG(base && p_tiles && u_rows && x_rows && invdiag && dof && err, "NULL pointer");
+  TFGB_CHECK_ARG(kmax >= 2 && kmax <= 8, "kmax must be in [2, 8]");
+  TFGB_CHECK_ARG(n > 0 && n_pad >= n && n_pad % 16 == 0, "n_pad must be >= n and a multiple of 16");
+  TFGB_CHECK_ARG(n_sc >= n && ld >= kmax && G >= 0 && n_rows >= 0 && w_stride >= 0, "bad sizes");
+  TFGB_CHECK_ARG(design_block == 16 || (design_block == 32 && kmax <= 5),
+                 "design_block must be 32 (kmax <= 5) or 16");
+  TFGB_CHECK_ARG((n_rows == 0 || program) && (w_stride == 0 || weights), "program / weights is NULL");
+  TFGB_CHECK_ARG(reinterpret_cast<uintptr_t>(p_tiles) % 16 == 0, "tiles must be 16-byte aligned");
+  if (G == 0) return TFCE_OK;
+  tfgb::ResidualDesignArgs a{};
+  a.base = base;
+  a.ld = ld;
+  a.rows = rows;
+  a.n = n;
+  a.n_pad = n_pad;
+  a.n_sc = n_sc;
+  a.G = G;
+  a.kmax = kmax;
+  a.DB = design_block;
+  a.centred = centred;
+  a.program = program;
+  a.n_rows = w_stride ? n_rows : 0;
+  a.w_stride = w_stride;
+  a.tiles = static_cast<__nv_bfloat16*>(p_tiles);
+  a.u = u_rows;
+  a.x = x_rows;
+  a.invdiag = invdiag;
+  a.dof = dof;
+  a.weights = weights;
+  a.err = err;
+  const unsigned grid = static_cast<unsigned>((G + design_block - 1) / design_block * design_block);
+  tfgb::residual_design_kernel<<<grid, tfgb::kDesignThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  TFGB_CUDA(cudaGetLastError());
+  return TFCE_OK;
+}
 
 int glm_qf_designs(const double* base, int64_t ld, int64_t stride, const int32_t* rows, const int32_t* cols,
                    int32_t share, int32_t n, int32_t n_pad, int32_t G, int32_t kmax, void* x_tiles, float* ginv,

@@ -54,8 +54,6 @@ constexpr int kTcK = 16;            // subjects per MMA K step / pipeline stage
 constexpr int kTcStages = 4;
 constexpr int kTcSubjChunk = 32;    // subjects per epilogue X chunk
 constexpr uint64_t kTcWaitNs = 2000000000ull;
-// output kinds of the programmed epilogue (mode 3)
-constexpr int kTcOutT = 0, kTcOutNegT = 1, kTcOutF = 2, kTcOutAmp = 3, kTcOutAcro = 4, kTcOutEss = 5;
 
 // designs per thread in the beta drain: 16 (32-design tiles, N = 256) or 8
 // (16-design tiles, N = 128); kmax > 5 always uses 8

@@ -215,6 +215,15 @@ class PermutationEngine:
     def _tmaps_of(self, perms):
         """t maps [P][C][V] of the permutation index rows."""
         P = perms.shape[0]
+        if self._program_on_device():
+            tc, out = self._tc, self._tbuf[:P]
+            base, _ = self._base()
+            rows = dev(self._index_rows(perms))
+            pt, u, x, invd, dof, wmat = tc.form_residual_designs(base, rows, P, self.k, self._centred, self._coef,
+                                                                 self.C, self._w_stride)
+            tc.stat(3, pt, u, x, invd, dof, P, self.k, self._coef, self.C, out, self.V, wmat=wmat,
+                    centred=self._centred)
+            return out
         if not self._graph_qf() or len(self.contrasts) > 8:
             return self.tmaps(self._designs(perms))
         tc, out = self._tc, self._tbuf[:P]
@@ -318,6 +327,12 @@ class PermutationEngine:
         tc = self._tc
         return (tc is not None and self.outputs is None and self._centred and tc.quadratic_form
                 and tc.yy is not None and 2 <= self.k <= 8 and min(self.contrasts) >= 1)
+
+    def _program_on_device(self):
+        """Whether a batch's designs of an output program are formed on the
+        device: rows of the design [1, pred_x] itself, permuted."""
+        return (self._tc is not None and self.outputs is not None and 2 <= self.k <= 8
+                and type(self)._designs is PermutationEngine._designs and bool(np.all(self.X[:, 0] == 1.0)))
 
     def _graph_form(self):
         """What a captured batch depends on: its size, the GLM's form and, with
