@@ -41,67 +41,118 @@ struct DesignArgs {
   int32_t* err;
 };
 
-__device__ inline double block_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  v = 0.0;
-  for (int w = 0; w < kDesignThreads / 32; ++w) v += red[w];
-  return v;
-}
+constexpr int kDesignSums = kDesignCols * (kDesignCols + 1) / 2;
 
 struct DesignShared {
-  double red[kDesignThreads / 32];
   double mean[kDesignCols], gram[kDesignCols][2 * kDesignCols];
+  double part[kDesignSums][kDesignThreads];  // the threads' sums
 };
 
-// Means and centred cross products of the columns entry(s, 0 .. kc).
+// Sum q of the threads' n_sums sums, in the first of each four threads.
+__device__ inline double gather_sums(const DesignShared& S, int n_sums) {
+  const int q = threadIdx.x >> 2, i0 = threadIdx.x & 3;
+  double v = 0.0;
+  if (q < n_sums)
+    for (int i = i0; i < kDesignThreads; i += 4) v += S.part[q][i];
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
+// Means and centred cross products of the columns entry(s, 0 .. kc), each all
+// at once: sum by sum, their 14 reductions (5 columns) took most of a design's
+// time.
 template <typename Entry>
 __device__ void centred_products(const Entry& entry, int kc, int n, DesignShared& S) {
+  static_assert(4 * kDesignSums <= kDesignThreads, "four threads add a sum up");
   const int tid = threadIdx.x;
-  for (int j = 0; j < kc; ++j) {
-    double s = 0.0;
-    for (int i = tid; i < n; i += kDesignThreads) s += entry(i, j);
-    s = block_sum(s, S.red);
-    if (tid == 0) S.mean[j] = s / n;
-  }
+  double sum[kDesignSums] = {};
+  for (int i = tid; i < n; i += kDesignThreads)
+#pragma unroll
+    for (int j = 0; j < kDesignCols; ++j)
+      if (j < kc) sum[j] += entry(i, j);
+#pragma unroll
+  for (int j = 0; j < kDesignCols; ++j)
+    if (j < kc) S.part[j][tid] = sum[j];
   __syncthreads();
-  for (int j = 0; j < kc; ++j)
-    for (int l = j; l < kc; ++l) {
-      double s = 0.0;
-      for (int i = tid; i < n; i += kDesignThreads) s += (entry(i, j) - S.mean[j]) * (entry(i, l) - S.mean[l]);
-      s = block_sum(s, S.red);
-      if (tid == 0) S.gram[j][l] = S.gram[l][j] = s;
-    }
+  const double total = gather_sums(S, kc);
+  if (tid % 4 == 0 && tid / 4 < kc) S.mean[tid / 4] = total / n;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kDesignSums; ++q) sum[q] = 0.0;
+  for (int i = tid; i < n; i += kDesignThreads) {
+    double c[kDesignCols];
+#pragma unroll
+    for (int j = 0; j < kDesignCols; ++j)
+      if (j < kc) c[j] = entry(i, j) - S.mean[j];
+#pragma unroll
+    for (int j = 0; j < kDesignCols; ++j)
+#pragma unroll
+      for (int l = 0; l <= j; ++l)
+        if (j < kc) sum[j * (j + 1) / 2 + l] += c[j] * c[l];
+  }
+#pragma unroll
+  for (int j = 0; j < kDesignCols; ++j)
+#pragma unroll
+    for (int l = 0; l <= j; ++l)
+      if (j < kc) S.part[j * (j + 1) / 2 + l][tid] = sum[j * (j + 1) / 2 + l];
+  __syncthreads();
+  const double product = gather_sums(S, kc * (kc + 1) / 2);
+  const int q = tid / 4;
+  if (tid % 4 == 0 && q < kc * (kc + 1) / 2) {
+    int j = 0;
+    while ((j + 1) * (j + 2) / 2 <= q) ++j;
+    const int l = q - j * (j + 1) / 2;
+    S.gram[j][l] = S.gram[l][j] = product;
+  }
   __syncthreads();
 }
 
 // Inverse of the w x w block at the left of g's rows of `ld` into the block
-// beside it, by Gauss-Jordan with row pivots (one thread).
+// beside it, by Gauss-Jordan with row pivots.  One warp, a lane per column.
 __device__ void invert(double* g, int ld, int w, int32_t* err) {
-  for (int j = 0; j < w; ++j)
-    for (int l = 0; l < w; ++l) g[j * ld + w + l] = (j == l) ? 1.0 : 0.0;
-  for (int j = 0; j < w; ++j) {
-    int p = j;
-    for (int r = j + 1; r < w; ++r)
-      if (fabs(g[r * ld + j]) > fabs(g[p * ld + j])) p = r;
-    if (p != j)
-      for (int l = 0; l < 2 * w; ++l) {
-        const double t = g[j * ld + l];
-        g[j * ld + l] = g[p * ld + l];
-        g[p * ld + l] = t;
-      }
-    const double pivot = g[j * ld + j];  // divided, so that equal columns leave an exact zero
-    if (pivot == 0.0) atomicCAS(err, 0, kDevSingular);
-    for (int l = 0; l < 2 * w; ++l) g[j * ld + l] = g[j * ld + l] / pivot;
-    for (int r = 0; r < w; ++r) {
-      if (r == j) continue;
-      const double f = g[r * ld + j];
-      if (f != 0.0)
-        for (int l = 0; l < 2 * w; ++l) g[r * ld + l] = fma(-f, g[j * ld + l], g[r * ld + l]);
-    }
+  constexpr int kMost = kDesignCols + 1;
+  const int lane = threadIdx.x & 31;
+  double c[kMost];
+#pragma unroll
+  for (int r = 0; r < kMost; ++r) {
+    c[r] = 0.0;
+    if (r < w && lane < w) c[r] = g[r * ld + lane];
+    else if (r < w && lane == w + r) c[r] = 1.0;
   }
+#pragma unroll
+  for (int j = 0; j < kMost; ++j) {
+    if (j >= w) break;
+    double f[kMost];  // the pivot's column
+#pragma unroll
+    for (int r = 0; r < kMost; ++r) f[r] = __shfl_sync(0xffffffffu, c[r], j);
+    int p = j;
+    double top = fabs(f[j]);
+#pragma unroll
+    for (int r = j + 1; r < kMost; ++r)
+      if (r < w && fabs(f[r]) > top) {
+        p = r;
+        top = fabs(f[r]);
+      }
+#pragma unroll
+    for (int r = j + 1; r < kMost; ++r)
+      if (r == p) {
+        const double x = c[j], y = f[j];
+        c[j] = c[r];
+        c[r] = x;
+        f[j] = f[r];
+        f[r] = y;
+      }
+    if (f[j] == 0.0 && lane == 0) atomicCAS(err, 0, kDevSingular);
+    c[j] = c[j] / f[j];  // divided, so that equal columns leave an exact zero
+#pragma unroll
+    for (int r = 0; r < kMost; ++r)
+      if (r != j && f[r] != 0.0) c[r] = fma(-f[r], c[j], c[r]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < kMost; ++r)
+    if (r < w && lane >= w && lane < 2 * w) g[r * ld + lane] = c[r];
+  __syncwarp();
 }
 
 __global__ void __launch_bounds__(kDesignThreads) design_kernel(DesignArgs a) {
@@ -130,14 +181,17 @@ __global__ void __launch_bounds__(kDesignThreads) design_kernel(DesignArgs a) {
   };
   if (live) centred_products(entry, kc, a.n, S);
   // a missing column keeps a zero row and column
-  if (tid == 0 && live) {
-    int k = 1;
-    for (int j = 0; j < kc; ++j) {
-      if (sCol[j] >= 0) ++k;
-      else gram[j][j] = 1.0;
+  if (tid < 32 && live) {
+    if (tid == 0) {
+      int k = 1;
+      for (int j = 0; j < kc; ++j) {
+        if (sCol[j] >= 0) ++k;
+        else gram[j][j] = 1.0;
+      }
+      a.dof[d] = static_cast<float>(a.n - k);
     }
+    __syncwarp();
     invert(&gram[0][0], 2 * kDesignCols, kc, a.err);
-    a.dof[d] = static_cast<float>(a.n - k);
   }
   // the split-BF16 tiles of glm_tile_split: 256-row blocks, 16-column steps of
   // [hi|lo][8-column block][row][8]
@@ -176,7 +230,7 @@ __global__ void __launch_bounds__(kDesignThreads) design_kernel(DesignArgs a) {
 // pseudoinverse rows, their sums, the negated design rows, inv(X'X)'s diagonal
 // and the weights of an output program.  The host formed and uploaded them
 // batch by batch: 1.1 of the 1.9 ms that 32 permutations of a rhythm model
-// over 82k vertices took; this takes 51 us.
+// over 82k vertices took; this takes 47 us.
 struct ResidualDesignArgs {
   const double* base;   // [n][ld]
   int64_t ld;
@@ -213,20 +267,24 @@ __global__ void __launch_bounds__(kDesignThreads) residual_design_kernel(Residua
   };
   if (live) {
     centred_products(entry, kc, a.n, S);
-    if (tid == 0) {
+    if (tid < 32) {
       invert(&S.gram[0][0], 2 * kDesignCols, kc, a.err);
-      double m0 = 1.0 / a.n;
-      for (int j = 0; j < kc; ++j) {
+      if (tid < kc) {
         double gm = 0.0;
         for (int l = 0; l < kc; ++l) {
-          full[j + 1][l + 1] = S.gram[j][kc + l];
-          gm = fma(S.gram[j][kc + l], S.mean[l], gm);
+          full[tid + 1][l + 1] = S.gram[tid][kc + l];
+          gm = fma(S.gram[tid][kc + l], S.mean[l], gm);
         }
-        full[0][j + 1] = full[j + 1][0] = -gm;
-        m0 = fma(S.mean[j], gm, m0);
+        full[0][tid + 1] = full[tid + 1][0] = -gm;
       }
-      full[0][0] = m0;
-      a.dof[d] = static_cast<float>(a.n - kmax);
+      __syncwarp();
+      if (tid == 0) {
+        double m0 = 1.0 / a.n;
+        for (int j = 0; j < kc; ++j) m0 = fma(-S.mean[j], full[0][j + 1], m0);
+        full[0][0] = m0;
+        a.dof[d] = static_cast<float>(a.n - kmax);
+      }
+      __syncwarp();
       float* w = a.weights + (int64_t)d * a.w_stride;
       for (int t = 0; t < a.n_rows; ++t) {
         const int kind = a.program[4 * t], j = a.program[4 * t + 1], width = a.program[4 * t + 2], o = a.program[4 * t + 3];
@@ -236,26 +294,22 @@ __global__ void __launch_bounds__(kDesignThreads) residual_design_kernel(Residua
         if (o < 0 || width < 1 || width > kAll || o + size > a.w_stride) continue;
         const bool inside = j >= 0 && j + width <= kmax;  // else the GLM returns NaN for the row
         if (inside && block_row) {
-          for (int p = 0; p < width; ++p)
-            for (int q = 0; q < width; ++q) block[p][q] = full[j + p][j + q];
+          for (int e = tid; e < size; e += 32) block[e / width][e % width] = full[j + e / width][j + e % width];
+          __syncwarp();
           invert(&block[0][0], 2 * kAll, width, a.err);
-          for (int p = 0; p < width; ++p)
-            for (int q = 0; q < width; ++q) w[o + p * width + q] = static_cast<float>(block[p][width + q]);
-        } else if (inside) {
-          w[o] = static_cast<float>(full[j][j]);
-          w[o + 1] = static_cast<float>(full[j][j + 1]);
-          w[o + 2] = static_cast<float>(full[j + 1][j + 1]);
+          for (int e = tid; e < size; e += 32) w[o + e] = static_cast<float>(block[e / width][width + e % width]);
+          __syncwarp();
         } else {
-          for (int e = 0; e < size; ++e) w[o + e] = 0.0f;
+          for (int e = tid; e < size; e += 32) w[o + e] = inside ? static_cast<float>(full[j + e / 2][j + (e + 1) / 2]) : 0.0f;
         }
       }
     }
     __syncthreads();
   }
-  // pseudoinverse entry (row j, subject s): inv(X'X) (1, x_s)'
+  // pseudoinverse entry (row j, subject s)
   auto pinv = [&](int j, int s) {
-    double v = full[j][0];
-    for (int l = 0; l < kc; ++l) v = fma(full[j][l + 1], entry(s, l), v);
+    double v = j == 0 ? 1.0 / a.n : 0.0;
+    for (int l = 0; l < kc; ++l) v = fma(full[j][l + 1], entry(s, l) - S.mean[l], v);
     return v;
   };
   const int rb = a.DB * 8, ks_count = a.n_pad / 16;
