@@ -787,6 +787,15 @@ struct StateArray {
       asm volatile("atom.relaxed.cta.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(glob(i)), "r"(v) : "memory");
     return old;
   }
+  // old, or `none` where `on` is false (a predicate, not a branch)
+  __device__ uint32_t add_if(bool on, uint32_t i, uint32_t v, uint32_t none) const {
+    uint32_t old = none;
+    if constexpr (kShared)
+      asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %3, 0;\n@p atom.relaxed.cta.shared.add.u32 %0, [%1], %2;\n}"
+                   : "+r"(old) : "r"(at(i)), "r"(v), "r"(static_cast<uint32_t>(on)) : "memory");
+    else if (on) old = add(i, v);
+    return old;
+  }
   __device__ void max_with(uint32_t i, uint32_t v) const {
     if constexpr (kShared) asm volatile("red.relaxed.cta.shared.max.u32 [%0], %1;" ::"r"(at(i)), "r"(v) : "memory");
     else asm volatile("red.relaxed.cta.global.max.u32 [%0], %1;" ::"l"(glob(i)), "r"(v) : "memory");
@@ -838,19 +847,25 @@ __device__ inline void hop(const Words& word, uint32_t& x, uint32_t& w) {
   w = up;
 }
 
-// The same for two walks of which at least one goes on, their loads together.
+// Roots of x and y, whose words are wx and wy, a hop of both at a time; kHalve
+// points x and y themselves to them (halving the path at each hop instead made
+// a hop 130 cycles of a lone warp, half of which are this: with the predicated
+// adds below 2.92 -> 2.72 ms for 2 x 1024 items of an L7 surface).
 template <bool kHalve, typename Words>
-__device__ inline void hop_two(const Words& word, uint32_t& x, uint32_t& wx, uint32_t& y, uint32_t& wy) {
-  const bool up_x = !(wx & kRoot), up_y = !(wy & kRoot);
-  uint32_t ux = wx, uy = wy;
-  if (up_x) ux = word.ld(wx);
-  if (up_y) uy = word.ld(wy);
-  if (kHalve && up_x && !(ux & kRoot)) word.st(x, ux);
-  if (kHalve && up_y && !(uy & kRoot)) word.st(y, uy);
-  if (up_x) x = wx;
-  if (up_y) y = wy;
-  wx = ux;
-  wy = uy;
+__device__ inline void find_two(const Words& word, uint32_t& x, uint32_t& wx, uint32_t& y, uint32_t& wy) {
+  const uint32_t x0 = x, y0 = y, x1 = wx, y1 = wy;
+  while (!(wx & wy & kRoot)) {
+    if (!(wx & kRoot)) {
+      x = wx;
+      wx = word.ld(x);
+    }
+    if (!(wy & kRoot)) {
+      y = wy;
+      wy = word.ld(y);
+    }
+  }
+  if (kHalve && !(x1 & kRoot) && x != x1) word.st(x0, x);
+  if (kHalve && !(y1 & kRoot) && y != y1) word.st(y0, y);
 }
 
 // Root of x, and its word.
@@ -864,6 +879,20 @@ template <bool kHalve, typename Words>
 __device__ inline uint32_t find_basin(const Words& word, uint32_t x) {
   uint32_t w;
   return find_basin<kHalve>(word, x, w);
+}
+
+__device__ inline int add_shared(uint32_t at, int v) {
+  int old;
+  asm volatile("atom.relaxed.cta.shared.add.s32 %0, [%1], %2;" : "=r"(old) : "r"(at), "r"(v) : "memory");
+  return old;
+}
+__device__ inline int load_shared(uint32_t at) {
+  int v;
+  asm volatile("ld.relaxed.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+  return v;
+}
+__device__ inline void store_shared(uint32_t at, int v) {
+  asm volatile("st.relaxed.cta.shared.s32 [%0], %1;" ::"r"(at), "r"(v) : "memory");
 }
 
 struct SweepShared {
@@ -946,7 +975,7 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
   }
   // the list of live basins, the other one, and their counters and a spare one
   auto live = st.list0, other = st.list1;
-  int *n_live = &S.n_live[0], *n_next = &S.n_live[1], *n_spare = &S.n_live[2];
+  uint32_t n_live = static_cast<uint32_t>(__cvta_generic_to_shared(&S.n_live[0])), n_next = n_live + 4, n_spare = n_live + 8;
 
   for (int i = 0; i < L; ++i) {
     Two my_ev[kAhead];
@@ -984,8 +1013,8 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
             py = st.word.ld(y);
           }
           for (int it = 0; it < kFindLimit; ++it) {
-            // both walks a hop at a time, their loads together
-            while (__any_sync(0xffffffffu, !(px & py & kRoot))) hop_two<kHalve>(st.word, x, px, y, py);
+            find_two<kHalve>(st.word, x, px, y, py);
+            __syncwarp();
             open = open && x != y;
             if (open) {
               const uint32_t ax = px >> 24, ay = py >> 24;
@@ -1061,7 +1090,7 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
           uint32_t wx = kRoot, wy = kRoot;
           if (on_x) wx = st.word.ld(x);
           if (on_y) wy = st.word.ld(y);
-          while (!(wx & wy & kRoot)) hop_two<kHalve>(st.word, x, wx, y, wy);
+          find_two<kHalve>(st.word, x, wx, y, wy);
         }
         if constexpr (kMode == kNodes) {
           if (on_x) a.vnode[eo + p - shift] = i * nb + x;
@@ -1072,14 +1101,13 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
         const uint32_t r0 = __shfl_sync(0xffffffffu, x, 0);
         const unsigned sx = __ballot_sync(0xffffffffu, on_x && x == r0), sy = __ballot_sync(0xffffffffu, on_y && y == r0);
         const bool leads = lane == __ffs(sx | sy) - 1;
-        uint32_t was_x = kExtent, was_y = kExtent, was_0 = kExtent;
-        if (leads) was_0 = st.word.add(r0, __popc(sx) + __popc(sy));
-        if (on_x && x != r0) was_x = st.word.add(x, 1u);
-        if (on_y && y != r0) was_y = st.word.add(y, 1u);
+        const uint32_t was_0 = st.word.add_if(leads, r0, __popc(sx) + __popc(sy), kExtent);
+        const uint32_t was_x = st.word.add_if(on_x && x != r0, x, 1u, kExtent);
+        const uint32_t was_y = st.word.add_if(on_y && y != r0, y, 1u, kExtent);
         // a component's first vertices: it goes live, with its age
         const bool new_0 = !(was_0 & kExtent), new_x = !(was_x & kExtent), new_y = !(was_y & kExtent);
         if (new_0 || new_x || new_y) {
-          int at = atomicAdd(n_live, int(new_0) + int(new_x) + int(new_y));
+          int at = add_shared(n_live, int(new_0) + int(new_x) + int(new_y));
           const uint32_t age = static_cast<uint32_t>(kMaxSteps - 1 - i) << 24;
           if (new_0) {
             live.st(at++, r0);
@@ -1106,7 +1134,7 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
     // (3) every live component adds its increment.  Linked ones drop out of
     // the list when it is packed, every eighth step.
     const float HH = S.HH[i];
-    const int n = *n_live;
+    const int n = load_shared(n_live);
     const bool pack = (i & 7) == 7;
     // (float)(extent^E * HH): one double product, one rounding
     // (fast_tfce.hpp:77); for E == 1 the double product of an integer below
@@ -1150,18 +1178,18 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
         }
         const unsigned m = __ballot_sync(0xffffffffu, root);
         int at = 0;
-        if (lane == 0 && m) at = atomicAdd(n_next, __popc(m));
+        if (lane == 0 && m) at = add_shared(n_next, __popc(m));
         at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
         if (root) other.st(at, c);
       }
     }
-    if (tid == 0 && pack) *n_spare = 0;  // the list before this one's: read before the last barrier
+    if (tid == 0 && pack) store_shared(n_spare, 0);  // the list before this one's: read before the last barrier
     __syncthreads();
     if (pack) {
       auto l = live;
       live = other;
       other = l;
-      int* c = n_live;
+      const uint32_t c = n_live;
       n_live = n_next;
       n_next = n_spare;
       n_spare = c;
@@ -1179,7 +1207,7 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
   float best = (L == 0 || S.ev[L] - S.ev[0] < Vs) ? __fmul_rn(0.0f, scale) : -INFINITY;
   if (Vs == 0) best = -INFINITY;
   if constexpr (kMode == kMaxima) {
-    const int n = *n_live;
+    const int n = load_shared(n_live);
     for (int q = tid; q < n; q += nth) best = fmaxf(best, __fmul_rn(__uint_as_float(st.w.ld(live.ld(q))), scale));
   }
   if constexpr (kMode == kPotential) {
