@@ -105,11 +105,12 @@ int tfce_adjset_set_threshold_groups(tfce_adjset* h, const int32_t* group);
  *      increment to a float accumulator at every threshold
  *      (fast_tfce.hpp:72-84), so results are bit-identical to the reference
  *      up to its libm's powf rounding (the default);
- *   1  per-component: each live component adds its increment once per
- *      threshold in double, and a vertex's value is resolved at the end along
- *      the chain of components it joined; the value is the float rounding of
- *      the exact sum of the same float increments, i.e. it differs from the
- *      reference by the reference's own float summation error (~1e-7 rel).
+ *   1  per-component: a component's sum is kept in double and brought up to a
+ *      threshold where its extent changes, and a vertex's value is resolved at
+ *      the end along the chain of components it joined; the value is the float
+ *      rounding of the double sum of extent^E * HH, i.e. it differs from the
+ *      reference by the reference's own float rounding of the increments and
+ *      their sum (~1e-7 rel).
  *   2  as 1, and maxima-only launches keep the potentials and resolve every
  *      vertex as well (for comparisons).
  * With 0 and 1 a launch that asks only for maxima (out_maps NULL) without

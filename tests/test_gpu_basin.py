@@ -149,3 +149,35 @@ def test_launches_of_three_sizes_at_once(weighted):
                     np.testing.assert_allclose(mx[:, k, s], want[pick], rtol=1e-5)
                 else:
                     np.testing.assert_array_equal(mx[:, k, s], want[pick])
+
+
+@pytest.mark.parametrize("E,H", [(1.0, 2.0), (0.5, 2.0), (2.0, 1.0), (0.0, 2.0), (1.0, 0.5)])
+def test_potentials_keep_the_precision_of_small_values(E, H):
+    """Weighted maps through the potentials against the oracle's float sums: a
+    value from single steps, far below the map's maximum, comes out as precise as
+    the double sum of its component allows (2^-53 of the largest, times the
+    steps)."""
+    rng = np.random.default_rng(3)
+    V = 6000
+    off, idx = _graph("ring", V, rng)
+    x = rng.standard_normal((1, V)).astype(np.float32)
+    x[0, :40] = 30.0 + np.arange(40)
+    adj = A.AdjacencySet((off, idx), H, E)
+    vd = np.ones(V, np.float32)
+    mx, om = _sweep(adj, x, 1, "component", vd, want_maps=True)
+    img = np.maximum(x[0], 0)
+    want = oracle.tfce(off, idx, img, H, E, hh_exact=True) * np.float32(img.max() / np.float32(100.0))
+    np.testing.assert_allclose(om[0, 0], want, rtol=1e-5, atol=200 * 2.0 ** -53 * want.max())
+    np.testing.assert_allclose(mx[0, 0, 0], want.max(), rtol=1e-5)
+
+
+def test_overflowing_thresholds_stay_infinite():
+    """Statistics whose squared thresholds leave float32: infinite where the sum
+    is, in the potentials too."""
+    V = 300
+    off, idx = _graph("ring", V, np.random.default_rng(0))
+    x = np.full((1, V), 1.0, np.float32)
+    x[0, 10:20] = 1e20
+    adj = A.AdjacencySet((off, idx), 2.0, 1.0)
+    mx, om = _sweep(adj, x, 1, "component", np.ones(V, np.float32), want_maps=True)
+    assert np.isinf(mx[0, 0, 0]) and np.isinf(om[0, 0, 10:20]).all()

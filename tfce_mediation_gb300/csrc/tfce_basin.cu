@@ -58,7 +58,7 @@ constexpr int kCrossChunk = kCrossThreads * kCrossPer;
 constexpr int kMaxSweepThreads = 1024;
 constexpr int kTileEntries = 120000;   // list entries per tile: pairs are counted in 16 bits
 constexpr int kSmBytes = 226 * 1024;   // shared memory of an SM's sweeps together
-constexpr int kSweepBytes = 3328;      // of a sweep besides its state
+constexpr int kSweepBytes = 4352;      // of a sweep besides its state
 constexpr int kFindLimit = 1 << 26;
 constexpr int kAhead = 4;              // pairs of events that a thread of the sweep loads a step ahead
 constexpr uint32_t kNone = 0xffffffffu;
@@ -820,9 +820,9 @@ struct BasinState {
   static constexpr bool kShared = kKind != kAllGlobal;
   using W = typename std::conditional<kMode == kPotential, double, uint32_t>::type;
   using Idx = typename std::conditional<kShared, uint16_t, uint32_t>::type;
-  StateArray<kShared, W> w;  // maxima: largest float sum (bits); potentials: sum, or offset to the parent
+  StateArray<kShared, W> w;  // maxima: largest float sum (bits); potentials: sum before step `last`, or offset to the parent
   StateArray<kShared, uint32_t> word;
-  StateArray<kKind == kAllShared, Idx> list0;  // live basins; they are packed from one list to the other
+  StateArray<kKind == kAllShared, Idx> list0;  // potentials: a root's `last`; else live basins; they are packed from one list to the other
   StateArray<kKind == kAllShared, Idx> list1;
   __device__ BasinState(char* smem, char* global, uint32_t n) {
     if constexpr (kShared) w.base = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
@@ -834,7 +834,7 @@ struct BasinState {
   }
 };
 constexpr int state_bytes_per_basin(int mode, int kind) {
-  return (mode == kPotential ? 8 : 4) + 4 + (kind == kAllShared ? 4 : kind == kAllGlobal ? 8 : 0);
+  return (mode == kPotential ? 12 : 8) + (kind == kListsGlobal ? 0 : (mode == kPotential ? 1 : 2) * (kind == kAllGlobal ? 4 : 2));
 }
 
 // One hop of a walk from x, whose word is w (not a root's); kHalve points x to
@@ -895,10 +895,56 @@ __device__ inline void store_shared(uint32_t at, int v) {
   asm volatile("st.relaxed.cta.shared.s32 [%0], %1;" ::"r"(at), "r"(v) : "memory");
 }
 
+// Potentials.  A component that keeps its extent from step a to step b gains
+// extent^E * (HH_a + .. + HH_b-1), so a root's sum is brought up to a step only
+// where its extent changes: it holds the sum before step `last`, and what it
+// gained since follows from the sums of HH from a step to the end (small to
+// large, so that late steps keep their precision).  Adding every live
+// component's increment at every step, in double, took 5,000 of a step's 8,200
+// cycles (6k basins, unsmoothed): two additions or conversions per SM and cycle.
+// 256 such items: 654 -> 363 us.
+__device__ inline double brought_up(double sum, const double* pw, const float* HH, const double* rest, uint32_t word,
+                                    int from, int to) {
+  const uint32_t ext = word & kExtent;
+  if (ext == 0u || from == to) return sum;
+  // an extent as a double, by way of a float, off the double pipe
+  const uint32_t u = __float_as_uint(static_cast<float>(ext));
+  const double power = pw ? pw[ext] : __hiloint2double(static_cast<int>((u >> 3) + 0x38000000u), static_cast<int>(u << 29));
+  double gain = rest[from] - rest[to];
+  if (!isfinite(rest[from])) {  // a threshold whose power overflows: added up as it comes
+    gain = 0.0;
+    for (int i = from; i < to; ++i) gain += static_cast<double>(HH[i]);
+  }
+  return fma(power, gain, sum);
+}
+
+// rest[i] of a table of L steps, by one warp.
+__device__ inline void sum_rest(const float* HH, int L, double* rest) {
+  constexpr int kPer = kMaxSteps / 32;
+  const int lane = threadIdx.x & 31;
+  double sum[kPer], later = 0.0;
+#pragma unroll
+  for (int k = kPer - 1; k >= 0; --k) {
+    const int i = lane * kPer + k;
+    later += i < L ? static_cast<double>(HH[i]) : 0.0;
+    sum[k] = later;
+  }
+  double mine = later;  // of this lane's steps and all later ones
+  for (int o = 1; o < 32; o <<= 1) {
+    const double v = __shfl_down_sync(0xffffffffu, mine, o);
+    if (lane + o < 32) mine += v;
+  }
+  const double beyond = __shfl_down_sync(0xffffffffu, mine, 1);
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) rest[lane * kPer + k] = sum[k] + (lane < 31 ? beyond : 0.0);
+  if (lane == 31) rest[kMaxSteps] = 0.0;
+}
+
 struct SweepShared {
   float T[kMaxSteps], HH[kMaxSteps];
   int ev[kMaxSteps + 1], pair[kMaxSteps + 1];  // first entries of the steps
   float red[32];
+  double rest[kMaxSteps + 1];  // potentials: sum of HH from a step to the last
   int L, item, n_basins;
   int n_live[3];  // by packs modulo 3: the list's, the packed one's, and one being cleared
 };
@@ -955,7 +1001,9 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
   for (int i = tid; i < nb; i += nth) {
     st.word.st(i, kRoot);
     st.w.st(i, 0);
+    if constexpr (kMode == kPotential) st.list0.st(i, 0);
   }
+  if (kMode == kPotential && tid < 32) sum_rest(S.HH, L, S.rest);
   if (tid == 0) S.n_live[0] = S.n_live[1] = S.n_live[2] = 0;
   __syncthreads();
   Node* nodes = (kMode == kNodes) ? a.nodes + item * a.node_cap : nullptr;
@@ -975,6 +1023,11 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
   }
   // the list of live basins, the other one, and their counters and a spare one
   auto live = st.list0, other = st.list1;
+  // potential of root r, whose word is given, before step i
+  auto potential = [&](uint32_t r, uint32_t word, int i) -> double {
+    if constexpr (kMode == kPotential) return brought_up(st.w.ld(r), pw, S.HH, S.rest, word, st.list0.ld(r), i);
+    return 0.0;
+  };
   uint32_t n_live = static_cast<uint32_t>(__cvta_generic_to_shared(&S.n_live[0])), n_next = n_live + 4, n_spare = n_live + 8;
 
   for (int i = 0; i < L; ++i) {
@@ -1038,11 +1091,19 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
         }
         __syncthreads();
         if constexpr (kMode == kPotential) {
+          uint32_t r = 0, was_r = 0;
+          double sum_r = 0.0;
           if (linked) {
-            const uint32_t r = find_basin<kHalve>(st.word, low);
-            if (ext) st.word.add(r, ext);
-            st.w.st(low, st.w.ld(low) - st.w.ld(r));
+            r = find_basin<kHalve>(st.word, low, was_r);
+            sum_r = potential(r, was_r, i);
+            st.w.st(low, potential(low, ext, i) - sum_r);
             st.word.st(low, r);
+          }
+          __syncthreads();
+          // the first to change r's extent brings its sum up to this step
+          if (linked && ext && st.word.add(r, ext) == was_r) {
+            st.w.st(r, sum_r);
+            st.list0.st(r, i);
           }
           __syncthreads();  // vertices climb by these
         } else {
@@ -1075,17 +1136,21 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
         const uint2 two = split(t);
         uint32_t x = two.x, y = two.y;
         const bool on_x = p >= ev0 && p < ev_end, on_y = p + 1 >= ev0 && p + 1 < ev_end;
+        uint32_t root_x = kRoot, root_y = kRoot;  // potentials: the roots' words and sums
+        double sum_x = 0.0, sum_y = 0.0;
         if constexpr (kMode == kPotential) {
-          auto climb = [&](uint32_t& r, int q) {
-            double sum = st.w.ld(r);
-            for (uint32_t up = st.word.ld(r); !(up & kRoot); up = st.word.ld(r)) {
-              r = up;
+          auto climb = [&](uint32_t& r, uint32_t& word, double& now, int q) {
+            double sum = 0.0;
+            for (word = st.word.ld(r); !(word & kRoot); word = st.word.ld(r)) {
               sum += st.w.ld(r);
+              r = word;
             }
-            a.base[eo + q - shift] = sum;
+            now = potential(r, word, i);
+            a.base[eo + q - shift] = sum + now;
           };
-          if (on_x) climb(x, p);
-          if (on_y) climb(y, p + 1);
+          if (on_x) climb(x, root_x, sum_x, p);
+          if (on_y) climb(y, root_y, sum_y, p + 1);
+          __syncthreads();
         } else {
           uint32_t wx = kRoot, wy = kRoot;
           if (on_x) wx = st.word.ld(x);
@@ -1106,7 +1171,19 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
         const uint32_t was_y = st.word.add_if(on_y && y != r0, y, 1u, kExtent);
         // a component's first vertices: it goes live, with its age
         const bool new_0 = !(was_0 & kExtent), new_x = !(was_x & kExtent), new_y = !(was_y & kExtent);
-        if (new_0 || new_x || new_y) {
+        if constexpr (kMode == kPotential) {
+          // the first to change a root's extent brings its sum up to this step
+          auto renew = [&](uint32_t r, uint32_t was, double sum) {
+            st.w.st(r, sum);
+            st.list0.st(r, i);
+            if (!(was & kExtent)) st.word.add(r, static_cast<uint32_t>(kMaxSteps - 1 - i) << 24);
+          };
+          const bool by_x = on_x && x == r0;
+          if (leads && was_0 == (by_x ? root_x : root_y)) renew(r0, was_0, by_x ? sum_x : sum_y);
+          if (on_x && x != r0 && was_x == root_x) renew(x, was_x, sum_x);
+          if (on_y && y != r0 && was_y == root_y) renew(y, was_y, sum_y);
+          __syncthreads();
+        } else if (new_0 || new_x || new_y) {
           int at = add_shared(n_live, int(new_0) + int(new_x) + int(new_y));
           const uint32_t age = static_cast<uint32_t>(kMaxSteps - 1 - i) << 24;
           if (new_0) {
@@ -1124,75 +1201,77 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
         }
       };
       const int even = ev0 & ~1;
+      const int ahead = kMode == kPotential ? 0 : wbase;  // the potentials' rounds have barriers
 #pragma unroll
       for (int k = 0; k < kAhead; ++k)
-        if (even + 2 * (wbase + k * nth) < ev_end) count_two(even + 2 * (tid + k * nth), my_ev[k]);
-      for (int p0 = even + 2 * (wbase + kAhead * nth); p0 < ev_end; p0 += 2 * nth)
-        count_two(p0 + 2 * lane, load_two(p0 + 2 * lane, ev0, ev_end));
-      __syncthreads();
+        if (even + 2 * (ahead + k * nth) < ev_end) count_two(even + 2 * (tid + k * nth), my_ev[k]);
+      for (int p0 = even + 2 * kAhead * nth; p0 + 2 * ahead < ev_end; p0 += 2 * nth)
+        count_two(p0 + 2 * tid, load_two(p0 + 2 * tid, ev0, ev_end));
+      if (kMode != kPotential) __syncthreads();
     }
-    // (3) every live component adds its increment.  Linked ones drop out of
-    // the list when it is packed, every eighth step.
-    const float HH = S.HH[i];
-    const int n = load_shared(n_live);
-    const bool pack = (i & 7) == 7;
-    // (float)(extent^E * HH): one double product, one rounding
-    // (fast_tfce.hpp:77); for E == 1 the double product of an integer below
-    // 2^24 and a float is exact, so a float product rounds alike
-    auto increment = [&](uint32_t word) {
-      const uint32_t ext = word & kExtent;
-      return pw ? __double2float_rn(__dmul_rn(pw[ext], static_cast<double>(HH))) : __fmul_rn(static_cast<float>(ext), HH);
-    };
-    auto grow = [&](uint32_t c, float inc) {
-      if constexpr (kMode == kMaxima) st.w.st(c, __float_as_uint(__fadd_rn(__uint_as_float(st.w.ld(c)), inc)));
-      if constexpr (kMode == kPotential) st.w.st(c, st.w.ld(c) + static_cast<double>(inc));
-      if constexpr (kMode == kNodes) nodes[(int64_t)i * nb + c] = Node{inc, c};
-    };
-    // nodes: a component that was linked at this step leads on to the one that
-    // it is part of now (before, it led on to itself).  A node's place follows
-    // from its step and basin, so that vertices know theirs as they join (a
-    // pass of its own for them cost a quarter of the sweep: 414 -> 342 us)
-    auto lead_on = [&](uint32_t c) {
-      if constexpr (kMode == kNodes) {
-        if (i > 0) nodes[(int64_t)(i - 1) * nb + c].next = find_basin<kHalve>(st.word, c);
-      }
-    };
-    if (!pack) {
-      for (int q = tid; q < n; q += nth) {
-        const uint32_t c = live.ld(q);
-        const uint32_t word = st.word.ld(c);
-        if (word & kRoot) grow(c, increment(word));
-        else lead_on(c);
-      }
-    } else {
-      for (int q0 = wbase; q0 < n; q0 += nth) {
-        const int q = q0 + lane;
-        bool root = false;
-        uint32_t c = 0;
-        if (q < n) {
-          c = live.ld(q);
+    if constexpr (kMode != kPotential) {
+      // (3) every live component adds its increment.  Linked ones drop out of
+      // the list when it is packed, every eighth step.
+      const float HH = S.HH[i];
+      const int n = load_shared(n_live);
+      const bool pack = (i & 7) == 7;
+      // (float)(extent^E * HH): one double product, one rounding
+      // (fast_tfce.hpp:77); for E == 1 the double product of an integer below
+      // 2^24 and a float is exact, so a float product rounds alike
+      auto increment = [&](uint32_t word) {
+        const uint32_t ext = word & kExtent;
+        return pw ? __double2float_rn(__dmul_rn(pw[ext], static_cast<double>(HH))) : __fmul_rn(static_cast<float>(ext), HH);
+      };
+      auto grow = [&](uint32_t c, float inc) {
+        if constexpr (kMode == kMaxima) st.w.st(c, __float_as_uint(__fadd_rn(__uint_as_float(st.w.ld(c)), inc)));
+        if constexpr (kMode == kNodes) nodes[(int64_t)i * nb + c] = Node{inc, c};
+      };
+      // nodes: a component that was linked at this step leads on to the one that
+      // it is part of now (before, it led on to itself).  A node's place follows
+      // from its step and basin, so that vertices know theirs as they join (a
+      // pass of its own for them cost a quarter of the sweep: 414 -> 342 us)
+      auto lead_on = [&](uint32_t c) {
+        if constexpr (kMode == kNodes) {
+          if (i > 0) nodes[(int64_t)(i - 1) * nb + c].next = find_basin<kHalve>(st.word, c);
+        }
+      };
+      if (!pack) {
+        for (int q = tid; q < n; q += nth) {
+          const uint32_t c = live.ld(q);
           const uint32_t word = st.word.ld(c);
-          root = word & kRoot;
-          if (root) grow(c, increment(word));
+          if (word & kRoot) grow(c, increment(word));
           else lead_on(c);
         }
-        const unsigned m = __ballot_sync(0xffffffffu, root);
-        int at = 0;
-        if (lane == 0 && m) at = add_shared(n_next, __popc(m));
-        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
-        if (root) other.st(at, c);
+      } else {
+        for (int q0 = wbase; q0 < n; q0 += nth) {
+          const int q = q0 + lane;
+          bool root = false;
+          uint32_t c = 0;
+          if (q < n) {
+            c = live.ld(q);
+            const uint32_t word = st.word.ld(c);
+            root = word & kRoot;
+            if (root) grow(c, increment(word));
+            else lead_on(c);
+          }
+          const unsigned m = __ballot_sync(0xffffffffu, root);
+          int at = 0;
+          if (lane == 0 && m) at = add_shared(n_next, __popc(m));
+          at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+          if (root) other.st(at, c);
+        }
       }
-    }
-    if (tid == 0 && pack) store_shared(n_spare, 0);  // the list before this one's: read before the last barrier
-    __syncthreads();
-    if (pack) {
-      auto l = live;
-      live = other;
-      other = l;
-      const uint32_t c = n_live;
-      n_live = n_next;
-      n_next = n_spare;
-      n_spare = c;
+      if (tid == 0 && pack) store_shared(n_spare, 0);  // the list before this one's: read before the last barrier
+      __syncthreads();
+      if (pack) {
+        auto l = live;
+        live = other;
+        other = l;
+        const uint32_t c = n_live;
+        n_live = n_next;
+        n_next = n_spare;
+        n_spare = c;
+      }
     }
     ev0 = ev_end;
     ev_end = ev2;
@@ -1211,6 +1290,11 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
     for (int q = tid; q < n; q += nth) best = fmaxf(best, __fmul_rn(__uint_as_float(st.w.ld(live.ld(q))), scale));
   }
   if constexpr (kMode == kPotential) {
+    for (int r = tid; r < nb; r += nth) {
+      const uint32_t word = st.word.ld(r);
+      if (word & kRoot) st.w.st(r, potential(r, word, L));
+    }
+    __syncthreads();
     float* omap = a.out_maps ? a.out_maps + (map * a.signs + sgn) * a.n_vertices : nullptr;
     const int end = L ? S.ev[L] : 0;
     for (int q = S.ev[0] + tid; q < end; q += nth) {
