@@ -54,6 +54,8 @@ constexpr int kProbes = 12;            // slots tried
 constexpr int kQueue = 96;              // neighbours that wait in a warp's queue: 31 and two rows' worth
 constexpr int kCrossThreads = 256;
 constexpr int kCrossPer = 4;
+constexpr int kCrossRows = 4;           // rows of neighbours whose loads are in flight together
+constexpr int kCrossQueue = 64;         // 31 and a row's worth
 constexpr int kCrossChunk = kCrossThreads * kCrossPer;
 constexpr int kMaxSweepThreads = 1024;
 constexpr int kTileEntries = 120000;   // list entries per tile: pairs are counted in 16 bits
@@ -482,10 +484,15 @@ __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a
 
 // Pairs that cross a tile boundary, and one-way entries: every boundary vertex
 // with the distinct basins of its listed neighbours that precede it by value
-// (ties by smaller vertex, the reference's insertion order).
+// (ties by smaller vertex, the reference's insertion order).  Bound by
+// instructions on voxel graphs (97k boundary vertices a map, 13 rows each);
+// inserting row by row, with a few lanes each, 48 maps took 331 us, with full
+// rounds from a queue 247.
 __global__ void __launch_bounds__(kCrossThreads) basin_cross_kernel(BasinArgs a) {
   __shared__ int cnt[kBuckets], total;
   __shared__ unsigned long long table[kCrossTable];  // {tile << 12 | basin, twice} << 8 | 128 - step
+  // pairs wait in a queue of the warp until there are 32 for a full round
+  __shared__ unsigned long long sQueue[kCrossThreads / 32 * kCrossQueue];
   const int chunk = blockIdx.x % a.n_chunks;
   const int64_t map = blockIdx.x / a.n_chunks;
   const ChunkInfo ci = a.chunks[chunk];
@@ -504,51 +511,75 @@ __global__ void __launch_bounds__(kCrossThreads) basin_cross_kernel(BasinArgs a)
     out[atomicAdd(&total, 1)] = make_uint2(((i << 4) & 0x7fff0000u) | ((b >> 4) << 12) | (i & 0xfffu),
                                            ((j << 4) & 0x7fff0000u) | ((b & 15u) << 12) | (j & 0xfffu));
   };
-#pragma unroll
+  unsigned long long* const queue = sQueue + (tid >> 5) * kCrossQueue;
+  int nq = 0;
+  auto insert = [&](unsigned long long e) {
+    uint32_t h = static_cast<uint32_t>(((e >> 8) * 0x9e3779b97f4a7c15ull) >> 54);
+    static_assert(kCrossTable == 1 << 10, "the hash gives 10 bits");
+    for (int t = 0;; ++t) {
+      unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&table[h]);
+      if (cur == 0) cur = atomicCAS(&table[h], 0ull, e);
+      if (cur == 0 || (cur ^ e) < 256) {
+        if (cur != 0 && cur < e) atomicMax(&table[h], e);
+        break;
+      }
+      if (t == kProbes) {
+        emit(e);
+        break;
+      }
+      h = (h + 1) & (kCrossTable - 1);
+    }
+  };
   for (int k = 0; k < kCrossPer; ++k) {
     const int q = tid + k * kCrossThreads;
-    if (q >= ci.nbnd) break;
-    const uint2 me = rec[ci.bnd0 + q];
-    if (me.y == kNone) continue;
-    const int vme = a.bnd_vert[ci.bnd0 + q];
+    if (q - lane >= ci.nbnd) break;
+    const uint2 me = q < ci.nbnd ? rec[ci.bnd0 + q] : make_uint2(0u, kNone);
+    const bool active = me.y != kNone;
+    if (!__any_sync(0xffffffffu, active)) continue;
+    const int vme = active ? a.bnd_vert[ci.bnd0 + q] : 0;
     const uint32_t s = me.x & 0x80000000u;
-    const uint32_t mine = (static_cast<uint32_t>(a.bnd_tile[ci.bnd0 + q]) << 12) | (me.y & 0xfffu);
-    const int own = static_cast<int>(me.x ^ s);
+    const uint32_t mine = (static_cast<uint32_t>(active ? a.bnd_tile[ci.bnd0 + q] : 0) << 12) | (me.y & 0xfffu);
+    const int own = active ? static_cast<int>(me.x ^ s) : 0x7fffffff;
     const uint32_t code = kMaxSteps - (me.y >> 16);
     const int sl = ci.slice0 + (q >> 5);
     uint32_t last = mine;  // (a one-way entry may lead to the vertex's own basin, which is no pair)
     const uint32_t o1 = a.cross_off[sl + 1];
-#pragma unroll 4
-    for (uint32_t o = a.cross_off[sl] + lane; o < o1; o += 32) {
-      const uint32_t ub = a.cross[o];
-      const uint2 r = rec[ub];
-      const int w = static_cast<int>(r.x ^ s);
-      if (w > own || (w == own && a.bnd_vert[ub] < vme)) {
-        const uint32_t other = (static_cast<uint32_t>(a.bnd_tile[ub]) << 12) | (r.y & 0xfffu);
-        if (other != last && other != mine) {
-          last = other;
+    for (uint32_t o = a.cross_off[sl] + lane; o < o1; o += 32 * kCrossRows) {
+      uint32_t ub[kCrossRows];
+      uint2 r[kCrossRows];
+#pragma unroll
+      for (int j = 0; j < kCrossRows; ++j) ub[j] = o + 32 * j < o1 ? a.cross[o + 32 * j] : 0xffffffffu;
+#pragma unroll
+      for (int j = 0; j < kCrossRows; ++j) r[j] = ub[j] != 0xffffffffu ? rec[ub[j]] : make_uint2(s, kNone);
+#pragma unroll
+      for (int j = 0; j < kCrossRows; ++j) {
+        if (o - lane + 32 * j >= o1) break;
+        const int w = static_cast<int>(r[j].x ^ s);
+        bool hit = w > own || (w == own && active && a.bnd_vert[ub[j]] < vme);
+        uint32_t other = 0;
+        if (hit) {
+          other = (static_cast<uint32_t>(a.bnd_tile[ub[j]]) << 12) | (r[j].y & 0xfffu);
+          hit = other != last && other != mine;
+          if (hit) last = other;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (hit) {
           const unsigned long long pair =
               (static_cast<unsigned long long>(min(mine, other) | (s >> 4)) << 28) | max(mine, other);
-          const unsigned long long e = (pair << 8) | code;
-          uint32_t h = static_cast<uint32_t>((pair * 0x9e3779b97f4a7c15ull) >> 54);
-          static_assert(kCrossTable == 1 << 10, "the hash gives 10 bits");
-          for (int t = 0;; ++t) {
-            unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&table[h]);
-            if (cur == 0) cur = atomicCAS(&table[h], 0ull, e);
-            if (cur == 0 || (cur ^ e) < 256) {
-              if (cur != 0 && cur < e) atomicMax(&table[h], e);
-              break;
-            }
-            if (t == kProbes) {
-              emit(e);
-              break;
-            }
-            h = (h + 1) & (kCrossTable - 1);
-          }
+          queue[nq + __popc(m & ((1u << lane) - 1u))] = (pair << 8) | code;
+        }
+        nq += __popc(m);
+        if (nq >= 32) {
+          __syncwarp();
+          insert(queue[nq - 32 + lane]);
+          nq -= 32;
+          __syncwarp();
         }
       }
     }
   }
+  __syncwarp();
+  if (lane < nq) insert(queue[lane]);
   __syncthreads();
   for (int i = tid; i < kCrossTable; i += kCrossThreads)
     if (table[i]) emit(table[i]);
