@@ -163,8 +163,20 @@ struct BasinArgs {
   int32_t most_first;   // basins of an item of the small class
   int32_t most_mid;     // of the middle class: all state in shared memory too
   int32_t mid;          // the launch takes the middle class
+  int32_t first_class;  // and is the first of the classes' launches
   int32_t most_narrow;  // basins of an item whose state (but the lists) is in shared memory
 };
+
+// The kernels of a call on few tiles are launched without waiting for one
+// another's end (programmatic dependent launch): each begins with this, which
+// waits for the one before, and lets the next one's CTAs start beside the last
+// of its own.  Up to a tile per SM a call gains 10 us (one map of 2,562 vertices
+// 214 -> 204 us, of 163,842 503 -> 490); launches that fill the chip lose 1 %
+// (the waiting CTAs' room) and go out plainly, where this does nothing.
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // ---------------------------------------------------------------------------
 __device__ inline float seg_maximum(const BasinArgs& a, int64_t map, int sgn, int seg) {
@@ -239,6 +251,7 @@ __device__ inline void scan_buckets(int* cnt, int* wsum) {
 // ---------------------------------------------------------------------------
 // Maxima of +x and -x of every (map, segment), finite values, at least 0.
 __global__ void __launch_bounds__(256) basin_max_kernel(BasinArgs a, int32_t parts) {
+  after_previous();
   __shared__ float red[32];
   const int64_t b = blockIdx.x;
   const int part = static_cast<int>(b % parts);
@@ -285,6 +298,7 @@ __global__ void __launch_bounds__(256) basin_max_kernel(BasinArgs a, int32_t par
 // The pairs' test reads the class of both words at once, and rows of an odd
 // width leave their last halves out (198 before).
 __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a) {
+  after_previous();
   __shared__ uint32_t key[kTile];
   __shared__ __align__(16) uint16_t lab[kTile];  // pointer, then root (2 * index in the tile)
   uint32_t* const table = reinterpret_cast<uint32_t*>(lab);  // distinct pairs, once lab is done with
@@ -489,6 +503,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a
 // inserting row by row, with a few lanes each, 48 maps took 331 us, with full
 // rounds from a queue 247.
 __global__ void __launch_bounds__(kCrossThreads) basin_cross_kernel(BasinArgs a) {
+  after_previous();
   __shared__ int cnt[kBuckets], total;
   __shared__ unsigned long long table[kCrossTable];  // {tile << 12 | basin, twice} << 8 | 128 - step
   // pairs wait in a queue of the warp until there are 32 for a full round
@@ -592,6 +607,7 @@ __global__ void __launch_bounds__(kCrossThreads) basin_cross_kernel(BasinArgs a)
 // chunks) before it, and the bucket starts of the segment's lists; first basin
 // number of every tile.  One CTA per (map, segment), one thread per bucket.
 __global__ void __launch_bounds__(kBuckets) basin_offset_kernel(BasinArgs a) {
+  after_previous();
   __shared__ int tot[kBuckets + 1], wsum[8];
   const int seg = blockIdx.x % a.n_seg;
   const int64_t map = blockIdx.x / a.n_seg;
@@ -662,6 +678,7 @@ __global__ void __launch_bounds__(kBuckets) basin_offset_kernel(BasinArgs a) {
 // sort in here, 387 with all loads issued before the first is used).
 template <bool kOrder>
 __global__ void __launch_bounds__(kTileThreads, 4) basin_order_kernel(BasinArgs a) {
+  after_previous();
   __shared__ uint32_t to_ev[kBuckets], to_pair[kBuckets];
   const int units = a.n_tiles + a.n_chunks;
   const int unit = blockIdx.x % units;
@@ -1371,7 +1388,8 @@ template <int kMode, bool kLarge>
 __global__ void __launch_bounds__(kLarge ? kMaxSweepThreads : 512, kLarge ? 1 : 2) basin_sweep_kernel(BasinArgs a) {
   __shared__ SweepShared S;
   extern __shared__ __align__(16) char dyn[];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (a.first_class) after_previous();
+  else asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x, nth = blockDim.x;
   const int cls = kLarge ? 2 : a.mid;
   int32_t* const counter = a.counter + 2 * cls;
@@ -1425,6 +1443,7 @@ __global__ void __launch_bounds__(kLarge ? kMaxSweepThreads : 512, kLarge ? 1 : 
 // Fills out_maps for the vertices that never become active: 0 scaled and
 // weighted as the others are.
 __global__ void basin_fill_kernel(BasinArgs a) {
+  after_previous();
   const int64_t V = a.n_vertices, n = (int64_t)a.n_maps * a.signs * V;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     float val = 0.0f;
@@ -1437,6 +1456,7 @@ __global__ void basin_fill_kernel(BasinArgs a) {
 // component from its own step on, added in float in threshold order
 // (fast_tfce.hpp:72-84), along the chain of nodes.
 __global__ void __launch_bounds__(256) basin_walk_kernel(BasinArgs a) {
+  after_previous();
   __shared__ float red[32];
   const int ms = blockIdx.y / a.n_seg, seg = blockIdx.y % a.n_seg;
   const int sgn = ms % a.signs;
@@ -1472,6 +1492,7 @@ __global__ void __launch_bounds__(256) basin_walk_kernel(BasinArgs a) {
 }
 
 __global__ void basin_max_out_kernel(BasinArgs a) {
+  after_previous();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < a.n_items; q += gridDim.x * blockDim.x) {
     const float best = dec_float(a.part_max[q]);
     a.out_max[q] = (best == -INFINITY) ? 0.0f : best;
@@ -1632,34 +1653,40 @@ SweepShape first_shape(const BasinPlan* p, int mode, int64_t items, bool dense) 
   return shape_of(p, per_basin, per_sm, per_sm == 4 ? 4096 : 65535, per_sm == 4 ? 256 : 512);
 }
 
-// `after`: the launch starts as soon as all CTAs of the one before it have.
-template <int kMode, bool kLarge>
-int launch_sweep_kernel(BasinArgs& a, const SweepShape& s, bool after, cudaStream_t st) {
-  auto* kern = basin_sweep_kernel<kMode, kLarge>;
-  TFGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmBytes - kSweepBytes));
+// Launches, `chain`: as one of a chain (see after_previous).
+template <typename Kernel, typename... Args>
+cudaError_t launch_after(bool chain, Kernel kern, dim3 grid, int threads, int smem, cudaStream_t st, const Args&... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(s.grid);
-  cfg.blockDim = dim3(s.threads);
-  cfg.dynamicSmemBytes = s.smem;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
-  cfg.numAttrs = after ? 1 : 0;
-  TFGB_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+  cfg.numAttrs = chain ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <int kMode, bool kLarge>
+int launch_sweep_kernel(BasinArgs& a, const SweepShape& s, bool first, bool chain, cudaStream_t st) {
+  auto* kern = basin_sweep_kernel<kMode, kLarge>;
+  TFGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmBytes - kSweepBytes));
+  a.first_class = first;
+  TFGB_CUDA(launch_after(chain || !first, kern, dim3(s.grid), s.threads, s.smem, st, a));
   return TFCE_OK;
 }
 
 template <int kMode>
 int launch_sweeps(BasinArgs& a, const SweepShape& first, const SweepShape& mid, const SweepShape& large,
-                  cudaStream_t st) {
+                  bool chain, cudaStream_t st) {
   int rc = TFCE_OK;
-  if (large.grid) rc = launch_sweep_kernel<kMode, true>(a, large, false, st);
+  if (large.grid) rc = launch_sweep_kernel<kMode, true>(a, large, true, chain, st);
   a.mid = 1;
-  if (!rc && mid.grid) rc = launch_sweep_kernel<kMode, false>(a, mid, large.grid > 0, st);
+  if (!rc && mid.grid) rc = launch_sweep_kernel<kMode, false>(a, mid, !large.grid, chain, st);
   a.mid = 0;
-  if (!rc) rc = launch_sweep_kernel<kMode, false>(a, first, large.grid || mid.grid, st);
+  if (!rc) rc = launch_sweep_kernel<kMode, false>(a, first, !large.grid && !mid.grid, chain, st);
   return rc;
 }
 
@@ -2117,6 +2144,7 @@ int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st) {
     a.out_max = r.out_max ? r.out_max + m0 * r.signs * p->n_seg : nullptr;
     a.out_maps = r.out_maps ? r.out_maps + m0 * r.signs * p->V : nullptr;
     a.n_items = static_cast<int32_t>(M * r.signs * p->n_seg);
+    const bool chain = M * p->n_tiles <= p->sms;
     TFGB_CUDA(cudaMemsetAsync(p->ws + lay.head, 0, 256 + M * 2 * p->n_seg * 4, st));
     // a block per (map, segment) reads about 8k values or, with many maps, all of a segment
     const int64_t pairs_ms = M * p->n_seg;
@@ -2125,30 +2153,33 @@ int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st) {
     basin_max_kernel<<<static_cast<unsigned>(pairs_ms * parts), 256, 0, st>>>(a, static_cast<int32_t>(parts));
     if (a.out_maps && r.out_mode == 1) {
       const int64_t n = M * r.signs * p->V;
-      basin_fill_kernel<<<static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, p->sms * 16)), 256, 0, st>>>(a);
+      TFGB_CUDA(launch_after(chain, basin_fill_kernel, dim3(static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, p->sms * 16))),
+                             256, 0, st, a));
     }
-    if (p->n_tiles) basin_tile_kernel<<<static_cast<unsigned>(M * p->n_tiles), kTileThreads, 0, st>>>(a);
+    if (p->n_tiles)
+      TFGB_CUDA(launch_after(chain, basin_tile_kernel, dim3(static_cast<unsigned>(M * p->n_tiles)), kTileThreads, 0, st, a));
     if (p->n_chunks)
-      basin_cross_kernel<<<static_cast<unsigned>(M * p->n_chunks), kCrossThreads, 0, st>>>(a);
-    basin_offset_kernel<<<static_cast<unsigned>(pairs_ms), kBuckets, 0, st>>>(a);
+      TFGB_CUDA(launch_after(chain, basin_cross_kernel, dim3(static_cast<unsigned>(M * p->n_chunks)), kCrossThreads, 0, st, a));
+    TFGB_CUDA(launch_after(chain, basin_offset_kernel, dim3(static_cast<unsigned>(pairs_ms)), kBuckets, 0, st, a));
     const unsigned units = static_cast<unsigned>(M * (p->n_tiles + p->n_chunks));
-    if (units && mode == kMaxima) basin_order_kernel<false><<<units, kTileThreads, 0, st>>>(a);
-    else if (units) basin_order_kernel<true><<<units, kTileThreads, 0, st>>>(a);
+    if (units)
+      TFGB_CUDA(launch_after(chain, mode == kMaxima ? basin_order_kernel<false> : basin_order_kernel<true>, dim3(units),
+                             kTileThreads, 0, st, a));
     TFGB_CUDA(cudaGetLastError());
     first.grid = std::min(first_ctas, a.n_items);
     mid.grid = std::min(mid_ctas, a.n_items);
     large.grid = std::min(large_ctas, a.n_items);
     int e;
-    if (mode == kMaxima) e = launch_sweeps<kMaxima>(a, first, mid, large, st);
-    else if (mode == kPotential) e = launch_sweeps<kPotential>(a, first, mid, large, st);
-    else e = launch_sweeps<kNodes>(a, first, mid, large, st);
+    if (mode == kMaxima) e = launch_sweeps<kMaxima>(a, first, mid, large, chain, st);
+    else if (mode == kPotential) e = launch_sweeps<kPotential>(a, first, mid, large, chain, st);
+    else e = launch_sweeps<kNodes>(a, first, mid, large, chain, st);
     if (e) return e;
     if (mode == kNodes) {
       const dim3 g(static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((p->vmax + 255) / 256, 1024))),
                    static_cast<unsigned>(a.n_items));
-      basin_walk_kernel<<<g, 256, 0, st>>>(a);
+      TFGB_CUDA(launch_after(chain, basin_walk_kernel, g, 256, 0, st, a));
       if (a.out_max)
-        basin_max_out_kernel<<<static_cast<unsigned>((a.n_items + 255) / 256), 256, 0, st>>>(a);
+        TFGB_CUDA(launch_after(chain, basin_max_out_kernel, dim3(static_cast<unsigned>((a.n_items + 255) / 256)), 256, 0, st, a));
       TFGB_CUDA(cudaGetLastError());
     }
   }
