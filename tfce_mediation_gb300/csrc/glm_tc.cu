@@ -200,6 +200,22 @@ __device__ inline void tmem_ld16(uint32_t taddr, float* out) {
   for (int i = 0; i < 16; ++i) out[i] = __uint_as_float(r[i]);
 }
 
+// The same in two halves: the registers may be read once the second has passed
+// them on.
+__device__ inline void tmem_ld16_start(uint32_t taddr, float* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]),
+        "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
+      : "r"(taddr));
+}
+__device__ inline void tmem_ld16_wait(float* r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]),
+                 "+f"(r[8]), "+f"(r[9]), "+f"(r[10]), "+f"(r[11]), "+f"(r[12]), "+f"(r[13]), "+f"(r[14]), "+f"(r[15])
+               :: "memory");
+}
+
 // --- operand pre-tiling -------------------------------------------------------
 // dst = the split-BF16 tiles of a [rows][cols] FP32 matrix (row stride ld_src;
 // transpose: the source is stored [cols][rows], e.g. the data n x V):
@@ -684,8 +700,12 @@ constexpr int kQfMaxCoef = 8;   // coefficients per design
 __host__ __device__ constexpr int qf_rows(int kc) { return kc <= 4 ? 4 : 8; }  // B rows per design
 __host__ __device__ constexpr int qf_db(int kc) { return kQfN / qf_rows(kc); }  // designs per tile
 __host__ __device__ constexpr int qf_stage() { return tc_y_stage() + kQfN * kTcK * 2 * 2; }
-__host__ __device__ constexpr int qf_smem() { return kTcStages * qf_stage() + 128; }
-static_assert(qf_smem() <= 113 * 1024, "two CTAs per SM");
+// the tile's constants: inv(Xc'Xc), the SE factors of the coefficients, dof
+__host__ __device__ constexpr int qf_const_floats(int kc) {
+  return qf_db(kc) * (qf_rows(kc) * qf_rows(kc) + kQfMaxCoef + 1);
+}
+__host__ __device__ constexpr int qf_smem(int kc) { return kTcStages * qf_stage() + 128 + 4 * qf_const_floats(kc); }
+static_assert(qf_smem(4) <= 112 * 1024 && qf_smem(7) <= 112 * 1024, "two CTAs per SM");
 
 struct QfArgs {
   const __nv_bfloat16* yt;  // pre-tiled centred data, 128-vertex row blocks
@@ -705,35 +725,37 @@ struct QfArgs {
 // design `dfirst` on (global index gbase + dfirst + ...), read from the TMEM
 // accumulator columns at `tacc` (lane quarter included) for vertex v of this
 // lane.  Every lane works on the same design at a time, so the per-design
-// constants are warp-uniform loads and the t stores coalesce over the vertices.
-template <int KC>
-__device__ __forceinline__ void qf_epilogue_warp(const QfArgs& a, uint32_t tacc, int dfirst, int gbase, int64_t v) {
+// constants are broadcast reads of shared memory (`ginv`, `se`, `dof`, staged
+// while the MMAs run) and the t stores coalesce over the vertices.  Bound by
+// the latency of a design's chain, four warps to a scheduler: the designs of a
+// 16-column load run side by side, and the next load is in flight meanwhile
+// (design by design, with the constants from global memory, 128 designs of 350
+// x 5 over 328k vertices took 592 us, so 412).  kInOrder: the coefficients are
+// 1, 2, ..
+template <int KC, bool kInOrder>
+__device__ __forceinline__ void qf_epilogue_warp(const QfArgs& a, const float* ginv, const float* se, const float* dof,
+                                                 const int* jc, uint32_t tacc, int dfirst, int gbase, int64_t v) {
   constexpr int R = qf_rows(KC), DB = qf_db(KC);
   const bool live = v < a.V;
   const float yyv = live ? __ldg(a.yy + v) : 0.0f;
-  int jc[kQfMaxCoef];  // the requested coefficients (uniform)
-#pragma unroll
-  for (int ci = 0; ci < kQfMaxCoef; ++ci) jc[ci] = (ci < a.n_coef) ? __ldg(a.coef + ci) : 0;
   constexpr int DPW = DB / 2;  // designs per warp
   constexpr int DPL = 16 / R;  // designs per 16-column load
-#pragma unroll 1
-  for (int d0 = 0; d0 < DPW; d0 += DPL) {
-    float cc[16];
-    tmem_ld16(tacc + d0 * R, cc);
+  float* out = a.t_out + (int64_t)(gbase + dfirst) * a.n_coef * a.ldt + v;
+  const int designs = min(DPW, a.G - gbase - dfirst);  // of this warp
+  auto group = [&](int d0, const float* cc) {
+    float b[DPL][KC], s2[DPL];
 #pragma unroll
     for (int dd = 0; dd < DPL; ++dd) {
-      const int g = gbase + dfirst + d0 + dd;
-      if (g >= a.G) break;
       // b = inv(Xc'Xc) c from the padded R x R inverse, rows as float4
-      const float4* gi = reinterpret_cast<const float4*>(a.ginv + (int64_t)g * R * R);
-      float b[KC];
+      const int d = dfirst + d0 + dd;
+      const float4* gi = reinterpret_cast<const float4*>(ginv + d * R * R);
       float qf = 0.0f;
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
         float row[R];
 #pragma unroll
         for (int r4 = 0; r4 < (KC + 3) / 4; ++r4) {
-          const float4 x4 = __ldg(gi + i * (R / 4) + r4);
+          const float4 x4 = gi[i * (R / 4) + r4];
           row[4 * r4] = x4.x;
           row[4 * r4 + 1] = x4.y;
           row[4 * r4 + 2] = x4.z;
@@ -742,23 +764,47 @@ __device__ __forceinline__ void qf_epilogue_warp(const QfArgs& a, uint32_t tacc,
         float s = 0.0f;
 #pragma unroll
         for (int j = 0; j < KC; ++j) s = fmaf(row[j], cc[dd * R + j], s);
-        b[i] = s;
+        b[dd][i] = s;
         qf = fmaf(cc[dd * R + i], s, qf);
       }
       // sigma^2 = RSS / dof; t_j = b_j / sqrt(sigma^2 inv(X'X)_jj)
-      const float s2 = fmaxf(yyv - qf, 0.0f) / __ldg(a.dof + g);
+      s2[dd] = fmaxf(yyv - qf, 0.0f) / dof[d];
+    }
 #pragma unroll
-      for (int ci = 0; ci < kQfMaxCoef; ++ci) {
-        if (ci >= a.n_coef) break;
-        const int j = jc[ci];
-        float bj = __int_as_float(0x7fc00000);  // NaN for a coefficient outside [1, KC]
+    for (int dd = 0; dd < DPL; ++dd) {
+      if (d0 + dd < designs) {
+        float* at = out + (int64_t)(d0 + dd) * a.n_coef * a.ldt;
+        const float* f = se + (dfirst + d0 + dd) * kQfMaxCoef;
 #pragma unroll
-        for (int jj = 0; jj < KC; ++jj)
-          if (jj + 1 == j) bj = b[jj];
-        const float dj = (j >= 1 && j <= KC) ? __ldg(a.invdiag + (int64_t)g * (KC + 1) + j) : 1.0f;
-        if (live) a.t_out[((int64_t)g * a.n_coef + ci) * a.ldt + v] = bj * rsqrtf(s2 * dj);
+        for (int ci = 0; ci < (kInOrder ? KC : kQfMaxCoef); ++ci) {
+          if (ci >= a.n_coef) break;
+          float bj = __int_as_float(0x7fc00000);  // NaN for a coefficient outside [1, KC]
+          if constexpr (kInOrder) {
+            bj = b[dd][ci];
+          } else {
+#pragma unroll
+            for (int jj = 0; jj < KC; ++jj)
+              if (jj + 1 == jc[ci]) bj = b[dd][jj];
+          }
+          if (live) *at = bj * rsqrtf(s2[dd] * f[ci]);
+          at += a.ldt;
+        }
       }
     }
+  };
+  float even[16], odd[16];
+  tmem_ld16_start(tacc, even);
+  tmem_ld16_wait(even);
+  static_assert(DPW % (2 * DPL) == 0, "loads go in pairs");
+#pragma unroll 1
+  for (int d0 = 0; d0 < designs; d0 += 2 * DPL) {
+    tmem_ld16_start(tacc + (d0 + DPL) * R, odd);
+    group(d0, even);
+    tmem_ld16_wait(odd);
+    const int next = d0 + 2 * DPL < DPW ? d0 + 2 * DPL : 0;
+    tmem_ld16_start(tacc + next * R, even);
+    group(d0 + DPL, odd);
+    tmem_ld16_wait(even);
   }
 }
 
@@ -770,6 +816,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) glm_tc_qf_kernel(QfArgs a) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kTcStages * qf_stage());  // full[4], empty[4], done
   uint32_t* sTmem = reinterpret_cast<uint32_t*>(bars + 2 * kTcStages + 1);
   int* sFail = reinterpret_cast<int*>(sTmem + 1);
+  float* sGinv = reinterpret_cast<float*>(sm + kTcStages * qf_stage() + 128);  // [DB][R][R]
+  float* sSe = sGinv + DB * R * R;                                             // [DB][kQfMaxCoef]
+  float* sDof = sSe + DB * kQfMaxCoef;                                         // [DB]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t vb = blockIdx.x / a.n_db;
   const int db = static_cast<int>(blockIdx.x % a.n_db);
@@ -777,9 +826,24 @@ __global__ void __launch_bounds__(kTcThreads, 2) glm_tc_qf_kernel(QfArgs a) {
   const uint32_t full0 = smem_addr(bars), empty0 = full0 + 8 * kTcStages, done = full0 + 16 * kTcStages;
   const uint32_t tmem = tc_setup<N>(sTmem, full0, empty0, done, sFail, warp, tid);
   const int KS = a.ks_count;
+  int jc[kQfMaxCoef];  // the requested coefficients (uniform)
+#pragma unroll
+  for (int ci = 0; ci < kQfMaxCoef; ++ci) jc[ci] = (ci < a.n_coef) ? __ldg(a.coef + ci) : 0;
 
   // the producer thread alone waits for the accumulator; the other warps
-  // wait at the CTA barrier (no issue slots spent polling)
+  // stage the constants and wait at the CTA barrier (no issue slots spent
+  // polling)
+  if (warp != 0) {
+    for (int i = tid - 32; i < DB * R * R; i += kTcThreads - 32)
+      sGinv[i] = db * DB + i / (R * R) < a.G ? __ldg(a.ginv + (int64_t)db * DB * R * R + i) : 0.0f;
+    for (int d = tid - 32; d < DB; d += kTcThreads - 32) {
+      const int64_t g = (int64_t)db * DB + d;
+      sDof[d] = g < a.G ? __ldg(a.dof + g) : 1.0f;
+#pragma unroll
+      for (int ci = 0; ci < kQfMaxCoef; ++ci)
+        sSe[d * kQfMaxCoef + ci] = (g < a.G && jc[ci] >= 1 && jc[ci] <= KC) ? __ldg(a.invdiag + g * (KC + 1) + jc[ci]) : 1.0f;
+    }
+  }
   if (tid == 0) {
     tc_gemm_pipeline<N>(reinterpret_cast<const unsigned char*>(a.yt) + (vb * KS) * (int64_t)YS,
                         reinterpret_cast<const unsigned char*>(a.xt) + ((int64_t)db * KS) * (int64_t)PS, sbase,
@@ -795,8 +859,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) glm_tc_qf_kernel(QfArgs a) {
 
   if (*sFail == 0) {
     const int q = warp & 3, half = warp >> 2;
-    qf_epilogue_warp<KC>(a, tmem + (static_cast<uint32_t>(q * 32) << 16) + half * (DB / 2) * R, half * (DB / 2),
-                         db * DB, vb * kTcM + q * 32 + lane);
+    const uint32_t tacc = tmem + (static_cast<uint32_t>(q * 32) << 16) + half * (DB / 2) * R;
+    const int64_t v = vb * kTcM + q * 32 + lane;
+    bool in_order = a.n_coef <= KC;
+#pragma unroll
+    for (int ci = 0; ci < KC; ++ci) in_order = in_order && (ci >= a.n_coef || jc[ci] == ci + 1);
+    if (in_order) qf_epilogue_warp<KC, true>(a, sGinv, sSe, sDof, jc, tacc, half * (DB / 2), db * DB, v);
+    else qf_epilogue_warp<KC, false>(a, sGinv, sSe, sDof, jc, tacc, half * (DB / 2), db * DB, v);
   }
   tc_fence_before();
   __syncthreads();
@@ -807,7 +876,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) glm_tc_qf_kernel(QfArgs a) {
 
 template <int KC>
 static int launch_tc_qf(const QfArgs& a, int64_t n_vb, cudaStream_t stream) {
-  const int smem = qf_smem();
+  const int smem = qf_smem(KC);
   TFGB_CUDA(cudaFuncSetAttribute(glm_tc_qf_kernel<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   glm_tc_qf_kernel<KC><<<static_cast<unsigned>(n_vb * a.n_db), kTcThreads, smem, stream>>>(a);
   TFGB_CUDA(cudaGetLastError());
