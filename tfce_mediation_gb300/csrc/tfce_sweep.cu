@@ -611,7 +611,12 @@ struct tfce_adjset {
   int64_t* d_seg_off = nullptr;
   float* d_H = nullptr;
   float* d_E = nullptr;
-  int32_t* d_ctrl = nullptr;  // [0] queue counter, [1] error word, [2] step count
+  int32_t* d_ctrl = nullptr;  // queue counter
+  // [0] error word, [1] step count: pinned host memory that the kernels write
+  // (an error, or once per recorded sweep), so that reading them takes a wait
+  // and no copy (8 us of a small map's 200)
+  volatile int32_t* report = nullptr;
+  cudaEvent_t reached = nullptr;  // for waits on the default stream
   char* d_ws = nullptr;
   int64_t ws_slot = 0;
   int32_t ws_slots = 0;
@@ -653,6 +658,8 @@ int release(tfce_adjset* h) {
   cudaFree(h->d_H);
   cudaFree(h->d_E);
   cudaFree(h->d_ctrl);
+  cudaFreeHost(const_cast<int32_t*>(h->report));  // after cudaFree has waited for the kernels
+  if (h->reached) cudaEventDestroy(h->reached);
   cudaFree(h->d_ws);
   cudaFree(h->d_img);
   cudaFree(h->d_enh);
@@ -724,7 +731,7 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
     r.d_E = h->d_E;
     r.d_seg_off = h->d_seg_off;
     r.seg_rank = h->d_segrank;
-    r.err = h->d_ctrl + 1;
+    r.err = const_cast<int32_t*>(h->report);
     if (tfgb::basin_takes(h->basin, r)) return tfgb::basin_sweep(h->basin, r, st);
   }
   int rs = resident_slots(h);
@@ -751,13 +758,13 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
   a.out_mode = out_mode;
   a.labels = labels;
   a.extents = extents;
-  a.n_steps_out = labels ? h->d_ctrl + 2 : nullptr;
+  a.n_steps_out = labels ? const_cast<int32_t*>(h->report) + 1 : nullptr;
   a.label_cap = label_cap;
   a.ws = h->d_ws;
   a.ws_slot_bytes = h->ws_slot;
   a.vcap = h->vmax_seg;
   a.counter = h->d_ctrl;
-  a.err = h->d_ctrl + 1;
+  a.err = const_cast<int32_t*>(h->report);
   a.n_items = items;
   a.item_order = nullptr;
   a.seg_rank = h->d_segrank;
@@ -788,12 +795,16 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
 
 // Reads and clears the sticky error word (synchronises the stream).
 int check_device_error(tfce_adjset* h, cudaStream_t st, int32_t* steps) {
-  int32_t ctrl[4];
-  TFGB_CUDA(cudaMemcpyAsync(ctrl, h->d_ctrl, sizeof(ctrl), cudaMemcpyDeviceToHost, st));
-  TFGB_CUDA(cudaStreamSynchronize(st));
-  if (steps) *steps = ctrl[2];
-  if (ctrl[1] != 0) TFGB_CUDA(cudaMemsetAsync(h->d_ctrl + 1, 0, sizeof(int32_t), st));
-  return tfgb::map_dev_err(ctrl[1]);
+  if (st) {
+    TFGB_CUDA(cudaStreamSynchronize(st));
+  } else {  // an event there waits for the blocking streams too, as a copy would
+    TFGB_CUDA(cudaEventRecord(h->reached, nullptr));
+    TFGB_CUDA(cudaEventSynchronize(h->reached));
+  }
+  const int32_t err = h->report[0];
+  if (steps) *steps = h->report[1];
+  if (err != 0) h->report[0] = 0;
+  return tfgb::map_dev_err(err);
 }
 
 int ensure_run_buffers(tfce_adjset* h, int32_t V) {
@@ -926,8 +937,13 @@ int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n
   TFGB_CUDA_H(cudaMalloc(&h->d_seg_off, sizeof(int64_t) * (n_seg + 1)));
   TFGB_CUDA_H(cudaMalloc(&h->d_H, sizeof(float) * n_seg));
   TFGB_CUDA_H(cudaMalloc(&h->d_E, sizeof(float) * n_seg));
-  TFGB_CUDA_H(cudaMalloc(&h->d_ctrl, sizeof(int32_t) * 4));
-  TFGB_CUDA_H(cudaMemset(h->d_ctrl, 0, sizeof(int32_t) * 4));
+  TFGB_CUDA_H(cudaMalloc(&h->d_ctrl, sizeof(int32_t)));
+  TFGB_CUDA_H(cudaMemset(h->d_ctrl, 0, sizeof(int32_t)));
+  int32_t* report = nullptr;
+  TFGB_CUDA_H(cudaHostAlloc(&report, sizeof(int32_t) * 2, cudaHostAllocPortable | cudaHostAllocMapped));
+  report[0] = report[1] = 0;
+  h->report = report;
+  TFGB_CUDA_H(cudaEventCreateWithFlags(&h->reached, cudaEventDisableTiming));
   TFGB_CUDA_H(cudaMemcpy(h->d_offsets, off.data(), sizeof(int64_t) * (V + 1), cudaMemcpyHostToDevice));
   if (!packed.empty())
     TFGB_CUDA_H(cudaMemcpy(h->d_indices, packed.data(), sizeof(uint32_t) * packed.size(),
