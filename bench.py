@@ -613,7 +613,7 @@ def run_config(kind, args, stash=None):
                     "d2h_bytes_per_step": int(P * C * signs * S * 4),
                     "note": "new data from pinned host memory every step (%s.run_stream)" %
                             ("MediationEngine" if kind == "config4a" else "PermutationEngine")},
-            "roofline": {"bound": "hbm", "kernel": "tfce_sweep_kernel", "achieved": achieved, "peak": hbm,
+            "roofline": {"bound": "hbm", "kernel": "basin_*_kernel (a batched sweep)", "achieved": achieved, "peak": hbm,
                          "unit": "GB/s", "frac": achieved / hbm, "peak_source": f"{peak_kind} hbm_gbs",
                          "traffic": None, "algorithmic_bytes_per_launch": alg, "ms_per_launch": ms,
                          "sweeps_per_launch": P * C * signs * S}}
@@ -961,9 +961,12 @@ def run_gpu(args):
                 T = np.asarray(T, np.float32)
                 upd.append(int(sum(int(np.count_nonzero(xs > t_)) for t_ in T)))
     updates_per_sweep = float(np.mean(upd))
-    per_sweep, traffic_note = profile_traffic("tfce_sweep")
+    per_sweep, traffic_note = profile_traffic("basin_sweep")
     traffic = None if per_sweep is None else per_sweep * sweeps_per_launch
     clocks = clk.summary()
+    # of a batched sweep: maxima, tiles, crossing pairs, offsets, order, and the
+    # size classes that the graph's bound on basins asks for (two at least here)
+    sweep_launches = 7
     if qf:
         # split-BF16 GEMM: 3 MMAs of M=V, N=R rows per design (the k-1 centred
         # columns padded to 4 or 8), K=n_pad; epilogue O(k^2) per vertex and design
@@ -978,7 +981,7 @@ def run_gpu(args):
                     "peak_source": f"{peak_kind} bf16_tflops_sustained (kernel timed inside a long step)",
                     "glm_ms_by_form": getattr(tc, "glm_timings", None),
                     "note": "tensor FLOPs count the three split-BF16 products on %d rows per design" % R}
-        launches = 3 * args.steps
+        launches = (2 + sweep_launches) * args.steps
     elif tc is not None:
         # split-BF16 GEMM: 3 MMAs of M=V, N=8 rows per design, K=n_pad; residual
         # epilogue: (k+1) FP32 FMAs per vertex, design and subject (k with the
@@ -994,12 +997,12 @@ def run_gpu(args):
                     "epilogue_fp32_tflops": epi_flop / (glm_avg / 1000) / 1e12,
                     "glm_ms_by_form": getattr(tc, "glm_timings", None),
                     "note": "tensor FLOPs count the three split-BF16 products on 8 padded rows per design"}
-        launches = 3 * args.steps
+        launches = (2 + sweep_launches) * args.steps
     else:
         glm_flop = 4.0 * n * eng.k * V * P  # beta + residual passes, FP32 CUDA cores
         glm_info = {"precision": "fp32", "kernels": "glm_tstat_kernel", "ms_per_launch": glm_avg,
                     "achieved_tflops_fp32": glm_flop / (glm_avg / 1000) / 1e12}
-        launches = 2 * args.steps
+        launches = (1 + sweep_launches) * args.steps
     line = {
         "metric": METRIC, "value": value, "unit": "perm/s", "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
@@ -1015,14 +1018,13 @@ def run_gpu(args):
                    "data_gen_s": round(gen_s, 1)},
         "e2e": {"value": e2e_value, "unit": "perm/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "steps": e2e_steps,
-                "note": "PermutationEngine.run_stream; per step: Y (pinned host) -> HBM and re-tiled, host "
-                        "FP64 design inverses (overlapped with the previous step), captured GLM + sweep, "
-                        "maxima -> host"},
+                "note": "PermutationEngine.run_stream; per step: Y (pinned host) -> HBM and re-tiled, index "
+                        "rows -> design operators formed on the device, captured GLM + sweep, maxima -> host"},
         "dropin": dropin,
         "job_api": {"value": job_value, "unit": "perm/s",
                     "note": "PermutationEngine.run_graph over %d permutations, Y resident" % (8 * P)},
         "gpu_launches": launches,
-        "roofline": {"bound": "hbm", "kernel": "tfce_sweep_kernel", "achieved": achieved, "peak": hbm,
+        "roofline": {"bound": "hbm", "kernel": "basin_*_kernel (a batched sweep)", "achieved": achieved, "peak": hbm,
                      "unit": "GB/s", "frac": achieved / hbm, "peak_source": f"{peak_kind} hbm_gbs",
                      "traffic": traffic, "traffic_note": traffic_note,
                      "algorithmic_bytes_per_launch": bytes_per_sweep * sweeps_per_launch,
