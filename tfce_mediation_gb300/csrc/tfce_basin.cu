@@ -24,10 +24,10 @@
 //
 // Measured on one GB300 against the vertex-by-vertex sweep that batched
 // launches ran before (its state, 5 MB an item, was walked at random in DRAM):
-// 512 maps x 2 hemispheres x +/- of the L7 icosphere, smooth: 21.9 -> 4.7 ms
-// (tile 2.3, sweep 1.5, order 0.5, cross 0.2, max 0.1); unsmoothed noise, 128
-// maps: 10.1 -> 2.9 ms; 48 maps of 242k voxels, 26 neighbours, E = 0.5: 9.8 ->
-// 1.3 ms; one map: 4.64 -> 0.40 ms.
+// 512 maps x 2 hemispheres x +/- of the L7 icosphere, smooth: 21.9 -> 4.35 ms
+// (tile 2.25, sweep 1.37, order 0.38, cross 0.18, max 0.11); unsmoothed noise,
+// 128 maps: 10.1 -> 2.75 ms; 48 maps of 242k voxels, 26 neighbours, E = 0.5: 9.8
+// -> 1.17 ms; one map: 4.64 -> 0.39 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

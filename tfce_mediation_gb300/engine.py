@@ -338,7 +338,7 @@ class PermutationEngine:
         """What a captured batch depends on: its size, the GLM's form and, with
         the residual epilogue, the designs per tile."""
         qf = self._graph_qf()
-        return self.batch, qf, None if qf or self._tc is None else self._tc.block(self.k)
+        return self.batch, qf, self._program_on_device(), None if qf or self._tc is None else self._tc.block(self.k)
 
     def _graph_slot(self, P):
         """One captured batch: pinned design operators -> device, glm_tstat,
@@ -348,14 +348,15 @@ class PermutationEngine:
         tc = self._tc
         slot = {"P": P, "form": self._graph_form()}
         qf = self._graph_qf()
-        slot["QF"] = qf
-        if qf:
+        program = not qf and self._program_on_device()
+        slot["on_device"] = qf or program  # designs formed on the device from index rows
+        if slot["on_device"]:
             keys = ()
             base, cols = self._base()
             slot["h_rows"] = t.empty((P, n), dtype=t.int32, pin_memory=True)
             slot["h_rows"].numpy()[...] = np.arange(n)
             slot["d_rows"] = t.empty((P, n), dtype=t.int32, device="cuda")
-            slot["ops"] = tc.design_buffers(P, kmax)
+            slot["ops"] = tc.design_buffers(P, kmax) if qf else tc.residual_buffers(P, kmax, self._w_stride)
         elif tc is not None:
             Gp, DB = tc.padded(P, kmax), tc.block(kmax)
             keys = ("P8", "U", "Xt", "invd", "dof") + (("W",) if self._w_stride else ())
@@ -371,7 +372,7 @@ class PermutationEngine:
             slot["h_pinv"] = t.zeros((P, kmax, n), dtype=t.float32, pin_memory=True)
             slot["h_X"] = t.zeros((P, n, kmax), dtype=t.float32, pin_memory=True)
         # the capture warm-up runs on these before the first fill: a harmless design
-        if not qf:
+        if not slot["on_device"]:
             slot["h_invd"] = t.ones((P, kmax), dtype=t.float32, pin_memory=True)
             slot["h_dof"] = t.ones((P,), dtype=t.float32, pin_memory=True)
         slot["h_max"] = t.empty((P, self.C, self.signs, self.n_seg), dtype=t.float32, pin_memory=True)
@@ -387,6 +388,12 @@ class PermutationEngine:
                 slot["d_rows"].copy_(slot["h_rows"], non_blocking=True)
                 tc.form_designs(base, cols, slot["d_rows"], P, kmax, slot["ops"])
                 tc.tstat_qf(*slot["ops"], P, kmax, self._coef, self.C, slot["d_t"], self.V)
+            elif program:
+                slot["d_rows"].copy_(slot["h_rows"], non_blocking=True)
+                tc.form_residual_designs(base, slot["d_rows"], P, kmax, self._centred, self._coef, self.C,
+                                         self._w_stride, out=slot["ops"])
+                *ops, wmat = slot["ops"]
+                tc.stat(3, *ops, P, kmax, self._coef, self.C, slot["d_t"], self.V, wmat=wmat, centred=self._centred)
             elif tc is not None:
                 tc.tile_designs(slot["d_P8"], P, kmax, out=slot["d_pt"])
                 tc.stat(3 if self.outputs is not None else 0, slot["d_pt"], slot["d_U"], slot["d_Xt"],
@@ -426,7 +433,7 @@ class PermutationEngine:
         return slot
 
     def _fill(self, slot, perms):
-        if slot["QF"]:
+        if slot["on_device"]:
             self._index_rows(perms, out=slot["h_rows"].numpy())
             return
         db = DesignBatch(self.X[perms])
@@ -444,8 +451,9 @@ class PermutationEngine:
 
     def run_graph(self, n_perm=None, seed=0, start=0, stop=None, perms=None):
         """Same result as run(), through two captured batch graphs replayed in
-        turn: while one batch runs on the GPU the host forms the next batch's
-        design inverses (run_stream over the batches)."""
+        turn: while one batch runs on the GPU the host fills in the next
+        batch's index rows, or its design operators where those are not formed
+        on the device (run_stream over the batches)."""
         if perms is None:
             stop = start + n_perm if stop is None else stop
             perms = permutations(self.n, seed, start, stop)
@@ -459,8 +467,8 @@ class PermutationEngine:
         vertex order (pinned memory keeps the copy asynchronous) or None to
         keep the resident data; perms: at most `batch` permutation index rows.
         Two captured batch slots are replayed in turn, each as a GLM graph and
-        a sweep graph.  The host forms a batch's design operators while the
-        GPU runs the previous batch; new data is copied and re-tiled on a side
+        a sweep graph.  The host fills in a batch's index rows (or design
+        operators) while the GPU runs the previous batch; new data is copied and re-tiled on a side
         stream once the previous batch's GLM (the last reader of the resident
         data) is done, so the upload overlaps that batch's sweep, and this
         batch's GLM waits for it; each batch's maxima come back when its slot

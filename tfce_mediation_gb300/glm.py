@@ -373,22 +373,29 @@ class TensorCoreOperands:
         self.form_designs(base, cols, None, G, k, out, stride=n * k)
         return out
 
-    def form_residual_designs(self, base, rows, G, kmax, centred, program, n_rows, w_stride):
-        """Operands of `stat` for G permuted intercept designs, formed on the
-        device (glm_tc_designs): (tiles, u, x, invdiag, dof, weights).  base: (n,
-        kmax) float64 design whose rows (G, n) int32 index; program: device rows
-        of output_program."""
+    def residual_buffers(self, G, kmax, w_stride):
+        """Device operands of `stat` for up to G designs: (tiles, u, x, invdiag,
+        dof, weights)."""
         t = self.t
         Gp, DB = self.padded(G, kmax), self.block(kmax)
         tiles = t.empty(int(self.lib.glm_tile_bytes(Gp * 8, DB * 8, self.n_pad)), dtype=t.uint8, device="cuda")
         # one allocation for the float operands
         sizes = [Gp * kmax, Gp * self.n_sc * kmax, G * kmax, G, G * w_stride]
         u, x, invd, dof, w = t.empty(sum(sizes), dtype=t.float32, device="cuda").split(sizes)
-        w = w.view(G, w_stride) if w_stride else None
+        return tiles, u, x, invd, dof, w.view(G, w_stride) if w_stride else None
+
+    def form_residual_designs(self, base, rows, G, kmax, centred, program, n_rows, w_stride, out=None):
+        """Operands of `stat` for G permuted intercept designs, formed on the
+        device (glm_tc_designs), in `out` (residual_buffers) when given.  base: (n,
+        kmax) float64 design whose rows (G, n) int32 index; program: device rows
+        of output_program."""
+        out = self.residual_buffers(G, kmax, w_stride) if out is None else out
+        tiles, u, x, invd, dof, w = out
         _lib.check(self.lib.glm_tc_designs(ptr(base), base.shape[-1], ptr(rows), self.n, self.n_pad, self.n_sc, G,
-                                           kmax, DB, int(centred), ptr(program), n_rows, w_stride, ptr(tiles), ptr(u),
-                                           ptr(x), ptr(invd), ptr(dof), ptr(w), ptr(self.err), stream_handle()))
-        return tiles, u, x, invd, dof, w
+                                           kmax, self.block(kmax), int(centred), ptr(program), n_rows, w_stride,
+                                           ptr(tiles), ptr(u), ptr(x), ptr(invd), ptr(dof), ptr(w), ptr(self.err),
+                                           stream_handle()))
+        return out
 
     def tstat_qf(self, x_tiles, ginv, invd, dof, G, kmax, coef_d, n_coef, out, ldt):
         _lib.check(self.lib.glm_tstat_tc_qf(ptr(self.yt), ptr(self.yy), self.n, self.n_pad, self.V, ptr(x_tiles),
