@@ -391,6 +391,10 @@ int glm_tc_designs(const double* base, int64_t ld, const int32_t* rows, int32_t 
                    int32_t G, int32_t kmax, int32_t design_block, int32_t centred, const int32_t* program,
                    int32_t n_rows, int32_t w_stride, void* p_tiles, float* u_rows, float* x_rows, float* invdiag,
                    float* dof, float* weights, int32_t* err, void* stream);
+/* The same designs for glm_tstat / glm_stat: pinv [G][kmax][n], X [G][n][kmax],
+ * invdiag [G][kmax] and dof [G] in float. */
+int glm_fp32_designs(const double* base, int64_t ld, const int32_t* rows, int32_t n, int32_t G, int32_t kmax,
+                     float* pinv, float* X, float* invdiag, float* dof, int32_t* err, void* stream);
 int glm_col_sumsq(const float* Y_centred, int64_t ldy, int32_t n, int64_t V, float* yy, void* stream);
 int glm_tstat_tc_qf(const void* y_tiles, const float* yy, int32_t n, int32_t n_pad, int64_t V,
                     const void* x_tiles, const float* ginv, const float* invdiag, const float* dof, int32_t G,

@@ -94,6 +94,8 @@ SIGNATURES = {
                                       c_vp]),
     "glm_tc_designs": (ctypes.c_int, [c_vp, ctypes.c_int64, c_vp] + [ctypes.c_int32] * 7 + [c_vp, ctypes.c_int32,
                                       ctypes.c_int32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "glm_fp32_designs": (ctypes.c_int, [c_vp, ctypes.c_int64, c_vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
+                                        c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "glm_tstat_tc_qf": (ctypes.c_int, [c_vp, c_vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int64, c_vp, c_vp,
                                        c_vp, c_vp, ctypes.c_int32, ctypes.c_int32, c_vp, ctypes.c_int32, c_vp,
                                        ctypes.c_int64, c_vp, c_vp]),

@@ -230,7 +230,8 @@ __global__ void __launch_bounds__(kDesignThreads) design_kernel(DesignArgs a) {
 // pseudoinverse rows, their sums, the negated design rows, inv(X'X)'s diagonal
 // and the weights of an output program.  The host formed and uploaded them
 // batch by batch: 1.1 of the 1.9 ms that 32 permutations of a rhythm model
-// over 82k vertices took; this takes 47 us.
+// over 82k vertices took; this takes 47 us.  The FP32 GLM's (glm_tstat) come
+// from here too: 32 weighted permutations 1.00 -> 0.81 ms.
 struct ResidualDesignArgs {
   const double* base;   // [n][ld]
   int64_t ld;
@@ -244,6 +245,9 @@ struct ResidualDesignArgs {
   float* invdiag;          // [G][kmax]
   float* dof;              // [G]
   float* weights;          // [G][w_stride]
+  // for the FP32 kernel (glm_tstat) instead of tiles, u and x
+  float* pinv;             // [G][kmax][n]
+  float* rows32;           // [G][n][kmax]
   int32_t* err;
 };
 
@@ -312,6 +316,15 @@ __global__ void __launch_bounds__(kDesignThreads) residual_design_kernel(Residua
     for (int l = 0; l < kc; ++l) v = fma(full[j][l + 1], entry(s, l) - S.mean[l], v);
     return v;
   };
+  if (a.pinv) {
+    for (int t = tid; t < kmax * a.n; t += kDesignThreads) {
+      a.pinv[(int64_t)d * kmax * a.n + t] = static_cast<float>(pinv(t / a.n, t % a.n));
+      const int s = t / kmax, j = t % kmax;
+      a.rows32[(int64_t)d * kmax * a.n + t] = j == 0 ? 1.0f : static_cast<float>(entry(s, j - 1));
+    }
+    if (tid < kmax) a.invdiag[(int64_t)d * kmax + tid] = static_cast<float>(full[tid][tid]);
+    return;
+  }
   const int rb = a.DB * 8, ks_count = a.n_pad / 16;
   for (int t = tid; t < 8 * (a.n_pad / 8); t += kDesignThreads) {
     const int j = t % 8, c0 = (t / 8) * 8;
@@ -351,6 +364,31 @@ __global__ void __launch_bounds__(kDesignThreads) residual_design_kernel(Residua
 }  // namespace tfgb
 
 extern "C" {
+
+int glm_fp32_designs(const double* base, int64_t ld, const int32_t* rows, int32_t n, int32_t G, int32_t kmax,
+                     float* pinv, float* X, float* invdiag, float* dof, int32_t* err, void* stream) {
+  tfgb::clear_error();
+  TFGB_CHECK_ARG(base && pinv && X && invdiag && dof && err, "NULL pointer");
+  TFGB_CHECK_ARG(kmax >= 2 && kmax <= 8, "kmax must be in [2, 8]");
+  TFGB_CHECK_ARG(n > 0 && ld >= kmax && G >= 0, "bad sizes");
+  if (G == 0) return TFCE_OK;
+  tfgb::ResidualDesignArgs a{};
+  a.base = base;
+  a.ld = ld;
+  a.rows = rows;
+  a.n = n;
+  a.G = G;
+  a.kmax = kmax;
+  a.DB = 1;
+  a.pinv = pinv;
+  a.rows32 = X;
+  a.invdiag = invdiag;
+  a.dof = dof;
+  a.err = err;
+  tfgb::residual_design_kernel<<<static_cast<unsigned>(G), tfgb::kDesignThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  TFGB_CUDA(cudaGetLastError());
+  return TFCE_OK;
+}
 
 int glm_tc_designs(const double* base, int64_t ld, const int32_t* rows, int32_t n, int32_t n_pad, int32_t n_sc,
                    int32_t G, int32_t kmax, int32_t design_block, int32_t centred, const int32_t* program,

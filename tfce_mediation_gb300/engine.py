@@ -224,6 +224,8 @@ class PermutationEngine:
             tc.stat(3, pt, u, x, invd, dof, P, self.k, self._coef, self.C, out, self.V, wmat=wmat,
                     centred=self._centred)
             return out
+        if self._fp32_on_device():
+            return self._tmaps_fp32(perms)
         if not self._graph_qf() or len(self.contrasts) > 8:
             return self.tmaps(self._designs(perms))
         tc, out = self._tc, self._tbuf[:P]
@@ -232,6 +234,28 @@ class PermutationEngine:
         ops = tc.design_buffers(P, self.k)
         tc.form_designs(base, cols, rows, P, self.k, ops)
         tc.tstat_qf(*ops, P, self.k, self._coef, self.C, out, self.V)
+        return out
+
+    def _fp32_on_device(self):
+        """Whether a batch's designs of the FP32 GLM are formed on the device:
+        rows of the design [1, pred_x] itself, permuted."""
+        return (self.precision == "fp32" and self.outputs is None and 2 <= self.k <= 8
+                and type(self)._designs is PermutationEngine._designs and bool(np.all(self.X[:, 0] == 1.0)))
+
+    def _tmaps_fp32(self, perms):
+        t, P, k, n = self.t, perms.shape[0], self.k, self.n
+        base, _ = self._base()
+        if not hasattr(self, "_design_err"):
+            self._design_err = t.zeros(1, dtype=t.int32, device="cuda")
+            self._design_err_host = t.zeros(1, dtype=t.int32, pin_memory=True)
+        rows, out = dev(self._index_rows(perms)), self._tbuf[:P]
+        pinv, X, invd, dof = t.empty(P * (2 * k * n + k + 1), dtype=t.float32, device="cuda").split(
+            [P * k * n, P * k * n, P * k, P])
+        _lib.check(self.lib.glm_fp32_designs(ptr(base), base.shape[-1], ptr(rows), n, P, k, ptr(pinv), ptr(X),
+                                             ptr(invd), ptr(dof), ptr(self._design_err), stream_handle()))
+        self._design_err_host.copy_(self._design_err, non_blocking=True)
+        _lib.check(self.lib.glm_tstat(ptr(self.Yd), self.V, n, self.V, ptr(pinv), ptr(X), ptr(invd), ptr(dof), P, k,
+                                      ptr(self._coef), self.C, ptr(out), self.V, stream_handle()))
         return out
 
     def tmaps(self, designs: DesignBatch, out=None, precision=None):
@@ -294,6 +318,10 @@ class PermutationEngine:
         self.adj.status()
         if self._tc is not None:
             self._tc.status()
+        if hasattr(self, "_design_err") and int(self._design_err_host[0]):
+            self._design_err.zero_()
+            self._design_err_host.zero_()
+            raise np.linalg.LinAlgError("Singular matrix")
 
     def run_batch(self, perms):
         """Maxima (P, C, signs, n_seg) for the permutation index rows `perms`."""
