@@ -59,7 +59,7 @@ const char* tfce_last_error(void);
  * into segments (hemispheres, surfaces of a multisurface study).  Entry b in
  * the list of a means "a is adjacent to b" exactly as the reference's
  * adjacencyList[a] (tfce_mediation/tfce.pyx:30-42).  Entries that point
- * outside [0, V) are rejected; self entries are dropped (the reference never
+ * outside [0, V) are rejected; repeated and self entries are dropped (the reference never
  * unions a vertex with itself); entries whose reverse is missing are marked so
  * the sweep applies the reference's insertion-order rule to them.
  * ------------------------------------------------------------------------- */

@@ -181,3 +181,19 @@ def test_overflowing_thresholds_stay_infinite():
     adj = A.AdjacencySet((off, idx), 2.0, 1.0)
     mx, om = _sweep(adj, x, 1, "component", np.ones(V, np.float32), want_maps=True)
     assert np.isinf(mx[0, 0, 0]) and np.isinf(om[0, 0, 10:20]).all()
+
+
+@pytest.mark.parametrize("V", [40, 4097])
+def test_repeated_entries_change_nothing(V):
+    """Lists that name a neighbour several times, from one side only, sweep as
+    the lists without the repeats."""
+    rng = np.random.default_rng(V)
+    off, idx = _graph("oneway", V, rng)
+    times = np.where(rng.random(len(idx)) < 0.3, 5, 1)
+    rows = np.repeat(np.repeat(np.arange(V), np.diff(off)), times)
+    again = (np.cumsum(np.r_[0, np.bincount(rows, minlength=V)]), np.repeat(idx, times))
+    maps = _maps(V, 4, rng)
+    vd = np.ones(V, np.float32)
+    got, want = (_sweep(A.AdjacencySet(g, 2.0, 1.0), maps, 2, "exact", vd, want_maps=True) for g in (again, (off, idx)))
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)

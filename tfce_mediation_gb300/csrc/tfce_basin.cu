@@ -34,18 +34,16 @@
 #include <map>
 
 #include "basin.cuh"
-#include "host_parallel.h"
+#include "basin_tables.h"
 #include "sweep_common.cuh"
 
 namespace tfgb {
 
-constexpr int kTile = 4096;            // vertices per tile at most (12 bits of a packed record)
 constexpr int kTileThreads = 512;
 constexpr int kPerThread = kTile / kTileThreads;
 constexpr int kBuckets = 256;          // sign * 128 + step
 constexpr int kTab = kBuckets + 2;     // bucket starts and the total
 constexpr uint32_t kNegative = 0x80000000u, kPositive = 0x40000000u;  // sign of a vertex of a tile
-constexpr uint32_t kOddRow = 0x80000000u;  // in edge_off: the second entries of the row's last words are padding
 constexpr uint32_t kRoot = 0x80000000u;
 constexpr uint32_t kExtent = 0x00ffffffu;
 constexpr int kPairTable = 2048;       // slots for the distinct pairs of basins of a tile
@@ -56,38 +54,13 @@ constexpr int kCrossThreads = 256;
 constexpr int kCrossPer = 4;
 constexpr int kCrossRows = 4;           // rows of neighbours whose loads are in flight together
 constexpr int kCrossQueue = 64;         // 31 and a row's worth
-constexpr int kCrossChunk = kCrossThreads * kCrossPer;
+static_assert(kCrossChunk == kCrossThreads * kCrossPer, "a CTA takes a chunk");
 constexpr int kMaxSweepThreads = 1024;
-constexpr int kTileEntries = 120000;   // list entries per tile: pairs are counted in 16 bits
 constexpr int kSmBytes = 226 * 1024;   // shared memory of an SM's sweeps together
 constexpr int kSweepBytes = 4352;      // of a sweep besides its state
 constexpr int kFindLimit = 1 << 26;
 constexpr int kAhead = 4;              // pairs of events that a thread of the sweep loads a step ahead
 constexpr uint32_t kNone = 0xffffffffu;
-
-struct TileInfo {
-  int32_t pos0;    // first list position (a multiple of 32)
-  int32_t nv;      // vertices
-  int32_t seg;
-  int32_t slice0;  // first slice (32 vertices each) of the neighbour and of the edge rows
-  int32_t bnd0;    // boundary vertices of the tile: [bnd0, bnd0 + nbnd)
-  int32_t nbnd;
-  int32_t pair0;   // first pair record
-  int32_t in_seg;  // index of the tile in its segment
-};
-
-struct ChunkInfo {
-  int32_t seg;
-  int32_t bnd0, nbnd;  // boundary vertices of the chunk
-  int32_t slice0;
-  int32_t pair0;       // first crossing-pair record
-  int32_t pad;
-};
-
-struct SegInfo {
-  int32_t tile0, ntiles, chunk0, nchunks;
-  int64_t pos0, pair0;  // first entries of the segment's ordered lists
-};
 
 struct Node {
   float inc;
@@ -1547,8 +1520,6 @@ int upload(BasinPlan* p, const std::vector<T>& h, T** d) {
   return TFCE_OK;
 }
 
-int64_t up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
-
 // workspace of a launch of M maps
 struct Layout {
   int64_t head, ev, pairs, cpairs, tab_ev, tab_pair, tab_cross, n_pairs, queue, n_basin, bnd, off_ev, off_pair, off_cross, base_of,
@@ -1560,7 +1531,7 @@ Layout layout_of(const BasinPlan* p, int64_t M, int signs, int mode, int64_t nod
   int64_t o = 0;
   auto take = [&](int64_t bytes) {
     const int64_t at = o;
-    o += up(bytes, 256);
+    o += round_up(bytes, 256);
     return at;
   };
   l.head = take(256 + M * 2 * p->n_seg * 4);
@@ -1699,293 +1670,36 @@ int basin_resident_items(const BasinPlan* p, bool dense) {
 int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_t>& packed,
                       const std::vector<int64_t>& seg, BasinPlan** out) {
   *out = nullptr;
-  const int64_t V = static_cast<int64_t>(off.size()) - 1;
-  const int n_seg = static_cast<int>(seg.size()) - 1;
-  const uint32_t kOne = 0x80000000u, kIdx = 0x7fffffffu;
-  // Tiles: patches grown breadth first from one vertex, so that few entries
-  // cross; a patch that cannot grow goes on from the next free vertex, so that
-  // all tiles of a segment but the last are full.  Inside a tile the vertices
-  // keep their order, so that the statistic is read in runs.
-  std::vector<int32_t> mark(V, -1), tile_of(V);
-  std::vector<std::vector<std::vector<int32_t>>> grown(n_seg);
-  parallel_for(n_seg, V, [&](int64_t s) {
-    constexpr int32_t kTaken = 0x7fffffff;  // in mark: in a tile; else the last tile that queued the vertex
-    std::vector<int32_t> queue(seg[s + 1] - seg[s] + 1), rim;
-    int64_t scan = seg[s], left = seg[s + 1] - seg[s];
-    while (left > 0) {
-      const int32_t id = static_cast<int32_t>(grown[s].size());
-      std::vector<int32_t> members;
-      members.reserve(std::min<int64_t>(left, kTile));
-      int64_t entries = 0;
-      bool full = false;
-      size_t rim_at = 0;  // of the free vertices beside the last tile
-      while (!full && left > 0) {
-        while (rim_at < rim.size() && mark[rim[rim_at]] == kTaken) ++rim_at;
-        size_t head = 0, tail = 1;
-        if (rim_at < rim.size()) {
-          queue[0] = rim[rim_at];
-        } else {
-          while (mark[scan] == kTaken) ++scan;
-          queue[0] = static_cast<int32_t>(scan);
-        }
-        mark[queue[0]] = id;
-        for (; head < tail; ++head) {
-          const int32_t v = queue[head];
-          const int64_t e0 = off[v], e1 = off[v + 1];
-          if (static_cast<int>(members.size()) == kTile || (entries > 0 && entries + e1 - e0 > kTileEntries)) {
-            full = true;
-            break;
-          }
-          entries += e1 - e0;
-          mark[v] = kTaken;
-          members.push_back(v);
-          --left;
-          for (int64_t e = e0; e < e1; ++e) {
-            const int32_t u = static_cast<int32_t>(packed[e] & kIdx);
-            if (mark[u] < id) {
-              mark[u] = id;
-              queue[tail++] = u;
-            }
-          }
-        }
-        if (full || left == 0) rim.assign(queue.begin() + head, queue.begin() + tail);
-      }
-      grown[s].push_back(std::move(members));
-    }
-  });
-  std::vector<TileInfo> tiles;
-  std::vector<SegInfo> segs(n_seg);
-  std::vector<std::vector<int32_t>*> members;
-  int32_t vmax = 1;
-  for (int s = 0; s < n_seg; ++s) {
-    vmax = std::max<int32_t>(vmax, static_cast<int32_t>(seg[s + 1] - seg[s]));
-    segs[s].tile0 = static_cast<int32_t>(tiles.size());
-    segs[s].ntiles = static_cast<int32_t>(grown[s].size());
-    if (segs[s].ntiles > 32767) return TFCE_OK;  // tile numbers are 15-bit
-    for (int t = 0; t < segs[s].ntiles; ++t) {
-      TileInfo ti{};
-      ti.seg = s;
-      ti.nv = static_cast<int32_t>(grown[s][t].size());
-      ti.in_seg = t;
-      tiles.push_back(ti);
-      members.push_back(&grown[s][t]);
-    }
-  }
-  const int nt = static_cast<int>(tiles.size());
-  std::vector<uint16_t> local(V, 0);
-  parallel_for(nt, V, [&](int64_t t) {
-    std::vector<int32_t>& mem = *members[t];
-    std::sort(mem.begin(), mem.end());
-    for (size_t i = 0; i < mem.size(); ++i) {
-      local[mem[i]] = static_cast<uint16_t>(i);
-      tile_of[mem[i]] = tiles[t].in_seg;
-    }
-  });
-  // entries that basin_cross_kernel takes: to another tile, or one-way
-  auto crosses = [&](int64_t v, uint32_t entry) { return (entry & kOne) || tile_of[entry & kIdx] != tile_of[v]; };
-  // rows of neighbours and of pairs of neighbours, by tile
-  struct Rows {
-    std::vector<uint32_t> nbr, nbr_end, edge, edge_end;
-    int64_t n_edges = 0, n_basins = 0;
-  };
-  std::vector<Rows> rows(nt);
-  std::vector<uint8_t> is_bnd(V, 0);
-  parallel_for(nt, V, [&](int64_t t) {
-    const std::vector<int32_t>& mem = *members[t];
-    const int nv = tiles[t].nv;
-    Rows& r = rows[t];
-    // rows of 32 lanes, two entries (4 * index) a lane; padding: the vertex itself
-    auto put = [&](std::vector<uint32_t>& out, std::vector<uint32_t>& ends, const std::vector<uint16_t>& list,
-                   const std::vector<int32_t>& at, const std::vector<int32_t>& count) {
-      for (int i = 0; i < nv; i += 32) {
-        int width = 0;
-        for (int v = i; v < std::min(nv, i + 32); ++v) width = std::max(width, count[v]);
-        size_t o = out.size();
-        out.resize(o + static_cast<size_t>((width + 1) / 2) * 32);
-        for (int j = 0; j < width; j += 2)
-          for (int v = i; v < i + 32; ++v) {
-            const uint32_t self = std::min(v, nv - 1);
-            const int c = v < nv ? count[v] : 0;
-            const uint32_t x = j < c ? list[at[v] + j] : self, y = j + 1 < c ? list[at[v] + j + 1] : self;
-            out[o++] = 4u * x | (4u * y << 16);
-          }
-        ends.push_back(static_cast<uint32_t>(out.size()) | (width & 1 ? kOddRow : 0u));
-      }
-    };
-    std::vector<int32_t> at(nv + 1, 0), count(nv, 0), held_count(nv, 0);
-    for (int i = 0; i < nv; ++i) at[i + 1] = at[i] + static_cast<int32_t>(off[mem[i] + 1] - off[mem[i]]);
-    std::vector<uint16_t> near(at[nv]), held(at[nv]);
-    auto hold = [&](int v, int u) { held[at[v] + held_count[v]++] = static_cast<uint16_t>(u); };
-    for (int i = 0; i < nv; ++i) {
-      const int32_t v = mem[i];
-      for (int64_t e = off[v]; e < off[v + 1]; ++e) {
-        if (crosses(v, packed[e])) {
-          __atomic_store_n(&is_bnd[packed[e] & kIdx], uint8_t{1}, __ATOMIC_RELAXED);
-          __atomic_store_n(&is_bnd[v], uint8_t{1}, __ATOMIC_RELAXED);
-          continue;
-        }
-        const uint16_t u = local[packed[e] & kIdx];
-        near[at[i] + count[i]++] = u;
-        if (u < i) continue;
-        // each pair of neighbours once, held by the one that holds fewer so far
-        if (held_count[u] < held_count[i]) hold(u, i);
-        else hold(i, u);
-        ++r.n_edges;
-      }
-    }
-    put(r.nbr, r.nbr_end, near, at, count);
-    for (int pass = 0; pass < 4; ++pass)  // even out: a vertex hands one to a neighbour that holds two fewer
-      for (int i = 0; i < nv; ++i)
-        for (int j = 0; j < held_count[i]; ++j) {
-          const int u = held[at[i] + j];
-          if (held_count[u] + 1 < held_count[i]) {
-            held[at[i] + j] = held[at[i] + --held_count[i]];
-            hold(u, i);
-          }
-        }
-    put(r.edge, r.edge_end, held, at, held_count);
-    // Basins at most: of vertices that are all neighbours of one another only
-    // the highest can start one.  Covered greedily by triples and pairs.
-    std::vector<uint8_t> covered(nv, 0);
-    for (int i = 0; i < nv; ++i) {
-      if (covered[i]) continue;
-      covered[i] = 1;
-      ++r.n_basins;
-      int u = -1, w = -1;
-      for (int j = 0; j < count[i] && w < 0; ++j) {
-        const int x = near[at[i] + j];
-        if (covered[x]) continue;
-        if (u < 0) u = x;
-        else if (std::find(near.begin() + at[x], near.begin() + at[x] + count[x], u) != near.begin() + at[x] + count[x])
-          w = x;
-      }
-      if (u >= 0) covered[u] = 1;
-      if (w >= 0) covered[w] = 1;
-    }
-  });
-  // the tiles one after the other
-  std::vector<int32_t> vert, bnd_vert, bnd_of(V, -1);
-  std::vector<uint32_t> slice_off(1, 0), nbr, edge_off(1, 0), edge;
-  std::vector<uint16_t> bnd_local, bnd_tile;
-  std::vector<int64_t> seg_pairs(n_seg, 0), seg_basins(n_seg, 0);
-  int64_t n_pair = 0;
-  for (int t = 0; t < nt; ++t) {
-    TileInfo& ti = tiles[t];
-    Rows& r = rows[t];
-    const std::vector<int32_t>& mem = *members[t];
-    ti.pos0 = static_cast<int32_t>(vert.size());
-    ti.slice0 = static_cast<int32_t>(slice_off.size()) - 1;
-    ti.bnd0 = static_cast<int32_t>(bnd_vert.size());
-    ti.pair0 = static_cast<int32_t>(n_pair);
-    for (size_t i = 0; i < r.nbr_end.size(); ++i) {
-      slice_off.push_back(static_cast<uint32_t>(nbr.size()) + (r.nbr_end[i] & ~kOddRow));
-      edge_off.push_back(static_cast<uint32_t>(edge.size()) + r.edge_end[i]);
-    }
-    nbr.insert(nbr.end(), r.nbr.begin(), r.nbr.end());
-    edge.insert(edge.end(), r.edge.begin(), r.edge.end());
-    if (r.n_edges > 65535) return TFCE_OK;  // pairs are counted in 16 bits
-    seg_basins[ti.seg] += r.n_basins;
-    seg_pairs[ti.seg] += up(r.n_edges, 8);  // pairs of basins: at most one per pair of neighbours
-    n_pair += up(r.n_edges, 8);
-    for (int i = 0; i < ti.nv; ++i) {
-      vert.push_back(mem[i]);
-      if (is_bnd[mem[i]]) {
-        bnd_of[mem[i]] = static_cast<int32_t>(bnd_vert.size());
-        bnd_local.push_back(static_cast<uint16_t>(i));
-        bnd_vert.push_back(mem[i]);
-        bnd_tile.push_back(static_cast<uint16_t>(ti.in_seg));
-      }
-    }
-    ti.nbnd = static_cast<int32_t>(bnd_vert.size()) - ti.bnd0;
-    while (vert.size() % 32) vert.push_back(0);
-    if (n_pair > 0x7fffffffLL || vert.size() > 0x7fffffffull || nbr.size() >= (1ull << 32) || edge.size() >= (1ull << 31)) return TFCE_OK;
-    r = Rows();
-  }
-  // crossing lists, in chunks of boundary vertices of one segment
-  std::vector<ChunkInfo> chunks;
-  for (int s = 0; s < n_seg; ++s) {
-    segs[s].chunk0 = static_cast<int32_t>(chunks.size());
-    if (segs[s].ntiles) {
-      const TileInfo& first = tiles[segs[s].tile0];
-      const TileInfo& last = tiles[segs[s].tile0 + segs[s].ntiles - 1];
-      for (int32_t b0 = first.bnd0; b0 < last.bnd0 + last.nbnd; b0 += kCrossChunk) {
-        ChunkInfo c{};
-        c.seg = s;
-        c.bnd0 = b0;
-        c.nbnd = std::min<int32_t>(kCrossChunk, last.bnd0 + last.nbnd - b0);
-        chunks.push_back(c);
-      }
-    }
-    segs[s].nchunks = static_cast<int32_t>(chunks.size()) - segs[s].chunk0;
-  }
-  const int n_chunks = static_cast<int>(chunks.size());
-  std::vector<Rows> crows(n_chunks);
-  parallel_for(n_chunks, V, [&](int64_t c) {
-    std::vector<uint32_t> list[32];
-    for (int i = 0; i < chunks[c].nbnd; i += 32) {
-      size_t width = 0;
-      for (int l = 0; l < 32; ++l) {
-        list[l].clear();
-        if (i + l >= chunks[c].nbnd) continue;
-        const int32_t v = bnd_vert[chunks[c].bnd0 + i + l];
-        for (int64_t e = off[v]; e < off[v + 1]; ++e)
-          if (crosses(v, packed[e])) list[l].push_back(static_cast<uint32_t>(bnd_of[packed[e] & kIdx]));
-        crows[c].n_edges += static_cast<int64_t>(list[l].size());
-        width = std::max(width, list[l].size());
-      }
-      for (size_t j = 0; j < width; ++j)
-        for (int l = 0; l < 32; ++l) {
-          const int self = std::min(i + l, chunks[c].nbnd - 1);  // padding: the vertex itself
-          crows[c].nbr.push_back(j < list[l].size() ? list[l][j] : static_cast<uint32_t>(chunks[c].bnd0 + self));
-        }
-      crows[c].nbr_end.push_back(static_cast<uint32_t>(crows[c].nbr.size()));
-    }
-  });
-  std::vector<uint32_t> cross_off(1, 0), cross;
-  int64_t n_cpair = 0;
-  for (int c = 0; c < n_chunks; ++c) {
-    chunks[c].slice0 = static_cast<int32_t>(cross_off.size()) - 1;
-    chunks[c].pair0 = static_cast<int32_t>(n_cpair);
-    for (uint32_t e : crows[c].nbr_end) cross_off.push_back(static_cast<uint32_t>(cross.size()) + e);
-    cross.insert(cross.end(), crows[c].nbr.begin(), crows[c].nbr.end());
-    n_cpair += up(crows[c].n_edges, 4);
-    seg_pairs[chunks[c].seg] += up(crows[c].n_edges, 4);
-    if (n_cpair > 0x7fffffffLL || cross.size() >= (1ull << 32)) return TFCE_OK;
-  }
-  int64_t n_opair = 0;
-  for (int s = 0; s < n_seg; ++s) {
-    segs[s].pos0 = seg[s];
-    segs[s].pair0 = n_opair;
-    n_opair += seg_pairs[s];
-  }
+  BasinTables t;
+  if (!build_basin_tables(off, packed, seg, &t)) return TFCE_OK;
   BasinPlan* p = new BasinPlan();
   cudaGetDevice(&p->device);
   cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
-  p->n_seg = n_seg;
-  p->vmax = vmax;
-  p->basins = static_cast<int32_t>(std::max<int64_t>(1, *std::max_element(seg_basins.begin(), seg_basins.end())));
-  p->V = V;
-  p->n_pos = static_cast<int64_t>(vert.size());
-  p->n_pair = n_pair;
-  p->n_cpair = n_cpair;
-  p->n_opair = n_opair;
-  p->n_tiles = nt;
-  p->n_chunks = static_cast<int32_t>(chunks.size());
-  p->n_bnd = static_cast<int32_t>(bnd_vert.size());
-  int rc = upload(p, tiles, &p->tiles);
-  if (!rc) rc = upload(p, chunks, &p->chunks);
-  if (!rc) rc = upload(p, segs, &p->segs);
-  if (!rc) rc = upload(p, vert, &p->vert);
-  if (!rc) rc = upload(p, slice_off, &p->slice_off);
-  if (!rc) rc = upload(p, nbr, &p->nbr);
-  if (!rc) rc = upload(p, edge_off, &p->edge_off);
-  if (!rc) rc = upload(p, edge, &p->edge);
-  if (!rc) rc = upload(p, bnd_local, &p->bnd_local);
-  if (!rc) rc = upload(p, bnd_vert, &p->bnd_vert);
-  if (!rc) rc = upload(p, bnd_tile, &p->bnd_tile);
-  if (!rc) rc = upload(p, cross_off, &p->cross_off);
-  if (!rc) rc = upload(p, cross, &p->cross);
-  std::vector<const double*> none(n_seg, nullptr);
+  p->n_seg = static_cast<int32_t>(seg.size()) - 1;
+  p->vmax = t.vmax;
+  p->basins = t.basins;
+  p->V = seg.back();
+  p->n_pos = static_cast<int64_t>(t.vert.size());
+  p->n_pair = t.n_pair;
+  p->n_cpair = t.n_cpair;
+  p->n_opair = t.n_opair;
+  p->n_tiles = static_cast<int32_t>(t.tiles.size());
+  p->n_chunks = static_cast<int32_t>(t.chunks.size());
+  p->n_bnd = static_cast<int32_t>(t.bnd_vert.size());
+  int rc = upload(p, t.tiles, &p->tiles);
+  if (!rc) rc = upload(p, t.chunks, &p->chunks);
+  if (!rc) rc = upload(p, t.segs, &p->segs);
+  if (!rc) rc = upload(p, t.vert, &p->vert);
+  if (!rc) rc = upload(p, t.slice_off, &p->slice_off);
+  if (!rc) rc = upload(p, t.nbr, &p->nbr);
+  if (!rc) rc = upload(p, t.edge_off, &p->edge_off);
+  if (!rc) rc = upload(p, t.edge, &p->edge);
+  if (!rc) rc = upload(p, t.bnd_local, &p->bnd_local);
+  if (!rc) rc = upload(p, t.bnd_vert, &p->bnd_vert);
+  if (!rc) rc = upload(p, t.bnd_tile, &p->bnd_tile);
+  if (!rc) rc = upload(p, t.cross_off, &p->cross_off);
+  if (!rc) rc = upload(p, t.cross, &p->cross);
+  std::vector<const double*> none(p->n_seg, nullptr);
   if (!rc) rc = upload(p, none, &p->seg_pow);
   if (rc) {
     basin_plan_destroy(p);
@@ -2065,7 +1779,7 @@ int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st) {
     if (const int cap_ctas = most_ctas()) large_ctas = std::min(large_ctas, cap_ctas);
     large_ctas = static_cast<int>(std::min<int64_t>(large_ctas, items_max));
   }
-  const int64_t state = !large_ctas ? 0 : up((int64_t)p->basins * state_bytes_per_basin(mode, kAllGlobal), 256);
+  const int64_t state = !large_ctas ? 0 : round_up((int64_t)p->basins * state_bytes_per_basin(mode, kAllGlobal), 256);
   const Layout lay = layout_of(p, per, r.signs, mode, cap);
   const int rc = ensure_ws(p, lay.total + large_ctas * state);
   if (rc) return rc;

@@ -34,15 +34,15 @@
 // Every walk and retry loop is bounded; a bound sets an error word and the
 // kernel runs on to its exit.
 #include <algorithm>
-#include <atomic>
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <string>
 #include <vector>
 
 #include "basin.cuh"
-#include "host_parallel.h"
+#include "basin_tables.h"
 #include "sweep_common.cuh"
 
 namespace tfgb {
@@ -52,8 +52,6 @@ constexpr int kBitmapMaxBytes = 48 * 1024;
 constexpr int kSweepThreads = 512;
 constexpr int kSweepMinBlocks = 3;  // 3 x 512 threads per SM (40 registers; a few spills)
 constexpr int kUBatch = 6;          // list entries of one vertex looked up together
-constexpr uint32_t kOneWay = 0x80000000u;   // entry whose reverse entry is missing
-constexpr uint32_t kIndexMask = 0x7fffffffu;
 constexpr uint32_t kInactiveKey = 0xffffffffu;
 constexpr int kPosBits = 24;                 // key = step << 24 | position
 constexpr int32_t kMaxSegVertices = (1 << kPosBits) - 1;
@@ -858,63 +856,21 @@ int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n
     TFGB_CHECK_ARG(std::isfinite(H[s]) && std::isfinite(E[s]), "H/E must be finite");
   }
 
-  // Clean the lists: validate, drop self entries, mark entries whose reverse
-  // is missing.  Neighbour order inside a list never changes the partition.
-  // An entry is rejected, the first of them, if it is outside the graph or its
-  // vertex's segment.
-  auto segment_of = [&](int64_t v) { return std::upper_bound(seg.begin(), seg.end(), v) - seg.begin() - 1; };
-  const int64_t blocks = (V + 4095) / 4096;
-  std::vector<int64_t> off(V + 1, 0), kept(blocks + 1, 0), bad(blocks, -1);
-  tfgb::parallel_for(blocks, D, [&](int64_t k) {
-    int64_t v = k * 4096, s = segment_of(v);
-    for (; v < std::min<int64_t>(V, (k + 1) * 4096); ++v) {
-      while (v >= seg[s + 1]) ++s;
-      int64_t n = 0;
-      for (int64_t e = offsets[v]; e < offsets[v + 1]; ++e) {
-        if ((indices[e] < seg[s] || indices[e] >= seg[s + 1]) && bad[k] < 0) bad[k] = e;
-        n += indices[e] != v;
-      }
-      kept[k + 1] += n;
-    }
-  });
-  for (int64_t e : bad) {
-    if (e < 0) continue;
-    const int32_t v = static_cast<int32_t>(std::upper_bound(offsets, offsets + V + 1, e) - offsets - 1);
-    if (indices[e] < 0 || indices[e] >= V) tfgb::set_error("adjacency entry %d of vertex %d outside [0, %d)", indices[e], v, V);
-    else tfgb::set_error("adjacency entry %d of vertex %d crosses segments", indices[e], v);
+  tfgb::CleanLists lists;
+  std::string error;
+  if (!tfgb::clean_lists(offsets, indices, V, seg, &lists, &error)) {
+    tfgb::set_error("%s", error.c_str());
     return TFCE_EINVAL;
   }
-  for (int64_t k = 0; k < blocks; ++k) kept[k + 1] += kept[k];
-  std::vector<int32_t> idx(kept[blocks]);
-  tfgb::parallel_for(blocks, D, [&](int64_t k) {
-    int64_t o = kept[k];
-    for (int64_t v = k * 4096; v < std::min<int64_t>(V, (k + 1) * 4096); ++v) {
-      const int64_t o0 = o;
-      for (int64_t e = offsets[v]; e < offsets[v + 1]; ++e)
-        if (indices[e] != v) idx[o++] = indices[e];
-      off[v + 1] = o;
-      if (!std::is_sorted(idx.begin() + o0, idx.begin() + o)) std::sort(idx.begin() + o0, idx.begin() + o);
-    }
-  });
-  std::vector<uint32_t> packed(idx.size());
-  std::atomic<bool> two_way{true};
-  tfgb::parallel_for(blocks, D, [&](int64_t k) {
-    for (int64_t v = k * 4096; v < std::min<int64_t>(V, (k + 1) * 4096); ++v)
-      for (int64_t e = off[v]; e < off[v + 1]; ++e) {
-        const int32_t b = idx[e];
-        const bool rev = std::binary_search(idx.begin() + off[b], idx.begin() + off[b + 1], static_cast<int32_t>(v));
-        packed[e] = static_cast<uint32_t>(b) | (rev ? 0u : tfgb::kOneWay);
-        if (!rev) two_way = false;
-      }
-  });
-  const bool symmetric = two_way;
+  const std::vector<int64_t>& off = lists.off;
+  const std::vector<uint32_t>& packed = lists.packed;
 
   tfce_adjset* h = new tfce_adjset();
   cudaGetDevice(&h->device);
   h->V = V;
   h->D = static_cast<int64_t>(packed.size());
   h->n_seg = n_seg;
-  h->symmetric = symmetric;
+  h->symmetric = lists.symmetric;
   h->vmax_seg = vmax;
   h->seg_off = seg;
   h->H.assign(H, H + n_seg);
