@@ -347,6 +347,12 @@ class AdjacencySet:
         _lib.check(self._lib.tfce_adjset_set_threshold_groups(self._h, _lib.ptr(g, _lib.c_i32p)))
         self.threshold_groups = g.copy()
 
+    def settings(self):
+        """What a captured sweep depends on besides its arguments (H and E are
+        read from the device): equal tuples sweep alike."""
+        g = self.threshold_groups
+        return self._h.value, self.accumulation, self.ctas_per_sm, None if g is None else tuple(g.tolist())
+
     def set_sweep_shape(self, ctas_per_sm: int):
         """Shape of the batched sweeps: 3 (more sweeps resident, each with room
         for 4,096 local maxima of its map in shared memory) or 2 (fewer, 9,300)."""

@@ -625,7 +625,8 @@ struct tfce_adjset {
   int32_t accumulation = 0;  // 0: reference arithmetic, 1: per-component
   bool no_max_only = false;  // accumulation 2: the potential form for maxima-only launches too
   int32_t sweep_shape = 3;   // 3: more sweeps resident, 2: fewer, with more shared state each
-  int32_t* d_group = nullptr;  // threshold group of every segment, or NULL
+  int32_t* d_group = nullptr;  // threshold group of every segment
+  bool grouped = false;        // the sweeps use them
   float* d_segmax = nullptr;   // segment maxima of the last grouped launch
   int64_t segmax_cap = 0;
   // Device buffers replaced by larger ones.  A launch captured into a CUDA
@@ -724,7 +725,7 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
     r.exact = !lazy;
     r.potentials = lazy && h->no_max_only;
     r.dense = h->sweep_shape == 3;
-    r.thr_group = h->d_group;
+    r.thr_group = h->grouped ? h->d_group : nullptr;
     r.d_H = h->d_H;
     r.d_E = h->d_E;
     r.d_seg_off = h->d_seg_off;
@@ -768,7 +769,7 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
   a.seg_rank = h->d_segrank;
   const int bm = tfgb::bitmap_bytes(h->vmax_seg);
   a.bm_words = bm / 4;
-  if (h->d_group) {
+  if (h->grouped) {
     const int64_t need = (int64_t)n_maps * signs * h->n_seg;
     if (h->segmax_cap < need) {
       const int64_t cap = std::max(need, 2 * h->segmax_cap);
@@ -959,14 +960,14 @@ int tfce_adjset_set_threshold_groups(tfce_adjset* h, const int32_t* group) {
   tfgb::clear_error();
   TFGB_CHECK_ARG(h != nullptr, "handle is NULL");
   std::lock_guard<std::mutex> lk(h->mu);
-  if (!group) {
-    cudaFree(h->d_group);
-    h->d_group = nullptr;
+  if (!group) {  // a captured launch may still read the ids: they stay until the handle goes
+    h->grouped = false;
     return TFCE_OK;
   }
   for (int s = 0; s < h->n_seg; ++s) TFGB_CHECK_ARG(group[s] >= 0 && group[s] < h->n_seg, "group id outside [0, n_seg)");
   if (!h->d_group) TFGB_CUDA(cudaMalloc(&h->d_group, sizeof(int32_t) * h->n_seg));
   TFGB_CUDA(cudaMemcpy(h->d_group, group, sizeof(int32_t) * h->n_seg, cudaMemcpyHostToDevice));
+  h->grouped = true;
   return TFCE_OK;
 }
 

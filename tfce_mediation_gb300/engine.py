@@ -205,11 +205,18 @@ class PermutationEngine:
         return out
 
     def _base(self):
-        """The design on the device, and its columns: every one permuted."""
+        """The design on the device, and its columns: every one permuted.  A
+        design that was changed goes up again, into the same memory (captured
+        batches read it)."""
         if not hasattr(self, "_X_d"):
-            np.linalg.inv(self.X.T @ self.X)  # a design without an inverse raises here
             self._cols_d = dev(np.arange(self.k, dtype=np.int32) + TensorCoreOperands.PERMUTED)
-            self._X_d = dev(self.X)
+            self._X_d = self.t.empty(self.X.shape, device="cuda", dtype=self.t.float64)
+            self._X_up = None
+        if self._X_up is None or not np.array_equal(self._X_up, self.X):
+            np.linalg.inv(self.X.T @ self.X)  # a design without an inverse raises here
+            X = np.array(self.X, np.float64)
+            self._X_d.copy_(self.t.from_numpy(X))
+            self._X_up = X
         return self._X_d, self._cols_d
 
     def _tmaps_of(self, perms):
@@ -364,9 +371,13 @@ class PermutationEngine:
 
     def _graph_form(self):
         """What a captured batch depends on: its size, the GLM's form and, with
-        the residual epilogue, the designs per tile."""
-        qf = self._graph_qf()
-        return self.batch, qf, self._program_on_device(), None if qf or self._tc is None else self._tc.block(self.k)
+        the residual epilogue, the designs per tile; what is tested; the sweep's
+        settings (the handle may be shared) and the memory it reads."""
+        qf, tc = self._graph_qf(), self._tc
+        return (self.batch, qf, self._program_on_device(), None if qf or tc is None else tc.block(self.k),
+                tuple(self.contrasts), self.signs, self.floor_zero, self.adj.settings(),
+                *(None if x is None else x.data_ptr() for x in (self.vd, self.Yd, self._coef)),
+                None if tc is None else tc.yt.data_ptr())
 
     def _graph_slot(self, P):
         """One captured batch: pinned design operators -> device, glm_tstat,
@@ -374,7 +385,7 @@ class PermutationEngine:
         t = self.t
         n, kmax = self.n, self.k
         tc = self._tc
-        slot = {"P": P, "form": self._graph_form()}
+        slot = {"P": P, "form": self._graph_form(), "held": (self.vd, self.Yd, self._coef, tc)}
         qf = self._graph_qf()
         program = not qf and self._program_on_device()
         slot["on_device"] = qf or program  # designs formed on the device from index rows
@@ -462,6 +473,7 @@ class PermutationEngine:
 
     def _fill(self, slot, perms):
         if slot["on_device"]:
+            self._base()
             self._index_rows(perms, out=slot["h_rows"].numpy())
             return
         db = DesignBatch(self.X[perms])
@@ -671,10 +683,12 @@ class MediationEngine:
         """Base columns of the path designs on the device -- pred_x, depend_y,
         covariates -- and the columns of each path ([1, x] and [1, dy, x] for
         'M', pyfunc.py:131-145), those of permuted variables flagged."""
-        if not hasattr(self, "_Z_d"):
-            x, dy = self.pred_x.reshape(self.n, -1), self.depend_y.reshape(self.n, -1)
-            cov = np.zeros((self.n, 0)) if self.cov is None else self.cov.reshape(self.n, -1)
-            nx, ny, nc = x.shape[1], dy.shape[1], cov.shape[1]
+        x, dy = self.pred_x.reshape(self.n, -1), self.depend_y.reshape(self.n, -1)
+        cov = np.zeros((self.n, 0)) if self.cov is None else self.cov.reshape(self.n, -1)
+        Z = np.hstack([x, dy, cov])
+        nx, ny, nc = x.shape[1], dy.shape[1], cov.shape[1]
+        key = self.medtype, nx, ny, nc
+        if getattr(self, "_paths_of", None) != key:
             cx = [j + TensorCoreOperands.PERMUTED for j in range(nx)]
             cy = [nx + j + (TensorCoreOperands.PERMUTED if self.medtype == "Y" else 0) for j in range(ny)]
             cc = [nx + ny + j for j in range(nc)]
@@ -682,8 +696,10 @@ class MediationEngine:
             cols = np.full((len(paths), self.kmax), -1, np.int32)
             for i, path in enumerate(paths):
                 cols[i, 1:1 + len(path)] = path
-            self._paths_d = dev(cols)
-            self._Z_d = dev(np.hstack([x, dy, cov]))
+            self._paths_d, self._paths_of = dev(cols), key
+            self._Z_up = None
+        if self._Z_up is None or not np.array_equal(self._Z_up, Z):
+            self._Z_d, self._Z_up = dev(Z), Z
         return self._Z_d, self._paths_d
 
     def _on_device(self):
