@@ -104,3 +104,23 @@ def test_mediation_designs_follow_changes():
     eng.depend_y = eng.depend_y + 3.0 * rng.standard_normal(40)
     eng.pred_x[:, 0] *= np.arange(40)
     np.testing.assert_array_equal(eng.run(perms=rows), fresh(eng.pred_x, eng.depend_y).run(perms=rows))
+
+
+@pytest.mark.parametrize("precision,outputs", [("bf16x3", None), ("fp32", None), ("bf16x3", [("t", 1)])])
+def test_a_subclass_forms_its_own_designs(precision, outputs):
+    """Designs that an engine of one's own hands out are the ones that are run."""
+    import torch
+
+    class Own(engine.PermutationEngine):
+        def _designs(self, perms):
+            return ("designs of", perms.shape[0])
+
+        def tmaps(self, designs, out=None, precision=None):
+            return designs
+
+    eng = _bare_engine(torch)
+    eng.__class__ = Own
+    eng.precision, eng.outputs = precision, outputs
+    if precision == "bf16x3":
+        eng._tc, eng._centred = types.SimpleNamespace(quadratic_form=True, yy=1), True
+    assert eng._tmaps_of(np.zeros((3, 4), np.int64)) == ("designs of", 3)

@@ -233,7 +233,8 @@ class PermutationEngine:
             return out
         if self._fp32_on_device():
             return self._tmaps_fp32(perms)
-        if not self._graph_qf() or len(self.contrasts) > 8:
+        if (not self._graph_qf() or len(self.contrasts) > 8
+                or type(self)._designs is not PermutationEngine._designs):  # a subclass forms its own
             return self.tmaps(self._designs(perms))
         tc, out = self._tc, self._tbuf[:P]
         base, cols = self._base()
