@@ -197,3 +197,33 @@ def test_repeated_entries_change_nothing(V):
     got, want = (_sweep(A.AdjacencySet(g, 2.0, 1.0), maps, 2, "exact", vd, want_maps=True) for g in (again, (off, idx)))
     for a, b in zip(got, want):
         np.testing.assert_array_equal(a, b)
+
+
+def test_infinities_are_inactive_in_both_forms():
+    """Infinite values between components, of either sign: the single map, its
+    labels, the batch and the allocation-free call leave them out alike."""
+    import torch
+    from tfce_mediation_gb300 import _lib
+    V = 300
+    off, idx = _graph("ring", V, np.random.default_rng(0))
+    x = (1.5 + np.sin(np.arange(V) / 7.0)).astype(np.float32)
+    x[[40, 41, 90]] = np.inf
+    x[[150, 200]] = -np.inf
+    x[[250, 260]] = -2.0
+    adj = A.AdjacencySet((off, idx), 2.0, 1.0)
+    one = np.zeros(V, np.float32)
+    adj.run(x, one)
+    img = np.where(np.isfinite(x), x, 0.0).astype(np.float32)
+    np.testing.assert_array_equal(one, oracle.tfce(off, idx, img, 2.0, 1.0, hh_exact=True))
+    enhn, labels, _ = adj.run_labels(x)
+    np.testing.assert_array_equal(enhn, one)
+    assert (labels[:, ~np.isfinite(x)] == -1).all()
+    mx, om = _sweep(adj, x[None], 2, "exact", None, want_maps=True)
+    np.testing.assert_array_equal(om[0, 0], (one * np.float32(img.max() / np.float32(100.0))).astype(np.float32))
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda()
+         for a in (off, idx, np.array([0, V]), np.array([2.0], np.float32), np.array([1.0], np.float32), x)]
+    out = torch.full((1, 2, 1), -1.0, device="cuda")
+    o, i, seg, H, E, xd = (a.data_ptr() for a in d)
+    _lib.check(_lib.load().tfce_sweep_batch_noalloc(o, i, V, len(idx), seg, 1, V, H, E, xd, V, 1, 2, None, 0,
+                                                    out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    np.testing.assert_array_equal(out.cpu().numpy(), mx)

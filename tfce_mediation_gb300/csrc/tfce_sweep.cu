@@ -291,8 +291,8 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepMinBlocks) tfce_sweep_ker
     // ---- 2. activation step per vertex, bucket histogram
     for (int32_t v = tid; v < Vs; v += nth) {
       const float xv = sign * x[v];
-      int lv = L;  // L == never active
-      if (L > 0 && xv > sT[L - 1]) {
+      int lv = L;  // L == never active: values that are not finite too
+      if (L > 0 && isfinite(xv) && xv > sT[L - 1]) {
         int lo = 0, hi = L - 1;  // smallest i with xv > T[i]; T decreasing
         while (lo < hi) {
           const int mid = (lo + hi) >> 1;
