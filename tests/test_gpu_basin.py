@@ -227,3 +227,24 @@ def test_infinities_are_inactive_in_both_forms():
     _lib.check(_lib.load().tfce_sweep_batch_noalloc(o, i, V, len(idx), seg, 1, V, H, E, xd, V, 1, 2, None, 0,
                                                     out.data_ptr(), torch.cuda.current_stream().cuda_stream))
     np.testing.assert_array_equal(out.cpu().numpy(), mx)
+
+
+def test_many_exponents_on_one_handle():
+    """A handle that is given one exponent after the other: every sweep uses its
+    own, earlier ones included, and the tables do not pile up."""
+    import torch
+    V = 50_000
+    off, idx = _graph("ring", V, np.random.default_rng(0))
+    x = np.abs(np.random.default_rng(1).standard_normal(V)).astype(np.float32)
+    adj = A.AdjacencySet((off, idx), 2.0, 1.0)
+    exps = [0.5] + [0.5 + i / 64 for i in range(1, 60)] + [0.5, 1.0, 2.0]
+    first = None
+    for i, E in enumerate(exps):
+        adj.set_params(2.0, E)
+        mx, _ = _sweep(adj, x[None], 1, "exact")
+        if E in (0.5, 1.0, 2.0):
+            raw = oracle.tfce(off, idx, x, 2.0, E, hh_exact=True)
+            assert mx[0, 0, 0] == (raw * np.float32(x.max() / np.float32(100.0))).max()
+        if i == 20:
+            first = torch.cuda.mem_get_info()[0]
+    assert first - torch.cuda.mem_get_info()[0] < 20 * 8 * (V + 1) + (8 << 20)

@@ -29,6 +29,24 @@ enum DevErr : int32_t {
 // output kinds of the programmed GLM epilogue (glm_stat_tc mode 3)
 constexpr int kTcOutT = 0, kTcOutNegT = 1, kTcOutF = 2, kTcOutAmp = 3, kTcOutAcro = 4, kTcOutEss = 5;
 
+// Makes a device current for its lifetime.
+class OnDevice {
+ public:
+  explicit OnDevice(int device) {
+    cudaGetDevice(&before_);
+    if (device != before_) cudaSetDevice(device);
+    else before_ = -1;
+  }
+  ~OnDevice() {
+    if (before_ >= 0) cudaSetDevice(before_);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+
+ private:
+  int before_ = -1;
+};
+
 inline int map_dev_err(int32_t e) {
   switch (e) {
     case kDevOk: return TFCE_OK;

@@ -1501,7 +1501,7 @@ struct BasinPlan {
   uint32_t* cross_off = nullptr;
   uint32_t* cross = nullptr;
   const double** seg_pow = nullptr;
-  std::map<float, double*> powers;  // extent^E tables; kept: a captured launch reads them through seg_pow
+  std::map<float, double*> powers;  // extent^E tables (read through seg_pow)
   // A buffer that is replaced by a larger one may still be used by a captured
   // launch: it is kept until the plan goes.  Growth is geometric.
   char* ws = nullptr;
@@ -1566,6 +1566,8 @@ Layout layout_of(const BasinPlan* p, int64_t M, int signs, int mode, int64_t nod
 }
 
 constexpr int64_t kWorkspaceBudget = 8LL << 30;  // maps are swept in as many launches as this asks for
+
+constexpr size_t kPowersKept = 16;  // tables of extent^E that a handle holds on to besides those in use
 
 int64_t node_capacity(const BasinPlan* p) { return (int64_t)p->basins * kMaxSteps; }
 
@@ -1723,6 +1725,7 @@ void basin_plan_destroy(BasinPlan* p) {
 }
 
 int basin_plan_set_exponents(BasinPlan* p, const float* E) {
+  const OnDevice on(p->device);
   std::vector<const double*> rows(p->n_seg, nullptr);
   for (int s = 0; s < p->n_seg; ++s) {
     if (E[s] == 1.0f) continue;
@@ -1731,14 +1734,27 @@ int basin_plan_set_exponents(BasinPlan* p, const float* E) {
       double* d = nullptr;
       const int64_t n = (int64_t)p->vmax + 1;
       TFGB_CUDA(cudaMalloc(&d, n * sizeof(double)));
-      it = p->powers.emplace(E[s], d).first;
       basin_power_kernel<<<static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, 1216)), 256>>>(d, n, E[s]);
-      TFGB_CUDA(cudaGetLastError());
-      TFGB_CUDA(cudaStreamSynchronize(nullptr));
+      cudaError_t e = cudaGetLastError();
+      if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+      if (e != cudaSuccess) cudaFree(d);  // a table that is not filled is not kept
+      TFGB_CUDA(e);
+      it = p->powers.emplace(E[s], d).first;
     }
     rows[s] = it->second;
   }
   TFGB_CUDA(cudaMemcpy(p->seg_pow, rows.data(), rows.size() * sizeof(double*), cudaMemcpyHostToDevice));
+  if (p->powers.size() > kPowersKept) {  // those of earlier exponents, once nothing reads them
+    TFGB_CUDA(cudaDeviceSynchronize());
+    for (auto it = p->powers.begin(); it != p->powers.end();) {
+      if (std::find(rows.begin(), rows.end(), it->second) != rows.end()) {
+        ++it;
+      } else {
+        cudaFree(it->second);
+        it = p->powers.erase(it);
+      }
+    }
+  }
   return TFCE_OK;
 }
 

@@ -794,6 +794,7 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
 
 // Reads and clears the sticky error word (synchronises the stream).
 int check_device_error(tfce_adjset* h, cudaStream_t st, int32_t* steps) {
+  const tfgb::OnDevice on(h->device);
   if (st) {
     TFGB_CUDA(cudaStreamSynchronize(st));
   } else {  // an event there waits for the blocking streams too, as a copy would
@@ -938,6 +939,7 @@ int tfce_adjset_set_params(tfce_adjset* h, const float* H, const float* E) {
   std::lock_guard<std::mutex> lk(h->mu);
   for (int s = 0; s < h->n_seg; ++s)
     TFGB_CHECK_ARG(std::isfinite(H[s]) && std::isfinite(E[s]), "H/E must be finite");
+  const tfgb::OnDevice on(h->device);
   h->H.assign(H, H + h->n_seg);
   h->E.assign(E, E + h->n_seg);
   TFGB_CUDA(cudaMemcpy(h->d_H, H, sizeof(float) * h->n_seg, cudaMemcpyHostToDevice));
@@ -965,6 +967,7 @@ int tfce_adjset_set_threshold_groups(tfce_adjset* h, const int32_t* group) {
     return TFCE_OK;
   }
   for (int s = 0; s < h->n_seg; ++s) TFGB_CHECK_ARG(group[s] >= 0 && group[s] < h->n_seg, "group id outside [0, n_seg)");
+  const tfgb::OnDevice on(h->device);
   if (!h->d_group) TFGB_CUDA(cudaMalloc(&h->d_group, sizeof(int32_t) * h->n_seg));
   TFGB_CUDA(cudaMemcpy(h->d_group, group, sizeof(int32_t) * h->n_seg, cudaMemcpyHostToDevice));
   h->grouped = true;
