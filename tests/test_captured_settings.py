@@ -124,3 +124,46 @@ def test_a_subclass_forms_its_own_designs(precision, outputs):
     if precision == "bf16x3":
         eng._tc, eng._centred = types.SimpleNamespace(quadratic_form=True, yy=1), True
     assert eng._tmaps_of(np.zeros((3, 4), np.int64)) == ("designs of", 3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("outputs", [None, [("t", 1), ("f", 1, 2)]])
+def test_maxima_of_a_singular_design_are_not_handed_on(outputs):
+    """A step whose designs have no inverse raises before its maxima reach
+    on_batch; the steps before it are handed on, and the engine goes on."""
+    st = synth.vertex_study(seed=2, level=2, n=40, passes=1, hemispheres=1, k=3, patches=((20, 0.8, 1),), name="s")
+    x = np.round(st.pred_x * 8)
+    eng = engine.PermutationEngine(st.Y, x, (st.offsets, st.indices), st.segments, 2.0, 1.0, batch=4, outputs=outputs)
+    rows = engine.permutations(st.n, 1, 0, 4)
+    bad = rows.copy()
+    bad[2] = 0  # one subject throughout
+    want = eng.run(perms=rows)
+    for order in ([rows, bad, rows, rows], [rows, rows, bad], [rows, rows, bad, rows]):
+        seen = []
+        with pytest.raises(np.linalg.LinAlgError):
+            eng.run_stream([(None, p) for p in order], on_batch=lambda i, m: seen.append((i, m)))
+        assert [i for i, _ in seen] == list(range([p is bad for p in order].index(True)))
+        for _, m in seen:
+            np.testing.assert_array_equal(m, want)
+    np.testing.assert_array_equal(eng.run_graph(perms=rows), want)
+
+
+@pytest.mark.gpu
+def test_mediation_steps_stop_at_a_singular_design():
+    st = synth.vertex_study(seed=2, level=2, n=40, passes=1, hemispheres=1, k=3, patches=((20, 0.8, 1),), name="s")
+    rng = np.random.default_rng(0)
+    eng = engine.MediationEngine(st.Y, np.round(rng.standard_normal((40, 1)) * 8), rng.standard_normal(40), "M",
+                                 (st.offsets, st.indices), st.segments, 2.0, 1.0, batch=4)
+    rows = engine.permutations(40, 1, 0, 4)
+    want = eng.run(perms=rows)
+    asked = []
+
+    def steps():
+        for i in range(6):
+            asked.append(i)
+            yield None, np.zeros_like(rows) if i == 1 else rows
+
+    with pytest.raises(np.linalg.LinAlgError):
+        eng.run_stream(steps())
+    assert asked[-1] < 5
+    np.testing.assert_array_equal(eng.run(perms=rows), want)

@@ -391,6 +391,7 @@ class PermutationEngine:
         program = not qf and self._program_on_device()
         slot["on_device"] = qf or program  # designs formed on the device from index rows
         if slot["on_device"]:
+            slot["h_err"] = t.zeros(1, dtype=t.int32, pin_memory=True)  # a design without an inverse, in this batch or before
             keys = ()
             base, cols = self._base()
             slot["h_rows"] = t.empty((P, n), dtype=t.int32, pin_memory=True)
@@ -449,6 +450,8 @@ class PermutationEngine:
             self.adj.sweep_batch(ptr(slot["d_t"]), self.V, P * self.C, self.signs, ptr(self.vd),
                                  int(self.floor_zero), ptr(slot["d_max"]), None, 0, stream_handle())
             slot["h_max"].copy_(slot["d_max"], non_blocking=True)
+            if slot["on_device"]:
+                slot["h_err"].copy_(tc.err, non_blocking=True)
 
         # warm-up outside capture (allocates the sweep workspace), then capture
         # two graphs: the GLM part (the last reader of the resident data) and
@@ -537,8 +540,10 @@ class PermutationEngine:
 
         def collect(slot):
             slot["event"].synchronize()
-            results[slot["order"]] = slot["h_max"].numpy()[: slot["rows"]].copy()
             slot["busy"] = False
+            if slot["on_device"] and int(slot["h_err"][0]):
+                self.status()  # raises: these maxima are not handed on
+            results[slot["order"]] = slot["h_max"].numpy()[: slot["rows"]].copy()
             if on_batch is not None:
                 on_batch(slot["order"], results[slot["order"]])
 
@@ -572,9 +577,8 @@ class PermutationEngine:
             slot["busy"], slot["order"], slot["rows"] = True, s_, rows
             prev = slot
             n_steps = s_ + 1
-        for slot in self._slots:
-            if slot.get("busy"):
-                collect(slot)
+        for slot in sorted((x for x in self._slots if x.get("busy")), key=lambda x: x["order"]):
+            collect(slot)
         self.status()
         return [results[i] for i in range(n_steps)]
 
@@ -790,6 +794,7 @@ class MediationEngine:
         if not hasattr(self, "_host_max"):
             self._host_max = [t.empty(self.batch * self.n_seg, dtype=t.float32, pin_memory=True) for _ in range(2)]
             self._max2 = [self._max.view(-1), t.empty_like(self._max.view(-1))]
+            self._host_err = t.zeros(2, dtype=t.int32, pin_memory=True)
             self._done = [t.cuda.Event(), t.cuda.Event()]
             self._glm_done = [t.cuda.Event(), t.cuda.Event()]
             self._up_stream = t.cuda.Stream()
@@ -800,6 +805,8 @@ class MediationEngine:
         def collect(item):
             k, P = item
             self._done[k].synchronize()
+            if int(self._host_err[k]):
+                inner.status()  # raises: a design without an inverse in this batch or before
             out.append(self._host_max[k][: P * self.n_seg].numpy().reshape(P, 1, 1, self.n_seg).copy())
 
         for i, (data, rows) in enumerate(steps):
@@ -824,6 +831,8 @@ class MediationEngine:
             inner.adj.sweep_batch(ptr(z), self.V, P, 1, ptr(inner.vd), int(inner.floor_zero),
                                   ptr(mx), None, 0, stream_handle())
             self._host_max[k][: P * self.n_seg].copy_(mx, non_blocking=True)
+            if inner._tc is not None:
+                self._host_err[k:k + 1].copy_(inner._tc.err, non_blocking=True)
             self._done[k].record(main)
             if prev is not None:
                 collect(prev)
