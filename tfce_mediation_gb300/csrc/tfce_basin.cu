@@ -61,6 +61,7 @@ constexpr int kSweepBytes = 4352;      // of a sweep besides its state
 constexpr int kFindLimit = 1 << 26;
 constexpr int kAhead = 4;              // pairs of events that a thread of the sweep loads a step ahead
 constexpr uint32_t kNone = 0xffffffffu;
+constexpr int kReady = 8;              // word of `counter`: the first of the sweep's launches sees the lists
 
 struct Node {
   float inc;
@@ -102,7 +103,7 @@ struct BasinArgs {
   int32_t n_tiles, n_chunks, n_bnd;
   // workspace
   uint32_t* seg_max;    // [maps][2][n_seg] bits of max(0, max)
-  int32_t* counter;     // items taken and, of the queued ones, there are: by class (2 * class, 2 * class + 1)
+  int32_t* counter;     // items taken and, of the queued ones, there are: by class (2 * class, 2 * class + 1); kReady
   uint32_t* ev;         // vertices of a tile by bucket: bucket << 24, index in the tile << 12, basin
   uint32_t* pairs;      // pairs of basins of a tile: bucket << 24, 12 bits each
   uint2* cpairs;        // crossing pairs: tile << 16 | 4 bits of the bucket << 12 | basin, twice
@@ -1361,9 +1362,23 @@ template <int kMode, bool kLarge>
 __global__ void __launch_bounds__(kLarge ? kMaxSweepThreads : 512, kLarge ? 1 : 2) basin_sweep_kernel(BasinArgs a) {
   __shared__ SweepShared S;
   extern __shared__ __align__(16) char dyn[];
-  if (a.first_class) after_previous();
-  else asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x, nth = blockDim.x;
+  // The lists are visible to the launch that waits for the kernel before it.  The
+  // launches beside it start after it has let them, and its release of `ready`
+  // before that makes the lists visible to whoever acquires it; should one find
+  // it unset, it waits for the launch before its own.
+  int32_t* const ready = a.counter + kReady;
+  if (a.first_class) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (tid == 0) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(ready), "r"(1) : "memory");
+    __syncthreads();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  } else {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    int32_t seen = 1;
+    if (tid == 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(ready) : "memory");
+    if (!__syncthreads_and(seen)) asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
   const int cls = kLarge ? 2 : a.mid;
   int32_t* const counter = a.counter + 2 * cls;
   const int32_t* const queue = a.queue + (kLarge ? a.n_items : 0);
