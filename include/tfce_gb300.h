@@ -143,7 +143,11 @@ int tfce_adjset_run_labels(tfce_adjset* h, const float* image, float* enhn, int3
  *             TFCE * (segment max / 100) * vdensity (pyfunc.py:116-118);
  *   out_maps  [n_maps][signs][V] or NULL; out_mode 1 writes the scaled map,
  *             out_mode 2 adds the raw sweep into out_maps (enhn semantics).
- * Uses a device workspace that the handle grows on demand. */
+ * Uses a device workspace that the handle grows on demand: at most 8 GiB (the
+ * maps are swept in several launches then; TFCE_SWEEP_WORKSPACE_MB caps it), half
+ * of the memory that is free for it, and less, down to a vertex-by-vertex sweep,
+ * where that is refused.  An outgrown workspace is freed (device-wide wait), or
+ * kept with the handle once a launch of the handle has been captured. */
 int tfce_sweep_batch(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t n_maps,
                      int32_t signs, const float* vdensity, int32_t floor_zero, float* out_max,
                      float* out_maps, int32_t out_mode, void* stream);

@@ -248,3 +248,59 @@ def test_many_exponents_on_one_handle():
         if i == 20:
             first = torch.cuda.mem_get_info()[0]
     assert first - torch.cuda.mem_get_info()[0] < 20 * 8 * (V + 1) + (8 << 20)
+
+
+@pytest.mark.parametrize("mode,weighted", [("component", False), ("exact", True)])
+def test_less_workspace_gives_the_same(mode, weighted, monkeypatch):
+    """Maps swept in one launch, in several (a small workspace), and vertex by
+    vertex (none): the same bits, for segments of uneven sizes and vertex values."""
+    rng = np.random.default_rng(8)
+    parts = [_graph(k, n, rng) for k, n in (("ring", 9000), ("isolated", 5), ("band", 4097), ("ring", 33))]
+    off, idx, seg = A.concat_csr(parts)
+    V = int(seg[-1])
+    maps = np.ascontiguousarray(rng.standard_normal((40, V)).astype(np.float32))
+    vd = (0.5 + rng.random(V)).astype(np.float32) if weighted else None
+    out = []
+    for mb in (None, "30", "5", "0"):
+        monkeypatch.delenv("TFCE_SWEEP_WORKSPACE_MB", raising=False)
+        if mb:
+            monkeypatch.setenv("TFCE_SWEEP_WORKSPACE_MB", mb)
+        adj = A.AdjacencySet((off, idx), 2.0, 1.0, seg)
+        out.append(_sweep(adj, maps, 2, mode, vd, want_maps=weighted))
+    for mx, om in out[1:]:
+        np.testing.assert_array_equal(mx, out[0][0])
+        if weighted:
+            np.testing.assert_array_equal(om, out[0][1])
+    for s, (o, i) in enumerate(parts):
+        img = np.ascontiguousarray(maps[7, seg[s]:seg[s + 1]])
+        raw = oracle.tfce(o, i, img, 2.0, 1.0, hh_exact=True)
+        val = (raw * np.float32(max(img.max(), 0) / np.float32(100.0))).astype(np.float32)
+        if weighted:
+            val = (val * vd[seg[s]:seg[s + 1]]).astype(np.float32)
+            np.testing.assert_array_equal(out[0][1][7, 0, seg[s]:seg[s + 1]], val)
+        assert out[0][0][7, 0, s] == val.max()
+
+
+def test_an_outgrown_workspace_is_given_back():
+    import torch
+    V = 40_000
+    off, idx = _graph("ring", V, np.random.default_rng(0))
+    maps = np.random.default_rng(1).standard_normal((64, V)).astype(np.float32)
+    adj = A.AdjacencySet((off, idx), 2.0, 1.0)
+    held = {}
+    for n in (1, 8, 64):
+        one = A.AdjacencySet((off, idx), 2.0, 1.0)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        _sweep(one, maps[:n], 2, "exact", np.ones(V, np.float32))
+        torch.cuda.empty_cache()
+        held[n] = before - torch.cuda.mem_get_info()[0]
+        del one
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    for n in (1, 8, 64):
+        want = _sweep(adj, maps[:n], 2, "exact", np.ones(V, np.float32))
+    torch.cuda.empty_cache()
+    # as much as the largest call alone takes (growth at least doubles: up to twice 8 maps' is no more than that)
+    assert before - torch.cuda.mem_get_info()[0] <= held[64] + (4 << 20)
+    np.testing.assert_array_equal(want[0][:8], _sweep(adj, maps[:8], 2, "exact", np.ones(V, np.float32))[0])

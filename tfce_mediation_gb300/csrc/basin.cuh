@@ -43,7 +43,8 @@ int basin_plan_set_exponents(BasinPlan* p, const float* E);
 // Whether the request can run in this form (the vertex values of the
 // reference's arithmetic need a node table that grows with the segment).
 bool basin_takes(const BasinPlan* p, const BasinRequest& r);
-int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st);
+// *refused: there was no memory for the workspace, and nothing was launched.
+int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st, bool* refused);
 // Items that a launch of many sweeps at once.
 int basin_resident_items(const BasinPlan* p, bool dense);
 

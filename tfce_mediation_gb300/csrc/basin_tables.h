@@ -112,6 +112,7 @@ struct ChunkInfo {
 struct SegInfo {
   int32_t tile0, ntiles, chunk0, nchunks;
   int64_t pos0, pair0;  // first entries of the segment's ordered lists
+  int64_t basin0;       // basins of one sign of the segments before it at most
 };
 inline int64_t round_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
@@ -126,6 +127,7 @@ struct BasinTables {
   int64_t n_pair = 0, n_cpair = 0, n_opair = 0;
   int32_t vmax = 1;    // vertices of the largest segment
   int32_t basins = 1;  // basins of one sign of a segment at most
+  int64_t all_basins = 0;  // of one sign of all segments
 };
 
 // The tables of cleaned lists (see CleanLists: a repeated entry would outgrow
@@ -393,6 +395,8 @@ inline bool build_basin_tables(const std::vector<int64_t>& off, const std::vecto
   for (int s = 0; s < n_seg; ++s) {
     segs[s].pos0 = seg[s];
     segs[s].pair0 = n_opair;
+    segs[s].basin0 = out->all_basins;
+    out->all_basins += seg_basins[s];
     n_opair += seg_pairs[s];
   }
   out->basins = static_cast<int32_t>(std::max<int64_t>(1, *std::max_element(seg_basins.begin(), seg_basins.end())));

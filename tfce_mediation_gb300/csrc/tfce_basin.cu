@@ -125,7 +125,7 @@ struct BasinArgs {
   int32_t* ord;         // ordered: vertex
   double* base;         // ordered: potential of the component before the vertex joined
   uint32_t* vnode;      // ordered: first node of the vertex
-  Node* nodes;          // [items][node_cap]: step * basins + basin
+  Node* nodes;          // [maps][signs][node_cap]; a segment's from basin0 * kMaxSteps: step * basins + basin
   uint32_t* part_max;   // [items] encoded maximum
   uint32_t* n_steps;    // [items]
   int64_t pos_per_map, pair_per_map, cpair_per_map, opair_per_map;
@@ -1028,7 +1028,7 @@ __device__ __forceinline__ void sweep_item(const BasinArgs& a, SweepShared& S, c
   if (kMode == kPotential && tid < 32) sum_rest(S.HH, L, S.rest);
   if (tid == 0) S.n_live[0] = S.n_live[1] = S.n_live[2] = 0;
   __syncthreads();
-  Node* nodes = (kMode == kNodes) ? a.nodes + item * a.node_cap : nullptr;
+  Node* nodes = (kMode == kNodes) ? a.nodes + (map * a.signs + sgn) * a.node_cap + si.basin0 * kMaxSteps : nullptr;
   // the thread's first entries of a step are loaded a step ahead
   int ev0 = S.ev[0], ev_end = S.ev[1], pr0 = S.pair[0], pr_end = S.pair[1];
   Two next_ev[kAhead] = {};
@@ -1453,7 +1453,7 @@ __global__ void __launch_bounds__(256) basin_walk_kernel(BasinArgs a) {
   const uint32_t* start = a.start_ev + (map * a.n_seg + seg) * kTab + sgn * kMaxSteps;
   const int lo = static_cast<int>(start[0]), hi = static_cast<int>(start[kMaxSteps]);
   const int64_t eo = map * a.n_vertices + a.segs[seg].pos0;
-  const Node* nodes = a.nodes + item * a.node_cap;
+  const Node* nodes = a.nodes + ms * a.node_cap + a.segs[seg].basin0 * kMaxSteps;
   const uint32_t nb = a.n_basins[(map * a.n_seg + seg) * 2 + sgn], L = a.n_steps[item];
   const float scale = __fdiv_rn(seg_maximum(a, map, sgn, seg), 100.0f);
   float* omap = a.out_maps ? a.out_maps + (int64_t)ms * a.n_vertices : nullptr;
@@ -1517,10 +1517,12 @@ struct BasinPlan {
   uint32_t* cross = nullptr;
   const double** seg_pow = nullptr;
   std::map<float, double*> powers;  // extent^E tables (read through seg_pow)
-  // A buffer that is replaced by a larger one may still be used by a captured
-  // launch: it is kept until the plan goes.  Growth is geometric.
+  int64_t all_basins = 0;  // of one sign of all segments
   char* ws = nullptr;
   int64_t ws_bytes = 0;
+  // Once a capture has been seen, a buffer that is replaced by a larger one is
+  // kept until the plan goes: captured launches use it.  Growth is geometric.
+  bool captured = false;
   std::vector<void*> retired;
 };
 
@@ -1573,7 +1575,7 @@ Layout layout_of(const BasinPlan* p, int64_t M, int signs, int mode, int64_t nod
   if (mode == kPotential) l.base = take(M * p->V * 8);
   if (mode == kNodes) {
     l.vnode = take(M * p->V * 4);
-    l.nodes = take(M * signs * p->n_seg * node_cap * 8);
+    l.nodes = take(M * signs * node_cap * 8);
     l.part = take(2 * M * signs * p->n_seg * 4);
   }
   l.total = o;
@@ -1581,16 +1583,41 @@ Layout layout_of(const BasinPlan* p, int64_t M, int signs, int mode, int64_t nod
 }
 
 constexpr int64_t kWorkspaceBudget = 8LL << 30;  // maps are swept in as many launches as this asks for
-
 constexpr size_t kPowersKept = 16;  // tables of extent^E that a handle holds on to besides those in use
 
-int64_t node_capacity(const BasinPlan* p) { return (int64_t)p->basins * kMaxSteps; }
+int64_t node_capacity(const BasinPlan* p) { return p->all_basins * kMaxSteps; }
 
-int ensure_ws(BasinPlan* p, int64_t bytes) {
+constexpr int64_t kStateBudget = 2LL << 30;  // state in global memory of the CTAs of the large class
+
+// tuning knob: the largest workspace that is asked for, in MB
+int64_t most_workspace() {
+  const char* env = std::getenv("TFCE_SWEEP_WORKSPACE_MB");
+  return env ? static_cast<int64_t>(std::max(0, std::atoi(env))) << 20 : INT64_MAX;
+}
+
+// A workspace of at least `bytes`.  An outgrown one goes first, or, if a capture
+// may have taken its address, with the plan.
+int ensure_ws(BasinPlan* p, int64_t bytes, int64_t most) {
   if (p->ws_bytes >= bytes) return TFCE_OK;
-  const int64_t want = std::max(bytes, std::min<int64_t>(2 * p->ws_bytes, kWorkspaceBudget));
+  if (bytes > most) {
+    set_error("sweep workspace of %lld bytes: more than TFCE_SWEEP_WORKSPACE_MB", static_cast<long long>(bytes));
+    return TFCE_ENOMEM;
+  }
+  int64_t want = std::max(bytes, std::min({2 * p->ws_bytes, most, kWorkspaceBudget}));
+  if (p->ws && !p->captured) {
+    TFGB_CUDA(cudaDeviceSynchronize());
+    cudaFree(p->ws);
+    p->ws = nullptr;
+    p->ws_bytes = 0;
+  }
   char* fresh = nullptr;
-  TFGB_CUDA(cudaMalloc(&fresh, want));
+  cudaError_t e = cudaMalloc(&fresh, want);
+  if (e == cudaErrorMemoryAllocation && want > bytes) {
+    cudaGetLastError();
+    e = cudaMalloc(&fresh, want = bytes);
+  }
+  if (e != cudaSuccess) cudaGetLastError();
+  TFGB_CUDA(e);
   if (p->ws) p->retired.push_back(p->ws);
   p->ws = fresh;
   p->ws_bytes = want;
@@ -1695,6 +1722,7 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
   p->n_seg = static_cast<int32_t>(seg.size()) - 1;
   p->vmax = t.vmax;
   p->basins = t.basins;
+  p->all_basins = t.all_basins;
   p->V = seg.back();
   p->n_pos = static_cast<int64_t>(t.vert.size());
   p->n_pair = t.n_pair;
@@ -1780,40 +1808,76 @@ bool basin_takes(const BasinPlan* p, const BasinRequest& r) {
   return layout_of(p, 1, r.signs, mode, cap).total <= kWorkspaceBudget;
 }
 
-int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st) {
+int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st, bool* refused) {
+  *refused = false;
   const int mode = mode_of(r);
   const int64_t cap = mode == kNodes ? node_capacity(p) : 0;
   const int64_t one = layout_of(p, 1, r.signs, mode, cap).total;
-  // as many maps per launch as the budget holds, in launches of equal size
-  int64_t most = std::max<int64_t>(1, kWorkspaceBudget / one);
-  most = std::min<int64_t>(most, std::max<int64_t>(1, 0x7fffffffLL / std::max(1, p->n_tiles + p->n_chunks)));
-  if (mode == kNodes)  // one grid row of the walk per item
-    most = std::min<int64_t>(most, std::max<int64_t>(1, 65535 / ((int64_t)r.signs * p->n_seg)));
-  const int64_t launches = (r.n_maps + most - 1) / most;
-  const int64_t per = (r.n_maps + launches - 1) / launches;
+  SweepShape first{}, mid{}, large{};
+  int first_ctas = 0, mid_ctas = 0, large_ctas = 0;
+  int64_t per = 0, state = 0;
+  Layout lay{};
+  // launches of equal size, of as many maps as `room` holds; the bytes they take
+  auto divide = [&](int64_t room) {
+    int64_t most = std::max<int64_t>(1, room / one);
+    most = std::min<int64_t>(most, std::max<int64_t>(1, 0x7fffffffLL / std::max(1, p->n_tiles + p->n_chunks)));
+    if (mode == kNodes)  // one grid row of the walk per item
+      most = std::min<int64_t>(most, std::max<int64_t>(1, 65535 / ((int64_t)r.signs * p->n_seg)));
+    const int64_t launches = (r.n_maps + most - 1) / most;
+    per = (r.n_maps + launches - 1) / launches;
 
-  const int64_t items_max = per * r.signs * p->n_seg;
-  SweepShape first = first_shape(p, mode, items_max, r.dense), mid{}, large{};
-  const int per_basin = state_bytes_per_basin(mode, kAllShared), per_basin_large = state_bytes_per_basin(mode, kListsGlobal);
-  const int first_ctas = first.grid;
-  int mid_ctas = 0, large_ctas = 0;
-  mid.basins = first.basins;
-  if (items_max > 2 * p->sms && r.dense && first.basins < p->basins) {
-    mid = shape_of(p, per_basin, 2, 65535, 512);
-    mid_ctas = mid.grid;
+    const int64_t items_max = per * r.signs * p->n_seg;
+    first = first_shape(p, mode, items_max, r.dense);
+    mid = large = SweepShape{};
+    const int per_basin = state_bytes_per_basin(mode, kAllShared), per_basin_large = state_bytes_per_basin(mode, kListsGlobal);
+    first_ctas = first.grid;
+    mid_ctas = large_ctas = 0;
+    state = 0;
+    mid.basins = first.basins;
+    if (items_max > 2 * p->sms && r.dense && first.basins < p->basins) {
+      mid = shape_of(p, per_basin, 2, 65535, 512);
+      mid_ctas = mid.grid;
+    }
+    if (mid.basins < p->basins) {
+      large.threads = kMaxSweepThreads;
+      large.basins = std::min({(kSmBytes - kSweepBytes) / per_basin_large, 65535, p->basins});
+      large.smem = large.basins * per_basin_large;
+      large_ctas = p->sms;
+      if (const int cap_ctas = most_ctas()) large_ctas = std::min(large_ctas, cap_ctas);
+      state = round_up((int64_t)p->basins * state_bytes_per_basin(mode, kAllGlobal), 256);
+      large_ctas = static_cast<int>(
+          std::min<int64_t>({large_ctas, items_max, std::max<int64_t>(1, std::min(room, kStateBudget) / state)}));
+    }
+    lay = layout_of(p, per, r.signs, mode, cap);
+    return lay.total + large_ctas * state;
+  };
+  // A call that has to grow the workspace asks for no more than half of the
+  // memory that there is for it (one map's is always asked for), and for less
+  // when that is refused; a captured one makes do with what it finds.
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) cudaGetLastError();
+  p->captured = p->captured || capturing != cudaStreamCaptureStatusNone;
+  const int64_t knob = most_workspace();
+  int64_t budget = std::min(kWorkspaceBudget, knob), need = divide(budget);
+  auto least = [&] { return per == 1 && large_ctas <= 1; };
+  auto less = [&] { need = divide(budget = std::min(budget, per * one + large_ctas * state) / 2); };
+  if (need > p->ws_bytes) {
+    int64_t limit = p->ws_bytes;
+    size_t unused = 0, total = 0;
+    if (capturing == cudaStreamCaptureStatusNone) {
+      if (cudaMemGetInfo(&unused, &total) != cudaSuccess) cudaGetLastError();
+      limit = std::max(limit, (static_cast<int64_t>(unused) + (p->captured ? 0 : p->ws_bytes)) / 2);
+    }
+    while (need > limit && !least()) less();
+    for (;;) {
+      const int rc = ensure_ws(p, need, knob);
+      if (rc == TFCE_OK) break;
+      *refused = rc == TFCE_ENOMEM;
+      if (rc != TFCE_ENOMEM || least()) return rc;
+      less();
+    }
+    *refused = false;
   }
-  if (mid.basins < p->basins) {
-    large.threads = kMaxSweepThreads;
-    large.basins = std::min({(kSmBytes - kSweepBytes) / per_basin_large, 65535, p->basins});
-    large.smem = large.basins * per_basin_large;
-    large_ctas = p->sms;
-    if (const int cap_ctas = most_ctas()) large_ctas = std::min(large_ctas, cap_ctas);
-    large_ctas = static_cast<int>(std::min<int64_t>(large_ctas, items_max));
-  }
-  const int64_t state = !large_ctas ? 0 : round_up((int64_t)p->basins * state_bytes_per_basin(mode, kAllGlobal), 256);
-  const Layout lay = layout_of(p, per, r.signs, mode, cap);
-  const int rc = ensure_ws(p, lay.total + large_ctas * state);
-  if (rc) return rc;
 
   BasinArgs a{};
   a.map_stride = r.map_stride;

@@ -731,7 +731,12 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
     r.d_seg_off = h->d_seg_off;
     r.seg_rank = h->d_segrank;
     r.err = const_cast<int32_t*>(h->report);
-    if (tfgb::basin_takes(h->basin, r)) return tfgb::basin_sweep(h->basin, r, st);
+    if (tfgb::basin_takes(h->basin, r)) {
+      bool refused = false;
+      const int rc = tfgb::basin_sweep(h->basin, r, st, &refused);
+      if (!refused) return rc;
+      tfgb::clear_error();  // vertex by vertex: a smaller workspace
+    }
   }
   int rs = resident_slots(h);
   if (rs) return rs;
