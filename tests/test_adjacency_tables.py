@@ -146,3 +146,37 @@ def test_bad_entries_are_named(program, tmp_path):
                          seg.tobytes() + np.asarray([u for x in lists for u in x], np.int32).tobytes())
         r = subprocess.run([program, str(path)], capture_output=True, text=True)
         assert want in r.stdout
+
+
+THROWS = r"""
+#include "host_parallel.h"
+#include <cstdio>
+#include <new>
+
+int main() {
+  std::atomic<int64_t> calls{0};
+  for (int64_t work : {int64_t{0}, int64_t{1} << 30})
+    try {
+      tfgb::parallel_for(100000, work, [&](int64_t i) {
+        ++calls;
+        if (i % 1000 == 999) throw std::bad_alloc();
+      });
+      return 1;
+    } catch (const std::bad_alloc&) {
+    }
+  if (calls >= 200000) return 2;
+  int64_t sum = 0;
+  tfgb::parallel_for(0, 1 << 30, [&](int64_t) { ++sum; });
+  return sum ? 3 : 0;
+}
+"""
+
+
+def test_out_of_memory_on_a_thread_reaches_the_caller(tmp_path):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        pytest.skip("no host compiler")
+    (tmp_path / "t.cpp").write_text(THROWS)
+    exe = str(tmp_path / "t")
+    subprocess.run([cxx, "-std=c++17", "-O1", "-pthread", "-I", CSRC, str(tmp_path / "t.cpp"), "-o", exe], check=True)
+    assert subprocess.run([exe]).returncode == 0

@@ -5,31 +5,38 @@
 
 #include <algorithm>
 #include <atomic>
+#include <exception>
 #include <thread>
 #include <vector>
 
 namespace tfgb {
 
 // f(i) for i in [0, n), on up to sixteen threads when `work` (in elements) is
-// worth starting them; on the calling thread alone when none can start.
+// worth starting them; on the calling thread alone when none can start.  What f
+// throws (out of memory) ends the loop and is thrown again on the calling thread.
 template <typename F>
 void parallel_for(int64_t n, int64_t work, const F& f) {
   const int64_t hw = std::max(1u, std::thread::hardware_concurrency());
   const int64_t threads = std::min<int64_t>({n, hw, 16, 1 + work / 8192});
   std::atomic<int64_t> next{0};
+  std::atomic<bool> failed{false};
+  std::exception_ptr thrown;
   auto run = [&] {
-    for (int64_t i = next.fetch_add(1); i < n; i = next.fetch_add(1)) f(i);
+    try {
+      for (int64_t i = next.fetch_add(1); i < n && !failed; i = next.fetch_add(1)) f(i);
+    } catch (...) {
+      if (!failed.exchange(true)) thrown = std::current_exception();
+    }
   };
   std::vector<std::thread> team;
-  for (int64_t t = 1; t < threads; ++t) {
-    try {
-      team.emplace_back(run);
-    } catch (...) {
-      break;
-    }
+  try {
+    team.reserve(std::max<int64_t>(threads, 1) - 1);
+    for (int64_t t = 1; t < threads; ++t) team.emplace_back(run);
+  } catch (...) {  // fewer then
   }
   run();
   for (std::thread& t : team) t.join();
+  if (thrown) std::rethrow_exception(thrown);
 }
 
 }  // namespace tfgb

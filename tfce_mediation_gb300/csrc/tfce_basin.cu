@@ -32,6 +32,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <map>
+#include <memory>
 
 #include "basin.cuh"
 #include "basin_tables.h"
@@ -1531,6 +1532,7 @@ namespace {
 template <typename T>
 int upload(BasinPlan* p, const std::vector<T>& h, T** d) {
   const size_t n = std::max<size_t>(1, h.size());
+  p->owned.reserve(p->owned.size() + 1);
   TFGB_CUDA(cudaMalloc(reinterpret_cast<void**>(d), n * sizeof(T)));
   p->owned.push_back(*d);
   if (!h.empty()) TFGB_CUDA(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
@@ -1716,7 +1718,11 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
   *out = nullptr;
   BasinTables t;
   if (!build_basin_tables(off, packed, seg, &t)) return TFCE_OK;
-  BasinPlan* p = new BasinPlan();
+  struct Destroy {
+    void operator()(BasinPlan* plan) const { basin_plan_destroy(plan); }
+  };
+  std::unique_ptr<BasinPlan, Destroy> own(new BasinPlan());
+  BasinPlan* const p = own.get();
   cudaGetDevice(&p->device);
   cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
   p->n_seg = static_cast<int32_t>(seg.size()) - 1;
@@ -1746,11 +1752,8 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
   if (!rc) rc = upload(p, t.cross, &p->cross);
   std::vector<const double*> none(p->n_seg, nullptr);
   if (!rc) rc = upload(p, none, &p->seg_pow);
-  if (rc) {
-    basin_plan_destroy(p);
-    return rc;
-  }
-  *out = p;
+  if (rc) return rc;
+  *out = own.release();
   return TFCE_OK;
 }
 

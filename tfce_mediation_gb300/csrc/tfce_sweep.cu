@@ -37,6 +37,8 @@
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
+#include <exception>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -824,14 +826,15 @@ int ensure_run_buffers(tfce_adjset* h, int32_t V) {
   return TFCE_OK;
 }
 
-}  // namespace
+struct Release {
+  void operator()(tfce_adjset* h) const {
+    release(h);
+    delete h;
+  }
+};
 
-extern "C" {
-
-int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n_vertices,
-                       const int64_t* seg_offsets, int32_t n_seg, const float* H, const float* E,
-                       tfce_adjset** out) {
-  tfgb::clear_error();
+int create_handle(const int64_t* offsets, const int32_t* indices, int32_t n_vertices, const int64_t* seg_offsets,
+                  int32_t n_seg, const float* H, const float* E, tfce_adjset** out) {
   TFGB_CHECK_ARG(out != nullptr, "out is NULL");
   *out = nullptr;
   TFGB_CHECK_ARG(n_vertices >= 0, "n_vertices < 0");
@@ -872,7 +875,8 @@ int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n
   const std::vector<int64_t>& off = lists.off;
   const std::vector<uint32_t>& packed = lists.packed;
 
-  tfce_adjset* h = new tfce_adjset();
+  std::unique_ptr<tfce_adjset, Release> own(new tfce_adjset());
+  tfce_adjset* const h = own.get();
   cudaGetDevice(&h->device);
   h->V = V;
   h->D = static_cast<int64_t>(packed.size());
@@ -882,38 +886,25 @@ int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n
   h->seg_off = seg;
   h->H.assign(H, H + n_seg);
   h->E.assign(E, E + n_seg);
-  auto fail = [&](int rc) {
-    release(h);
-    delete h;
-    return rc;
-  };
-#define TFGB_CUDA_H(call)                                                           \
-  do {                                                                              \
-    cudaError_t _e = (call);                                                        \
-    if (_e != cudaSuccess) {                                                        \
-      tfgb::set_error("%s: %s", #call, cudaGetErrorString(_e));                     \
-      return fail(_e == cudaErrorMemoryAllocation ? TFCE_ENOMEM : TFCE_EDEVICE);    \
-    }                                                                               \
-  } while (0)
-  TFGB_CUDA_H(cudaMalloc(&h->d_offsets, sizeof(int64_t) * (V + 1)));
-  TFGB_CUDA_H(cudaMalloc(&h->d_indices, sizeof(uint32_t) * std::max<size_t>(1, packed.size())));
-  TFGB_CUDA_H(cudaMalloc(&h->d_seg_off, sizeof(int64_t) * (n_seg + 1)));
-  TFGB_CUDA_H(cudaMalloc(&h->d_H, sizeof(float) * n_seg));
-  TFGB_CUDA_H(cudaMalloc(&h->d_E, sizeof(float) * n_seg));
-  TFGB_CUDA_H(cudaMalloc(&h->d_ctrl, sizeof(int32_t)));
-  TFGB_CUDA_H(cudaMemset(h->d_ctrl, 0, sizeof(int32_t)));
+  TFGB_CUDA(cudaMalloc(&h->d_offsets, sizeof(int64_t) * (V + 1)));
+  TFGB_CUDA(cudaMalloc(&h->d_indices, sizeof(uint32_t) * std::max<size_t>(1, packed.size())));
+  TFGB_CUDA(cudaMalloc(&h->d_seg_off, sizeof(int64_t) * (n_seg + 1)));
+  TFGB_CUDA(cudaMalloc(&h->d_H, sizeof(float) * n_seg));
+  TFGB_CUDA(cudaMalloc(&h->d_E, sizeof(float) * n_seg));
+  TFGB_CUDA(cudaMalloc(&h->d_ctrl, sizeof(int32_t)));
+  TFGB_CUDA(cudaMemset(h->d_ctrl, 0, sizeof(int32_t)));
   int32_t* report = nullptr;
-  TFGB_CUDA_H(cudaHostAlloc(&report, sizeof(int32_t) * 2, cudaHostAllocPortable | cudaHostAllocMapped));
+  TFGB_CUDA(cudaHostAlloc(&report, sizeof(int32_t) * 2, cudaHostAllocPortable | cudaHostAllocMapped));
   report[0] = report[1] = 0;
   h->report = report;
-  TFGB_CUDA_H(cudaEventCreateWithFlags(&h->reached, cudaEventDisableTiming));
-  TFGB_CUDA_H(cudaMemcpy(h->d_offsets, off.data(), sizeof(int64_t) * (V + 1), cudaMemcpyHostToDevice));
+  TFGB_CUDA(cudaEventCreateWithFlags(&h->reached, cudaEventDisableTiming));
+  TFGB_CUDA(cudaMemcpy(h->d_offsets, off.data(), sizeof(int64_t) * (V + 1), cudaMemcpyHostToDevice));
   if (!packed.empty())
-    TFGB_CUDA_H(cudaMemcpy(h->d_indices, packed.data(), sizeof(uint32_t) * packed.size(),
+    TFGB_CUDA(cudaMemcpy(h->d_indices, packed.data(), sizeof(uint32_t) * packed.size(),
                            cudaMemcpyHostToDevice));
-  TFGB_CUDA_H(cudaMemcpy(h->d_seg_off, seg.data(), sizeof(int64_t) * (n_seg + 1), cudaMemcpyHostToDevice));
-  TFGB_CUDA_H(cudaMemcpy(h->d_H, H, sizeof(float) * n_seg, cudaMemcpyHostToDevice));
-  TFGB_CUDA_H(cudaMemcpy(h->d_E, E, sizeof(float) * n_seg, cudaMemcpyHostToDevice));
+  TFGB_CUDA(cudaMemcpy(h->d_seg_off, seg.data(), sizeof(int64_t) * (n_seg + 1), cudaMemcpyHostToDevice));
+  TFGB_CUDA(cudaMemcpy(h->d_H, H, sizeof(float) * n_seg, cudaMemcpyHostToDevice));
+  TFGB_CUDA(cudaMemcpy(h->d_E, E, sizeof(float) * n_seg, cudaMemcpyHostToDevice));
   bool uneven = false;
   for (int s = 0; s + 1 < n_seg; ++s) uneven = uneven || (seg[s + 1] - seg[s] != seg[s + 2] - seg[s + 1]);
   if (uneven) {
@@ -921,15 +912,30 @@ int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n
     for (int32_t s = 0; s < n_seg; ++s) rank[s] = s;
     std::stable_sort(rank.begin(), rank.end(),
                      [&](int32_t x, int32_t y) { return seg[x + 1] - seg[x] > seg[y + 1] - seg[y]; });
-    TFGB_CUDA_H(cudaMalloc(&h->d_segrank, sizeof(int32_t) * n_seg));
-    TFGB_CUDA_H(cudaMemcpy(h->d_segrank, rank.data(), sizeof(int32_t) * n_seg, cudaMemcpyHostToDevice));
+    TFGB_CUDA(cudaMalloc(&h->d_segrank, sizeof(int32_t) * n_seg));
+    TFGB_CUDA(cudaMemcpy(h->d_segrank, rank.data(), sizeof(int32_t) * n_seg, cudaMemcpyHostToDevice));
   }
-#undef TFGB_CUDA_H
   int rc = tfgb::basin_plan_create(off, packed, seg, &h->basin);
   if (!rc && h->basin) rc = tfgb::basin_plan_set_exponents(h->basin, E);
-  if (rc) return fail(rc);
-  *out = h;
+  if (rc) return rc;
+  *out = own.release();
   return TFCE_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int tfce_adjset_create(const int64_t* offsets, const int32_t* indices, int32_t n_vertices,
+                       const int64_t* seg_offsets, int32_t n_seg, const float* H, const float* E,
+                       tfce_adjset** out) {
+  tfgb::clear_error();
+  try {
+    return create_handle(offsets, indices, n_vertices, seg_offsets, n_seg, H, E, out);
+  } catch (const std::exception& e) {
+    tfgb::set_error("tfce_adjset_create: %s", e.what());
+    return TFCE_ENOMEM;
+  }
 }
 
 void tfce_adjset_destroy(tfce_adjset* h) {
