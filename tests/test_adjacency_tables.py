@@ -32,14 +32,14 @@ int main(int, char** argv) {
     for (int64_t e = c.off[v]; e < c.off[v + 1]; ++e)
       printf("list %d %d %d\n", (int)v, (int)(c.packed[e] & kIndexMask), (int)(c.packed[e] >> 31));
   BasinTables t;
-  if (!build_basin_tables(c.off, c.packed, seg, &t)) return puts("no tables"), 0;
+  if (!build_basin_tables(c, seg, &t)) return puts("no tables"), 0;
   printf("basins %d 0\n", t.basins);
-  for (size_t i = 0; i < t.tiles.size(); ++i) {
+  for (int64_t i = 0; i < t.tiles.size(); ++i) {
     const TileInfo ti = t.tiles[i];
     for (int v = 0; v < ti.nv; ++v) {
       printf("vertex %d %d\n", t.vert[ti.pos0 + v], (int)i);
       const int s = ti.slice0 + (v >> 5);
-      auto rows = [&](const char* name, const std::vector<uint32_t>& off, const std::vector<uint32_t>& of) {
+      auto rows = [&](const char* name, const auto& off, const auto& of) {
         for (uint32_t o = (off[s] & ~kOddRow) + (v & 31); o < (off[s + 1] & ~kOddRow); o += 32)
           for (uint32_t u : {(of[o] & 0xffffu) >> 2, of[o] >> 18})
             if ((int)u != v) printf("%s %d %d\n", name, t.vert[ti.pos0 + v], t.vert[ti.pos0 + u]);

@@ -8,6 +8,7 @@
 
 namespace tfgb {
 
+struct CleanLists;
 struct BasinPlan;  // tiles, neighbour slices, boundary tables and workspaces of one adjacency handle
 
 // What one tfce_sweep_batch call asks for (device pointers).
@@ -32,11 +33,9 @@ struct BasinRequest {
   int32_t* err;
 };
 
-// Tiles of a validated CSR: off [V+1], packed [off[V]] (bit 31: one-way
-// entry), seg [n_seg+1].  *out stays NULL (and TFCE_OK is returned) for graphs
+// Tiles of cleaned lists, seg [n_seg+1].  *out stays NULL (and TFCE_OK is returned) for graphs
 // that the form does not take.
-int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_t>& packed,
-                      const std::vector<int64_t>& seg, BasinPlan** out);
+int basin_plan_create(const CleanLists& lists, const std::vector<int64_t>& seg, BasinPlan** out);
 void basin_plan_destroy(BasinPlan* p);
 // Tables of extent^E of the segments' exponents (host array of n_seg).
 int basin_plan_set_exponents(BasinPlan* p, const float* E);

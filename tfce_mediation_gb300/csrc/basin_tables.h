@@ -7,8 +7,9 @@
 
 #include <algorithm>
 #include <atomic>
+#include <memory>
 #include <string>
-#include <utility>
+#include <type_traits>
 #include <vector>
 
 #include "host_parallel.h"
@@ -22,12 +23,33 @@ constexpr int kTileEntries = 120000;          // list entries per tile: pairs ar
 constexpr int kCrossChunk = 1024;             // boundary vertices of a chunk
 constexpr uint32_t kOddRow = 0x80000000u;     // in edge_off: the second entries of the row's last words are padding
 
+// An array that starts unwritten: its pages are first touched by the threads
+// that fill it.
+template <typename T>
+class Raw {
+ public:
+  Raw() = default;
+  explicit Raw(int64_t n) : p_(new T[n]), n_(n) {}
+  int64_t size() const { return n_; }
+  T* data() const { return p_.get(); }
+  T& operator[](int64_t i) const {
+#ifdef _GLIBCXX_ASSERTIONS
+    if (i < 0 || i >= n_) __builtin_trap();
+#endif
+    return p_[i];
+  }
+
+ private:
+  std::unique_ptr<T[]> p_;
+  int64_t n_ = 0;
+};
+
 // Adjacency lists as the kernels read them: sorted, without self entries and
 // repeats (which never change the partition), entries whose reverse is missing
 // flagged (kOneWay).
 struct CleanLists {
-  std::vector<int64_t> off;      // [V + 1]
-  std::vector<uint32_t> packed;  // [off[V]]
+  Raw<int64_t> off;      // [V + 1]
+  Raw<uint32_t> packed;  // [off[V]]
   bool symmetric = true;
 };
 
@@ -37,10 +59,11 @@ inline bool clean_lists(const int64_t* offsets, const int32_t* indices, int32_t 
                         CleanLists* out, std::string* error) {
   auto segment_of = [&](int64_t v) { return std::upper_bound(seg.begin(), seg.end(), v) - seg.begin() - 1; };
   const int64_t D = offsets[V], blocks = (V + 4095) / 4096;
-  std::vector<int64_t>& off = out->off;
-  off.assign(V + 1, 0);
+  out->off = Raw<int64_t>(V + 1);
+  Raw<int64_t>& off = out->off;
+  off[0] = 0;
   std::vector<int64_t> bad(blocks, -1);
-  std::vector<int32_t> idx(D);
+  const Raw<int32_t> idx(D);
   // every list in the place that it came in, and its length (in off[v + 1])
   parallel_for(blocks, D, [&](int64_t k) {
     int64_t v = k * 4096, s = segment_of(v);
@@ -72,7 +95,7 @@ inline bool clean_lists(const int64_t* offsets, const int32_t* indices, int32_t 
     return false;
   }
   for (int32_t v = 0; v < V; ++v) off[v + 1] += off[v];
-  out->packed.resize(off[V]);
+  out->packed = Raw<uint32_t>(off[V]);
   std::atomic<bool> two_way{true};
   parallel_for(blocks, D, [&](int64_t k) {
     for (int64_t v = k * 4096; v < std::min<int64_t>(V, (k + 1) * 4096); ++v) {
@@ -116,82 +139,115 @@ struct SegInfo {
 };
 inline int64_t round_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
-// What basin_plan_create uploads, and the sizes that its workspaces follow from.
+// An array of the tables' memory.
+template <typename T>
+struct TableArray {
+  T* p = nullptr;
+  int64_t n = 0, at = 0;  // entries; bytes before it
+  int64_t size() const { return n; }
+  T* begin() const { return p; }
+  T* end() const { return p + n; }
+  T& operator[](int64_t i) const {
+#ifdef _GLIBCXX_ASSERTIONS
+    if (i < 0 || i >= n) __builtin_trap();
+#endif
+    return p[i];
+  }
+};
+
+// What basin_plan_create uploads (in one piece), and the sizes that its
+// workspaces follow from.
 struct BasinTables {
-  std::vector<TileInfo> tiles;
-  std::vector<ChunkInfo> chunks;
-  std::vector<SegInfo> segs;
-  std::vector<int32_t> vert, bnd_vert;
-  std::vector<uint32_t> slice_off, nbr, edge_off, edge, cross_off, cross;
-  std::vector<uint16_t> bnd_local, bnd_tile;
+  TableArray<TileInfo> tiles;
+  TableArray<ChunkInfo> chunks;
+  TableArray<SegInfo> segs;
+  TableArray<int32_t> vert, bnd_vert;
+  TableArray<uint32_t> slice_off, nbr, edge_off, edge, cross_off, cross;
+  TableArray<uint16_t> bnd_local, bnd_tile;
+  std::unique_ptr<char[]> memory;  // not cleared: threads write their parts first
+  int64_t bytes = 0;
   int64_t n_pair = 0, n_cpair = 0, n_opair = 0;
   int32_t vmax = 1;    // vertices of the largest segment
   int32_t basins = 1;  // basins of one sign of a segment at most
   int64_t all_basins = 0;  // of one sign of all segments
+
+  template <typename F>
+  void each(const F& f) {
+    f(tiles), f(chunks), f(segs), f(vert), f(bnd_vert), f(slice_off), f(nbr), f(edge_off), f(edge), f(cross_off), f(cross);
+    f(bnd_local), f(bnd_tile);
+  }
 };
 
 // The tables of cleaned lists (see CleanLists: a repeated entry would outgrow
 // its row).  False for graphs that the basin form does not take.
-inline bool build_basin_tables(const std::vector<int64_t>& off, const std::vector<uint32_t>& packed,
-                               const std::vector<int64_t>& seg, BasinTables* out) {
-  const int64_t V = static_cast<int64_t>(off.size()) - 1;
+//
+// Part of making a handle, so a program that sweeps one map pays for it too.
+// Handle and first map of an icosphere L5 / L6 / L7 / a 91 x 109 x 91 mask, 16
+// cores: 1.6 / 3.2 / 9.7 / 29 ms, of which the tables take 0.5 / 1.7 / 6.5 / 21
+// (sorted tile by tile, joined by one thread and uploaded table by table: 2.0 /
+// 5.1 / 12.5 / 32); swept vertex by vertex, without tables and the lists cleaned
+// by one thread, 1.4 / 3.3 / 12.0 / 60.
+inline bool build_basin_tables(const CleanLists& lists, const std::vector<int64_t>& seg, BasinTables* out) {
+  const Raw<int64_t>& off = lists.off;
+  const Raw<uint32_t>& packed = lists.packed;
+  const int64_t V = off.size() - 1;
   const int n_seg = static_cast<int>(seg.size()) - 1;
   // Tiles: patches grown breadth first from one vertex, so that few entries
   // cross; a patch that cannot grow goes on from the next free vertex, so that
   // all tiles of a segment but the last are full.  Inside a tile the vertices
   // keep their order, so that the statistic is read in runs.
-  std::vector<int32_t> mark(V, -1), tile_of(V);
-  std::vector<std::vector<std::vector<int32_t>>> grown(n_seg);
+  const Raw<int32_t> tile_of(V);  // 2 t + 1: in tile t of the segment; 2 t: queued by it last, or kFree
+  constexpr int32_t kFree = -2;
+  std::vector<std::vector<int32_t>> grown(n_seg);  // vertices of a segment's tiles
   parallel_for(n_seg, V, [&](int64_t s) {
-    constexpr int32_t kTaken = 0x7fffffff;  // in mark: in a tile; else the last tile that queued the vertex
-    std::vector<int32_t> queue(seg[s + 1] - seg[s] + 1), rim;
+    std::fill(tile_of.data() + seg[s], tile_of.data() + seg[s + 1], kFree);
+    std::vector<int32_t> queue(2 * kTile), rim;
     int64_t scan = seg[s], left = seg[s + 1] - seg[s];
     while (left > 0) {
       const int32_t id = static_cast<int32_t>(grown[s].size());
-      std::vector<int32_t> members;
-      members.reserve(std::min<int64_t>(left, kTile));
+      int32_t members = 0;
       int64_t entries = 0;
       bool full = false;
       size_t rim_at = 0;  // of the free vertices beside the last tile
       while (!full && left > 0) {
-        while (rim_at < rim.size() && mark[rim[rim_at]] == kTaken) ++rim_at;
+        while (rim_at < rim.size() && (tile_of[rim[rim_at]] & 1)) ++rim_at;
         size_t head = 0, tail = 1;
         if (rim_at < rim.size()) {
           queue[0] = rim[rim_at];
         } else {
-          while (mark[scan] == kTaken) ++scan;
+          while (tile_of[scan] & 1) ++scan;
           queue[0] = static_cast<int32_t>(scan);
         }
-        mark[queue[0]] = id;
+        tile_of[queue[0]] = 2 * id;
         for (; head < tail; ++head) {
           const int32_t v = queue[head];
           const int64_t e0 = off[v], e1 = off[v + 1];
-          if (static_cast<int>(members.size()) == kTile || (entries > 0 && entries + e1 - e0 > kTileEntries)) {
+          if (members == kTile || (entries > 0 && entries + e1 - e0 > kTileEntries)) {
             full = true;
             break;
           }
           entries += e1 - e0;
-          mark[v] = kTaken;
-          members.push_back(v);
+          tile_of[v] = 2 * id + 1;
+          ++members;
           --left;
-          for (int64_t e = e0; e < e1; ++e) {
-            const int32_t u = static_cast<int32_t>(packed[e] & kIndexMask);
-            if (mark[u] < id) {
-              mark[u] = id;
-              queue[tail++] = u;
-            }
+          if (tail + (e1 - e0) >= queue.size()) queue.resize(2 * (tail + (e1 - e0)));
+          for (int64_t e = e0; e < e1; ++e) {  // (no branches: they would be coin tosses)
+            const int32_t u = static_cast<int32_t>(packed[e] & kIndexMask), was = tile_of[u];
+            const bool fresh = !(was & 1) & (was < 2 * id);
+            tile_of[u] = fresh ? 2 * id : was;
+            queue[tail] = u;
+            tail += fresh;
           }
         }
         if (full || left == 0) rim.assign(queue.begin() + head, queue.begin() + tail);
       }
-      grown[s].push_back(std::move(members));
+      grown[s].push_back(members);
     }
   });
-  std::vector<TileInfo>& tiles = out->tiles;
-  std::vector<SegInfo>& segs = out->segs;
-  segs.resize(n_seg);
-  std::vector<std::vector<int32_t>*> members;
+  std::vector<TileInfo> tiles;
+  std::vector<SegInfo> segs(n_seg);
   int32_t& vmax = out->vmax;
+  int64_t n_vert = 0;
   for (int s = 0; s < n_seg; ++s) {
     vmax = std::max<int32_t>(vmax, static_cast<int32_t>(seg[s + 1] - seg[s]));
     segs[s].tile0 = static_cast<int32_t>(tiles.size());
@@ -200,24 +256,33 @@ inline bool build_basin_tables(const std::vector<int64_t>& off, const std::vecto
     for (int t = 0; t < segs[s].ntiles; ++t) {
       TileInfo ti{};
       ti.seg = s;
-      ti.nv = static_cast<int32_t>(grown[s][t].size());
+      ti.nv = grown[s][t];
       ti.in_seg = t;
+      ti.pos0 = static_cast<int32_t>(n_vert);
+      n_vert = round_up(n_vert + ti.nv, 32);
+      if (n_vert > 0x7fffffffLL) return false;
       tiles.push_back(ti);
-      members.push_back(&grown[s][t]);
     }
   }
   const int nt = static_cast<int>(tiles.size());
-  std::vector<uint16_t> local(V, 0);
-  parallel_for(nt, V, [&](int64_t t) {
-    std::vector<int32_t>& mem = *members[t];
-    std::sort(mem.begin(), mem.end());
-    for (size_t i = 0; i < mem.size(); ++i) {
-      local[mem[i]] = static_cast<uint16_t>(i);
-      tile_of[mem[i]] = tiles[t].in_seg;
+  const Raw<int32_t> vert(n_vert);  // (a tile's last slice is filled up with vertex 0)
+  // a vertex's place: its tile in the segment, and its index there (12 bits)
+  const Raw<int32_t>& place = tile_of;
+  parallel_for(n_seg, V, [&](int64_t s) {
+    std::vector<int32_t> filled(segs[s].ntiles, 0);
+    for (int64_t v = seg[s]; v < seg[s + 1]; ++v) {
+      const int32_t t = tile_of[v] >> 1, i = filled[t]++;
+      place[v] = t << 12 | i;
+      vert[tiles[segs[s].tile0 + t].pos0 + i] = static_cast<int32_t>(v);
+    }
+    for (int32_t t = 0; t < segs[s].ntiles; ++t) {
+      const TileInfo& ti = tiles[segs[s].tile0 + t];
+      std::fill(vert.data() + ti.pos0 + ti.nv, vert.data() + round_up(ti.pos0 + ti.nv, 32), 0);
     }
   });
   // entries that basin_cross_kernel takes: to another tile, or one-way
-  auto crosses = [&](int64_t v, uint32_t entry) { return (entry & kOneWay) || tile_of[entry & kIndexMask] != tile_of[v]; };
+  static_assert(kTile == 1 << 12, "the index in a tile has 12 bits");
+  auto crosses = [&](int64_t v, uint32_t entry) { return (entry & kOneWay) || ((place[entry & kIndexMask] ^ place[v]) >> 12) != 0; };
   // rows of neighbours and of pairs of neighbours, by tile
   struct Rows {
     std::vector<uint32_t> nbr, nbr_end, edge, edge_end;
@@ -225,18 +290,23 @@ inline bool build_basin_tables(const std::vector<int64_t>& off, const std::vecto
   };
   std::vector<Rows> rows(nt);
   std::vector<uint8_t> is_bnd(V, 0);
-  parallel_for(nt, V, [&](int64_t t) {
-    const std::vector<int32_t>& mem = *members[t];
+  parallel_for(nt, off[V], [&](int64_t t) {
+    const int32_t* const mem = vert.data() + tiles[t].pos0;
     const int nv = tiles[t].nv;
     Rows& r = rows[t];
     // rows of 32 lanes, two entries (4 * index) a lane; padding: the vertex itself
     auto put = [&](std::vector<uint32_t>& out, std::vector<uint32_t>& ends, const std::vector<uint16_t>& list,
                    const std::vector<int32_t>& at, const std::vector<int32_t>& count) {
+      size_t words = 0;
       for (int i = 0; i < nv; i += 32) {
-        int width = 0;
-        for (int v = i; v < std::min(nv, i + 32); ++v) width = std::max(width, count[v]);
-        size_t o = out.size();
-        out.resize(o + static_cast<size_t>((width + 1) / 2) * 32);
+        const int width = *std::max_element(count.begin() + i, count.begin() + std::min(nv, i + 32));
+        words += static_cast<size_t>((width + 1) / 2) * 32;
+        ends.push_back(static_cast<uint32_t>(words) | (width & 1 ? kOddRow : 0u));
+      }
+      out.resize(words);
+      size_t o = 0;
+      for (int i = 0; i < nv; i += 32) {
+        const int width = *std::max_element(count.begin() + i, count.begin() + std::min(nv, i + 32));
         for (int j = 0; j < width; j += 2)
           for (int v = i; v < i + 32; ++v) {
             const uint32_t self = std::min(v, nv - 1);
@@ -244,7 +314,6 @@ inline bool build_basin_tables(const std::vector<int64_t>& off, const std::vecto
             const uint32_t x = j < c ? list[at[v] + j] : self, y = j + 1 < c ? list[at[v] + j + 1] : self;
             out[o++] = 4u * x | (4u * y << 16);
           }
-        ends.push_back(static_cast<uint32_t>(out.size()) | (width & 1 ? kOddRow : 0u));
       }
     };
     std::vector<int32_t> at(nv + 1, 0), count(nv, 0), held_count(nv, 0);
@@ -259,7 +328,7 @@ inline bool build_basin_tables(const std::vector<int64_t>& off, const std::vecto
           __atomic_store_n(&is_bnd[v], uint8_t{1}, __ATOMIC_RELAXED);
           continue;
         }
-        const uint16_t u = local[packed[e] & kIndexMask];
+        const uint16_t u = place[packed[e] & kIndexMask] & (kTile - 1);
         near[at[i] + count[i]++] = u;
         if (u < i) continue;
         // each pair of neighbours once, held by the one that holds fewer so far
@@ -298,49 +367,40 @@ inline bool build_basin_tables(const std::vector<int64_t>& off, const std::vecto
       if (w >= 0) covered[w] = 1;
     }
   });
-  // the tiles one after the other
-  std::vector<int32_t>&vert = out->vert, &bnd_vert = out->bnd_vert;
-  std::vector<uint32_t>&slice_off = out->slice_off, &nbr = out->nbr, &edge_off = out->edge_off, &edge = out->edge;
-  std::vector<uint16_t>&bnd_local = out->bnd_local, &bnd_tile = out->bnd_tile;
-  std::vector<int32_t> bnd_of(V, -1);
-  slice_off.assign(1, 0);
-  edge_off.assign(1, 0);
-  std::vector<int64_t> seg_pairs(n_seg, 0), seg_basins(n_seg, 0);
-  int64_t& n_pair = out->n_pair;
+  // where the tiles' parts go, and the boundary vertices
+  std::vector<int32_t> bnd_vert;
+  const Raw<int32_t> bnd_of(V);  // of boundary vertices
+  std::vector<uint16_t> bnd_local, bnd_tile;
+  std::vector<int64_t> nbr0(nt), edge0(nt), seg_pairs(n_seg, 0), seg_basins(n_seg, 0);
+  int64_t &n_pair = out->n_pair, n_nbr = 0, n_edge = 0, n_slice = 0;
   for (int t = 0; t < nt; ++t) {
     TileInfo& ti = tiles[t];
-    Rows& r = rows[t];
-    const std::vector<int32_t>& mem = *members[t];
-    ti.pos0 = static_cast<int32_t>(vert.size());
-    ti.slice0 = static_cast<int32_t>(slice_off.size()) - 1;
+    const Rows& r = rows[t];
+    ti.slice0 = static_cast<int32_t>(n_slice);
     ti.bnd0 = static_cast<int32_t>(bnd_vert.size());
     ti.pair0 = static_cast<int32_t>(n_pair);
-    for (size_t i = 0; i < r.nbr_end.size(); ++i) {
-      slice_off.push_back(static_cast<uint32_t>(nbr.size()) + (r.nbr_end[i] & ~kOddRow));
-      edge_off.push_back(static_cast<uint32_t>(edge.size()) + r.edge_end[i]);
-    }
-    nbr.insert(nbr.end(), r.nbr.begin(), r.nbr.end());
-    edge.insert(edge.end(), r.edge.begin(), r.edge.end());
+    nbr0[t] = n_nbr;
+    edge0[t] = n_edge;
+    n_slice += static_cast<int64_t>(r.nbr_end.size());
+    n_nbr += static_cast<int64_t>(r.nbr.size());
+    n_edge += static_cast<int64_t>(r.edge.size());
     if (r.n_edges > 65535) return false;  // pairs are counted in 16 bits
     seg_basins[ti.seg] += r.n_basins;
     seg_pairs[ti.seg] += round_up(r.n_edges, 8);  // pairs of basins: at most one per pair of neighbours
     n_pair += round_up(r.n_edges, 8);
+    if (n_pair > 0x7fffffffLL || n_nbr >= (1LL << 32) || n_edge >= (1LL << 31)) return false;
+    const int32_t* const mem = vert.data() + ti.pos0;
     for (int i = 0; i < ti.nv; ++i) {
-      vert.push_back(mem[i]);
-      if (is_bnd[mem[i]]) {
-        bnd_of[mem[i]] = static_cast<int32_t>(bnd_vert.size());
-        bnd_local.push_back(static_cast<uint16_t>(i));
-        bnd_vert.push_back(mem[i]);
-        bnd_tile.push_back(static_cast<uint16_t>(ti.in_seg));
-      }
+      if (!is_bnd[mem[i]]) continue;
+      bnd_of[mem[i]] = static_cast<int32_t>(bnd_vert.size());
+      bnd_local.push_back(static_cast<uint16_t>(i));
+      bnd_vert.push_back(mem[i]);
+      bnd_tile.push_back(static_cast<uint16_t>(ti.in_seg));
     }
     ti.nbnd = static_cast<int32_t>(bnd_vert.size()) - ti.bnd0;
-    while (vert.size() % 32) vert.push_back(0);
-    if (n_pair > 0x7fffffffLL || vert.size() > 0x7fffffffull || nbr.size() >= (1ull << 32) || edge.size() >= (1ull << 31)) return false;
-    r = Rows();
   }
   // crossing lists, in chunks of boundary vertices of one segment
-  std::vector<ChunkInfo>& chunks = out->chunks;
+  std::vector<ChunkInfo> chunks;
   for (int s = 0; s < n_seg; ++s) {
     segs[s].chunk0 = static_cast<int32_t>(chunks.size());
     if (segs[s].ntiles) {
@@ -358,7 +418,7 @@ inline bool build_basin_tables(const std::vector<int64_t>& off, const std::vecto
   }
   const int n_chunks = static_cast<int>(chunks.size());
   std::vector<Rows> crows(n_chunks);
-  parallel_for(n_chunks, V, [&](int64_t c) {
+  parallel_for(n_chunks, 16 * static_cast<int64_t>(bnd_vert.size()), [&](int64_t c) {
     std::vector<uint32_t> list[32];
     for (int i = 0; i < chunks[c].nbnd; i += 32) {
       size_t width = 0;
@@ -379,17 +439,17 @@ inline bool build_basin_tables(const std::vector<int64_t>& off, const std::vecto
       crows[c].nbr_end.push_back(static_cast<uint32_t>(crows[c].nbr.size()));
     }
   });
-  std::vector<uint32_t>&cross_off = out->cross_off, &cross = out->cross;
-  cross_off.assign(1, 0);
-  int64_t& n_cpair = out->n_cpair;
+  std::vector<int64_t> cross0(n_chunks);
+  int64_t &n_cpair = out->n_cpair, n_cross = 0, n_cross_slice = 0;
   for (int c = 0; c < n_chunks; ++c) {
-    chunks[c].slice0 = static_cast<int32_t>(cross_off.size()) - 1;
+    chunks[c].slice0 = static_cast<int32_t>(n_cross_slice);
     chunks[c].pair0 = static_cast<int32_t>(n_cpair);
-    for (uint32_t e : crows[c].nbr_end) cross_off.push_back(static_cast<uint32_t>(cross.size()) + e);
-    cross.insert(cross.end(), crows[c].nbr.begin(), crows[c].nbr.end());
+    cross0[c] = n_cross;
+    n_cross_slice += static_cast<int64_t>(crows[c].nbr_end.size());
+    n_cross += static_cast<int64_t>(crows[c].nbr.size());
     n_cpair += round_up(crows[c].n_edges, 4);
     seg_pairs[chunks[c].seg] += round_up(crows[c].n_edges, 4);
-    if (n_cpair > 0x7fffffffLL || cross.size() >= (1ull << 32)) return false;
+    if (n_cpair > 0x7fffffffLL || n_cross >= (1LL << 32)) return false;
   }
   int64_t& n_opair = out->n_opair;
   for (int s = 0; s < n_seg; ++s) {
@@ -400,6 +460,49 @@ inline bool build_basin_tables(const std::vector<int64_t>& off, const std::vecto
     n_opair += seg_pairs[s];
   }
   out->basins = static_cast<int32_t>(std::max<int64_t>(1, *std::max_element(seg_basins.begin(), seg_basins.end())));
+  // all of it in one piece of memory
+  BasinTables& o = *out;
+  o.tiles.n = nt;
+  o.chunks.n = n_chunks;
+  o.segs.n = n_seg;
+  o.vert.n = n_vert;
+  o.slice_off.n = o.edge_off.n = n_slice + 1;
+  o.nbr.n = n_nbr;
+  o.edge.n = n_edge;
+  o.cross_off.n = n_cross_slice + 1;
+  o.cross.n = n_cross;
+  o.bnd_vert.n = o.bnd_local.n = o.bnd_tile.n = static_cast<int64_t>(bnd_vert.size());
+  o.each([&](auto& a) {
+    a.at = o.bytes;
+    o.bytes += round_up(a.n * static_cast<int64_t>(sizeof(*a.p)), 256);
+  });
+  o.memory.reset(new char[o.bytes]);
+  o.each([&](auto& a) { a.p = reinterpret_cast<std::remove_reference_t<decltype(a.p)>>(o.memory.get() + a.at); });
+  auto copy = [](const auto& from, auto* to) { std::copy(from.begin(), from.end(), to); };
+  copy(tiles, o.tiles.p);
+  copy(chunks, o.chunks.p);
+  copy(segs, o.segs.p);
+  std::copy(vert.data(), vert.data() + n_vert, o.vert.p);
+  copy(bnd_vert, o.bnd_vert.p);
+  copy(bnd_local, o.bnd_local.p);
+  copy(bnd_tile, o.bnd_tile.p);
+  o.slice_off[0] = o.edge_off[0] = o.cross_off[0] = 0;
+  parallel_for(nt + n_chunks, (n_nbr + n_edge + n_cross) / 16, [&](int64_t u) {
+    if (u < nt) {
+      const Rows& r = rows[u];
+      copy(r.nbr, o.nbr.p + nbr0[u]);
+      copy(r.edge, o.edge.p + edge0[u]);
+      for (size_t i = 0; i < r.nbr_end.size(); ++i) {
+        o.slice_off[tiles[u].slice0 + 1 + i] = static_cast<uint32_t>(nbr0[u]) + (r.nbr_end[i] & ~kOddRow);
+        o.edge_off[tiles[u].slice0 + 1 + i] = static_cast<uint32_t>(edge0[u]) + r.edge_end[i];
+      }
+    } else {
+      const int64_t c = u - nt;
+      copy(crows[c].nbr, o.cross.p + cross0[c]);
+      for (size_t i = 0; i < crows[c].nbr_end.size(); ++i)
+        o.cross_off[chunks[c].slice0 + 1 + i] = static_cast<uint32_t>(cross0[c]) + crows[c].nbr_end[i];
+    }
+  });
   return true;
 }
 

@@ -1502,7 +1502,7 @@ struct BasinPlan {
   int32_t basins = 0;  // of one sign of a segment at most
   int64_t V = 0, n_pos = 0, n_pair = 0, n_cpair = 0, n_opair = 0;
   int32_t n_tiles = 0, n_chunks = 0, n_bnd = 0;
-  std::vector<void*> owned;  // device tables
+  char* tables = nullptr;  // those below, in one piece
   TileInfo* tiles = nullptr;
   ChunkInfo* chunks = nullptr;
   SegInfo* segs = nullptr;
@@ -1528,16 +1528,6 @@ struct BasinPlan {
 };
 
 namespace {
-
-template <typename T>
-int upload(BasinPlan* p, const std::vector<T>& h, T** d) {
-  const size_t n = std::max<size_t>(1, h.size());
-  p->owned.reserve(p->owned.size() + 1);
-  TFGB_CUDA(cudaMalloc(reinterpret_cast<void**>(d), n * sizeof(T)));
-  p->owned.push_back(*d);
-  if (!h.empty()) TFGB_CUDA(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-  return TFCE_OK;
-}
 
 // workspace of a launch of M maps
 struct Layout {
@@ -1713,11 +1703,10 @@ int basin_resident_items(const BasinPlan* p, bool dense) {
   return first_shape(p, kMaxima, int64_t{1} << 30, dense).grid;
 }
 
-int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_t>& packed,
-                      const std::vector<int64_t>& seg, BasinPlan** out) {
+int basin_plan_create(const CleanLists& lists, const std::vector<int64_t>& seg, BasinPlan** out) {
   *out = nullptr;
   BasinTables t;
-  if (!build_basin_tables(off, packed, seg, &t)) return TFCE_OK;
+  if (!build_basin_tables(lists, seg, &t)) return TFCE_OK;
   struct Destroy {
     void operator()(BasinPlan* plan) const { basin_plan_destroy(plan); }
   };
@@ -1737,22 +1726,25 @@ int basin_plan_create(const std::vector<int64_t>& off, const std::vector<uint32_
   p->n_tiles = static_cast<int32_t>(t.tiles.size());
   p->n_chunks = static_cast<int32_t>(t.chunks.size());
   p->n_bnd = static_cast<int32_t>(t.bnd_vert.size());
-  int rc = upload(p, t.tiles, &p->tiles);
-  if (!rc) rc = upload(p, t.chunks, &p->chunks);
-  if (!rc) rc = upload(p, t.segs, &p->segs);
-  if (!rc) rc = upload(p, t.vert, &p->vert);
-  if (!rc) rc = upload(p, t.slice_off, &p->slice_off);
-  if (!rc) rc = upload(p, t.nbr, &p->nbr);
-  if (!rc) rc = upload(p, t.edge_off, &p->edge_off);
-  if (!rc) rc = upload(p, t.edge, &p->edge);
-  if (!rc) rc = upload(p, t.bnd_local, &p->bnd_local);
-  if (!rc) rc = upload(p, t.bnd_vert, &p->bnd_vert);
-  if (!rc) rc = upload(p, t.bnd_tile, &p->bnd_tile);
-  if (!rc) rc = upload(p, t.cross_off, &p->cross_off);
-  if (!rc) rc = upload(p, t.cross, &p->cross);
-  std::vector<const double*> none(p->n_seg, nullptr);
-  if (!rc) rc = upload(p, none, &p->seg_pow);
-  if (rc) return rc;
+  const int64_t pow_at = t.bytes;  // the segments' tables of extent^E: none yet
+  TFGB_CUDA(cudaMalloc(&p->tables, t.bytes + p->n_seg * sizeof(double*)));
+  TFGB_CUDA(cudaMemcpy(p->tables, t.memory.get(), t.bytes, cudaMemcpyHostToDevice));
+  TFGB_CUDA(cudaMemset(p->tables + pow_at, 0, p->n_seg * sizeof(double*)));
+  auto on_device = [&](const auto& a, auto*& d) { d = reinterpret_cast<std::remove_reference_t<decltype(d)>>(p->tables + a.at); };
+  on_device(t.tiles, p->tiles);
+  on_device(t.chunks, p->chunks);
+  on_device(t.segs, p->segs);
+  on_device(t.vert, p->vert);
+  on_device(t.slice_off, p->slice_off);
+  on_device(t.nbr, p->nbr);
+  on_device(t.edge_off, p->edge_off);
+  on_device(t.edge, p->edge);
+  on_device(t.bnd_local, p->bnd_local);
+  on_device(t.bnd_vert, p->bnd_vert);
+  on_device(t.bnd_tile, p->bnd_tile);
+  on_device(t.cross_off, p->cross_off);
+  on_device(t.cross, p->cross);
+  p->seg_pow = reinterpret_cast<const double**>(p->tables + pow_at);
   *out = own.release();
   return TFCE_OK;
 }
@@ -1762,7 +1754,7 @@ void basin_plan_destroy(BasinPlan* p) {
   int dev = 0;
   cudaGetDevice(&dev);
   cudaSetDevice(p->device);
-  for (void* d : p->owned) cudaFree(d);
+  cudaFree(p->tables);
   for (auto& kv : p->powers) cudaFree(kv.second);
   for (void* d : p->retired) cudaFree(d);
   cudaFree(p->ws);

@@ -606,12 +606,18 @@ struct tfce_adjset {
   int32_t vmax_seg = 0;
   std::vector<int64_t> seg_off;
   std::vector<float> H, E;
+  char* tables = nullptr;  // one piece of device memory: the arrays down to d_segrank
   int64_t* d_offsets = nullptr;
   uint32_t* d_indices = nullptr;
   int64_t* d_seg_off = nullptr;
   float* d_H = nullptr;
   float* d_E = nullptr;
   int32_t* d_ctrl = nullptr;  // queue counter
+  // Segments of uneven sizes: the segments by decreasing size, so items are
+  // handed out largest segment first (every map of the largest segment, then
+  // the next) and a launch does not end on a few long sweeps.  NULL when all
+  // segments have the same size.
+  int32_t* d_segrank = nullptr;
   // [0] error word, [1] step count: pinned host memory that the kernels write
   // (an error, or once per recorded sweep), so that reading them takes a wait
   // and no copy (8 us of a small map's 200)
@@ -637,11 +643,6 @@ struct tfce_adjset {
   // tfce_adjset_destroy.  Growth is geometric, so the retired total stays
   // below the live buffer's size.
   std::vector<void*> retired;
-  // Segments of uneven sizes: the segments by decreasing size, so items are
-  // handed out largest segment first (every map of the largest segment, then
-  // the next) and a launch does not end on a few long sweeps.  NULL when all
-  // segments have the same size.
-  int32_t* d_segrank = nullptr;
   tfgb::BasinPlan* basin = nullptr;  // NULL: a graph that form does not take
   std::mutex mu;
 };
@@ -653,12 +654,7 @@ int release(tfce_adjset* h) {
   int dev = 0;
   cudaGetDevice(&dev);
   cudaSetDevice(h->device);
-  cudaFree(h->d_offsets);
-  cudaFree(h->d_indices);
-  cudaFree(h->d_seg_off);
-  cudaFree(h->d_H);
-  cudaFree(h->d_E);
-  cudaFree(h->d_ctrl);
+  cudaFree(h->tables);
   cudaFreeHost(const_cast<int32_t*>(h->report));  // after cudaFree has waited for the kernels
   if (h->reached) cudaEventDestroy(h->reached);
   cudaFree(h->d_ws);
@@ -666,7 +662,6 @@ int release(tfce_adjset* h) {
   cudaFree(h->d_enh);
   cudaFree(h->d_group);
   cudaFree(h->d_segmax);
-  cudaFree(h->d_segrank);
   tfgb::basin_plan_destroy(h->basin);
   for (void* p : h->retired) cudaFree(p);
   h->retired.clear();
@@ -872,51 +867,63 @@ int create_handle(const int64_t* offsets, const int32_t* indices, int32_t n_vert
     tfgb::set_error("%s", error.c_str());
     return TFCE_EINVAL;
   }
-  const std::vector<int64_t>& off = lists.off;
-  const std::vector<uint32_t>& packed = lists.packed;
 
   std::unique_ptr<tfce_adjset, Release> own(new tfce_adjset());
   tfce_adjset* const h = own.get();
   cudaGetDevice(&h->device);
   h->V = V;
-  h->D = static_cast<int64_t>(packed.size());
+  h->D = lists.packed.size();
   h->n_seg = n_seg;
   h->symmetric = lists.symmetric;
   h->vmax_seg = vmax;
   h->seg_off = seg;
   h->H.assign(H, H + n_seg);
   h->E.assign(E, E + n_seg);
-  TFGB_CUDA(cudaMalloc(&h->d_offsets, sizeof(int64_t) * (V + 1)));
-  TFGB_CUDA(cudaMalloc(&h->d_indices, sizeof(uint32_t) * std::max<size_t>(1, packed.size())));
-  TFGB_CUDA(cudaMalloc(&h->d_seg_off, sizeof(int64_t) * (n_seg + 1)));
-  TFGB_CUDA(cudaMalloc(&h->d_H, sizeof(float) * n_seg));
-  TFGB_CUDA(cudaMalloc(&h->d_E, sizeof(float) * n_seg));
-  TFGB_CUDA(cudaMalloc(&h->d_ctrl, sizeof(int32_t)));
-  TFGB_CUDA(cudaMemset(h->d_ctrl, 0, sizeof(int32_t)));
   int32_t* report = nullptr;
   TFGB_CUDA(cudaHostAlloc(&report, sizeof(int32_t) * 2, cudaHostAllocPortable | cudaHostAllocMapped));
   report[0] = report[1] = 0;
   h->report = report;
   TFGB_CUDA(cudaEventCreateWithFlags(&h->reached, cudaEventDisableTiming));
-  TFGB_CUDA(cudaMemcpy(h->d_offsets, off.data(), sizeof(int64_t) * (V + 1), cudaMemcpyHostToDevice));
-  if (!packed.empty())
-    TFGB_CUDA(cudaMemcpy(h->d_indices, packed.data(), sizeof(uint32_t) * packed.size(),
-                           cudaMemcpyHostToDevice));
-  TFGB_CUDA(cudaMemcpy(h->d_seg_off, seg.data(), sizeof(int64_t) * (n_seg + 1), cudaMemcpyHostToDevice));
-  TFGB_CUDA(cudaMemcpy(h->d_H, H, sizeof(float) * n_seg, cudaMemcpyHostToDevice));
-  TFGB_CUDA(cudaMemcpy(h->d_E, E, sizeof(float) * n_seg, cudaMemcpyHostToDevice));
   bool uneven = false;
   for (int s = 0; s + 1 < n_seg; ++s) uneven = uneven || (seg[s + 1] - seg[s] != seg[s + 2] - seg[s + 1]);
-  if (uneven) {
-    std::vector<int32_t> rank(n_seg);
-    for (int32_t s = 0; s < n_seg; ++s) rank[s] = s;
-    std::stable_sort(rank.begin(), rank.end(),
-                     [&](int32_t x, int32_t y) { return seg[x + 1] - seg[x] > seg[y + 1] - seg[y]; });
-    TFGB_CUDA(cudaMalloc(&h->d_segrank, sizeof(int32_t) * n_seg));
-    TFGB_CUDA(cudaMemcpy(h->d_segrank, rank.data(), sizeof(int32_t) * n_seg, cudaMemcpyHostToDevice));
-  }
-  int rc = tfgb::basin_plan_create(off, packed, seg, &h->basin);
+  std::vector<int32_t> rank(uneven ? n_seg : 0);
+  for (int32_t s = 0; s < static_cast<int32_t>(rank.size()); ++s) rank[s] = s;
+  std::stable_sort(rank.begin(), rank.end(),
+                   [&](int32_t x, int32_t y) { return seg[x + 1] - seg[x] > seg[y + 1] - seg[y]; });
+  // one allocation; the short arrays go up together
+  std::vector<char> small;
+  auto add = [&small](const void* from, size_t bytes) {
+    const size_t at = small.size();
+    small.resize(tfgb::round_up(at + bytes, 256));
+    if (bytes) std::memcpy(small.data() + at, from, bytes);
+    return at;
+  };
+  const int32_t zero = 0;
+  const size_t at_ctrl = add(&zero, sizeof(zero)), at_seg = add(seg.data(), sizeof(int64_t) * (n_seg + 1)),
+               at_H = add(H, sizeof(float) * n_seg), at_E = add(E, sizeof(float) * n_seg),
+               at_rank = add(rank.data(), sizeof(int32_t) * rank.size());
+  const size_t at_off = small.size(), at_idx = at_off + tfgb::round_up(sizeof(int64_t) * (V + 1), 256);
+  TFGB_CUDA(cudaMalloc(&h->tables, at_idx + sizeof(uint32_t) * std::max<int64_t>(1, lists.packed.size())));
+  auto at = [&](auto*& p, size_t o) { p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(h->tables + o); };
+  at(h->d_ctrl, at_ctrl);
+  at(h->d_seg_off, at_seg);
+  at(h->d_H, at_H);
+  at(h->d_E, at_E);
+  if (uneven) at(h->d_segrank, at_rank);
+  at(h->d_offsets, at_off);
+  at(h->d_indices, at_idx);
+  TFGB_CUDA(cudaMemcpy(h->tables, small.data(), small.size(), cudaMemcpyHostToDevice));
+  TFGB_CUDA(cudaMemcpy(h->d_offsets, lists.off.data(), sizeof(int64_t) * (V + 1), cudaMemcpyHostToDevice));
+  if (h->D) TFGB_CUDA(cudaMemcpy(h->d_indices, lists.packed.data(), sizeof(uint32_t) * h->D, cudaMemcpyHostToDevice));
+  int rc = tfgb::basin_plan_create(lists, seg, &h->basin);
   if (!rc && h->basin) rc = tfgb::basin_plan_set_exponents(h->basin, E);
+  if (rc == TFCE_ENOMEM) {  // the handle sweeps vertex by vertex
+    cudaGetLastError();
+    tfgb::clear_error();
+    tfgb::basin_plan_destroy(h->basin);
+    h->basin = nullptr;
+    rc = TFCE_OK;
+  }
   if (rc) return rc;
   *out = own.release();
   return TFCE_OK;
