@@ -183,7 +183,7 @@ struct BasinTables {
 //
 // Part of making a handle, so a program that sweeps one map pays for it too.
 // Handle and first map of an icosphere L5 / L6 / L7 / a 91 x 109 x 91 mask, 16
-// cores: 1.6 / 3.2 / 9.7 / 29 ms, of which the tables take 0.5 / 1.7 / 6.5 / 21
+// cores: 1.7 / 3.1 / 8.2 / 24 ms, of which the tables take 0.5 / 1.6 / 5 / 19
 // (sorted tile by tile, joined by one thread and uploaded table by table: 2.0 /
 // 5.1 / 12.5 / 32); swept vertex by vertex, without tables and the lists cleaned
 // by one thread, 1.4 / 3.3 / 12.0 / 60.

@@ -890,6 +890,18 @@ int create_handle(const int64_t* offsets, const int32_t* indices, int32_t n_vert
   for (int32_t s = 0; s < static_cast<int32_t>(rank.size()); ++s) rank[s] = s;
   std::stable_sort(rank.begin(), rank.end(),
                    [&](int32_t x, int32_t y) { return seg[x + 1] - seg[x] > seg[y + 1] - seg[y]; });
+  // (before the lists go up: the tables are grown along them, and that took 4.0 ms
+  // instead of 2.5 for an L7 surface after the copy had read them)
+  int rc = tfgb::basin_plan_create(lists, seg, &h->basin);
+  if (!rc && h->basin) rc = tfgb::basin_plan_set_exponents(h->basin, E);
+  if (rc == TFCE_ENOMEM) {  // the handle sweeps vertex by vertex
+    cudaGetLastError();
+    tfgb::clear_error();
+    tfgb::basin_plan_destroy(h->basin);
+    h->basin = nullptr;
+    rc = TFCE_OK;
+  }
+  if (rc) return rc;
   // one allocation; the short arrays go up together
   std::vector<char> small;
   auto add = [&small](const void* from, size_t bytes) {
@@ -915,16 +927,6 @@ int create_handle(const int64_t* offsets, const int32_t* indices, int32_t n_vert
   TFGB_CUDA(cudaMemcpy(h->tables, small.data(), small.size(), cudaMemcpyHostToDevice));
   TFGB_CUDA(cudaMemcpy(h->d_offsets, lists.off.data(), sizeof(int64_t) * (V + 1), cudaMemcpyHostToDevice));
   if (h->D) TFGB_CUDA(cudaMemcpy(h->d_indices, lists.packed.data(), sizeof(uint32_t) * h->D, cudaMemcpyHostToDevice));
-  int rc = tfgb::basin_plan_create(lists, seg, &h->basin);
-  if (!rc && h->basin) rc = tfgb::basin_plan_set_exponents(h->basin, E);
-  if (rc == TFCE_ENOMEM) {  // the handle sweeps vertex by vertex
-    cudaGetLastError();
-    tfgb::clear_error();
-    tfgb::basin_plan_destroy(h->basin);
-    h->basin = nullptr;
-    rc = TFCE_OK;
-  }
-  if (rc) return rc;
   *out = own.release();
   return TFCE_OK;
 }
