@@ -109,3 +109,55 @@ def test_candidates_fill_whole_waves(ctas):
     for P in A.candidates(eng, 256):
         assert 4 <= P <= 256
         assert P in (16, 32, 64, 128, 256) or (P * per_perm) % ctas == 0
+
+
+def test_key_names_what_was_timed(monkeypatch):
+    """A stored choice holds for the kernels, sweep mode and GLM it was timed on."""
+    import torch
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda *_: "gpu")
+    eng = _Eng()
+    eng.adj.accumulation, eng.vd, eng.outputs = "component", None, None
+    keys = [A._key(eng)]
+
+    def changed():
+        keys.append(A._key(eng))
+        assert keys[-1] not in keys[:-1]
+
+    eng.vd = object()
+    changed()
+    eng.adj.accumulation = "exact"
+    changed()
+    eng.outputs = [("f", 1, 2)]
+    changed()
+    eng.outputs = [("t", 1)]
+    changed()
+    monkeypatch.setattr(A, "source_digest", lambda: "other kernels")
+    changed()
+
+
+def test_batches_are_timed_as_they_are_run(monkeypatch):
+    """time_batch and time_glm ask for a batch's t maps as run_batch does."""
+    import numpy as np
+    import torch
+    asked = []
+
+    class Event:
+        def __init__(self, **_):
+            pass
+
+        def record(self):
+            pass
+
+        def elapsed_time(self, other):
+            return 3.0
+
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda: None)
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: empty(*a, dtype=k["dtype"]))
+    eng = _Eng()
+    eng._tmaps_of = lambda perms, out=None: asked.append(np.asarray(perms).shape)
+    eng.sweep_max = lambda *a, **k: None
+    eng.status = lambda: None
+    assert A.time_batch(eng, 4) == 1.0 and A.time_glm(eng, 4) == 1.0
+    assert asked and set(asked) == {(4, eng.n)}

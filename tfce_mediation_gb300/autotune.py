@@ -15,8 +15,8 @@ values of P fill the persistent sweep grid evenly: one launch has P x
 contrasts x signs x segments sweep items spread over the resident CTAs
 (tfce_sweep_resident_slots), so P where that count is a multiple of the CTA
 count avoids a ragged last wave.  Results are cached per (GPU, n, k, V,
-entries, segments, contrasts, signs, precision) in
-~/.cache/tfce_mediation_gb300/autotune.json.
+entries, segments, contrasts, signs, precision, accumulation, weights, output
+program, native sources) in ~/.cache/tfce_mediation_gb300/autotune.json.
 """
 from __future__ import annotations
 
@@ -25,6 +25,8 @@ import os
 
 import numpy as np
 
+from .build import source_digest
+
 CACHE = os.path.join(os.path.expanduser("~"), ".cache", "tfce_mediation_gb300", "autotune.json")
 
 
@@ -32,7 +34,9 @@ def _key(eng):
     import torch
     name = torch.cuda.get_device_name()
     return "|".join(str(x) for x in (name, eng.n, eng.k, eng.V, eng.adj.n_entries, eng.n_seg, eng.C, eng.signs,
-                                     getattr(eng, "precision", "fp32")))
+                                     getattr(eng, "precision", "fp32"), eng.adj.accumulation,
+                                     "weighted" if eng.vd is not None else "unweighted", eng.outputs or "t",
+                                     source_digest()))
 
 
 def _load():
@@ -72,21 +76,20 @@ def candidates(eng, max_p=256):
 
 
 def time_batch(eng, P, seed=12345, repeats=3):
-    """Milliseconds per batch of P permutations (GLM + sweep), device time."""
+    """Milliseconds per batch of P permutations (the batch's own way to its t
+    maps, and the sweep), device time."""
     import torch
     from .engine import permutations
-    from .glm import DesignBatch
     perms = permutations(eng.n, seed, 0, P)
-    ops = DesignBatch(eng.X[perms])
     t = torch.empty((P, eng.C, eng.V), device="cuda", dtype=torch.float32)
     mx = torch.empty(P * eng.C * eng.signs * eng.n_seg, device="cuda", dtype=torch.float32)
-    eng.tmaps(ops, out=t)
+    eng._tmaps_of(perms, out=t)
     eng.sweep_max(t, P * eng.C, out=mx)
     torch.cuda.synchronize()
     a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     a.record()
     for _ in range(repeats):
-        eng.tmaps(ops, out=t)
+        eng._tmaps_of(perms, out=t)
         eng.sweep_max(t, P * eng.C, out=mx)
     b.record()
     torch.cuda.synchronize()
@@ -98,15 +101,14 @@ def time_glm(eng, P, seed=12345, repeats=3):
     """Milliseconds of the GLM of one batch of P permutations (device time)."""
     import torch
     from .engine import permutations
-    from .glm import DesignBatch
-    ops = DesignBatch(eng.X[permutations(eng.n, seed, 0, P)])
+    perms = permutations(eng.n, seed, 0, P)
     t = torch.empty((P, eng.C, eng.V), device="cuda", dtype=torch.float32)
-    eng.tmaps(ops, out=t)
+    eng._tmaps_of(perms, out=t)
     torch.cuda.synchronize()
     a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     a.record()
     for _ in range(repeats):
-        eng.tmaps(ops, out=t)
+        eng._tmaps_of(perms, out=t)
     b.record()
     torch.cuda.synchronize()
     eng.status()

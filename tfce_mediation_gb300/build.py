@@ -9,6 +9,8 @@ container and on the aarch64 GPU hosts.
 from __future__ import annotations
 
 import concurrent.futures as cf
+import functools
+import hashlib
 import os
 import shutil
 import subprocess
@@ -30,6 +32,17 @@ def nvcc() -> str:
         if cand and os.path.exists(cand):
             return cand
     raise RuntimeError("nvcc not found: the CUDA toolkit is required to build tfce_mediation_gb300")
+
+
+@functools.lru_cache(maxsize=None)
+def source_digest() -> str:
+    """A short digest of the native sources: what was measured on the kernels of
+    one digest does not hold for another."""
+    h = hashlib.sha256()
+    for f in sorted(os.listdir(CSRC)):
+        with open(os.path.join(CSRC, f), "rb") as fh:
+            h.update(f.encode() + b"\0" + fh.read())
+    return h.hexdigest()[:12]
 
 
 def _stale(extra=()) -> bool:

@@ -219,11 +219,11 @@ class PermutationEngine:
             self._X_up = X
         return self._X_d, self._cols_d
 
-    def _tmaps_of(self, perms):
+    def _tmaps_of(self, perms, out=None):
         """t maps [P][C][V] of the permutation index rows."""
         P = perms.shape[0]
         if self._program_on_device():
-            tc, out = self._tc, self._tbuf[:P]
+            tc, out = self._tc, self._tbuf[:P] if out is None else out
             base, _ = self._base()
             rows = dev(self._index_rows(perms))
             pt, u, x, invd, dof, wmat = tc.form_residual_designs(base, rows, P, self.k, self._centred, self._coef,
@@ -232,11 +232,11 @@ class PermutationEngine:
                     centred=self._centred)
             return out
         if self._fp32_on_device():
-            return self._tmaps_fp32(perms)
+            return self._tmaps_fp32(perms, out)
         if (not self._graph_qf() or len(self.contrasts) > 8
                 or type(self)._designs is not PermutationEngine._designs):  # a subclass forms its own
-            return self.tmaps(self._designs(perms))
-        tc, out = self._tc, self._tbuf[:P]
+            return self.tmaps(self._designs(perms), out=out)
+        tc, out = self._tc, self._tbuf[:P] if out is None else out
         base, cols = self._base()
         rows = dev(self._index_rows(perms))
         ops = tc.design_buffers(P, self.k)
@@ -250,13 +250,13 @@ class PermutationEngine:
         return (self.precision == "fp32" and self.outputs is None and 2 <= self.k <= 8
                 and type(self)._designs is PermutationEngine._designs and bool(np.all(self.X[:, 0] == 1.0)))
 
-    def _tmaps_fp32(self, perms):
+    def _tmaps_fp32(self, perms, out=None):
         t, P, k, n = self.t, perms.shape[0], self.k, self.n
         base, _ = self._base()
         if not hasattr(self, "_design_err"):
             self._design_err = t.zeros(1, dtype=t.int32, device="cuda")
             self._design_err_host = t.zeros(1, dtype=t.int32, pin_memory=True)
-        rows, out = dev(self._index_rows(perms)), self._tbuf[:P]
+        rows, out = dev(self._index_rows(perms)), self._tbuf[:P] if out is None else out
         pinv, X, invd, dof = t.empty(P * (2 * k * n + k + 1), dtype=t.float32, device="cuda").split(
             [P * k * n, P * k * n, P * k, P])
         _lib.check(self.lib.glm_fp32_designs(ptr(base), base.shape[-1], ptr(rows), n, P, k, ptr(pinv), ptr(X),
