@@ -316,12 +316,18 @@ __global__ void __launch_bounds__(256) glm_f64_kernel(
       low = __fsub_rn(low, __fsub_rn(t, sum));
       sum = t;
     }
-    // A residual is off by at most 2^-47 of its terms' sum per term and
-    // operation (8 per column), a sum of n squares by n 2^-47.
+    // With u = 2^-24 and M = top + reach, which no partial sum exceeds: x and b as
+    // pairs and the product of their low parts left out cost 3 u^2 |x b| a
+    // column.  After j columns |rl| <= (j + 3) u M (a two-sum's error is at most u
+    // M, the three low products of a column u |x b| each), and a column rounds
+    // four times, u times (u M + u |x b|) and three times |rl|: in all
+    // u^2 M (1.5 K^2 + 11.5 K + 4), below 0.75 K (K + 8) + 8 times 2^-47 M.  RSS is
+    // off by (3 n + 6) u^2 of itself (two roundings of at most u times 2 u of the
+    // sum a subject, and those of a square's low part), its root by half of that.
     if (fits && sum >= 0x1p-60f && sum <= 0x1p100f) {
       rss = (double)sum + (double)low;
       const float root = sqrtf(__fdiv_rn(sum, (float)n));
-      eps = 0x1p-43 + (double)(0x1p-47f * ((float)n + (8.0f * KMAX + 8.0f) * ((top + reach) / root)));
+      eps = 0x1p-43 + (double)(0x1p-47f * ((float)n + (0.75f * KMAX * (KMAX + 8) + 8.0f) * ((top + reach) / root)));
     }
   }
   auto rss_double = [&]() {
