@@ -873,12 +873,14 @@ def run_gpu(args):
         dist.barrier()
     torch.cuda.synchronize()
     start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    sweep_launches = -eng.adj.launches()
     with ClockSampler(local) as clk:
         start.record(stream)
         for s in range(args.steps):
             step(args.warmup + s, evs[s])
         stop.record(stream)
         torch.cuda.synchronize()
+    sweep_launches += eng.adj.launches()  # kernels of the timed steps' sweeps
     eng.status()
     ms = start.elapsed_time(stop)
     glm_ms = [e[0].elapsed_time(e[1]) for e in evs]
@@ -916,7 +918,7 @@ def run_gpu(args):
     slot = eng._slots[0]
     h2d = st.Y.nbytes + sum(v.numel() * v.element_size() for k_, v in slot.items()
                             if k_.startswith("h_") and k_ != "h_max")
-    d2h = P * C * 2 * S * 4
+    d2h = P * C * 2 * S * 4 + (slot["err_back"].nbytes if slot["on_device"] else 0)
     dropin = dropin_rate(st, P) if (rank == 0 and not args.no_configs) else None
 
     if rank != 0:
@@ -964,9 +966,6 @@ def run_gpu(args):
     per_sweep, traffic_note = profile_traffic("basin_sweep")
     traffic = None if per_sweep is None else per_sweep * sweeps_per_launch
     clocks = clk.summary()
-    # of a batched sweep: maxima, tiles, crossing pairs, offsets, order, and the
-    # size classes that the graph's bound on basins asks for (two at least here)
-    sweep_launches = 7
     if qf:
         # split-BF16 GEMM: 3 MMAs of M=V, N=R rows per design (the k-1 centred
         # columns padded to 4 or 8), K=n_pad; epilogue O(k^2) per vertex and design
@@ -981,7 +980,7 @@ def run_gpu(args):
                     "peak_source": f"{peak_kind} bf16_tflops_sustained (kernel timed inside a long step)",
                     "glm_ms_by_form": getattr(tc, "glm_timings", None),
                     "note": "tensor FLOPs count the three split-BF16 products on %d rows per design" % R}
-        launches = (2 + sweep_launches) * args.steps
+        launches = 2 * args.steps + sweep_launches
     elif tc is not None:
         # split-BF16 GEMM: 3 MMAs of M=V, N=8 rows per design, K=n_pad; residual
         # epilogue: (k+1) FP32 FMAs per vertex, design and subject (k with the
@@ -997,12 +996,12 @@ def run_gpu(args):
                     "epilogue_fp32_tflops": epi_flop / (glm_avg / 1000) / 1e12,
                     "glm_ms_by_form": getattr(tc, "glm_timings", None),
                     "note": "tensor FLOPs count the three split-BF16 products on 8 padded rows per design"}
-        launches = (2 + sweep_launches) * args.steps
+        launches = 2 * args.steps + sweep_launches
     else:
         glm_flop = 4.0 * n * eng.k * V * P  # beta + residual passes, FP32 CUDA cores
         glm_info = {"precision": "fp32", "kernels": "glm_tstat_kernel", "ms_per_launch": glm_avg,
                     "achieved_tflops_fp32": glm_flop / (glm_avg / 1000) / 1e12}
-        launches = (1 + sweep_launches) * args.steps
+        launches = args.steps + sweep_launches
     line = {
         "metric": METRIC, "value": value, "unit": "perm/s", "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
@@ -1011,7 +1010,7 @@ def run_gpu(args):
         "config": {"workload": WORKLOAD, "perms_per_step": P, "sweeps_per_step": sweeps_per_launch,
                    "l2": "inputs larger than L2 (Y 459 MB, t maps %d MB per step)" % (P * C * V * 4 // 2 ** 20),
                    "parallelism": f"replicas over permutation ranges x{ws}",
-                   "sweep_ctas_per_sm": getattr(eng.adj, "ctas_per_sm", None),
+                   "sweep_shape": getattr(eng.adj, "ctas_per_sm", None),
                    "glm_designs_per_tile": (int(tc.lib.glm_qf_design_block(eng.k)) if qf else
                                             getattr(tc, "design_block", None) if tc is not None else None),
                    "glm_form": "quadratic" if qf else "residual" if tc is not None else "fp32",

@@ -160,6 +160,8 @@ int tfce_sweep_status(tfce_adjset* h, void* stream);
  * persistent grid (resident CTAs per SM x SMs; TFCE_SWEEP_MAX_CTAS caps it).
  * A launch of n items runs in ceil(n / slots) waves. */
 int tfce_sweep_resident_slots(tfce_adjset* h, int32_t* slots);
+/* Kernels that the handle's sweeps have launched (or captured) so far. */
+int tfce_sweep_launches(tfce_adjset* h, int64_t* kernels);
 
 /* Allocation-free form of tfce_sweep_batch.  No counterpart in the reference.
  *

@@ -315,7 +315,7 @@ class AdjacencySet:
         self.H = Hs.copy()
         self.E = Es.copy()
         self.accumulation = "exact"  # the native handle's defaults
-        self.ctas_per_sm = 3
+        self.ctas_per_sm = 3  # the sweep shape (set_sweep_shape), not a count
         self.threshold_groups = None
 
     @property
@@ -354,8 +354,8 @@ class AdjacencySet:
         return self._h.value, self.accumulation, self.ctas_per_sm, None if g is None else tuple(g.tolist())
 
     def set_sweep_shape(self, ctas_per_sm: int):
-        """Shape of the batched sweeps: 3 (more sweeps resident, each with room
-        for 4,096 local maxima of its map in shared memory) or 2 (fewer, 9,300)."""
+        """Shape of the batched sweeps: 3 (four CTAs per SM, each with room for
+        4,096 local maxima of its map in shared memory) or 2 (two, 9,300)."""
         _lib.check(self._lib.tfce_adjset_set_sweep_shape(self._h, int(ctas_per_sm)))
         self.ctas_per_sm = int(ctas_per_sm)
 
@@ -400,6 +400,12 @@ class AdjacencySet:
         """Sweep items run at once (the persistent grid's CTAs)."""
         n = ctypes.c_int32(0)
         _lib.check(self._lib.tfce_sweep_resident_slots(self._h, ctypes.byref(n)))
+        return int(n.value)
+
+    def launches(self):
+        """Kernels launched (or captured) by the sweeps so far."""
+        n = ctypes.c_int64(0)
+        _lib.check(self._lib.tfce_sweep_launches(self._h, ctypes.byref(n)))
         return int(n.value)
 
     def status(self, stream=None):

@@ -18,7 +18,6 @@ struct BasinRequest {
   int32_t n_maps;
   int32_t signs;
   const float* vdensity;
-  int32_t floor_zero;
   float* out_max;
   float* out_maps;
   int32_t out_mode;
@@ -27,7 +26,6 @@ struct BasinRequest {
   int32_t dense;      // 1: more items resident with less shared state each; 0: fewer, larger
   const int32_t* thr_group;
   const float* d_H;
-  const float* d_E;
   const int64_t* d_seg_off;
   const int32_t* seg_rank;
   int32_t* err;
@@ -44,6 +42,7 @@ int basin_plan_set_exponents(BasinPlan* p, const float* E);
 bool basin_takes(const BasinPlan* p, const BasinRequest& r);
 // *refused: there was no memory for the workspace, and nothing was launched.
 int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st, bool* refused);
+int64_t basin_launched(const BasinPlan* p);  // kernels, so far
 // Items that a launch of many sweeps at once.
 int basin_resident_items(const BasinPlan* p, bool dense);
 

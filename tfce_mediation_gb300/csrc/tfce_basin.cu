@@ -1524,6 +1524,7 @@ struct BasinPlan {
   // Once a capture has been seen, a buffer that is replaced by a larger one is
   // kept until the plan goes: captured launches use it.  Growth is geometric.
   bool captured = false;
+  int64_t launched = 0;  // kernels
   std::vector<void*> retired;
 };
 
@@ -1749,6 +1750,8 @@ int basin_plan_create(const CleanLists& lists, const std::vector<int64_t>& seg, 
   return TFCE_OK;
 }
 
+int64_t basin_launched(const BasinPlan* p) { return p ? p->launched : 0; }
+
 void basin_plan_destroy(BasinPlan* p) {
   if (!p) return;
   int dev = 0;
@@ -1955,6 +1958,9 @@ int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st, bool* refu
     const int64_t parts = std::max<int64_t>(
         1, std::min<int64_t>((p->vmax + 8191) / 8192, (8 * p->sms + pairs_ms - 1) / pairs_ms));
     basin_max_kernel<<<static_cast<unsigned>(pairs_ms * parts), 256, 0, st>>>(a, static_cast<int32_t>(parts));
+    p->launched += 3 + (a.out_maps && r.out_mode == 1) + (p->n_tiles > 0) + (p->n_chunks > 0) +
+                   (p->n_tiles + p->n_chunks > 0) + (mid_ctas > 0) + (large_ctas > 0) +
+                   (mode == kNodes ? 1 + (a.out_max != nullptr) : 0);
     if (a.out_maps && r.out_mode == 1) {
       const int64_t n = M * r.signs * p->V;
       TFGB_CUDA(launch_after(chain, basin_fill_kernel, dim3(static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, p->sms * 16))),

@@ -644,6 +644,7 @@ struct tfce_adjset {
   // below the live buffer's size.
   std::vector<void*> retired;
   tfgb::BasinPlan* basin = nullptr;  // NULL: a graph that form does not take
+  int64_t launched = 0;              // kernels of vertex sweeps
   std::mutex mu;
 };
 
@@ -715,7 +716,6 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
     r.n_maps = n_maps;
     r.signs = signs;
     r.vdensity = vdensity;
-    r.floor_zero = floor_zero;
     r.out_max = out_max;
     r.out_maps = out_maps;
     r.out_mode = out_mode;
@@ -724,7 +724,6 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
     r.dense = h->sweep_shape == 3;
     r.thr_group = h->grouped ? h->d_group : nullptr;
     r.d_H = h->d_H;
-    r.d_E = h->d_E;
     r.d_seg_off = h->d_seg_off;
     r.seg_rank = h->d_segrank;
     r.err = const_cast<int32_t*>(h->report);
@@ -790,6 +789,7 @@ int launch_sweep(tfce_adjset* h, const float* stats, int64_t map_stride, int32_t
     a.seg_max = h->d_segmax;
   }
   tfgb::tfce_sweep_kernel<false><<<slots, tfgb::kSweepThreads, bm, st>>>(a);
+  h->launched += 1 + h->grouped;
   TFGB_CUDA(cudaGetLastError());
   return TFCE_OK;
 }
@@ -1109,6 +1109,14 @@ int tfce_sweep_resident_slots(tfce_adjset* h, int32_t* slots) {
   const int rc = resident_slots(h);
   if (rc) return rc;
   *slots = h->max_slots;
+  return TFCE_OK;
+}
+
+int tfce_sweep_launches(tfce_adjset* h, int64_t* kernels) {
+  tfgb::clear_error();
+  TFGB_CHECK_ARG(h != nullptr && kernels != nullptr, "NULL pointer");
+  std::lock_guard<std::mutex> lk(h->mu);
+  *kernels = h->launched + tfgb::basin_launched(h->basin);
   return TFCE_OK;
 }
 

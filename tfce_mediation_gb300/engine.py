@@ -391,7 +391,7 @@ class PermutationEngine:
         program = not qf and self._program_on_device()
         slot["on_device"] = qf or program  # designs formed on the device from index rows
         if slot["on_device"]:
-            slot["h_err"] = t.zeros(1, dtype=t.int32, pin_memory=True)  # a design without an inverse, in this batch or before
+            slot["err_back"] = t.zeros(1, dtype=t.int32, pin_memory=True)  # a design without an inverse, in this batch or before
             keys = ()
             base, cols = self._base()
             slot["h_rows"] = t.empty((P, n), dtype=t.int32, pin_memory=True)
@@ -451,7 +451,7 @@ class PermutationEngine:
                                  int(self.floor_zero), ptr(slot["d_max"]), None, 0, stream_handle())
             slot["h_max"].copy_(slot["d_max"], non_blocking=True)
             if slot["on_device"]:
-                slot["h_err"].copy_(tc.err, non_blocking=True)
+                slot["err_back"].copy_(tc.err, non_blocking=True)
 
         # warm-up outside capture (allocates the sweep workspace), then capture
         # two graphs: the GLM part (the last reader of the resident data) and
@@ -541,7 +541,7 @@ class PermutationEngine:
         def collect(slot):
             slot["event"].synchronize()
             slot["busy"] = False
-            if slot["on_device"] and int(slot["h_err"][0]):
+            if slot["on_device"] and int(slot["err_back"][0]):
                 self.status()  # raises: these maxima are not handed on
             results[slot["order"]] = slot["h_max"].numpy()[: slot["rows"]].copy()
             if on_batch is not None:
