@@ -22,3 +22,12 @@ def test_fit_is_scipys_maximum(n, xi):
         assert loglik(*got) >= loglik(c, s) - 1e-6 * n
         np.testing.assert_allclose(got, (c, s), rtol=2e-3, atol=2e-3)
     assert gpd._profile_fit(np.linspace(1.0, 2.0, 40)) is None or got[1] > 0
+
+
+@pytest.mark.parametrize("y", [np.linspace(1.0, 2.0, 40), np.linspace(0.01, 1.0, 40)])
+def test_likelihoods_that_rise_to_the_boundary_go_to_scipy(y):
+    """The profile has no maximum above xi = -0.9: the fit is scipy's, clipped."""
+    from scipy.stats import genpareto
+    assert gpd._profile_fit(y) is None
+    c, _, s = genpareto.fit(y, floc=0)
+    assert c < -0.9 and gpd.fit_gpd(y) == (-0.9, float(s))
