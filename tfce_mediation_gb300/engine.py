@@ -5,8 +5,10 @@ vertex_tfce_mediation_randomise.py:79-91,
 tfce_mediation/tm_func.py:144-185 and 269-305).
 
 Per launch, P permutations:
-  1. host: permutation indices RandomState(seed + p).permutation(n) and, in
-     float64, each permuted design's inv(X'X) X' and diag(inv(X'X));
+  1. host: permutation indices RandomState(seed + p).permutation(n); each
+     permuted design's operators (centred columns, inv(X'X), ...) are formed
+     from them on the device in float64, or on the host for the forms that the
+     device kernels do not take;
   2. device: one GLM launch -> t maps [P][C][V] (float32, resident): the
      tcgen05 split-BF16 GEMM with the fused residual epilogue (precision
      'bf16x3', default) or the FP32 CUDA-core kernel ('fp32'); with
@@ -16,8 +18,8 @@ Per launch, P permutations:
      -> the scaled per-segment maximum of every sweep;
   4. host: max over segments (hemispheres) gives the reference's per-permutation
      CSV values (2 per contrast: + then -).
-Y stays resident in HBM for the whole run; per launch only the P design
-operators go up and P x C x 2 x S maxima come down.
+Y stays resident in HBM for the whole run; per launch only the P index rows
+(or design operators) go up and P x C x 2 x S maxima come down.
 """
 from __future__ import annotations
 
@@ -720,7 +722,11 @@ class MediationEngine:
         DesignBatch of the path designs (FP64 inverses)."""
         if self._on_device():
             rows = np.ascontiguousarray(index_rows(perms, self.n, self.pred_x), np.int32)
-            return rows, (np.asarray(self._paths(perms)[2], np.float32) if self.medtype == "Y" else None)
+            if self.medtype != "Y":
+                return rows, None
+            from .pyfunc import path_a_scalar
+            return rows, np.asarray([path_a_scalar(self.pred_x[p], self.depend_y[p], self.n, self.cov) for p in perms],
+                                    np.float32)
         A, B, ta = self._paths(perms)
         if self.medtype == "Y":
             return DesignBatch(B, kmax=self.kmax), np.asarray(ta, np.float32)
@@ -770,8 +776,9 @@ class MediationEngine:
 
     def run(self, n_perm=None, seed=0, start=0, stop=None, perms=None):
         """Null maxima (n_perm, 1, 1, n_seg).  A batch's maxima are read back
-        after the next batch is queued, so the host forms the next batch's
-        path designs (FP64 inverses) while the GPU runs the current one."""
+        after the next batch is queued, so the host checks the next batch's
+        index rows (or forms its path designs, where the device does not) while
+        the GPU runs the current one."""
         if perms is None:
             stop = start + n_perm if stop is None else stop
             perms = permutations(self.n, seed, start, stop)
@@ -783,8 +790,8 @@ class MediationEngine:
         batch per item (data, perms) of `steps` -- data: new (n, V) mediator
         data from the host (pinned memory keeps the copy asynchronous) or None
         to keep the resident data; perms: at most `batch` permutation rows.
-        A batch's path designs are formed on the host while the previous batch
-        runs on the device; new data is copied and re-tiled on a side stream
+        A batch's path designs are formed on the device from its index rows (or
+        on the host, while the previous batch runs on the device); new data is copied and re-tiled on a side stream
         once the previous batch's GLM (the last reader of the resident data)
         is done, and this batch's GLM waits for it; each batch's maxima are
         read back after the next batch is queued.  Returns the per-batch

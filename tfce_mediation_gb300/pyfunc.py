@@ -146,17 +146,23 @@ def mediation_designs(medtype, pred_x, depend_y, n, covariates=None):
     if medtype == "M":
         return np.hstack([one, x] + cov), np.hstack([one, dy, x] + cov), None
     if medtype == "Y":
-        if covariates is None:
-            from scipy.stats import linregress
-            lr = linregress(np.asarray(pred_x, np.float64).ravel(), np.asarray(depend_y, np.float64).ravel())
-            return None, np.hstack([one, dy, x]), lr.slope / lr.stderr
-        Xa = np.hstack([one, x] + cov)
-        inv = np.linalg.inv(Xa.T @ Xa)
-        y = dy[:, 0]
-        a = inv @ Xa.T @ y
-        sigma2 = np.sum((y - Xa @ a) ** 2) / (n - Xa.shape[1])
-        return None, np.hstack([one, dy, x] + cov), a[1] / np.sqrt(sigma2 * inv[1, 1])
+        return None, np.hstack([one, dy, x] + cov), path_a_scalar(pred_x, depend_y, n, covariates)
     raise ValueError("Invalid mediation type")
+
+
+def path_a_scalar(pred_x, depend_y, n, covariates=None):
+    """t of path a of medtype 'Y' (pyfunc.py:141-145)."""
+    if covariates is None:
+        from scipy.stats import linregress
+        lr = linregress(np.asarray(pred_x, np.float64).ravel(), np.asarray(depend_y, np.float64).ravel())
+        return lr.slope / lr.stderr
+    Xa = np.hstack([np.ones((n, 1)), np.asarray(pred_x, np.float64).reshape(n, -1),
+                    np.asarray(covariates, np.float64).reshape(n, -1)])
+    inv = np.linalg.inv(Xa.T @ Xa)
+    y = np.asarray(depend_y, np.float64).reshape(n, -1)[:, 0]
+    a = inv @ Xa.T @ y
+    sigma2 = np.sum((y - Xa @ a) ** 2) / (n - Xa.shape[1])
+    return a[1] / np.sqrt(sigma2 * inv[1, 1])
 
 
 def sobel_from_t(ta, tb, alg="aroian", ta_scalar=None):
