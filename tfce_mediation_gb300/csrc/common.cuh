@@ -15,9 +15,10 @@ namespace tfgb {
 void set_error(const char* fmt, ...);
 void clear_error();
 
-// Device-side error codes written into a flag word by the kernels.  Every
-// loop that waits on or walks shared state is bounded; hitting a bound sets a
-// code here and the kernel carries on to its exit instead of trapping.
+// Device-side error codes written into a flag word by the kernels.  Every loop
+// that waits or tries again is bounded; hitting a bound sets a code here and the
+// kernel carries on to its exit instead of trapping.  Walks along parents or
+// pointers that strictly grow in their order end by themselves.
 enum DevErr : int32_t {
   kDevOk = 0,
   kDevBadIndex = 1,   // adjacency entry outside its segment

@@ -9,8 +9,9 @@
 //   beta_j = sum_s pinv[g][j][s] * y[s][v]                (cy_lin_lstsqr_mat)
 //   rss    = sum_s (y[s][v] - sum_j X[g][s][j] beta_j)^2  (residuals, never Y'Y)
 //   t_j    = beta_j / sqrt(rss / dof_g * invdiag[g][j])   (se_of_slope, tval_int)
-// in FP32 with FMA accumulation; the FP64 k x k inverse and pseudoinverse are
-// formed on the host.
+// in FP32 with FMA accumulation; the k x k inverse and pseudoinverse are formed
+// in FP64, on the device for an engine's batches (glm_design.cu), else on the
+// host.
 //
 // Also: the indirect-effect (Sobel/Aroian/Goodman) combination of two path t
 // maps (tfce_mediation/pyfunc.py:146-161).

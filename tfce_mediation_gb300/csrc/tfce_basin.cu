@@ -253,9 +253,7 @@ __global__ void __launch_bounds__(256) basin_max_kernel(BasinArgs a, int32_t par
 }
 
 // ---------------------------------------------------------------------------
-// Activation steps, basins and pairs of basins of one tile of one map.  Bound
-// by instruction issue (IPC 3.2 of 4; 425 warp instructions per 32 vertices,
-// a sixth each for steps, pointers and roots, the rest for the pairs).
+// Activation steps, basins and pairs of basins of one tile of one map.
 //
 // A vertex is one 32-bit word in shared memory: sign, 127 - step, place inside
 // the step (12 bits) and 4095 - index (12 bits).  Words of one sign order the
@@ -268,10 +266,11 @@ __global__ void __launch_bounds__(256) basin_max_kernel(BasinArgs a, int32_t par
 // pair of neighbours with different roots is a pair of basins, joined at the
 // later step of the two.
 //
-// Bound by instructions (3.3 a cycle, 420 per 32 vertices of a mesh: keys 71,
-// neighbours 81, pointers 71, pairs 154, sort 53): 2.25 ms for 512 maps x 2 L7.
-// The pairs' test reads the class of both words at once, and rows of an odd
-// width leave their last halves out (198 before).
+// Bound by instruction issue (3.3 of 4 a cycle; 430 warp instructions per 32
+// vertices of a mesh: keys 71, neighbours 81, pointers 71, pairs 154, sort 53):
+// 2.25 ms for 512 maps x 2 L7.  The pairs' test reads the class of both words at
+// once, and rows of an odd width leave their last halves out (198 for the pairs
+// before).
 __global__ void __launch_bounds__(kTileThreads, 4) basin_tile_kernel(BasinArgs a) {
   after_previous();
   __shared__ uint32_t key[kTile];
