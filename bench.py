@@ -918,7 +918,7 @@ def run_gpu(args):
     slot = eng._slots[0]
     h2d = st.Y.nbytes + sum(v.numel() * v.element_size() for k_, v in slot.items()
                             if k_.startswith("h_") and k_ != "h_max")
-    d2h = P * C * 2 * S * 4 + (slot["err_back"].nbytes if slot["on_device"] else 0)
+    d2h = P * C * 2 * S * 4
     dropin = dropin_rate(st, P) if (rank == 0 and not args.no_configs) else None
 
     if rank != 0:

@@ -62,7 +62,7 @@ constexpr int kSweepBytes = 4352;      // of a sweep besides its state
 constexpr int kFindLimit = 1 << 26;
 constexpr int kAhead = 4;              // pairs of events that a thread of the sweep loads a step ahead
 constexpr uint32_t kNone = 0xffffffffu;
-constexpr int kReady = 8;              // word of `counter`: the first of the sweep's launches sees the lists
+constexpr int kReady = 1 << 30;         // in a class's counter: the first of the sweep's launches sees the lists
 
 struct Node {
   float inc;
@@ -104,7 +104,7 @@ struct BasinArgs {
   int32_t n_tiles, n_chunks, n_bnd;
   // workspace
   uint32_t* seg_max;    // [maps][2][n_seg] bits of max(0, max)
-  int32_t* counter;     // items taken and, of the queued ones, there are: by class (2 * class, 2 * class + 1); kReady
+  int32_t* counter;     // items taken and, of the queued ones, there are: by class (2 * class, 2 * class + 1)
   uint32_t* ev;         // vertices of a tile by bucket: bucket << 24, index in the tile << 12, basin
   uint32_t* pairs;      // pairs of basins of a tile: bucket << 24, 12 bits each
   uint2* cpairs;        // crossing pairs: tile << 16 | 4 bits of the bucket << 12 | basin, twice
@@ -1364,29 +1364,38 @@ __global__ void __launch_bounds__(kLarge ? kMaxSweepThreads : 512, kLarge ? 1 : 
   extern __shared__ __align__(16) char dyn[];
   const int tid = threadIdx.x, nth = blockDim.x;
   // The lists are visible to the launch that waits for the kernel before it.  The
-  // launches beside it start after it has let them, and its release of `ready`
-  // before that makes the lists visible to whoever acquires it; should one find
-  // it unset, it waits for the launch before its own.
-  int32_t* const ready = a.counter + kReady;
+  // launches beside it start after it has let them, and before that it adds
+  // kReady to their counters, a release that their first item's acquire meets;
+  // a CTA that does not find it waits for the launch before its own.  (A word of
+  // its own, released by every CTA and acquired before the first item, made a
+  // call of three classes 10 us longer.)
   if (a.first_class) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (tid == 0) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(ready), "r"(1) : "memory");
-    __syncthreads();
+    if (blockIdx.x == 0) {
+      if (tid < 2 && tid < (kLarge ? 2 : a.mid))
+        asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(a.counter + 2 * tid), "r"(kReady) : "memory");
+      __syncthreads();
+    }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   } else {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    int32_t seen = 1;
-    if (tid == 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(ready) : "memory");
-    if (!__syncthreads_and(seen)) asm volatile("griddepcontrol.wait;" ::: "memory");
   }
   const int cls = kLarge ? 2 : a.mid;
   int32_t* const counter = a.counter + 2 * cls;
   const int32_t* const queue = a.queue + (kLarge ? a.n_items : 0);
-  const int n_items = cls ? counter[1] : a.n_items;
+  bool ready = a.first_class;
   for (;;) {
-    if (tid == 0) S.item = atomicAdd(counter, 1);
+    if (tid == 0) {
+      int32_t at;
+      if (ready) at = atomicAdd(counter, 1);
+      else asm volatile("atom.acquire.gpu.global.add.s32 %0, [%1], 1;" : "=r"(at) : "l"(counter) : "memory");
+      S.item = at;
+    }
     __syncthreads();
-    const int qi = S.item;
+    if (!ready && !(S.item & kReady)) asm volatile("griddepcontrol.wait;" ::: "memory");
+    ready = true;
+    const int n_items = cls ? counter[1] : a.n_items;
+    const int qi = S.item & (kReady - 1);
     if (qi >= n_items) break;
     int64_t out;  // (map * signs + sign) * n_seg + segment
     if (cls) {

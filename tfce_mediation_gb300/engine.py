@@ -214,11 +214,11 @@ class PermutationEngine:
             self._cols_d = dev(np.arange(self.k, dtype=np.int32) + TensorCoreOperands.PERMUTED)
             self._X_d = self.t.empty(self.X.shape, device="cuda", dtype=self.t.float64)
             self._X_up = None
-        if self._X_up is None or not np.array_equal(self._X_up, self.X):
+        up = self.X.tobytes()
+        if up != self._X_up:
             np.linalg.inv(self.X.T @ self.X)  # a design without an inverse raises here
-            X = np.array(self.X, np.float64)
-            self._X_d.copy_(self.t.from_numpy(X))
-            self._X_up = X
+            self._X_d.copy_(self.t.from_numpy(np.array(self.X, np.float64)))
+            self._X_up = up
         return self._X_d, self._cols_d
 
     def _tmaps_of(self, perms, out=None):
@@ -393,7 +393,8 @@ class PermutationEngine:
         program = not qf and self._program_on_device()
         slot["on_device"] = qf or program  # designs formed on the device from index rows
         if slot["on_device"]:
-            slot["err_back"] = t.zeros(1, dtype=t.int32, pin_memory=True)  # a design without an inverse, in this batch or before
+            slot["err"] = t.zeros(1, dtype=t.int32, pin_memory=True)  # written by the designs' kernel
+            slot["err_host"] = slot["err"].numpy()
             keys = ()
             base, cols = self._base()
             slot["h_rows"] = t.empty((P, n), dtype=t.int32, pin_memory=True)
@@ -429,12 +430,12 @@ class PermutationEngine:
                 slot["d_" + key].copy_(slot["h_" + key], non_blocking=True)
             if qf:
                 slot["d_rows"].copy_(slot["h_rows"], non_blocking=True)
-                tc.form_designs(base, cols, slot["d_rows"], P, kmax, slot["ops"])
+                tc.form_designs(base, cols, slot["d_rows"], P, kmax, slot["ops"], err=slot["err"])
                 tc.tstat_qf(*slot["ops"], P, kmax, self._coef, self.C, slot["d_t"], self.V)
             elif program:
                 slot["d_rows"].copy_(slot["h_rows"], non_blocking=True)
                 tc.form_residual_designs(base, slot["d_rows"], P, kmax, self._centred, self._coef, self.C,
-                                         self._w_stride, out=slot["ops"])
+                                         self._w_stride, out=slot["ops"], err=slot["err"])
                 *ops, wmat = slot["ops"]
                 tc.stat(3, *ops, P, kmax, self._coef, self.C, slot["d_t"], self.V, wmat=wmat, centred=self._centred)
             elif tc is not None:
@@ -452,8 +453,6 @@ class PermutationEngine:
             self.adj.sweep_batch(ptr(slot["d_t"]), self.V, P * self.C, self.signs, ptr(self.vd),
                                  int(self.floor_zero), ptr(slot["d_max"]), None, 0, stream_handle())
             slot["h_max"].copy_(slot["d_max"], non_blocking=True)
-            if slot["on_device"]:
-                slot["err_back"].copy_(tc.err, non_blocking=True)
 
         # warm-up outside capture (allocates the sweep workspace), then capture
         # two graphs: the GLM part (the last reader of the resident data) and
@@ -536,6 +535,8 @@ class PermutationEngine:
             if slot.get("busy"):  # left by a call that raised: drain it, its maxima are not this call's
                 slot["event"].synchronize()
                 slot["busy"] = False
+                if slot["on_device"]:
+                    slot["err_host"][0] = 0
         main = t.cuda.current_stream()
         results = {}
         prev = None
@@ -543,8 +544,9 @@ class PermutationEngine:
         def collect(slot):
             slot["event"].synchronize()
             slot["busy"] = False
-            if slot["on_device"] and int(slot["err_back"][0]):
-                self.status()  # raises: these maxima are not handed on
+            if slot["on_device"] and slot["err_host"][0]:  # a design without an inverse: not handed on
+                e, slot["err_host"][0] = int(slot["err_host"][0]), 0
+                self._tc.raise_code(e)
             results[slot["order"]] = slot["h_max"].numpy()[: slot["rows"]].copy()
             if on_batch is not None:
                 on_batch(slot["order"], results[slot["order"]])
@@ -690,12 +692,11 @@ class MediationEngine:
         """Base columns of the path designs on the device -- pred_x, depend_y,
         covariates -- and the columns of each path ([1, x] and [1, dy, x] for
         'M', pyfunc.py:131-145), those of permuted variables flagged."""
-        x, dy = self.pred_x.reshape(self.n, -1), self.depend_y.reshape(self.n, -1)
-        cov = np.zeros((self.n, 0)) if self.cov is None else self.cov.reshape(self.n, -1)
-        Z = np.hstack([x, dy, cov])
-        nx, ny, nc = x.shape[1], dy.shape[1], cov.shape[1]
-        key = self.medtype, nx, ny, nc
-        if getattr(self, "_paths_of", None) != key:
+        arrays = self.pred_x, self.depend_y, self.cov
+        up = self.medtype, *(None if a is None else (a.shape, a.tobytes()) for a in arrays)
+        if up != getattr(self, "_Z_up", None):
+            x, dy, cov = (np.zeros((self.n, 0)) if a is None else a.reshape(self.n, -1) for a in arrays)
+            nx, ny, nc = x.shape[1], dy.shape[1], cov.shape[1]
             cx = [j + TensorCoreOperands.PERMUTED for j in range(nx)]
             cy = [nx + j + (TensorCoreOperands.PERMUTED if self.medtype == "Y" else 0) for j in range(ny)]
             cc = [nx + ny + j for j in range(nc)]
@@ -703,10 +704,8 @@ class MediationEngine:
             cols = np.full((len(paths), self.kmax), -1, np.int32)
             for i, path in enumerate(paths):
                 cols[i, 1:1 + len(path)] = path
-            self._paths_d, self._paths_of = dev(cols), key
-            self._Z_up = None
-        if self._Z_up is None or not np.array_equal(self._Z_up, Z):
-            self._Z_d, self._Z_up = dev(Z), Z
+            self._paths_d, self._Z_d = dev(cols), dev(np.hstack([x, dy, cov]))
+            self._Z_up = up
         return self._Z_d, self._paths_d
 
     def _on_device(self):
@@ -732,7 +731,7 @@ class MediationEngine:
             return DesignBatch(B, kmax=self.kmax), np.asarray(ta, np.float32)
         return DesignBatch([m for pair in zip(A, B) for m in pair], kmax=self.kmax), None
 
-    def _zmaps_from(self, db, ta, P, out=None):
+    def _zmaps_from(self, db, ta, P, out=None, err=None):
         inner = self.inner
         z = self._z[:P] if out is None else out
         lib = inner.lib
@@ -742,7 +741,7 @@ class MediationEngine:
             G = P * paths.shape[0]
             ops = tc.design_buffers(G, self.kmax)
             rows = dev(db)
-            tc.form_designs(base, paths, rows, G, self.kmax, ops, share=paths.shape[0])
+            tc.form_designs(base, paths, rows, G, self.kmax, ops, share=paths.shape[0], err=err)
             tm = inner._tbuf[:G]
             tc.tstat_qf(*ops, G, self.kmax, inner._coef, 1, tm, inner.V)
         else:
@@ -801,19 +800,26 @@ class MediationEngine:
         if not hasattr(self, "_host_max"):
             self._host_max = [t.empty(self.batch * self.n_seg, dtype=t.float32, pin_memory=True) for _ in range(2)]
             self._max2 = [self._max.view(-1), t.empty_like(self._max.view(-1))]
-            self._host_err = t.zeros(2, dtype=t.int32, pin_memory=True)
+            self._err = [t.zeros(1, dtype=t.int32, pin_memory=True) for _ in range(2)]  # of the designs' kernel
+            self._err_host = [e.numpy() for e in self._err]
+            self._open = False
             self._done = [t.cuda.Event(), t.cuda.Event()]
             self._glm_done = [t.cuda.Event(), t.cuda.Event()]
             self._up_stream = t.cuda.Stream()
             self._up_done = t.cuda.Event()
         main = t.cuda.current_stream()
+        if self._open:  # a call that raised may have left batches behind
+            t.cuda.synchronize()
+            for e in self._err_host:
+                e[0] = 0
+        self._open = True
         out, prev = [], None
 
         def collect(item):
             k, P = item
             self._done[k].synchronize()
-            if int(self._host_err[k]):
-                inner.status()  # raises: a design without an inverse in this batch or before
+            if self._err_host[k][0]:  # a design without an inverse
+                inner._tc.raise_code(int(self._err_host[k][0]))
             out.append(self._host_max[k][: P * self.n_seg].numpy().reshape(P, 1, 1, self.n_seg).copy())
 
         for i, (data, rows) in enumerate(steps):
@@ -832,14 +838,12 @@ class MediationEngine:
                     inner.upload(data)
                 self._up_done.record(up)
                 main.wait_event(self._up_done)
-            z = self._zmaps_from(db, ta, P)
+            z = self._zmaps_from(db, ta, P, err=self._err[k])
             self._glm_done[k].record(main)
             mx = self._max2[k][: P * self.n_seg]
             inner.adj.sweep_batch(ptr(z), self.V, P, 1, ptr(inner.vd), int(inner.floor_zero),
                                   ptr(mx), None, 0, stream_handle())
             self._host_max[k][: P * self.n_seg].copy_(mx, non_blocking=True)
-            if inner._tc is not None:
-                self._host_err[k:k + 1].copy_(inner._tc.err, non_blocking=True)
             self._done[k].record(main)
             if prev is not None:
                 collect(prev)
@@ -847,6 +851,7 @@ class MediationEngine:
         if prev is not None:
             collect(prev)
         inner.status()
+        self._open = False
         return out
 
     def observed(self):

@@ -264,7 +264,8 @@ class TensorCoreOperands:
         # the data minus its centre: residuals of intercept designs skip the intercept term
         self.Yc = t.empty_like(Yd) if centre else None
         self.yy = t.empty(self.V, dtype=t.float32, device="cuda") if centre else None
-        self.err = t.zeros(1, dtype=t.int32, device="cuda")
+        # pinned memory that the kernels write on an error: read after a wait, no copy
+        self.err = t.zeros(1, dtype=t.int32, pin_memory=True)
         # t of coefficients >= 1 of intercept designs through the quadratic
         # form (False: the residual epilogue; the autotuner times both)
         self.quadratic_form = True
@@ -353,15 +354,16 @@ class TensorCoreOperands:
                 t.empty((Gp, R, R), dtype=t.float32, device="cuda"),
                 t.empty((G, kmax), dtype=t.float32, device="cuda"), t.empty(G, dtype=t.float32, device="cuda"))
 
-    def form_designs(self, base, cols, rows, G, kmax, out, stride=0, share=1):
+    def form_designs(self, base, cols, rows, G, kmax, out, stride=0, share=1, err=None):
         """Form the operators of G designs on the device (glm_qf_designs).  base:
         (n, c) float64, or one matrix per design `stride` apart; cols: (share,
         kmax) int32 base columns (+ PERMUTED); rows: (G / share, n) int32 or
-        None; out: design_buffers."""
+        None; out: design_buffers; err: an int32 word of these designs' own (pinned
+        host memory will do) instead of the operands'."""
         tiles, ginv, invd, dof = out
         _lib.check(self.lib.glm_qf_designs(ptr(base), base.shape[-1], stride, ptr(rows), ptr(cols), share, self.n,
                                            self.n_pad, G, kmax, ptr(tiles), ptr(ginv), ptr(invd), ptr(dof),
-                                           ptr(self.err), stream_handle()))
+                                           ptr(self.err if err is None else err), stream_handle()))
 
     def form_stacked(self, X64, out=None):
         """Operators of designs stacked as host float64 (G, n, k), the first
@@ -384,17 +386,17 @@ class TensorCoreOperands:
         u, x, invd, dof, w = t.empty(sum(sizes), dtype=t.float32, device="cuda").split(sizes)
         return tiles, u, x, invd, dof, w.view(G, w_stride) if w_stride else None
 
-    def form_residual_designs(self, base, rows, G, kmax, centred, program, n_rows, w_stride, out=None):
+    def form_residual_designs(self, base, rows, G, kmax, centred, program, n_rows, w_stride, out=None, err=None):
         """Operands of `stat` for G permuted intercept designs, formed on the
         device (glm_tc_designs), in `out` (residual_buffers) when given.  base: (n,
         kmax) float64 design whose rows (G, n) int32 index; program: device rows
-        of output_program."""
+        of output_program; err as form_designs."""
         out = self.residual_buffers(G, kmax, w_stride) if out is None else out
         tiles, u, x, invd, dof, w = out
         _lib.check(self.lib.glm_tc_designs(ptr(base), base.shape[-1], ptr(rows), self.n, self.n_pad, self.n_sc, G,
                                            kmax, self.block(kmax), int(centred), ptr(program), n_rows, w_stride,
-                                           ptr(tiles), ptr(u), ptr(x), ptr(invd), ptr(dof), ptr(w), ptr(self.err),
-                                           stream_handle()))
+                                           ptr(tiles), ptr(u), ptr(x), ptr(invd), ptr(dof), ptr(w),
+                                           ptr(self.err if err is None else err), stream_handle()))
         return out
 
     def tstat_qf(self, x_tiles, ginv, invd, dof, G, kmax, coef_d, n_coef, out, ldt):
@@ -458,14 +460,19 @@ class TensorCoreOperands:
                                               ptr(wmat), w_stride, ptr(out), ldt, ptr(self.err), stream_handle()))
 
     def status(self):
+        self.t.cuda.current_stream().synchronize()
         e = int(self.err.item())
         if e:
             self.err.zero_()
-            if e == 4:
-                raise np.linalg.LinAlgError("Singular matrix")
-            if e == 1:
-                raise IndexError("a permutation index is out of bounds")
-            raise RuntimeError("tensor-core GLM: a copy or MMA completion wait ran out (device code %d)" % e)
+            self.raise_code(e)
+
+    @staticmethod
+    def raise_code(e):
+        if e == 4:
+            raise np.linalg.LinAlgError("Singular matrix")
+        if e == 1:
+            raise IndexError("a permutation index is out of bounds")
+        raise RuntimeError("tensor-core GLM: a copy or MMA completion wait ran out (device code %d)" % e)
 
 
 def glm_tstat_tc(Y, designs, coef, ops=None, centre=True, quadratic_form=None):
