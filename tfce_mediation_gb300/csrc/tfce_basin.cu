@@ -1588,6 +1588,7 @@ constexpr size_t kPowersKept = 16;  // tables of extent^E that a handle holds on
 
 int64_t node_capacity(const BasinPlan* p) { return p->all_basins * kMaxSteps; }
 
+constexpr int64_t kAskAtOnce = 256LL << 20;  // a workspace that is asked for without a look at free memory (20 us)
 constexpr int64_t kStateBudget = 2LL << 30;  // state in global memory of the CTAs of the large class
 
 // tuning knob: the largest workspace that is asked for, in MB
@@ -1869,10 +1870,13 @@ int basin_sweep(BasinPlan* p, const BasinRequest& r, cudaStream_t st, bool* refu
   auto less = [&] { need = divide(budget = std::min(budget, per * one + large_ctas * state) / 2); };
   if (need > p->ws_bytes) {
     int64_t limit = p->ws_bytes;
-    size_t unused = 0, total = 0;
     if (capturing == cudaStreamCaptureStatusNone) {
-      if (cudaMemGetInfo(&unused, &total) != cudaSuccess) cudaGetLastError();
-      limit = std::max(limit, (static_cast<int64_t>(unused) + (p->captured ? 0 : p->ws_bytes)) / 2);
+      limit = std::max(limit, kAskAtOnce);
+      size_t unused = 0, total = 0;
+      if (need > limit) {
+        if (cudaMemGetInfo(&unused, &total) != cudaSuccess) cudaGetLastError();
+        limit = std::max(limit, (static_cast<int64_t>(unused) + (p->captured ? 0 : p->ws_bytes)) / 2);
+      }
     }
     while (need > limit && !least()) less();
     for (;;) {
